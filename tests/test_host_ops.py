@@ -1,0 +1,68 @@
+"""The native host path (module _gsq_ops): its routing against the Python table that is API, and on the GPU the fused
+layer of several runs against one product per run, direct calls against the custom ops."""
+
+import pytest
+import torch
+import torch.utils._python_dispatch
+
+import gsq_b200  # noqa: F401
+from gsq_b200 import _gsq_ops, synth
+from gsq_b200.quantization import iq3_pack, linear
+
+TYPES = {**synth.TYPE_IDS, **synth.LOW_BIT_TYPE_IDS}
+
+
+def test_native_routing_is_the_python_table():
+    bad = []
+    for t in TYPES.values():
+        for packed in (False, True):
+            pk = packed and t in iq3_pack.PACKABLE_TYPES
+            for n in (1, 2, 3, 5, 6, 7, 8, 9, 16, 17, 32, 33, 48, 49, 300):
+                for rows in (1024, 2048, 2049, 5120, 12288, 17408):
+                    for k in (512, 5120, 17408):
+                        want = linear._lcpp_op(n, t, rows, k, pk)
+                        if pk and t == 14:
+                            want = "gsq_mul_mat_vec_q6k_packed" if want == "lcpp_mul_mat_vec_q" else "gsq_mul_mat_q6k_packed"
+                        if _gsq_ops.route(n, t, rows, k, pk) != want:
+                            bad.append((n, t, rows, k, pk))
+    assert not bad, bad[:5]
+
+
+def test_native_errors_are_python_exceptions():
+    x, w = torch.zeros(70, 512, dtype=torch.bfloat16), torch.zeros(16, 112, dtype=torch.uint8)
+    with pytest.raises(NotImplementedError, match="no kernel for ggml type 29 at 70"):
+        _gsq_ops.linear(x, w, 29, None, False)
+    with pytest.raises(NotImplementedError, match="Unsupported GGUF quantization type"):
+        _gsq_ops.linear(x, w, 8, None, False)
+    with pytest.raises(RuntimeError, match="must be CUDA tensors"):
+        _gsq_ops.linear_runs(x[:4], w, [0, 16, 112, 29], False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 4, 8, 9, 40, 70])
+@pytest.mark.parametrize("names", [("IQ3_S", "IQ3_S", "Q6_K"), ("Q4_K", "IQ4_XS", "Q4_K"), ("IQ3_S", "IQ2_XS", "Q2_K")])
+def test_runs_of_a_fused_layer(m, names):
+    k, rows = 1024, (160, 48, 64)
+    layer, method = torch.nn.Module(), linear.GGUFLinearMethod(None)
+    method.create_weights(layer, k, list(rows), k, sum(rows), torch.bfloat16)
+    for i, (sid, name, r) in enumerate(zip("qkv", names, rows)):
+        layer.weight.load_shard(torch.from_numpy(synth.make_weight(TYPES[name], r, k, 20 + i)).cuda(), sid)
+        layer.weight_type.shard_weight_type[sid] = TYPES[name]
+    method.process_weights_after_loading(layer)
+    x = torch.from_numpy(synth.make_activation(m, k, 30 + m)).to(torch.bfloat16).cuda()
+    got = method.apply(layer, x)
+    w = layer.weight
+    packed = getattr(w, "iq3_packed", False)
+    want = torch.cat([linear._fused_mul_mat_gguf(x, v, t, None, packed)
+                      for v, t in linear._shard_runs(w, ["q", "k", "v"], [TYPES[n] for n in names])], dim=1)
+    assert torch.equal(got, want)
+    seen = []
+
+    class Watch(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Watch():   # someone intercepts: through the custom op, same result
+        assert torch.equal(method.apply(layer, x), want)
+    assert "_C_gguf.gsq_linear_runs.default" in seen

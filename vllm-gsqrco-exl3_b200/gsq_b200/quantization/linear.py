@@ -10,6 +10,10 @@ same names, argument meaning and error behaviour -- so it can stand in for that 
   GGUFLinearMethod.{create_weights, process_weights_after_loading, apply}  347-570
   torch.ops.vllm._fused_mul_mat_gguf / _quantize_x_q8_1       307-325     custom ops with fake impls
 
+The functions below say what the custom ops do and serve them on CPU tensors (where every call ends in a guard's
+message); on CUDA tensors the ops are implemented in native code (csrc/gsq_torch.cpp), and apply() calls that directly
+when nothing is tracing.
+
 Differences, all deliberate: there is one route (the reference's "Route L"), no stock / Triton /
 dequantise fallback, and only the four ggml types with an sm_100a kernel compute; a type outside
 that set raises. The op names `_lcpp_op` returns are API (tests and `_quantize_x_q8_1` key on
@@ -24,7 +28,7 @@ from itertools import groupby
 
 import torch
 
-from .. import lcpp_ops, ops
+from .. import _gsq_ops, ops
 from . import iq3_pack
 from .params import GGUFWeightParameter, GGUFWeightTypeParameter, _gguf_ordered_shard_ids
 
@@ -47,6 +51,7 @@ _FP32_DST_BUDGET = 256 << 20
 _MMA_K_ON = os.environ.get("VLLM_GGUF_MMA_K", "1") != "0"
 _IQ3_TILED_ON = os.environ.get("VLLM_GGUF_IQ3_TILED", "1") != "0"
 _IQ1M_MMVQ_ON = os.environ.get("VLLM_GGUF_IQ1M_MMVQ", "1") != "0"
+_gsq_ops.set_switches(ops.LCPP_ENABLED, _MMA_K_ON, _IQ3_TILED_ON, _IQ1M_MMVQ_ON)
 
 
 def _mma_k_wins(weight_type: int, n: int, rows: int, k: int) -> bool:
@@ -197,7 +202,7 @@ def _register_python_ops():
     for name, schema, fn, fake in specs:
         try:
             _VLLM_LIB.define(name + schema)
-            _VLLM_LIB.impl(name, fn, "CUDA")
+            _gsq_ops.implement_vllm(name)
             _VLLM_LIB.impl(name, fn, "CPU")
             _VLLM_LIB._register_fake(name, fake)
             out[name] = getattr(torch.ops.vllm, name)
@@ -312,24 +317,51 @@ class GGUFLinearMethod:
         new.shard_offset_map = offsets
         layer.register_parameter("weight", new)
 
+    @staticmethod
+    def _plan(layer: torch.nn.Module, weight) -> tuple:
+        """(type, None) of a layer that is one product, (None, runs) of one that is several, runs = start row, rows, row
+        bytes and type of each in one flat list (gsq_linear_runs), or (None, None) if one of them is not quantised.
+        Worked out at the first call on a weight and kept with it."""
+        shard_id = weight.shard_id
+        if not shard_id:
+            return layer.weight_type.weight_type, None
+        shard_id = ["q", "k", "v"] if "q" in shard_id else shard_id
+        fallback = layer.weight_type.weight_type
+        types = [layer.weight_type.shard_weight_type.get(i, fallback) for i in shard_id]
+        if len(set(types)) == 1:
+            return types[0], None
+        if any(t in ops.UNQUANTIZED_TYPES for t in types) or not weight.is_contiguous():
+            return None, None
+        runs, offsets = [], weight.shard_offset_map
+        for t, run in groupby(zip(shard_id, types), key=lambda p: p[1]):
+            ids = [i for i, _ in run]
+            start, _, size = offsets[ids[0]]
+            runs += [start, offsets[ids[-1]][1] - start, size, t]
+        return None, runs
+
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         if self.layout is not None:
             x = self.layout.input_to_gguf(x)
         weight = layer.weight
-        shard_id = weight.shard_id
         packed = getattr(weight, "iq3_packed", False)
-        if shard_id:
-            shard_id = ["q", "k", "v"] if "q" in shard_id else shard_id
-            fallback = layer.weight_type.weight_type
-            types = [layer.weight_type.shard_weight_type.get(i, fallback) for i in shard_id]
-            if len(set(types)) == 1:
-                out = fused_mul_mat_gguf(x, weight, types[0], None, packed)
-            else:
-                runs = list(_shard_runs(weight, shard_id, types))
-                x_q8 = quantize_x_q8_1(x, [t for _, t in runs], [w.shape[0] for w, _ in runs], packed)
-                out = torch.cat([fused_mul_mat_gguf(x, w, t, x_q8, packed) for w, t in runs], dim=1)
+        plan = getattr(weight, "gsq_plan", None)
+        if plan is None:
+            plan = self._plan(layer, weight)
+            if weight.numel():
+                weight.gsq_plan = plan
+        weight_type, runs = plan
+        # a plain CUDA tensor and nobody tracing or intercepting: straight to the native code under the custom ops
+        direct = type(x) is torch.Tensor and x.is_cuda and not torch.compiler.is_compiling() and not torch._C._len_torch_dispatch_stack()
+        if weight_type is not None:
+            out = (_gsq_ops.linear if direct else fused_mul_mat_gguf)(x, weight, weight_type, None, packed)
+        elif runs is not None:
+            out = (_gsq_ops.linear_runs if direct else torch.ops._C_gguf.gsq_linear_runs)(x, weight, runs, packed)
         else:
-            out = fused_mul_mat_gguf(x, weight, layer.weight_type.weight_type, None, packed)
+            types = layer.weight_type.shard_weight_type
+            shard_id = ["q", "k", "v"] if "q" in weight.shard_id else weight.shard_id
+            runs = list(_shard_runs(weight, shard_id, [types.get(i, layer.weight_type.weight_type) for i in shard_id]))
+            x_q8 = quantize_x_q8_1(x, [t for _, t in runs], [w.shape[0] for w, _ in runs], packed)
+            out = torch.cat([fused_mul_mat_gguf(x, w, t, x_q8, packed) for w, t in runs], dim=1)
         if bias is not None:
             out.add_(bias)
         return out
