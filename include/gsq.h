@@ -60,7 +60,7 @@ extern "C" {
 #define GSQ_KERNEL_GEMV 1 /* dp4a streaming GEMV, 1..8 activation rows per launch, reads block_q8_1 */
 #define GSQ_KERNEL_GEMM 2 /* tcgen05 kind::i8 GEMM, 64-token tiles in lockstep, reads 128-value q8_1 blocks */
 #define GSQ_KERNEL_MMV 3  /* register-operand tensor-core kernel, 1..48 activation rows per launch */
-#define GSQ_KERNEL_GEMM_PREFILL 4 /* warp-specialised tcgen05 kind::i8 GEMM, 256-token blocks, reads operand tiles */
+#define GSQ_KERNEL_GEMM_PREFILL 4 /* tcgen05 prefill GEMMs: weights expanded to fp16 operands, or (integer sums) decoded in the kernel */
 
 const char* gsq_strerror(int status);
 /* cudaError_t of the last failing CUDA call made by this library on this thread (0 if none). */
@@ -222,11 +222,13 @@ int gsq_mul_mat_q8(const void* w, int64_t row_bytes, int64_t rows, int ggml_type
 /*
  * The whole product from X as it is, any number of activation rows: quantises X into `scratch` in the layout of
  * the kernel it then runs (the small-batch tensor-core kernel up to 48 rows, the warp-specialised tcgen05 GEMM
- * above, the dp4a kernel for Q6_K and IQ3_S in GGUF order). Replaces what the reference's self-quantising ops do
+ * above; Q6_K, IQ3_S in GGUF order and the low-bit types: their small-batch kernels while that takes few launches, then
+ * the same GEMM). Replaces what the reference's self-quantising ops do
  * in one call: lcpp_mul_mat_q, lcpp_mul_mat_mma_k, lcpp_mul_mat_iq3_packed (lcpp_shim.cu:626-671, 753-909, whose
  * scratch comes from torch's allocator, :250-263).
  *   x            [m, k] in x_dtype, row stride x_row_stride elements
- *   scratch      gsq_linear_scratch_bytes(...) bytes, 256-byte aligned; need not be initialised, not preserved
+ *   scratch      gsq_linear_scratch_bytes(...) bytes, 256-byte aligned; need not be initialised, not preserved. The
+ *                prefill GEMM keeps the expanded weights there: 2 bytes per weight (4 for Q6_K), at most 512 MB at a time
  */
 size_t gsq_linear_scratch_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed);
 int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype,
@@ -234,8 +236,9 @@ int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, in
                size_t scratch_bytes, void* stream);
 
 /*
- * How gsq_linear forms the prefill product of repacked IQ3_S, of IQ4_XS and of Q4_K (256 tokens and up; the other
- * routes are not affected).
+ * How gsq_linear forms the prefill product of repacked IQ3_S, of IQ4_XS and of Q4_K (256 tokens and up, 128 on tall
+ * weights). Q6_K, IQ3_S in GGUF order and the low-bit types have the accuracy of the split form in the first two modes
+ * and their small-batch kernels' integer sums in the third; the other routes are not affected.
  * The reference's kernels keep an exact int32 sum per 32-value slice and scale it in fp32
  * (lcpp_owned_iq3_mma.cu:768-970, mmq.cuh:961-1385). Sets the mode, returns the previous one:
  *   GSQ_PREFILL_ROUNDED (default)  d_x * q goes into the tensor-core operand as one fp16 number and tensor memory
@@ -318,7 +321,8 @@ int gsq_peer_reduce_error_flag(int* flag);
 
 /*
  * Kernel family that serves (activation rows m, type, weight rows, k, packed) on B200: GSQ_KERNEL_*, the choice
- * gsq_mul_mat_vec_q8 and gsq_linear make. The op-level routing table of the reference (_lcpp_op,
+ * gsq_mul_mat_vec_q8 and, for repacked IQ3_S, IQ4_XS and Q4_K, gsq_linear make (for the other types: the small-batch
+ * kernel; gsq_linear leaves it for the prefill GEMM once it would take several launches). The op-level routing table of the reference (_lcpp_op,
  * quantization/linear.py:85-114) stays in the Python layer because its op names are API; this is the choice made
  * underneath those names.
  */

@@ -1,0 +1,84 @@
+"""The two-step product (weights expanded to fp16 operand tiles, then the tcgen05 GEMM on pairs of CTAs): every weight
+kind at the edges of its tiles (row tiles of 128 in pairs, token blocks of a multiple of 16, superblocks, parts of K),
+against the float64 product of the dequantised weights and the q8_1 activations.
+
+Q6_K, IQ3_S in GGUF order and the low-bit types carry 22 bits of d_x * q and exact weights: 3e-6 of a row's norm. (The
+small-row kernels of the low-bit types truncate integer divisions as the reference's do; the many-row form, like the
+reference's, does not.)"""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import gsq_b200  # noqa: F401
+from gsq_b200 import _cabi, synth
+from gsq_b200.quantization import iq3_pack
+from oracle import blocks, blocks_f1, product, q8_1
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+TYPES = {**synth.TYPE_IDS, **synth.LOW_BIT_TYPE_IDS}
+
+
+def _run(t, packed, raw, x, rows, ldy=None):
+    w = torch.from_numpy(raw).to(DEV)
+    if packed:
+        iq3_pack.pack_(w, t)
+    lib, (m, k) = _cabi.lib, x.shape
+    n = lib.gsq_linear_scratch_bytes(rows, m, k, t, int(packed))
+    scratch = torch.full((n,), 0xFF, dtype=torch.uint8, device=DEV)     # nothing may rely on what it holds
+    ldy = ldy or rows
+    y = torch.full((m, ldy), float("nan"), dtype=torch.float32, device=DEV)
+    rc = lib.gsq_linear(w.data_ptr(), w.shape[1], rows, t, int(packed), x.data_ptr(), 0, m, k, x.stride(0), y.data_ptr(), 0, ldy,
+                        scratch.data_ptr(), n, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, lib.gsq_strerror(rc)
+    torch.cuda.synchronize()
+    assert bool(torch.isnan(y[:, rows:]).all())
+    flag = ctypes.c_int(-1)
+    assert lib.gsq_device_error_flag(ctypes.byref(flag)) == 0 and flag.value == 0
+    return y[:, :rows].cpu().numpy()
+
+
+def _dense(raw, t):
+    return product.product_full(raw, t, np.eye(_k(raw, t), dtype=np.float32)).T if t in synth.TYPE_IDS.values() else blocks_f1.product_full(
+        raw, t, np.eye(_k(raw, t), dtype=np.float32)).T
+
+
+def _k(raw, t):
+    return raw.shape[1] // synth.BLOCK_BYTES[t] * 256
+
+
+CASES = [("Q6_K", True), ("Q6_K", False), ("IQ3_S", False)] + [(n, False) for n in synth.LOW_BIT_TYPE_IDS]
+
+
+@pytest.mark.parametrize("name,packed", CASES)
+@pytest.mark.parametrize("rows,k,m", [(16, 256, 130), (144, 512, 257), (400, 1024, 99), (272, 4608, 300)])
+def test_full_precision_kinds(name, packed, rows, k, m):
+    t = TYPES[name]
+    raw = synth.make_weight(t, rows, k, 60 + rows)
+    xa = synth.make_activation(m, k, 61 + m)
+    xa[3, :64] = 0.0
+    xa[7, :] = 0.0
+    xa[5, 7] = 300.0
+    x = synth.nudge_ties_torch(torch.from_numpy(xa).to(torch.bfloat16)).float()
+    q, d, _ = q8_1.quantize_q8_1(x.numpy())
+    xq = (q.reshape(m, k // 32, 32).astype(np.float64) * d.astype(np.float64).reshape(m, k // 32, 1)).reshape(m, k)
+    want = xq @ _dense(raw, t).astype(np.float64).T
+    got = _run(t, packed, raw, x.to(DEV), rows, rows + 5)
+    assert np.isfinite(got).all() and not got[7].any()
+    assert product.rel_err(got, want) <= 3e-6
+
+
+@pytest.mark.parametrize("m", [256, 257, 272, 511, 529])
+@pytest.mark.parametrize("name", ["IQ3_S", "IQ4_XS", "Q4_K"])
+def test_rounded_kinds_over_token_blocks(name, m):
+    """Ragged token counts and a K that is cut into parts: the model of the rounded form's own arithmetic."""
+    from oracle import prefill_forms
+
+    t, rows, k = TYPES[name], 400, 4096
+    raw = synth.make_weight(t, rows, k, 70)
+    x = synth.nudge_ties_torch(torch.from_numpy(synth.make_activation(m, k, 71 + m)).to(torch.bfloat16)).float()
+    got = _run(t, name == "IQ3_S", raw, x.to(DEV), rows)
+    assert product.rel_err(got, prefill_forms.product(raw, t, x.numpy())) <= 3e-6

@@ -22,8 +22,16 @@ __host__ __device__ constexpr int f1_block_bytes(int kind) {
 // values per integer sub-scale (what the debug dump is grouped by)
 __host__ __device__ constexpr int f1_group(int kind) { return (kind == F1_IQ2XXS || kind == F1_IQ3XXS) ? 32 : 16; }
 
+// a block's bytes from global memory (streaming loads), or from shared memory (SH: the block is staged there)
+template <bool SH>
+__device__ __forceinline__ uint32_t f1_u8(const uint8_t* p) { return SH ? *p : ldg_stream_u8(p); }
+template <bool SH>
+__device__ __forceinline__ uint32_t f1_u16(const uint8_t* p) { return SH ? *reinterpret_cast<const uint16_t*>(p) : ldg_stream_u16(p); }
+template <bool SH>
+__device__ __forceinline__ uint32_t f1_u32(const uint8_t* p) { return SH ? *reinterpret_cast<const uint32_t*>(p) : ldg_stream_u32(p); }
+template <bool SH>
 __device__ __forceinline__ uint32_t ld32_h(const uint8_t* p) {   // 32 bits from a 2-byte aligned address
-  return ldg_stream_u16(p) | (ldg_stream_u16(p + 2) << 16);
+  return f1_u16<SH>(p) | (f1_u16<SH>(p + 2) << 16);
 }
 // the 4 low bits of `bits` say which bytes of g to negate (no byte of these codebooks is zero, so ~g + 1 per byte
 // never carries)
@@ -40,39 +48,39 @@ template <int KIND>
 struct Raw {
   uint32_t r[KIND == F1_Q2K ? 10 : KIND == F1_IQ2S ? 5 : 4];
 
+  template <bool SH = false>
   __device__ __forceinline__ void fetch(const uint8_t* b, int s) {
     if (KIND == F1_IQ2XXS) {
-      r[0] = ldg_stream_u16(b);
-      r[1] = ld32_h(b + 2 + 8 * s);
-      r[2] = ld32_h(b + 6 + 8 * s);
+      r[0] = f1_u16<SH>(b);
+      r[1] = ld32_h<SH>(b + 2 + 8 * s);
+      r[2] = ld32_h<SH>(b + 6 + 8 * s);
     } else if (KIND == F1_IQ2XS) {
-      r[0] = ldg_stream_u16(b);
-      r[1] = ld32_h(b + 2 + 8 * s);
-      r[2] = ld32_h(b + 6 + 8 * s);
-      r[3] = ldg_stream_u8(b + 66 + s);
+      r[0] = f1_u16<SH>(b);
+      r[1] = ld32_h<SH>(b + 2 + 8 * s);
+      r[2] = ld32_h<SH>(b + 6 + 8 * s);
+      r[3] = f1_u8<SH>(b + 66 + s);
     } else if (KIND == F1_IQ2S) {
-      r[0] = ldg_stream_u16(b);
-      r[1] = ld32_h(b + 2 + 4 * s);
-      r[2] = ld32_h(b + 34 + 4 * s);
-      r[3] = ldg_stream_u8(b + 66 + s);
-      r[4] = ldg_stream_u8(b + 74 + s);
+      r[0] = f1_u16<SH>(b);
+      r[1] = ld32_h<SH>(b + 2 + 4 * s);
+      r[2] = ld32_h<SH>(b + 34 + 4 * s);
+      r[3] = f1_u8<SH>(b + 66 + s);
+      r[4] = f1_u8<SH>(b + 74 + s);
     } else if (KIND == F1_IQ3XXS) {
-      r[0] = ldg_stream_u16(b);
-      r[1] = ld32_h(b + 2 + 8 * s);
-      r[2] = ld32_h(b + 6 + 8 * s);
-      r[3] = ld32_h(b + 66 + 4 * s);
+      r[0] = f1_u16<SH>(b);
+      r[1] = ld32_h<SH>(b + 2 + 8 * s);
+      r[2] = ld32_h<SH>(b + 6 + 8 * s);
+      r[3] = ld32_h<SH>(b + 66 + 4 * s);
     } else if (KIND == F1_Q2K) {
       const int h = s >> 2;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) r[e] = ldg_stream_u32(b + 16 + 32 * h + 4 * e);
-      r[8] = ldg_stream_u16(b + 2 * s);
-      r[9] = ldg_stream_u32(b + 80);
+      for (int e = 0; e < 8; ++e) r[e] = f1_u32<SH>(b + 16 + 32 * h + 4 * e);
+      r[8] = f1_u16<SH>(b + 2 * s);
+      r[9] = f1_u32<SH>(b + 80);
     } else {  // IQ1_M
-      r[0] = ldg_stream_u32(b + 4 * s);
-      r[1] = ldg_stream_u16(b + 32 + 2 * s);
-      const uint2 sa = ldg_stream_v2(b + 48);
-      r[2] = sa.x;
-      r[3] = sa.y;
+      r[0] = f1_u32<SH>(b + 4 * s);
+      r[1] = f1_u16<SH>(b + 32 + 2 * s);
+      r[2] = f1_u32<SH>(b + 48);
+      r[3] = f1_u32<SH>(b + 52);
     }
   }
 };

@@ -19,10 +19,13 @@ int gemm2_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, in
                int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream);
 // gsq_gemm3.cu
 bool gemm3_applies(int ggml_type, int packed, int64_t rows);
-bool gemm3_acc_applies(int ggml_type, int packed, int64_t rows);
-size_t gemm3_tile_bytes(int64_t m, int64_t k, int acc, int sums);
+size_t gemm3_tile_bytes(int64_t m, int64_t k);
 int gemm3_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x_tiles, int64_t m,
-               int64_t k, void* y, int y_dtype, int64_t y_row_stride, int acc, int pair, void* stream);
+               int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream);
+// gsq_gemm4.cu
+size_t gemm4_scratch_bytes(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu);
+int gemm4_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
+                 int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* scratch, int hu, void* stream);
 // gsq_quantize.cu
 int quantize_tiles_host(const void* x, int x_dtype, int64_t m, int64_t k, int64_t stride, int layout, void* out, void* stream);
 // gsq_gemm.cu
@@ -33,6 +36,53 @@ static size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 static int g_prefill_precision = GSQ_PREFILL_ROUNDED;
 
+// The kernels of a product above the small-batch tensor-core kernel's rows (or of a type or shape it does not serve).
+enum Way {
+  W_PLANES1,    // two steps, operands expanded to fp16: one plane of scaled activations (rounded)
+  W_PLANES2,    // the same with the activations as hi + lo: fp32 accuracy
+  W_IQ3_INT,    // gsq_gemm3.cu: fp16 operands, integer slice sums
+  W_I8,         // gsq_gemm2.cu: int8 prefill GEMM
+  W_LOCKSTEP,   // gsq_gemm.cu: 64-token tiles, split K
+  W_MMV_LOOP,   // repacked Q6_K: the small-batch kernel, 48 rows per launch
+  W_GEMV_LOOP   // GGUF-order blocks: the dp4a kernels, 8 rows per launch
+};
+
+static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m) {
+  const int variant = gemm_variant();
+  const bool dump = gemm_dump_pointer() != nullptr;   // (per-slice integer sums: only the integer forms have them)
+  if (gemm2_applies(ggml_type, packed, rows)) {
+    // Repacked IQ3_S, IQ4_XS, Q4_K. The prefill forms from 256 tokens on, and from 128 where the weight alone gives half
+    // an SM count of row tiles; the int8 one, where integer sums are asked for, from 512 and 192. Below, the lockstep kernel.
+    const bool tall = (rows + 127) / 128 >= 74, iq3 = gemm3_applies(ggml_type, packed, rows);
+    const bool big3 = m >= 256 || (m >= 128 && tall), big = m >= 512 || (m >= 192 && tall);
+    if (variant == 3 || variant >= 5 || (variant == 0 && big3)) {
+      int planes = g_prefill_precision == GSQ_PREFILL_ROUNDED ? 1 : g_prefill_precision == GSQ_PREFILL_SPLIT && iq3 ? 2 : 0;
+      if (variant == 5 || variant == 9) planes = ggml_type == GSQ_TYPE_Q4_K ? 1 : 2;
+      if (variant == 6 || variant == 8) planes = 1;
+      if (variant == 7 || dump) planes = 0;
+      if (planes) return planes == 1 ? W_PLANES1 : W_PLANES2;
+      if (iq3) return W_IQ3_INT;
+    }
+    return variant == 3 || variant == 4 || variant >= 5 || (variant == 0 && big) ? W_I8 : W_LOCKSTEP;
+  }
+  const bool q6 = ggml_type == GSQ_TYPE_Q6_K, q6_packed = q6 && packed && rows % 16 == 0;
+  // Q6_K, IQ3_S in GGUF order and the low-bit types: the two steps once they cost less than the repeated launches of the
+  // small-batch kernels (48 or 8 rows each), at fp32 accuracy, unless integer sums are asked for.
+  if (!dump && g_prefill_precision != GSQ_PREFILL_INTEGER && m >= (q6_packed ? 97 : q6 || ggml_type == GSQ_TYPE_IQ3_S ? 25 : 9)) return W_PLANES2;
+  return q6_packed ? W_MMV_LOOP : W_GEMV_LOOP;
+}
+
+static size_t way_scratch(Way way, int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
+  switch (way) {
+    case W_PLANES1: return gemm4_scratch_bytes(ggml_type, packed, rows, m, k, 1);
+    case W_PLANES2: return gemm4_scratch_bytes(ggml_type, packed, rows, m, k, 2);
+    case W_IQ3_INT: return gemm3_tile_bytes(m, k);
+    case W_I8: return gemm2_tile_bytes(m, k, ggml_type);
+    case W_LOCKSTEP: return (size_t)(k / 128) * (size_t)m * 144;
+    default: return (size_t)(k / 32) * (size_t)m * 36;
+  }
+}
+
 }  // namespace gsq
 
 extern "C" int gsq_prefill_precision(int mode) {
@@ -42,21 +92,13 @@ extern "C" int gsq_prefill_precision(int mode) {
 }
 
 extern "C" size_t gsq_linear_scratch_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
-  if (m <= 0 || k <= 0) return 0;
-  const size_t mmq = (size_t)(k / 128) * (size_t)m * 144, q81 = (size_t)(k / 32) * (size_t)m * 36;
-  size_t tiles = gsq::gemm3_applies(ggml_type, packed, rows) ? 0 : gsq::gemm2_tile_bytes(m, k, ggml_type);
-  if (gsq::gemm3_acc_applies(ggml_type, packed, rows)) {
-    // the fp16-operand forms: one plane of scaled products per slice, two where the split form is selected (or forced
-    // through the debug switch); and the integer-sum form's units, which the dump of those sums selects
-    const int v = gsq::gemm_variant();
-    const int planes = (gsq::g_prefill_precision == GSQ_PREFILL_SPLIT || v == 5 || v == 9) ? 2 : 1;
-    const size_t t3 = gsq::gemm3_tile_bytes(m, k, planes, ggml_type == GSQ_TYPE_Q4_K), t0 = gsq::gemm3_tile_bytes(m, k, 0, 0);
-    tiles = tiles > t3 ? tiles : t3;
-    tiles = tiles > t0 ? tiles : t0;
-  }
-  size_t b = mmq > tiles ? mmq : tiles;
-  b = b > q81 ? b : q81;
-  return gsq::align256(b);
+  using namespace gsq;
+  if (m <= 0 || k <= 0 || rows <= 0) return 0;
+  size_t b = way_scratch(choose_way(ggml_type, packed, rows, m), rows, m, k, ggml_type, packed);
+  // (the small-batch kernel takes 128-value blocks, and may decline the shape)
+  const size_t mmq = mmv_applies(ggml_type, packed, rows, m) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
+  b = b > mmq ? b : mmq;
+  return align256(b > 0 ? b : 1);
 }
 
 extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x,
@@ -78,75 +120,41 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
     rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, 1, m, k, y, y_dtype, y_row_stride, stream, gemm_dump_pointer());
     if (rc != 1000) return rc;  // 1000: declined, the activations of this shape do not fit its staging area
   }
-  // The prefill GEMMs on operand-ordered units, where their 128-row x 256-token items can occupy the GPU. Measured
-  // against the lockstep kernel (64-token tiles, K split over a cluster when tiles are few) on 17408 x 5120,
-  // 5120 x 5120 and 5120 x 17408: the fp16-operand kernel wins from 256 tokens on, and from 128 where the weight
-  // alone gives half an SM count of row tiles; the int8 one from 512, and from 192 on the tall weights.
-  const int variant = gemm_variant();
-  const bool tall = (rows + 127) / 128 >= 74;
-  const bool big3 = m >= 256 || (m >= 128 && tall);
-  const bool big = m >= 512 || (m >= 192 && tall);
-  // repacked IQ3_S and IQ4_XS: the kernels with the sub-scales folded into fp16 operands (variant 4 keeps the int8
-  // kernel for them)
-  if (gemm3_acc_applies(ggml_type, packed, rows) && (variant == 3 || variant >= 5 || (variant == 0 && big3))) {
-    // the form that accumulates over a superblock in tensor memory, on one or two fp16 planes of scaled products, or the
-    // one with integer slice sums (also whenever the debug dump of those sums is on); variants 5 / 6 / 7 force one
-    int acc = g_prefill_precision == GSQ_PREFILL_ROUNDED ? 1 : g_prefill_precision == GSQ_PREFILL_SPLIT ? 2 : 0;
-    // IQ4_XS: (ls - 32) * value reaches 4064 and is not always exact in fp16, so only the rounded form is offered on
-    // fp16 operands; the split setting takes the int8 kernel's integer sums instead
-    // (and Q4_K, whose minimum term is folded in with one rounding of dmin / d * m)
-    if ((ggml_type == GSQ_TYPE_IQ4_XS || ggml_type == GSQ_TYPE_Q4_K) && acc == 2) acc = 0;
-    int pair = 0;
-    if (variant == 5 || variant == 9) acc = 2;
-    if (variant == 6 || variant == 8) acc = 1;
-    if (variant == 8 || variant == 9) pair = gemm3_applies(ggml_type, packed, rows) ? 1 : 0;
-    if (variant == 7 || gemm_dump_pointer()) acc = 0;
-    if (acc || gemm3_applies(ggml_type, packed, rows)) {
-      rc = quantize_tiles_host(x, x_dtype, m, k, x_row_stride,
-                               acc == 2 ? Q8_TILES_F16S2 : acc == 1 ? (ggml_type == GSQ_TYPE_Q4_K ? Q8_TILES_F16SD : Q8_TILES_F16S) : Q8_TILES_H16,
-                               scratch, stream);
+  const Way way = choose_way(ggml_type, packed, rows, m);
+  const int64_t ysz = y_dtype == GSQ_F32 ? 4 : 2;
+  switch (way) {
+    case W_PLANES1:
+    case W_PLANES2:
+      return gemm4_linear(w, row_bytes, rows, ggml_type, packed, x, x_dtype, m, k, x_row_stride, y, y_dtype, y_row_stride, scratch,
+                          way == W_PLANES1 ? 1 : 2, stream);
+    case W_IQ3_INT:
+      rc = quantize_tiles_host(x, x_dtype, m, k, x_row_stride, Q8_TILES_H16, scratch, stream);
       if (rc != GSQ_OK) return rc;
-      return gemm3_host(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, acc, pair, stream);
-    }
-    // (IQ4_XS with integer sums: the int8 kernel below)
+      return gemm3_host(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, stream);
+    case W_I8:
+      rc = quantize_tiles_host(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
+      if (rc != GSQ_OK) return rc;
+      return gemm2_host(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, stream);
+    case W_LOCKSTEP:
+      rc = gsq_quantize_q8_1_mmq(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
+      if (rc != GSQ_OK) return rc;
+      return gsq_mul_mat_q8(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, nullptr, 0, stream);
+    default: break;
   }
-  if (gemm2_applies(ggml_type, packed, rows) && variant == 4) {
-    rc = quantize_tiles_host(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
-    if (rc != GSQ_OK) return rc;
-    return gemm2_host(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, stream);
-  }
-  if (gemm2_applies(ggml_type, packed, rows) && (variant == 3 || variant >= 5 || (variant == 0 && big))) {
-    rc = quantize_tiles_host(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
-    if (rc != GSQ_OK) return rc;
-    return gemm2_host(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, stream);
-  }
-  if (gemm2_applies(ggml_type, packed, rows)) {
-    rc = gsq_quantize_q8_1_mmq(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
-    if (rc != GSQ_OK) return rc;
-    return gsq_mul_mat_q8(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, nullptr, 0, stream);
-  }
-  if (ggml_type == GSQ_TYPE_Q6_K && packed) {
-    // repacked Q6_K above 48 rows: the small-batch kernel, 48 rows per launch, on 36-byte blocks of the whole X
-    rc = gsq_quantize_q8_1(x, x_dtype, m, k, x_row_stride, scratch, stream);
-    if (rc != GSQ_OK) return rc;
-    const int64_t ysz6 = y_dtype == GSQ_F32 ? 4 : 2;
-    for (int64_t i = 0; i < m; i += 48) {
-      const int64_t c = m - i < 48 ? m - i : 48;
-      rc = mmv_host(w, row_bytes, rows, ggml_type, packed, (const uint8_t*)scratch + i * (k / 32) * 36, 0, c, k,
-                    (uint8_t*)y + i * y_row_stride * ysz6, y_dtype, y_row_stride, stream, nullptr);
-      if (rc != GSQ_OK) return rc == 1000 ? GSQ_ERR_TOO_LARGE : rc;
-    }
-    return GSQ_OK;
-  }
-  // Q6_K and IQ3_S in GGUF order: the dp4a kernel on 36-byte blocks, as many rows per launch as it takes
+  // as many rows per launch as the kernel takes, on 36-byte blocks of the whole X
   rc = gsq_quantize_q8_1(x, x_dtype, m, k, x_row_stride, scratch, stream);
   if (rc != GSQ_OK) return rc;
-  const int step = gsq_mul_mat_vec_max_rows(ggml_type, packed);
-  const int64_t ysz = y_dtype == GSQ_F32 ? 4 : 2;
+  const int64_t step = way == W_MMV_LOOP ? 48 : gsq_mul_mat_vec_max_rows(ggml_type, packed);
   for (int64_t i = 0; i < m; i += step) {
     const int64_t c = m - i < step ? m - i : step;
-    rc = gsq_mul_mat_vec_q8(w, row_bytes, rows, ggml_type, packed, (const uint8_t*)scratch + i * (k / 32) * 36, c, k,
-                            (uint8_t*)y + i * y_row_stride * ysz, y_dtype, y_row_stride, stream);
+    const uint8_t* xq = (const uint8_t*)scratch + i * (k / 32) * 36;
+    uint8_t* yi = (uint8_t*)y + i * y_row_stride * ysz;
+    if (way == W_MMV_LOOP) {
+      rc = mmv_host(w, row_bytes, rows, ggml_type, packed, xq, 0, c, k, yi, y_dtype, y_row_stride, stream, nullptr);
+      if (rc == 1000) return GSQ_ERR_TOO_LARGE;
+    } else {
+      rc = gsq_mul_mat_vec_q8(w, row_bytes, rows, ggml_type, packed, xq, c, k, yi, y_dtype, y_row_stride, stream);
+    }
     if (rc != GSQ_OK) return rc;
   }
   return GSQ_OK;

@@ -8,50 +8,9 @@
 // 32-value block. The block sum is formed in the same order as the reference's 16,8,4,2,1
 // xor-shuffle tree over one value per lane (common.cuh:468-475): lane offsets 16 and 8 become
 // thread offsets 2 and 1, offsets 4,2,1 become a tree inside the thread.
-#include "gsq_common.cuh"
+#include "gsq_quant.cuh"
 
 namespace gsq {
-
-__device__ __forceinline__ float div_approx(float a, float b) {
-  float r;
-  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float rcp_approx(float a) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ float to_f32(T v);
-template <>
-__device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
-template <>
-__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-// 8 consecutive values of row `row` starting at column c (c % 8 == 0). VEC: 16-byte aligned rows.
-// Loads go to L2 (ld.global.cg): launched as a programmatic dependent, this kernel can be resident while the
-// kernel that writes X still runs, so X is not read-only for its lifetime and the non-coherent path is not valid.
-template <typename T, bool VEC>
-__device__ __forceinline__ void load8(const T* __restrict__ x, int64_t off, float (&v)[8]) {
-  if constexpr (VEC && sizeof(T) == 2) {
-    const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(x + off));
-    const T* p = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = to_f32<T>(p[e]);
-  } else if constexpr (VEC && sizeof(T) == 4) {
-    const float4 a = __ldcg(reinterpret_cast<const float4*>(x + off));
-    const float4 b = __ldcg(reinterpret_cast<const float4*>(x + off + 4));
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = to_f32<T>(__ldcg(x + off + e));
-  }
-}
 
 __device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d) {
   // float -> int8 as the C conversion in the reference (round toward zero of an already rounded value)
@@ -169,41 +128,6 @@ __global__ void __launch_bounds__(256) quantize_q8_1_mmq_kernel(const T* __restr
   }
 }
 
-// Per token (one warp each) the power of two that brings its largest magnitude over all of k to [2^13, 2^14), stored as
-// its reciprocal; tokens past m get 0, a token of zeros 1. For the scaled-product units below.
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(256) row_scale_kernel(const T* __restrict__ x, float* __restrict__ inv_scale, int64_t m,
-                                                       int64_t mpad, int64_t k, int64_t stride) {
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row >= mpad) return;
-  if (row >= m) {
-    if (lane == 0) inv_scale[row] = 0.0f;
-    return;
-  }
-  float amax = 0.0f;
-  for (int64_t c = 8 * lane; c < k; c += 256) {
-    float v[8];
-    load8<T, VEC>(x, row * stride + c, v);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-  if (lane == 0) {
-    float inv = 1.0f;
-    if (amax > 0.0f && amax <= 3.0e38f) {
-      int e;
-      frexpf(amax, &e);                        // amax = f * 2^e, f in [0.5, 1)
-      const int up = min(max(14 - e, -100), 100);
-      inv = ldexpf(1.0f, -up);
-    }
-    inv_scale[row] = inv;
-  }
-}
-
 // Activation units of the prefill GEMMs (gsq_gemm2.cu, gsq_gemm3.cu): the same quantisation as
 // quantize_q8_1_mmq_kernel (32-value blocks, d = 1 / (127 / amax), D4 or DS4 scales), written in the shared-memory layout
 // of the tensor-core operand so that one bulk copy brings a unit into place. A unit is one 32-value slice of a block
@@ -214,17 +138,6 @@ __global__ void __launch_bounds__(256) row_scale_kernel(const T* __restrict__ x,
 //   fp16 operands (LAYOUT = Q8_TILES_H16): the same quants as fp16 numbers
 //                   [32 token groups][4 K chunks of 8][8 tokens][8 fp16] quants          (16384 bytes)
 //                   [256 tokens] float d                                                 (1024 bytes)
-//   scaled products (LAYOUT = Q8_TILES_F16S / _F16S2): in the fp16 operand order, hi = fp16(d * q * 2^e[token]) (16384
-//                   bytes) and, for _F16S2, lo = fp16(d * q * 2^e - hi) (16384 more); after the last unit one float
-//                   per token of the padded range, 2^-e[token] (row_scale_kernel: 2^e brings the token's largest
-//                   magnitude to [2^13, 2^14), so no product overflows fp16 and hi + lo carries 22 bits of each)
-//   ... with sums (LAYOUT = Q8_TILES_F16SD, for Q4_K): d and sum x rounded to halves as the reference's DS4 blocks
-//                   keep them; between the last unit and the per-token floats one 8 KB unit per token block and
-//                   superblock, [32 token groups][2 K chunks of 8][8 tokens][8 fp16], for the 8 slices:
-//                   chunk 0 = half(sum x) * 2^(e - 4) (exact, below 2^15: the minimum term's activations);
-//                   chunk 1 = (sum of the slice's exact products - sum of the rounded ones) * 2^-4, what the rounding
-//                   took from the slice in total. Q4_K's quants are all of one sign (0..15), so the roundings would
-//                   add up along a slice as 8 sc * (sum of the errors); the kernel adds that amount back.
 // Tokens past m (up to the end of the last block) are written as zeros. One CUDA block = 64 tokens x one slice:
 // warp w holds token group w of the 64, lane = (token % 8) * 4 + 8-value piece, so a warp writes whole core matrices.
 template <typename T, bool VEC, int LAYOUT>
@@ -232,10 +145,8 @@ __global__ void __launch_bounds__(256) quantize_q8_1_tiles_kernel(const T* __res
                                                                  int64_t m, int64_t k, int64_t stride) {
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  constexpr bool SD = LAYOUT == Q8_TILES_F16SD;
-  constexpr bool DS = LAYOUT == GSQ_Q8_LAYOUT_DS4 || SD, H16 = LAYOUT == Q8_TILES_H16;
-  constexpr bool F16S = LAYOUT == Q8_TILES_F16S || LAYOUT == Q8_TILES_F16S2 || SD, LO = LAYOUT == Q8_TILES_F16S2;
-  constexpr int UB = F16S ? (LO ? 32768 : 16384) : H16 ? 16384 + 1024 : 8192 + (DS ? 2048 : 1024);
+  constexpr bool DS = LAYOUT == GSQ_Q8_LAYOUT_DS4, H16 = LAYOUT == Q8_TILES_H16;
+  constexpr int UB = H16 ? 16384 + 1024 : 8192 + (DS ? 2048 : 1024);
   const int slice = blockIdx.x;              // 32-value slice along k
   const int64_t tt = blockIdx.y;             // token tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -268,45 +179,10 @@ __global__ void __launch_bounds__(256) quantize_q8_1_tiles_kernel(const T* __res
   float q[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) q[e] = live && amax > 0.0f ? roundf(v[e] * d_inv) : 0.0f;   // (a block of zeros: 0 * inf)
-  float d = live ? rcp_approx(d_inv) : 0.0f;
+  const float d = live ? rcp_approx(d_inv) : 0.0f;
   const int sb = slice >> 3, s = slice & 7;
   const int rb = (int)(tt & 3) * 64 + r;   // token within its block of 256
   uint8_t* unit = out + (((tt >> 2) * (k >> 8) + sb) * 8 + s) * UB;
-  if constexpr (F16S) {
-    uint8_t* behind = out + (int64_t)gridDim.y / 4 * (k >> 8) * 8 * UB;     // what follows the last unit
-    const float* inv_scale = reinterpret_cast<const float*>(behind + (SD ? (int64_t)gridDim.y / 4 * (k >> 8) * 8192 : 0));
-    const float up = live ? 1.0f / inv_scale[row] : 0.0f;         // 2^e, a power of two: the products below are exact
-    float sum_half = 0.0f;
-    if constexpr (SD) {
-      const float2 dsum = __half22float2(__floats2half2_rn(d, sum));   // the reference keeps half2(d, sum)
-      d = dsum.x;
-      sum_half = dsum.y;
-    }
-    const float ds = d * up;
-    uint8_t* dst = unit + (rb >> 3) * 512 + piece * 128 + (rb & 7) * 16;
-    __half2 hi[4], lo[4];
-    float lost = 0.0f;   // exact products minus rounded ones, this lane's 8 values
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float p0 = ds * q[2 * e], p1 = ds * q[2 * e + 1];
-      hi[e] = __floats2half2_rn(p0, p1);
-      const float2 back = __half22float2(hi[e]);
-      lo[e] = __floats2half2_rn(p0 - back.x, p1 - back.y);
-      lost += (p0 - back.x) + (p1 - back.y);
-    }
-    if constexpr (SD) {
-      lost += __shfl_xor_sync(0xFFFFFFFFu, lost, 2);
-      lost += __shfl_xor_sync(0xFFFFFFFFu, lost, 1);
-      if (piece == 0) {
-        uint8_t* su = behind + ((tt >> 2) * (k >> 8) + sb) * 8192 + (rb >> 3) * 256 + (rb & 7) * 16;
-        reinterpret_cast<__half*>(su)[s] = __float2half_rn(sum_half * up * 0.0625f);
-        reinterpret_cast<__half*>(su + 128)[s] = __float2half_rn(lost * 0.0625f);
-      }
-    }
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(hi);
-    if constexpr (LO) *reinterpret_cast<uint4*>(dst + 16384) = *reinterpret_cast<const uint4*>(lo);
-    return;
-  }
   if constexpr (H16) {
     // the lane's 8 values are one 16-byte row of a core matrix (integers up to 127 in magnitude: exact in fp16)
     uint8_t* dst = unit + (rb >> 3) * 512 + piece * 128 + (rb & 7) * 16;
@@ -482,17 +358,6 @@ template <typename T, int LAYOUT>
 static int launch_q8_1_tiles(const void* x, int64_t m, int64_t k, int64_t stride, void* out, cudaStream_t st) {
   if (m == 0) return GSQ_OK;
   const bool vec = ((uintptr_t)x % 16 == 0) && ((stride * (int64_t)sizeof(T)) % 16 == 0);
-  if constexpr (LAYOUT == Q8_TILES_F16S || LAYOUT == Q8_TILES_F16S2 || LAYOUT == Q8_TILES_F16SD) {
-    // first the per-token scales, behind the last unit (and the units of sums)
-    const int64_t mpad = (m + 255) / 256 * 256;
-    float* inv_scale = reinterpret_cast<float*>((uint8_t*)out + mpad / 256 * (k >> 8) *
-                                                                    (8 * (LAYOUT == Q8_TILES_F16S2 ? 32768 : 16384) +
-                                                                     (LAYOUT == Q8_TILES_F16SD ? 8192 : 0)));
-    const unsigned grid = (unsigned)(mpad / 8);
-    const int rc = vec ? launch_pdl(row_scale_kernel<T, true>, grid, st, (const T*)x, inv_scale, m, mpad, k, stride)
-                       : launch_pdl(row_scale_kernel<T, false>, grid, st, (const T*)x, inv_scale, m, mpad, k, stride);
-    if (rc != GSQ_OK) return rc;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(k >> 5), (unsigned)((m + 255) / 256 * 4));   // whole blocks of 256 tokens
   cfg.blockDim = dim3(256);
@@ -516,9 +381,6 @@ int quantize_tiles_host(const void* x, int x_dtype, int64_t m, int64_t k, int64_
   cudaStream_t st = (cudaStream_t)stream;
 #define GSQ_TILES_CASE(T)                                                                                  \
   return layout == Q8_TILES_H16      ? launch_q8_1_tiles<T, Q8_TILES_H16>(x, m, k, stride, out, st)     \
-         : layout == Q8_TILES_F16S   ? launch_q8_1_tiles<T, Q8_TILES_F16S>(x, m, k, stride, out, st)    \
-         : layout == Q8_TILES_F16S2  ? launch_q8_1_tiles<T, Q8_TILES_F16S2>(x, m, k, stride, out, st)   \
-         : layout == Q8_TILES_F16SD  ? launch_q8_1_tiles<T, Q8_TILES_F16SD>(x, m, k, stride, out, st)   \
          : layout == GSQ_Q8_LAYOUT_D4 ? launch_q8_1_tiles<T, GSQ_Q8_LAYOUT_D4>(x, m, k, stride, out, st) \
                                       : launch_q8_1_tiles<T, GSQ_Q8_LAYOUT_DS4>(x, m, k, stride, out, st)
   switch (x_dtype) {
