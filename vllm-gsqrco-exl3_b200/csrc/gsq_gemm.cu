@@ -889,9 +889,10 @@ static int g_gemm_variant = 0;  // behind gsq_linear: 0 = choose by shape, 3 = a
 int gemm2_error_flag(int* flag);  // gsq_gemm2.cu
 int gemm3_error_flag(int* flag);  // gsq_gemm3.cu
 int gemm4_error_flag(int* flag);  // gsq_gemm4.cu
+int gemm5_error_flag(int* flag);  // gsq_gemm5.cu
 
 int gemm_error_flag(int* flag) {
-  int a = 0, b = 0, c = 0, d = 0;
+  int a = 0, b = 0, c = 0, d = 0, e = 0;
   GSQ_CUDA_TRY(cudaMemcpyFromSymbol(&a, g_gemm_error, sizeof(int)));
   int rc = gemm2_error_flag(&b);
   if (rc != GSQ_OK) return rc;
@@ -899,7 +900,9 @@ int gemm_error_flag(int* flag) {
   if (rc != GSQ_OK) return rc;
   rc = gemm4_error_flag(&d);
   if (rc != GSQ_OK) return rc;
-  *flag = a | b | c | d;
+  rc = gemm5_error_flag(&e);
+  if (rc != GSQ_OK) return rc;
+  *flag = a | b | c | d | e;
   return GSQ_OK;
 }
 
@@ -960,7 +963,7 @@ extern "C" int gsq_debug_swap_descriptor_strides(int on) {
 
 extern "C" int gsq_debug_gemm_variant(int v) {
   const int old = gsq::g_gemm_variant;
-  gsq::g_gemm_variant = (v >= 1 && v <= 9) ? v : 0;
+  gsq::g_gemm_variant = (v >= 1 && v <= 10) ? v : 0;
   return old;
 }
 

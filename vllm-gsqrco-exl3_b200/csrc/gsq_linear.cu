@@ -22,6 +22,11 @@ bool gemm3_applies(int ggml_type, int packed, int64_t rows);
 size_t gemm3_tile_bytes(int64_t m, int64_t k);
 int gemm3_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x_tiles, int64_t m,
                int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream);
+// gsq_gemm5.cu
+bool gemm5_applies(int ggml_type, int packed, int64_t rows, int64_t m);
+size_t gemm5_scratch_bytes(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k);
+int gemm5_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
+                 int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* scratch, void* stream);
 // gsq_gemm4.cu
 size_t gemm4_scratch_bytes(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu);
 int gemm4_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
@@ -42,6 +47,7 @@ enum Way {
   W_PLANES2,    // the same with the activations as hi + lo: fp32 accuracy
   W_IQ3_INT,    // gsq_gemm3.cu: fp16 operands, integer slice sums
   W_I8,         // gsq_gemm2.cu: int8 prefill GEMM
+  W_BATCH,      // gsq_gemm5.cu: up to 256 rows, int8 operands decoded in the kernel, work cut evenly over the SMs
   W_LOCKSTEP,   // gsq_gemm.cu: 64-token tiles, split K
   W_MMV_LOOP,   // repacked Q6_K: the small-batch kernel, 48 rows per launch
   W_GEMV_LOOP   // GGUF-order blocks: the dp4a kernels, 8 rows per launch
@@ -50,9 +56,12 @@ enum Way {
 static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m) {
   const int variant = gemm_variant();
   const bool dump = gemm_dump_pointer() != nullptr;   // (per-slice integer sums: only the integer forms have them)
+  if (variant == 10 && !dump && gemm5_applies(ggml_type, packed, rows, m)) return W_BATCH;
   if (gemm2_applies(ggml_type, packed, rows)) {
     // Repacked IQ3_S, IQ4_XS, Q4_K. The prefill forms from 256 tokens on, and from 128 where the weight alone gives half
-    // an SM count of row tiles; the int8 one, where integer sums are asked for, from 512 and 192. Below, the lockstep kernel.
+    // an SM count of row tiles; the int8 one, where integer sums are asked for, from 512 and 192. Below, the kernel with
+    // integer sums and evenly cut work (100 rows, us, it / the lockstep kernel: IQ3_S 17408 x 5120 82 / 158, IQ4_XS
+    // 5120 x 17408 90 / 261, Q4_K 2048 x 2048 17 / 21).
     const bool tall = (rows + 127) / 128 >= 74, iq3 = gemm3_applies(ggml_type, packed, rows);
     const bool big3 = m >= 256 || (m >= 128 && tall), big = m >= 512 || (m >= 192 && tall);
     if (variant == 3 || variant >= 5 || (variant == 0 && big3)) {
@@ -63,7 +72,8 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m) {
       if (planes) return planes == 1 ? W_PLANES1 : W_PLANES2;
       if (iq3) return W_IQ3_INT;
     }
-    return variant == 3 || variant == 4 || variant >= 5 || (variant == 0 && big) ? W_I8 : W_LOCKSTEP;
+    if (variant == 3 || variant == 4 || variant >= 5 || (variant == 0 && big)) return W_I8;
+    return variant == 0 && !dump && gemm5_applies(ggml_type, packed, rows, m) ? W_BATCH : W_LOCKSTEP;
   }
   const bool q6 = ggml_type == GSQ_TYPE_Q6_K, q6_packed = q6 && packed && rows % 16 == 0;
   // Q6_K, IQ3_S in GGUF order and the low-bit types: the two steps once they cost less than the repeated launches of the
@@ -72,12 +82,22 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m) {
   return q6_packed ? W_MMV_LOOP : W_GEMV_LOOP;
 }
 
+// Whether the small-batch tensor-core kernel is tried first. It serves 1..48 rows; for the types in GGUF order, whose
+// decoding it repeats per lane, the kernel with evenly cut work is faster from 33 rows on (48 rows, us: IQ4_XS 5120 x 17408
+// 64 -> 58, Q4_K 17408 x 5120 59 -> 52, 2048 x 2048 16.5 -> 13.5; at 32 rows they are level; repacked IQ3_S 44 against 54).
+static bool small_batch(int ggml_type, int packed, int64_t rows, int64_t m) {
+  if (gemm_variant() == 10 || !mmv_applies(ggml_type, packed, rows, m)) return false;
+  const bool gguf = ggml_type == GSQ_TYPE_IQ4_XS || ggml_type == GSQ_TYPE_Q4_K;
+  return !(gguf && m > 32 && gemm_variant() == 0 && !gemm_dump_pointer());
+}
+
 static size_t way_scratch(Way way, int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
   switch (way) {
     case W_PLANES1: return gemm4_scratch_bytes(ggml_type, packed, rows, m, k, 1);
     case W_PLANES2: return gemm4_scratch_bytes(ggml_type, packed, rows, m, k, 2);
     case W_IQ3_INT: return gemm3_tile_bytes(m, k);
     case W_I8: return gemm2_tile_bytes(m, k, ggml_type);
+    case W_BATCH: return gemm5_scratch_bytes(ggml_type, packed, rows, m, k);
     case W_LOCKSTEP: return (size_t)(k / 128) * (size_t)m * 144;
     default: return (size_t)(k / 32) * (size_t)m * 36;
   }
@@ -96,7 +116,7 @@ extern "C" size_t gsq_linear_scratch_bytes(int64_t rows, int64_t m, int64_t k, i
   if (m <= 0 || k <= 0 || rows <= 0) return 0;
   size_t b = way_scratch(choose_way(ggml_type, packed, rows, m), rows, m, k, ggml_type, packed);
   // (the small-batch kernel takes 128-value blocks, and may decline the shape)
-  const size_t mmq = mmv_applies(ggml_type, packed, rows, m) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
+  const size_t mmq = small_batch(ggml_type, packed, rows, m) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
   b = b > mmq ? b : mmq;
   return align256(b > 0 ? b : 1);
 }
@@ -114,7 +134,7 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
   const int layout = gsq_q8_layout_for_type(ggml_type);
   int rc;
   // 1..48 rows: the small-batch tensor-core kernel on 128-value blocks, where it serves the type and the shape fits
-  if (mmv_applies(ggml_type, packed, rows, m)) {
+  if (small_batch(ggml_type, packed, rows, m)) {
     rc = gsq_quantize_q8_1_mmq(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
     if (rc != GSQ_OK) return rc;
     rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, 1, m, k, y, y_dtype, y_row_stride, stream, gemm_dump_pointer());
@@ -135,6 +155,8 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
       rc = quantize_tiles_host(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
       if (rc != GSQ_OK) return rc;
       return gemm2_host(w, row_bytes, rows, ggml_type, packed, scratch, m, k, y, y_dtype, y_row_stride, stream);
+    case W_BATCH:
+      return gemm5_linear(w, row_bytes, rows, ggml_type, packed, x, x_dtype, m, k, x_row_stride, y, y_dtype, y_row_stride, scratch, stream);
     case W_LOCKSTEP:
       rc = gsq_quantize_q8_1_mmq(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
       if (rc != GSQ_OK) return rc;
