@@ -227,10 +227,13 @@ int gsq_mul_mat_q8(const void* w, int64_t row_bytes, int64_t rows, int ggml_type
  * in one call: lcpp_mul_mat_q, lcpp_mul_mat_mma_k, lcpp_mul_mat_iq3_packed (lcpp_shim.cu:626-671, 753-909, whose
  * scratch comes from torch's allocator, :250-263).
  *   x            [m, k] in x_dtype, row stride x_row_stride elements
- *   scratch      gsq_linear_scratch_bytes(...) bytes, 256-byte aligned; need not be initialised, not preserved. The
- *                prefill GEMM keeps the expanded weights there: 2 bytes per weight (4 for Q6_K), at most 512 MB at a time
+ *   scratch      256-byte aligned; need not be initialised, not preserved. With gsq_linear_workspace_bytes(...) bytes the
+ *                fastest kernels run: the prefill GEMM then keeps the expanded weights there, 2 bytes per weight (4 for
+ *                Q6_K), at most 512 MB at a time. gsq_linear_scratch_bytes(...) bytes, the least, have no room for that:
+ *                the kernels that decode the weights as they go run instead
  */
 size_t gsq_linear_scratch_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed);
+size_t gsq_linear_workspace_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed);
 int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype,
                int64_t m, int64_t k, int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* scratch,
                size_t scratch_bytes, void* stream);

@@ -44,7 +44,7 @@ def test_batch_kernel(name, rows, k, m):
     lib = _cabi.lib
     old = lib.gsq_debug_gemm_variant(10)
     try:
-        n = lib.gsq_linear_scratch_bytes(rows, m, k, t, int(packed))
+        n = lib.gsq_linear_workspace_bytes(rows, m, k, t, int(packed))
         scratch = torch.full((n,), 0xFF, dtype=torch.uint8, device=DEV)
         y = torch.full((m, rows + 3), float("nan"), dtype=torch.float32, device=DEV)
         xd = x.to(DEV)

@@ -22,12 +22,12 @@ DEV = "cuda:0"
 TYPES = {**synth.TYPE_IDS, **synth.LOW_BIT_TYPE_IDS}
 
 
-def _run(t, packed, raw, x, rows, ldy=None):
+def _run(t, packed, raw, x, rows, ldy=None, least=False):
     w = torch.from_numpy(raw).to(DEV)
     if packed:
         iq3_pack.pack_(w, t)
     lib, (m, k) = _cabi.lib, x.shape
-    n = lib.gsq_linear_scratch_bytes(rows, m, k, t, int(packed))
+    n = (lib.gsq_linear_scratch_bytes if least else lib.gsq_linear_workspace_bytes)(rows, m, k, t, int(packed))
     scratch = torch.full((n,), 0xFF, dtype=torch.uint8, device=DEV)     # nothing may rely on what it holds
     ldy = ldy or rows
     y = torch.full((m, ldy), float("nan"), dtype=torch.float32, device=DEV)
@@ -82,3 +82,17 @@ def test_rounded_kinds_over_token_blocks(name, m):
     x = synth.nudge_ties_torch(torch.from_numpy(synth.make_activation(m, k, 71 + m)).to(torch.bfloat16)).float()
     got = _run(t, name == "IQ3_S", raw, x.to(DEV), rows)
     assert product.rel_err(got, prefill_forms.product(raw, t, x.numpy())) <= 3e-6
+
+
+@pytest.mark.parametrize("name,packed,m", [("IQ3_S", True, 256), ("IQ4_XS", False, 300), ("Q4_K", False, 520), ("Q6_K", True, 99),
+                                           ("Q6_K", False, 26)])
+def test_least_scratch(name, packed, m):
+    """A caller whose scratch has no room for expanded weights gets the kernels that need none."""
+    t, rows, k = TYPES[name], 272, 1024
+    raw = synth.make_weight(t, rows, k, 72)
+    x = synth.nudge_ties_torch(torch.from_numpy(synth.make_activation(m, k, 73 + m)).to(torch.bfloat16)).float()
+    lib = _cabi.lib
+    assert lib.gsq_linear_scratch_bytes(rows, m, k, t, int(packed)) < lib.gsq_linear_workspace_bytes(rows, m, k, t, int(packed))
+    got = _run(t, packed, raw, x.to(DEV), rows, least=True)
+    q, d, _ = q8_1.quantize_q8_1(x.numpy())
+    assert product.rel_err(got, product.product_q81(blocks.decode(raw, t), q, d)) <= 3e-3   # (d in half or in fp32; Q4_K: sums of x or of q)

@@ -53,7 +53,8 @@ enum Way {
   W_GEMV_LOOP   // GGUF-order blocks: the dp4a kernels, 8 rows per launch
 };
 
-static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m) {
+// small: the scratch has no room for expanded weights: the forms that need none instead, none less exact
+static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, bool small) {
   const int variant = gemm_variant();
   const bool dump = gemm_dump_pointer() != nullptr;   // (per-slice integer sums: only the integer forms have them)
   if (variant == 10 && !dump && gemm5_applies(ggml_type, packed, rows, m)) return W_BATCH;
@@ -69,7 +70,7 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m) {
       if (variant == 5 || variant == 9) planes = ggml_type == GSQ_TYPE_Q4_K ? 1 : 2;
       if (variant == 6 || variant == 8) planes = 1;
       if (variant == 7 || dump) planes = 0;
-      if (planes) return planes == 1 ? W_PLANES1 : W_PLANES2;
+      if (planes && !(planes == 1 && small)) return planes == 1 ? W_PLANES1 : W_PLANES2;
       if (iq3) return W_IQ3_INT;
     }
     if (variant == 3 || variant == 4 || variant >= 5 || (variant == 0 && big)) return W_I8;
@@ -78,7 +79,7 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m) {
   const bool q6 = ggml_type == GSQ_TYPE_Q6_K, q6_packed = q6 && packed && rows % 16 == 0;
   // Q6_K, IQ3_S in GGUF order and the low-bit types: the two steps once they cost less than the repeated launches of the
   // small-batch kernels (48 or 8 rows each), at fp32 accuracy, unless integer sums are asked for.
-  if (!dump && g_prefill_precision != GSQ_PREFILL_INTEGER && m >= (q6_packed ? 97 : q6 || ggml_type == GSQ_TYPE_IQ3_S ? 25 : 9)) return W_PLANES2;
+  if (!small && !dump && g_prefill_precision != GSQ_PREFILL_INTEGER && m >= (q6_packed ? 97 : q6 || ggml_type == GSQ_TYPE_IQ3_S ? 25 : 9)) return W_PLANES2;
   return q6_packed ? W_MMV_LOOP : W_GEMV_LOOP;
 }
 
@@ -111,14 +112,27 @@ extern "C" int gsq_prefill_precision(int mode) {
   return old;
 }
 
-extern "C" size_t gsq_linear_scratch_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
+static size_t linear_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed, bool small) {
   using namespace gsq;
   if (m <= 0 || k <= 0 || rows <= 0) return 0;
-  size_t b = way_scratch(choose_way(ggml_type, packed, rows, m), rows, m, k, ggml_type, packed);
+  const Way way = choose_way(ggml_type, packed, rows, m, small);
+  size_t b = way_scratch(way, rows, m, k, ggml_type, packed);
+  if (small && gemm2_applies(ggml_type, packed, rows) && choose_way(ggml_type, packed, rows, m, false) == W_PLANES1) {
+    // one fp16 plane of activations (and Q4_K's block sums): room for any of the forms of the default precision
+    const size_t plane = gemm3_tile_bytes(m, k) + (ggml_type == GSQ_TYPE_Q4_K ? (size_t)((m + 255) / 256) * (k / 256) * 8192 : 0);
+    b = b > plane ? b : plane;
+  }
   // (the small-batch kernel takes 128-value blocks, and may decline the shape)
   const size_t mmq = small_batch(ggml_type, packed, rows, m) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
   b = b > mmq ? b : mmq;
   return align256(b > 0 ? b : 1);
+}
+extern "C" size_t gsq_linear_scratch_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
+  const size_t small = linear_bytes(rows, m, k, ggml_type, packed, true), full = linear_bytes(rows, m, k, ggml_type, packed, false);
+  return small < full ? small : full;
+}
+extern "C" size_t gsq_linear_workspace_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
+  return linear_bytes(rows, m, k, ggml_type, packed, false);
 }
 
 extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x,
@@ -140,7 +154,7 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
     rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, 1, m, k, y, y_dtype, y_row_stride, stream, gemm_dump_pointer());
     if (rc != 1000) return rc;  // 1000: declined, the activations of this shape do not fit its staging area
   }
-  const Way way = choose_way(ggml_type, packed, rows, m);
+  const Way way = choose_way(ggml_type, packed, rows, m, scratch_bytes < gsq_linear_workspace_bytes(rows, m, k, ggml_type, packed));
   const int64_t ysz = y_dtype == GSQ_F32 ? 4 : 2;
   switch (way) {
     case W_PLANES1:

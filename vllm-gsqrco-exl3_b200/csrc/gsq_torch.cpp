@@ -193,7 +193,7 @@ void product(const Spec& s, const Weight& w, const Tensor& x, int64_t i0, int64_
     }
     return;
   }
-  const size_t need = gsq_linear_scratch_bytes(row, n, k, (int)type, s.packed);
+  const size_t need = gsq_linear_workspace_bytes(row, n, k, (int)type, s.packed);
   Tensor scratch = bytes(std::max<int64_t>((int64_t)need, 1), x);
   const int64_t xs = row_stride(x, k);
   const char* xp = (const char*)x.const_data_ptr() + i0 * xs * es;
