@@ -1,0 +1,67 @@
+"""Small products that quantise X inside the product kernel: the quantiser kernels' values (so the two-call result up to the
+order of the fp32 sums), ragged rows of Y and column counts, strided and unaligned X, each data type."""
+
+import numpy as np
+import pytest
+import torch
+
+import gsq_b200  # noqa: F401
+from gsq_b200 import _cabi, synth
+from gsq_b200.quantization import iq3_pack
+from oracle import blocks, product, q8_1
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+TYPES = {"IQ3_S": 21, "IQ4_XS": 23, "Q4_K": 12, "Q6_K": 14}
+DTYPES = {"fp32": (0, torch.float32), "fp16": (1, torch.float16), "bf16": (2, torch.bfloat16)}
+UNSUPPORTED = -3
+
+
+@pytest.mark.parametrize("name", list(TYPES))
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("rows,k,ms", [(16, 256, (1, 5, 8, 16)), (1040, 2304, (1, 2, 7, 8, 9, 15)), (2064, 5120, (1, 3, 4))])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_quantised_in_the_product(name, dtype, rows, k, ms, pad):
+    t = TYPES[name]
+    lib, code, tdt = _cabi.lib, DTYPES[dtype][0], DTYPES[dtype][1]
+    raw = synth.make_weight(t, rows, k, 90 + rows)
+    dec = blocks.decode(raw, t)
+    w = torch.from_numpy(raw).to(DEV)
+    packed = name in ("IQ3_S", "Q6_K")
+    if packed:
+        iq3_pack.pack_(w, t)
+    st = torch.cuda.current_stream().cuda_stream
+    for m in ms:
+        xa = synth.make_activation(m, k, 91 + m)
+        xa[0, :64] = 0.0
+        xa[m - 1, 40] = 300.0
+        x = synth.nudge_ties_torch(torch.from_numpy(xa).to(tdt))
+        buf = torch.empty((m, k + pad), dtype=tdt, device=DEV)   # pad: rows that are not 16-byte aligned
+        buf[:, :k] = x.to(DEV)
+        xn = x.float().numpy()
+        if m <= 8:
+            y = torch.full((m, rows + 3), float("nan"), dtype=torch.float32, device=DEV)
+            rc = lib.gsq_linear_vec(w.data_ptr(), w.shape[1], rows, t, int(packed), buf.data_ptr(), code, m, k, k + pad, y.data_ptr(), 0,
+                                    rows + 3, st)
+            if rc == UNSUPPORTED:   # the dp4a kernel's products
+                assert name in ("IQ4_XS", "Q4_K") and rows > 2000 and m < 4 or m * k > 10000
+            else:
+                assert rc == 0, lib.gsq_strerror(rc)
+                q, d = q8_1.quantize_q8_1(xn)[:2]
+                want = product.product_q81(dec, q, d)
+                assert bool(torch.isnan(y[:, rows:]).all())
+                assert product.rel_err(y[:, :rows].cpu().numpy(), want) <= 2e-6
+        layout = q8_1.LAYOUT_DS4 if name == "Q4_K" else q8_1.LAYOUT_D4
+        q, d, s = q8_1.quantize_mmq(xn, layout)
+        n = lib.gsq_linear_workspace_bytes(rows, m, k, t, int(packed))
+        scratch = torch.full((n,), 0xFF, dtype=torch.uint8, device=DEV)
+        y = torch.full((m, rows + 3), float("nan"), dtype=torch.float32, device=DEV)
+        rc = lib.gsq_linear(w.data_ptr(), w.shape[1], rows, t, int(packed), buf.data_ptr(), code, m, k, k + pad, y.data_ptr(), 0, rows + 3,
+                            scratch.data_ptr(), n, st)
+        assert rc == 0, lib.gsq_strerror(rc)
+        if name == "Q4_K":
+            want = product.product_xsum(dec, q, d.astype(np.float16), s.astype(np.float16))
+        else:
+            want = product.product_q81(dec, q, d)
+        assert bool(torch.isnan(y[:, rows:]).all())
+        assert product.rel_err(y[:, :rows].cpu().numpy(), want) <= 2e-6

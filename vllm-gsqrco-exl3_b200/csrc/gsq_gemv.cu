@@ -940,7 +940,8 @@ bool mmv_applies(int ggml_type, int packed, int64_t rows, int64_t m);
 bool mmv_early_trigger();
 int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* xq, int x_layout,
              int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
-             const gsq_peer_reduce* pr = nullptr);
+             const gsq_peer_reduce* pr = nullptr, int x_dtype = GSQ_BF16,
+             int64_t x_row_stride = 0);
 
 static int gemv_host_dp4a(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x_q8,
                           int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,

@@ -9,9 +9,11 @@ namespace gsq {
 
 // gsq_mmv.cu
 bool mmv_applies(int ggml_type, int packed, int64_t rows, int64_t m);
+bool mmv_raw_applies(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int vec);
 int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* xq, int x_layout,
              int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
-             const gsq_peer_reduce* pr = nullptr);
+             const gsq_peer_reduce* pr = nullptr, int x_dtype = GSQ_BF16,
+             int64_t x_row_stride = 0);
 // gsq_gemm2.cu
 bool gemm2_applies(int ggml_type, int packed, int64_t rows);
 size_t gemm2_tile_bytes(int64_t m, int64_t k, int ggml_type);
@@ -149,6 +151,10 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
   int rc;
   // 1..48 rows: the small-batch tensor-core kernel on 128-value blocks, where it serves the type and the shape fits
   if (small_batch(ggml_type, packed, rows, m)) {
+    if (!gemm_dump_pointer() && mmv_raw_applies(ggml_type, packed, rows, m, k, 0)) {
+      rc = mmv_host(w, row_bytes, rows, ggml_type, packed, x, 3, m, k, y, y_dtype, y_row_stride, stream, nullptr, nullptr, x_dtype, x_row_stride);
+      if (rc != 1000) return rc;
+    }
     rc = gsq_quantize_q8_1_mmq(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
     if (rc != GSQ_OK) return rc;
     rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, 1, m, k, y, y_dtype, y_row_stride, stream, gemm_dump_pointer());
@@ -211,4 +217,15 @@ extern "C" int gsq_linear_allreduce(const void* w, int64_t row_bytes, int64_t ro
   if (rc != GSQ_OK) return rc;
   rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, 1, m, k, y, y_dtype, y_row_stride, stream, nullptr, pr);
   return rc == 1000 ? GSQ_ERR_UNSUPPORTED : rc;   // 1000: the shape does not fit the kernel's staging area
+}
+
+extern "C" int gsq_linear_vec(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype,
+                              int64_t m, int64_t k, int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* stream) {
+  using namespace gsq;
+  if (m == 0 || rows == 0) return GSQ_OK;
+  if (m < 0 || m > 8 || rows < 0 || k <= 0 || k % 256 != 0 || !w || !x || !y) return GSQ_ERR_UNSUPPORTED;
+  if (!mmv_raw_applies(ggml_type, packed, rows, m, k, 1)) return GSQ_ERR_UNSUPPORTED;
+  const int rc = mmv_host(w, row_bytes, rows, ggml_type, packed, x, 2, m, k, y, y_dtype, y_row_stride, stream, nullptr, nullptr, x_dtype,
+                          x_row_stride);
+  return rc == 1000 ? GSQ_ERR_UNSUPPORTED : rc;
 }

@@ -47,10 +47,34 @@ bool mmv_applies(int ggml_type, int packed, int64_t rows, int64_t m) {
   return m >= (g_mmv_min_rows > 0 ? g_mmv_min_rows : min_rows);
 }
 
+// Whether X itself (quantised while it is staged) may be served here: as block_q8_1 (vec) 1..8 rows, as block_q8_1_mmq
+// 1..16. A quantiser kernel in front costs 1 to 2 us of GPU time and, where the host is what limits, 2.5 us of its time;
+// quantising in every CTA costs about 0.5 us per 1000 values of a CTA's share. Level at 16000 values of X, with IQ3_S at 10000
+// (GPU us, here / two kernels: Q6_K 5120 x 5120 1 row 10.6 / 11.3, 4 rows 11.0 / 11.4, 8 rows 12.0 / 11.8; Q4_K
+// 17408 x 5120 2 rows 17.1 / 17.4, 4 rows 17.9 / 17.6; IQ3_S 17408 x 5120 1 row 18.2 / 18.7, 4 rows 18.9 / 18.6); on small
+// products at 40000 (1024 x 5120 8 rows Q6_K 7.8 / 8.2), where the host's share counts too (1024 x 2048 called one by one
+// 5.4 / 8.0).
+bool mmv_raw_applies(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int vec) {
+  if (g_mmv_mode == 1 || m > (vec ? 8 : 16) || m > g_mmv_max_rows || m < g_mmv_min_rows) return false;
+  const bool small = rows * k <= (8 << 20), iq3 = ggml_type == GSQ_TYPE_IQ3_S;
+  if (m * k > (small ? 40960 : iq3 ? 10240 : 16384)) return false;
+  switch (ggml_type) {
+    case GSQ_TYPE_Q4_K:
+    case GSQ_TYPE_IQ4_XS:
+      // (at these row counts the dp4a kernel is faster, 8.0 / 11.9 us at 5120 x 5120, but for the launch that it costs)
+      if (m < (ggml_type == GSQ_TYPE_Q4_K ? 2 : 4) && rows * k > (3 << 20)) return false;
+      return !packed;
+    case GSQ_TYPE_IQ3_S:
+    case GSQ_TYPE_Q6_K: return packed && rows % 16 == 0;
+    default: return false;
+  }
+}
+
 // x_layout: 0 = block_q8_1, 1 = block_q8_1_mmq. Returns MMV_DECLINED when the shape does not fit.
+// x_layout 2 / 3: xq is X itself (x_dtype, rows x_row_stride elements apart), up to 8 / 16 rows.
 int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* xq, int x_layout,
              int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
-             const gsq_peer_reduce* pr) {
+             const gsq_peer_reduce* pr, int x_dtype, int64_t x_row_stride) {
   if (pr && (m == 0 || rows == 0)) return GSQ_ERR_UNSUPPORTED;   // every rank must launch: nothing to skip
   if (m == 0 || rows == 0) return GSQ_OK;
   if (m < 0 || m > 48 || rows < 0 || k <= 0 || k % 256 != 0 || !w || !xq || !y) return GSQ_ERR_UNSUPPORTED;
@@ -83,6 +107,10 @@ int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int 
   a.pr_rank = 0;
   a.pr_world = 1;
   a.pr_slot_bytes = 0;
+  a.x_dtype = x_dtype;
+  a.x_stride = x_row_stride;
+  a.x_vec = (uintptr_t)xq % 16 == 0 && (x_row_stride * (x_dtype == GSQ_F32 ? 4 : 2)) % 16 == 0;
+  if (x_layout >= XL_XQ81 && ((x_dtype != GSQ_F32 && x_dtype != GSQ_F16 && x_dtype != GSQ_BF16) || dump || pr)) return GSQ_ERR_UNSUPPORTED;
   if (pr) {
     const int64_t esz = y_dtype == GSQ_F32 ? 4 : 2;
     if (!pr->slots || !pr->flags || !pr->state || pr->world < 2 || pr->world > 8 || pr->rank < 0 || pr->rank >= pr->world ||

@@ -34,6 +34,7 @@
 #include <cstdio>
 
 #include "gsq_common.cuh"
+#include "gsq_quant.cuh"
 #include "gsq_tables.h"
 
 namespace cg = cooperative_groups;
@@ -41,7 +42,9 @@ namespace cg = cooperative_groups;
 namespace gsq {
 
 enum { MK_Q4K = 0, MK_IQ3S = 1, MK_IQ4XS = 2, MK_Q6K = 3 };
-enum { XL_Q81 = 0, XL_MMQ = 1 };
+// what the activations come as: block_q8_1, block_q8_1_mmq, or X itself, quantised while it is staged with the arithmetic
+// of the one (XL_XQ81) or the other (XL_XMMQ)
+enum { XL_Q81 = 0, XL_MMQ = 1, XL_XQ81 = 2, XL_XMMQ = 3 };
 
 constexpr int MMV_WARPS = 16;
 constexpr int MMV_THREADS = MMV_WARPS * 32;
@@ -72,6 +75,11 @@ struct MmvArgs {
   // ([0]) and with nsr_lo + 1 ([1]: K does not split evenly); 16-byte pieces per row of block_q8_1_mmq blocks
   int nsr_lo;
   uint32_t inv_gpc[2], inv_nkb[2], inv_per;
+  // XL_XQ81 / XL_XMMQ: xq is X [m, k] in x_dtype, rows x_stride elements apart, x_vec: 16-byte aligned; fast_div_inv of
+  // the 8-value pieces per staged column
+  int x_dtype, x_vec;
+  int64_t x_stride;
+  uint32_t inv_ppc[2];
   unsigned long long* prof;  // debug: per CTA 8 time stamps (ns) at the phase boundaries
   // Sum over GPUs of the partial results of a K-sharded product, inside this kernel (pr_world > 1; see the end of
   // mmv_kernel): every rank's slot area [2][world][pr_slot_bytes] and flag area [world], the same offsets on every
@@ -233,6 +241,27 @@ __device__ __forceinline__ void stage_x_pad(int m, int nkb, int colb, uint8_t* x
 template <bool PERM>
 __device__ __forceinline__ int x_slot(int w) { return PERM ? ((w & 3) << 1) | (w >> 2) : w; }
 
+// what multiplies the minimums with block_q8_1 activations: d * (integer sum of the block's quants), from the staged quants
+template <int MC>
+__device__ __forceinline__ void stage_x_sums(const MmvArgs& a, int nkb, int colb, const uint8_t* xq, const float* xd, float* xs, int tid) {
+  const uint32_t inv_nkb = nkb == a.nsr_lo * 8 ? a.inv_nkb[0] : a.inv_nkb[1];
+  __syncthreads();
+  for (int i = tid; i < nkb * a.m; i += MMV_THREADS) {
+    const int col = fast_div(i, inv_nkb), kb = i - col * nkb;
+    const uint4* q = reinterpret_cast<const uint4*>(xq + col * colb + kb * 32);
+    const uint4 lo = q[0], hi = q[1];
+    int sum = dp4a(0x01010101, (int)lo.x, 0);
+    sum = dp4a(0x01010101, (int)lo.y, sum);
+    sum = dp4a(0x01010101, (int)lo.z, sum);
+    sum = dp4a(0x01010101, (int)lo.w, sum);
+    sum = dp4a(0x01010101, (int)hi.x, sum);
+    sum = dp4a(0x01010101, (int)hi.y, sum);
+    sum = dp4a(0x01010101, (int)hi.z, sum);
+    sum = dp4a(0x01010101, (int)hi.w, sum);
+    xs[kb * MC + col] = xd[kb * MC + col] * (float)sum;
+  }
+}
+
 template <int MC, bool DS, bool PERM, typename AfterIssue>
 __device__ __forceinline__ void stage_x_q81(const MmvArgs& a, int kb0, int nkb, int colb, uint8_t* xq, float* xd, float* xs,
                                             int tid, AfterIssue after_issue) {
@@ -241,7 +270,6 @@ __device__ __forceinline__ void stage_x_q81(const MmvArgs& a, int kb0, int nkb, 
   const int total = gpc * a.m;
   const int which = nkb == a.nsr_lo * 8 ? 0 : 1;
   const uint32_t inv = which ? a.inv_gpc[1] : a.inv_gpc[0];
-  const uint32_t inv_nkb = which ? a.inv_nkb[1] : a.inv_nkb[0];
   constexpr int U = 4;
   for (int i0 = tid; i0 < total || i0 == tid; i0 += U * MMV_THREADS) {
     uint4 v[U];
@@ -275,23 +303,7 @@ __device__ __forceinline__ void stage_x_q81(const MmvArgs& a, int kb0, int nkb, 
   }
   mmv_stamp(a, 7);
   stage_x_pad<MC, DS>(a.m, nkb, colb, xq, xd, xs, tid);
-  if (DS) {
-    __syncthreads();
-    for (int i = tid; i < nkb * a.m; i += MMV_THREADS) {
-      const int col = fast_div(i, inv_nkb), kb = i - col * nkb;
-      const uint4* q = reinterpret_cast<const uint4*>(xq + col * colb + kb * 32);
-      const uint4 lo = q[0], hi = q[1];
-      int sum = dp4a(0x01010101, (int)lo.x, 0);
-      sum = dp4a(0x01010101, (int)lo.y, sum);
-      sum = dp4a(0x01010101, (int)lo.z, sum);
-      sum = dp4a(0x01010101, (int)lo.w, sum);
-      sum = dp4a(0x01010101, (int)hi.x, sum);
-      sum = dp4a(0x01010101, (int)hi.y, sum);
-      sum = dp4a(0x01010101, (int)hi.z, sum);
-      sum = dp4a(0x01010101, (int)hi.w, sum);
-      xs[kb * MC + col] = xd[kb * MC + col] * (float)sum;
-    }
-  }
+  if (DS) stage_x_sums<MC>(a, nkb, colb, xq, xd, xs, tid);
 }
 
 // block_q8_1_mmq source (144-byte blocks, [K/128][column]: 16 scale bytes = 4 x half2(d, sum) (DS) or 4 x float
@@ -341,6 +353,100 @@ __device__ __forceinline__ void stage_x_mmq(const MmvArgs& a, int kb0, int nkb, 
     }
   }
   stage_x_pad<MC, DS>(a.m, nkb, colb, xq, xd, xs, tid);
+}
+
+// X itself (fp32 / fp16 / bf16): every CTA quantises its share of K for itself, to the quantisers' values
+// (gsq_quantize.cu): a thread takes 8 consecutive values, four neighbouring threads a 32-value block. See mmv_raw_wins for
+// what this costs against a quantiser kernel in front.
+__device__ __forceinline__ void load_x8(const MmvArgs& a, int64_t off, float (&v)[8]) {
+  if (a.x_dtype == GSQ_F32) {
+    if (a.x_vec) load8<float, true>(reinterpret_cast<const float*>(a.xq), off, v);
+    else load8<float, false>(reinterpret_cast<const float*>(a.xq), off, v);
+  } else if (a.x_dtype == GSQ_F16) {
+    if (a.x_vec) load8<__half, true>(reinterpret_cast<const __half*>(a.xq), off, v);
+    else load8<__half, false>(reinterpret_cast<const __half*>(a.xq), off, v);
+  } else {
+    if (a.x_vec) load8<__nv_bfloat16, true>(reinterpret_cast<const __nv_bfloat16*>(a.xq), off, v);
+    else load8<__nv_bfloat16, false>(reinterpret_cast<const __nv_bfloat16*>(a.xq), off, v);
+  }
+}
+__device__ __forceinline__ uint32_t pack_q4(const float* q) {
+  return (uint32_t)((int)q[0] & 0xFF) | ((uint32_t)((int)q[1] & 0xFF) << 8) | ((uint32_t)((int)q[2] & 0xFF) << 16) | ((uint32_t)(int)q[3] << 24);
+}
+template <int MC, bool DS, bool PERM, bool MMQ>
+__device__ __forceinline__ void stage_x_raw(const MmvArgs& a, int kb0, int nkb, int colb, uint8_t* xq, float* xd, float* xs, int tid) {
+  const int ppc = nkb * 4, total = ppc * a.m;
+  const uint32_t inv = nkb == a.nsr_lo * 8 ? a.inv_ppc[0] : a.inv_ppc[1];
+  constexpr int U = 4;
+#pragma unroll 1
+  for (int i0 = tid; (i0 & ~31) < total; i0 += U * MMV_THREADS) {   // (whole warps: shuffles)
+    float v[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * MMV_THREADS;
+      if (i < total) {
+        const int col = fast_div(i, inv), p = i - col * ppc;
+        load_x8(a, (int64_t)col * a.x_stride + (int64_t)kb0 * 32 + p * 8, v[u]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[u][e] = 0.0f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * MMV_THREADS;
+      if ((i & ~31) >= total) break;
+      const int col = fast_div(i, inv), p = i - col * ppc, kb = p >> 2, piece = p & 3;
+      float amax = 0.0f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[u][e]));
+      amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+      amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+      float d, q[8], sum = 0.0f;
+      if (MMQ) {
+        if (DS) {
+          // the reference sums 4 values per thread, then lane offsets 4, 2, 1 over 8 threads
+          float pa = ((v[u][0] + v[u][1]) + v[u][2]) + v[u][3];
+          float pb = ((v[u][4] + v[u][5]) + v[u][6]) + v[u][7];
+          pa += __shfl_xor_sync(0xFFFFFFFFu, pa, 2);
+          pb += __shfl_xor_sync(0xFFFFFFFFu, pb, 2);
+          pa += __shfl_xor_sync(0xFFFFFFFFu, pa, 1);
+          pb += __shfl_xor_sync(0xFFFFFFFFu, pb, 1);
+          sum = pa + pb;
+        }
+        const float d_inv = div_approx(127.0f, amax);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q[e] = roundf(v[u][e] * d_inv);
+        d = rcp_approx(d_inv);
+        if (DS) {
+          const float2 h = __half22float2(__floats2half2_rn(d, sum));
+          d = h.x;
+          sum = h.y;
+        }
+      } else {
+        // (one reciprocal for the block: eight divisions per thread would queue up at the special-function unit)
+        const float df = div_approx(amax, 127.0f), inv_d = rcp_approx(df);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q[e] = amax == 0.0f ? 0.0f : roundf(v[u][e] * inv_d);
+        d = __half2float(__float2half_rn(df));
+      }
+      if (i < total) {
+        uint8_t* dst = xq + col * colb + kb * 32;
+        if (PERM) {
+          *reinterpret_cast<uint32_t*>(dst + x_slot<true>(2 * piece) * 4) = pack_q4(q);
+          *reinterpret_cast<uint32_t*>(dst + x_slot<true>(2 * piece + 1) * 4) = pack_q4(q + 4);
+        } else {
+          *reinterpret_cast<uint2*>(dst + 8 * piece) = make_uint2(pack_q4(q), pack_q4(q + 4));
+        }
+        if (piece == 0) {
+          xd[kb * MC + col] = d;
+          if (MMQ && DS) xs[kb * MC + col] = sum;
+        }
+      }
+    }
+  }
+  stage_x_pad<MC, DS>(a.m, nkb, colb, xq, xd, xs, tid);
+  if (DS && !MMQ) stage_x_sums<MC>(a, nkb, colb, xq, xd, xs, tid);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -957,7 +1063,9 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
   const uint32_t epoch = fused ? *reinterpret_cast<volatile uint32_t*>(a.pr_state) + 1u : 0u;
   const int64_t push_off = fused ? (int64_t)((epoch & 1u) * a.pr_world + a.pr_rank) * a.pr_slot_bytes : 0;
   auto nothing = []() {};
-  if (XL == XL_Q81) {
+  if (XL == XL_XQ81 || XL == XL_XMMQ) {
+    stage_x_raw<MC, DS, MmvKind<KIND>::PERM, XL == XL_XMMQ>(a, sb0 * 8, nkb, colb, xq, xd, xs, tid);
+  } else if (XL == XL_Q81) {
     stage_x_q81<MC, DS, MmvKind<KIND>::PERM>(a, sb0 * 8, nkb, colb, xq, xd, xs, tid, nothing);
   } else {
     stage_x_mmq<MC, DS, MmvKind<KIND>::PERM>(a, sb0 * 8, nkb, colb, xq, xd, xs, tid, nothing);
@@ -1362,6 +1470,7 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
   for (int i = 0; i < 2; ++i) {
     a.inv_gpc[i] = fast_div_inv((a.nsr_lo + i) * 18);
     a.inv_nkb[i] = fast_div_inv((a.nsr_lo + i) * 8);
+    a.inv_ppc[i] = fast_div_inv((a.nsr_lo + i) * 32);
   }
   a.inv_per = fast_div_inv(a.m * 9);
   a.tiles_base = a.ntiles / best_clusters;
@@ -1393,7 +1502,7 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
   cfg.attrs = attr;
   cfg.numAttrs = g_mmv_pdl ? 2 : 1;
   if (a.pr_world > 1) {
-    if constexpr (DUMP) {
+    if constexpr (DUMP || XL == XL_XQ81 || XL == XL_XMMQ) {
       return GSQ_ERR_UNSUPPORTED;
     } else {
       static bool configured[32];
@@ -1416,31 +1525,42 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
 template <int KIND, int XL>
 static int mmv_launch_n(const MmvArgs& a, int sm_count, int max_smem, cudaStream_t st) {
   const int ntl = (a.m + 7) / 8;
-  if (a.dump) {
+  if constexpr (XL == XL_XQ81) {
+    return ntl == 1 ? mmv_launch_t<KIND, 1, XL, false>(a, sm_count, max_smem, st) : MMV_DECLINED;
+  } else if constexpr (XL == XL_XMMQ) {
+    return ntl == 1   ? mmv_launch_t<KIND, 1, XL, false>(a, sm_count, max_smem, st)
+           : ntl == 2 ? mmv_launch_t<KIND, 2, XL, false>(a, sm_count, max_smem, st)
+                      : MMV_DECLINED;
+  } else {
+    if (a.dump) {
+      switch (ntl) {
+        case 1: return mmv_launch_t<KIND, 1, XL, true>(a, sm_count, max_smem, st);
+        case 2: return mmv_launch_t<KIND, 2, XL, true>(a, sm_count, max_smem, st);
+        case 3: return mmv_launch_t<KIND, 3, XL, true>(a, sm_count, max_smem, st);
+        case 4: return mmv_launch_t<KIND, 4, XL, true>(a, sm_count, max_smem, st);
+        case 5:
+        case 6: return mmv_launch_t<KIND, 6, XL, true>(a, sm_count, max_smem, st);
+        default: return MMV_DECLINED;
+      }
+    }
     switch (ntl) {
-      case 1: return mmv_launch_t<KIND, 1, XL, true>(a, sm_count, max_smem, st);
-      case 2: return mmv_launch_t<KIND, 2, XL, true>(a, sm_count, max_smem, st);
-      case 3: return mmv_launch_t<KIND, 3, XL, true>(a, sm_count, max_smem, st);
-      case 4: return mmv_launch_t<KIND, 4, XL, true>(a, sm_count, max_smem, st);
+      case 1: return mmv_launch_t<KIND, 1, XL, false>(a, sm_count, max_smem, st);
+      case 2: return mmv_launch_t<KIND, 2, XL, false>(a, sm_count, max_smem, st);
+      case 3: return mmv_launch_t<KIND, 3, XL, false>(a, sm_count, max_smem, st);
+      case 4: return mmv_launch_t<KIND, 4, XL, false>(a, sm_count, max_smem, st);
       case 5:
-      case 6: return mmv_launch_t<KIND, 6, XL, true>(a, sm_count, max_smem, st);
+      case 6: return mmv_launch_t<KIND, 6, XL, false>(a, sm_count, max_smem, st);
       default: return MMV_DECLINED;
     }
-  }
-  switch (ntl) {
-    case 1: return mmv_launch_t<KIND, 1, XL, false>(a, sm_count, max_smem, st);
-    case 2: return mmv_launch_t<KIND, 2, XL, false>(a, sm_count, max_smem, st);
-    case 3: return mmv_launch_t<KIND, 3, XL, false>(a, sm_count, max_smem, st);
-    case 4: return mmv_launch_t<KIND, 4, XL, false>(a, sm_count, max_smem, st);
-    case 5:
-    case 6: return mmv_launch_t<KIND, 6, XL, false>(a, sm_count, max_smem, st);
-    default: return MMV_DECLINED;
   }
 }
 
 template <int KIND>
 static int mmv_launch_kind(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st) {
-  return x_layout == XL_Q81 ? mmv_launch_n<KIND, XL_Q81>(a, sm_count, max_smem, st) : mmv_launch_n<KIND, XL_MMQ>(a, sm_count, max_smem, st);
+  return x_layout == XL_Q81    ? mmv_launch_n<KIND, XL_Q81>(a, sm_count, max_smem, st)
+         : x_layout == XL_MMQ  ? mmv_launch_n<KIND, XL_MMQ>(a, sm_count, max_smem, st)
+         : x_layout == XL_XQ81 ? mmv_launch_n<KIND, XL_XQ81>(a, sm_count, max_smem, st)
+                               : mmv_launch_n<KIND, XL_XMMQ>(a, sm_count, max_smem, st);
 }
 static int mmv_peer_error(int* flag) {
   GSQ_CUDA_TRY(cudaMemcpyFromSymbol(flag, g_mmv_peer_error, sizeof(int)));

@@ -184,6 +184,13 @@ void product(const Spec& s, const Weight& w, const Tensor& x, int64_t i0, int64_
   const int dt = dtype_code(x.scalar_type());
   const int64_t es = x.element_size();
   if (s.vec) {
+    if (!x_q8.defined() && n <= 8) {
+      // quantised inside the product kernel where that is the faster way
+      const int64_t xs = row_stride(x, k);
+      const int rc = gsq_linear_vec(w.data, w.size1, row, (int)type, s.packed, (const char*)x.const_data_ptr() + i0 * xs * es, dt, n, k, xs, y,
+                                    dt, ldy, stream);
+      if (rc != GSQ_ERR_UNSUPPORTED) return check(rc, "gsq_linear_vec");
+    }
     if (!x_q8.defined()) x_q8 = quantize_blocks(x, k, stream);
     const int64_t per_row = k / 32 * 36, step = gsq_mul_mat_vec_max_rows((int)type, s.packed);
     for (int64_t i = 0; i < n; i += step) {
