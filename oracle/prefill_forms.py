@@ -1,5 +1,5 @@
 """CPU model (numpy) of the arithmetic of the prefill kernels that put the scales into fp16 tensor-core operands
-(gsq_gemm3.cu: gemm3_acc_kernel, with the activation units of quantize_q8_1_tiles_kernel). Test infrastructure: only
+(gsq_gemm4.cu on the operands that gsq_expand.cu and gsq_planes.cu write). Test infrastructure: only
 tests/ import this.
 
 These kernels are not a restatement of a reference kernel: the reference forms exact int32 sums per 32-value slice and
