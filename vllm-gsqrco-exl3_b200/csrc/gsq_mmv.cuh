@@ -584,15 +584,20 @@ __device__ __forceinline__ void process(const RecQ4K& r, const MmvArgs& ar, int 
 // ---------------------------------------------------------------------------------------------
 // IQ3_S in the fragment-ordered layout of gsq_iq3s_repack (see gsq_repack.cu): per lane 9 words of 9-bit
 // codebook indices (field f = 4 s + 2 h + e at bit 9 f), 4 words of sign bits, the sub-scale nibbles and d of
-// rows g, g + 8. The codebook copy in shared memory holds, per entry and per lane-mod-16 replica, the pair
-// (g, -g) of packed int8x4 words (entry i of replica r at byte 128 i + 8 r): a field's signed word is one
-// 64-bit load and one byte permute whose selector comes from the sign bits.
+// rows g, g + 8. The codebook copy in shared memory holds, per entry and per lane-mod-16 replica, up to 24 columns
+// the pair (g, -g) of packed int8x4 words (entry i of replica r at byte 128 i + 8 r): a field's signed word is one
+// 64-bit load and one byte permute whose selector comes from the sign bits. From 25 columns on g alone (at byte
+// 64 i + 4 r): see iq3_single.
 
 static __device__ const uint32_t g_iq3s_grid_mmv[512] = GSQ_IQ3S_GRID_INIT;
 
-// 16 replicas (64 KB) keep the lookups free of bank conflicts; from 25 activation rows on the staged activations
-// need the room and 8 replicas (32 KB, two lanes per replica) are used
-__host__ __device__ constexpr int iq3_replica_shift(int ntl) { return ntl >= 4 ? 3 : 4; }
+// Up to 24 activation rows 16 replicas of (g, -g) (64 KB) keep the look-ups free of bank conflicts. From 25 rows on the
+// staged activations need the room: 32 KB, as 16 replicas of g alone. The bytes of g are odd, so -g is g ^ 0xFE: one more
+// logic instruction per look-up, but half the shared-memory wavefronts of 8 replicas of (g, -g), where two lanes
+// shared each replica. There shared memory is the busiest unit (76 % of its wavefronts at 32 rows; 17408 x 5120 35.0 ->
+// 32.8 us); below, the logic pipe is (at 8 rows the single form measured 20.3 against 19.1 us).
+__host__ __device__ constexpr bool iq3_single(int ntl) { return ntl >= 4; }
+constexpr int IQ3_REPLICAS = 16;
 
 struct RecIQ3S {
   uint32_t idx[9], sg[4];
@@ -616,17 +621,24 @@ struct RecIQ3S {
   }
 };
 
-// RS: log2 of the codebook replicas in shared memory (entry i of replica r at byte (8 << RS) i + 8 r)
-template <int F, int RS>
+// SINGLE: entries of 4 bytes (g) instead of 8 (g, -g)
+template <int F, bool SINGLE>
 __device__ __forceinline__ uint32_t iq3_field(const RecIQ3S& r, const char* gbase, uint32_t lane_off) {
-  constexpr int bit = 9 * F, word = bit >> 5, off = bit & 31, P = 3 + RS;  // the index goes to bits P .. P + 8
+  constexpr int bit = 9 * F, word = bit >> 5, off = bit & 31, P = SINGLE ? 6 : 7;  // the index goes to bits P .. P + 8
   uint32_t t;
   if (off + 9 <= 32) {
     t = off >= P ? r.idx[word] >> (off >= P ? off - P : 0) : r.idx[word] << (off < P ? P - off : 0);
   } else {
     t = __funnelshift_r(r.idx[word], r.idx[word + 1], off - P);
   }
-  const uint2 gp = *reinterpret_cast<const uint2*>(gbase + and_or(t, 0x1FFu << P, lane_off));
+  const char* entry = gbase + and_or(t, 0x1FFu << P, lane_off);
+  uint2 gp;
+  if constexpr (SINGLE) {
+    gp.x = *reinterpret_cast<const uint32_t*>(entry);
+    gp.y = gp.x ^ 0xFEFEFEFEu;
+  } else {
+    gp = *reinterpret_cast<const uint2*>(entry);
+  }
   constexpr int fl = F & 7, sh = 16 * (fl >> 2) + (fl & 3) - 2;
   const uint32_t sgs = sh >= 0 ? r.sg[F >> 3] >> (sh >= 0 ? sh : 0) : r.sg[F >> 3] << (sh < 0 ? -sh : 0);
   return mprmt(gp.x, gp.y, and_or(sgs, 0x4444u, 0x3210u));
@@ -639,11 +651,11 @@ __device__ __forceinline__ void iq3_slice(const RecIQ3S& r, const MmvArgs& ar, i
   constexpr int MC = 8 * NTL;
   constexpr bool DEFER = NTL <= 2;
   uint32_t a[4];
-  constexpr int RS = iq3_replica_shift(NTL);
-  a[0] = iq3_field<4 * S + 0, RS>(r, gbase, lane_off);   // (row g, group 2t)
-  a[1] = iq3_field<4 * S + 2, RS>(r, gbase, lane_off);   // (row g + 8, group 2t)
-  a[2] = iq3_field<4 * S + 1, RS>(r, gbase, lane_off);   // (row g, group 2t + 1)
-  a[3] = iq3_field<4 * S + 3, RS>(r, gbase, lane_off);   // (row g + 8, group 2t + 1)
+  constexpr bool SINGLE = iq3_single(NTL);
+  a[0] = iq3_field<4 * S + 0, SINGLE>(r, gbase, lane_off);   // (row g, group 2t)
+  a[1] = iq3_field<4 * S + 2, SINGLE>(r, gbase, lane_off);   // (row g + 8, group 2t)
+  a[2] = iq3_field<4 * S + 1, SINGLE>(r, gbase, lane_off);   // (row g, group 2t + 1)
+  a[3] = iq3_field<4 * S + 3, SINGLE>(r, gbase, lane_off);   // (row g + 8, group 2t + 1)
   // 2 * nibble + 1 of slice S: byte S / 2 of the even- or odd-slice word
   const uint64_t nm2 = pk2(-MAGIC_F, -MAGIC_F);
   if constexpr (mmv_float_scale(NTL)) {
@@ -687,7 +699,7 @@ __device__ __forceinline__ void process(const RecIQ3S& r, const MmvArgs& ar, int
                                         const uint8_t* grid, uint64_t (&acc)[NTL][2]) {
   constexpr bool DEFER = NTL <= 2;
   const char* gbase = reinterpret_cast<const char*>(grid);
-  const uint32_t lane_off = (uint32_t)(lane & ((1 << iq3_replica_shift(NTL)) - 1)) << 3;
+  const uint32_t lane_off = (uint32_t)(lane & (IQ3_REPLICAS - 1)) << (iq3_single(NTL) ? 2 : 3);
   uint32_t iscw[2][2];  // [row half][even / odd slices]: bytes 2 * nibble + 1
   uint64_t d2[2];
 #pragma unroll
@@ -952,7 +964,7 @@ template <>
 struct MmvKind<MK_IQ3S> {
   using Rec = RecIQ3S;
   static constexpr bool DS = false;
-  static constexpr int grid_bytes(int ntl) { return 512 * (8 << iq3_replica_shift(ntl)); }
+  static constexpr int grid_bytes(int ntl) { return 512 * IQ3_REPLICAS * (iq3_single(ntl) ? 4 : 8); }
   static constexpr bool PERM = false;
 };
 template <>
@@ -1049,12 +1061,13 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
     }
   }
   if (GRID) {
-    // one global load per thread (512 threads, 512 entries), then the replicas of its (g, -g) pair; no byte
-    // of the codebook is zero, so ~g + 1 per byte never carries
+    // one global load per thread (512 threads, 512 entries), then the replicas of its entry; the bytes of
+    // the codebook are odd, so the negative of each is its xor with 0xFE
     const uint32_t gv = g_iq3s_grid_mmv[tid & 511];
     uint4* dst = reinterpret_cast<uint4*>(smem + (tid & 511) * (GRID / 512));
 #pragma unroll
-    for (int r2 = 0; r2 < GRID / 512 / 16; ++r2) dst[r2] = make_uint4(gv, ~gv + 0x01010101u, gv, ~gv + 0x01010101u);
+    for (int r2 = 0; r2 < GRID / 512 / 16; ++r2)
+      dst[r2] = iq3_single(NTL) ? make_uint4(gv, gv, gv, gv) : make_uint4(gv, gv ^ 0xFEFEFEFEu, gv, gv ^ 0xFEFEFEFEu);
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // fused sum over GPUs: this call's number (the same in every CTA and on every rank) picks the slot pair. Read after
