@@ -1083,15 +1083,17 @@ extern "C" int gsq_debug_force_cluster_size(int cs) {
 
 namespace gsq {
 int gemm_error_flag(int* flag);  // gsq_gemm.cu
+int mmv_error_flags(int* peer, int* copy);  // gsq_mmv.cu
 }
 
 extern "C" int gsq_device_error_flag(int* flag) {
   if (!flag) return GSQ_ERR_UNSUPPORTED;
-  int a = 0, b = 0;
+  int a = 0, b = 0, c = 0, peer = 0;
   GSQ_CUDA_TRY(cudaMemcpyFromSymbol(&a, gsq::g_gemv_error, sizeof(int)));
-  const int rc = gsq::gemm_error_flag(&b);
+  int rc = gsq::gemm_error_flag(&b);
+  if (rc == GSQ_OK) rc = gsq::mmv_error_flags(&peer, &c);
   if (rc != GSQ_OK) return rc;
-  *flag = a | b;
+  *flag = a | b | c;
   return GSQ_OK;
 }
 

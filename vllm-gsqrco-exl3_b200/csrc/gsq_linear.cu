@@ -9,6 +9,10 @@ namespace gsq {
 
 // gsq_mmv.cu
 bool mmv_applies(int ggml_type, int packed, int64_t rows, int64_t m);
+int mmv_rows_columns(int64_t m);
+size_t mmv_rows_bytes(int ggml_type, int64_t m, int64_t k);
+bool mmv_rows_wins(int ggml_type, int64_t rows, int64_t m, int64_t k);
+int quantize_rows_host(const void* x, int x_dtype, int64_t m, int mc, int64_t k, int64_t stride, int ggml_type, void* out, void* stream);
 bool mmv_raw_applies(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int vec);
 int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* xq, int x_layout,
              int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
@@ -125,7 +129,8 @@ static size_t linear_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, in
     b = b > plane ? b : plane;
   }
   // (the small-batch kernel takes 128-value blocks, and may decline the shape)
-  const size_t mmq = small_batch(ggml_type, packed, rows, m) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
+  size_t mmq = small_batch(ggml_type, packed, rows, m) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
+  if (mmq && !small && mmv_rows_wins(ggml_type, rows, m, k) && mmv_rows_bytes(ggml_type, m, k) > mmq) mmq = mmv_rows_bytes(ggml_type, m, k);
   b = b > mmq ? b : mmq;
   return align256(b > 0 ? b : 1);
 }
@@ -155,9 +160,13 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
       rc = mmv_host(w, row_bytes, rows, ggml_type, packed, x, 3, m, k, y, y_dtype, y_row_stride, stream, nullptr, nullptr, x_dtype, x_row_stride);
       if (rc != 1000) return rc;
     }
-    rc = gsq_quantize_q8_1_mmq(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
+    const int mc = mmv_rows_columns(m);
+    const bool in_rows = mmv_rows_wins(ggml_type, rows, m, k) && !gemm_dump_pointer() && scratch_bytes >= mmv_rows_bytes(ggml_type, m, k) &&
+                         (uintptr_t)scratch % 16 == 0;
+    rc = in_rows ? quantize_rows_host(x, x_dtype, m, mc, k, x_row_stride, ggml_type, scratch, stream)
+                 : gsq_quantize_q8_1_mmq(x, x_dtype, m, k, x_row_stride, layout, scratch, stream);
     if (rc != GSQ_OK) return rc;
-    rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, 1, m, k, y, y_dtype, y_row_stride, stream, gemm_dump_pointer());
+    rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, in_rows ? 4 : 1, m, k, y, y_dtype, y_row_stride, stream, gemm_dump_pointer());
     if (rc != 1000) return rc;  // 1000: declined, the activations of this shape do not fit its staging area
   }
   const Way way = choose_way(ggml_type, packed, rows, m, scratch_bytes < gsq_linear_workspace_bytes(rows, m, k, ggml_type, packed));

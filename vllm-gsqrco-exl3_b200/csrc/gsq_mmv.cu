@@ -18,13 +18,13 @@ int g_mmv_trace = 0;     // one line per launch plan on stderr
 bool mmv_early_trigger() { return g_mmv_pdl >= 2; }
 
 int mmv_launch_q4k(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st);   // gsq_mmv_q4k.cu
-int mmv_peer_error_q4k(int* flag);
+int mmv_errors_q4k(int* peer, int* copy);
 int mmv_launch_iq4xs(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st);   // gsq_mmv_iq4xs.cu
-int mmv_peer_error_iq4xs(int* flag);
+int mmv_errors_iq4xs(int* peer, int* copy);
 int mmv_launch_iq3s(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st);   // gsq_mmv_iq3s.cu
-int mmv_peer_error_iq3s(int* flag);
+int mmv_errors_iq3s(int* peer, int* copy);
 int mmv_launch_q6k(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st);   // gsq_mmv_q6k.cu
-int mmv_peer_error_q6k(int* flag);
+int mmv_errors_q6k(int* peer, int* copy);
 
 // Whether (type, packed, m) may be served here (mmv_host can still decline a shape: MMV_DECLINED).
 bool mmv_applies(int ggml_type, int packed, int64_t rows, int64_t m) {
@@ -71,7 +71,7 @@ bool mmv_raw_applies(int ggml_type, int packed, int64_t rows, int64_t m, int64_t
 }
 
 // x_layout: 0 = block_q8_1, 1 = block_q8_1_mmq. Returns MMV_DECLINED when the shape does not fit.
-// x_layout 2 / 3: xq is X itself (x_dtype, rows x_row_stride elements apart), up to 8 / 16 rows.
+// x_layout 4: quantize_rows_host's. x_layout 2 / 3: xq is X itself (x_dtype, rows x_row_stride elements apart), up to 8 / 16 rows.
 int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* xq, int x_layout,
              int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
              const gsq_peer_reduce* pr, int x_dtype, int64_t x_row_stride) {
@@ -110,7 +110,8 @@ int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int 
   a.x_dtype = x_dtype;
   a.x_stride = x_row_stride;
   a.x_vec = (uintptr_t)xq % 16 == 0 && (x_row_stride * (x_dtype == GSQ_F32 ? 4 : 2)) % 16 == 0;
-  if (x_layout >= XL_XQ81 && ((x_dtype != GSQ_F32 && x_dtype != GSQ_F16 && x_dtype != GSQ_BF16) || dump || pr)) return GSQ_ERR_UNSUPPORTED;
+  if (x_layout == XL_ROWS && (dump || pr || (uintptr_t)xq % 16 != 0)) return GSQ_ERR_UNSUPPORTED;
+  if ((x_layout == XL_XQ81 || x_layout == XL_XMMQ) && ((x_dtype != GSQ_F32 && x_dtype != GSQ_F16 && x_dtype != GSQ_BF16) || dump || pr)) return GSQ_ERR_UNSUPPORTED;
   if (pr) {
     const int64_t esz = y_dtype == GSQ_F32 ? 4 : 2;
     if (!pr->slots || !pr->flags || !pr->state || pr->world < 2 || pr->world > 8 || pr->rank < 0 || pr->rank >= pr->world ||
@@ -134,17 +135,39 @@ int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int 
   }
 }
 
+// Sticky flags of bounded waits that gave up: on a peer GPU, on a bulk copy.
+int mmv_error_flags(int* peer, int* copy) {
+  int p[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
+  int rc = mmv_errors_q4k(&p[0], &c[0]);
+  if (rc == GSQ_OK) rc = mmv_errors_iq4xs(&p[1], &c[1]);
+  if (rc == GSQ_OK) rc = mmv_errors_iq3s(&p[2], &c[2]);
+  if (rc == GSQ_OK) rc = mmv_errors_q6k(&p[3], &c[3]);
+  *peer = p[0] | p[1] | p[2] | p[3];
+  *copy = c[0] | c[1] | c[2] | c[3];
+  return rc;
+}
+
+// The activations in the order of the staging area (quantize_rows_host): padded columns, bytes.
+int mmv_rows_columns(int64_t m) {
+  const int64_t ntl = (m + 7) / 8;
+  return (int)(8 * (ntl == 5 ? 6 : ntl));
+}
+// Whether that order is the faster one: it is once a CTA's share of a column is some hundred bytes. Small weights are split
+// over clusters of 8 and each copy is short (1024 x 2048 IQ3_S at 40 rows 11.1 us from blocks, 11.9 from rows); above 32 rows
+// the scales of 48 columns and the more copies leave a gain only for the large products of Q6_K (17408 x 5120 at 48
+// rows 60.3 -> 56.1; IQ3_S 47.0 -> 47.5).
+bool mmv_rows_wins(int ggml_type, int64_t rows, int64_t m, int64_t k) {
+  return rows * k > (4 << 20) && k <= (1 << 24) && (m <= 32 || (ggml_type == GSQ_TYPE_Q6_K && rows * k > (16 << 20)));
+}
+size_t mmv_rows_bytes(int ggml_type, int64_t m, int64_t k) {
+  return (size_t)(m * k) + (size_t)(k / 32) * mmv_rows_columns(m) * (ggml_type == GSQ_TYPE_Q4_K ? 8 : 4);
+}
+
 }  // namespace gsq
 
 extern "C" int gsq_peer_reduce_error_flag(int* flag) {
-  if (!flag) return GSQ_ERR_UNSUPPORTED;
-  int f[4] = {0, 0, 0, 0};
-  int rc = gsq::mmv_peer_error_q4k(&f[0]);
-  if (rc == GSQ_OK) rc = gsq::mmv_peer_error_iq4xs(&f[1]);
-  if (rc == GSQ_OK) rc = gsq::mmv_peer_error_iq3s(&f[2]);
-  if (rc == GSQ_OK) rc = gsq::mmv_peer_error_q6k(&f[3]);
-  *flag = f[0] | f[1] | f[2] | f[3];
-  return rc;
+  int copy;
+  return flag ? gsq::mmv_error_flags(flag, &copy) : GSQ_ERR_UNSUPPORTED;
 }
 
 extern "C" int gsq_debug_mmv_mode(int mode) {

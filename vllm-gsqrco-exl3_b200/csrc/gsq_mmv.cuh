@@ -43,8 +43,9 @@ namespace gsq {
 
 enum { MK_Q4K = 0, MK_IQ3S = 1, MK_IQ4XS = 2, MK_Q6K = 3 };
 // what the activations come as: block_q8_1, block_q8_1_mmq, or X itself, quantised while it is staged with the arithmetic
-// of the one (XL_XQ81) or the other (XL_XMMQ)
-enum { XL_Q81 = 0, XL_MMQ = 1, XL_XQ81 = 2, XL_XMMQ = 3 };
+// of the one (XL_XQ81) or the other (XL_XMMQ), or the values of block_q8_1_mmq in the staging area's own order (XL_ROWS:
+// quantize_q8_1_rows_kernel)
+enum { XL_Q81 = 0, XL_MMQ = 1, XL_XQ81 = 2, XL_XMMQ = 3, XL_ROWS = 4 };
 
 constexpr int MMV_WARPS = 16;
 constexpr int MMV_THREADS = MMV_WARPS * 32;
@@ -91,6 +92,8 @@ struct MmvArgs {
   int64_t pr_slot_bytes;
 };
 
+// set (sticky) when a bounded wait on a bulk copy gave up
+static __device__ int g_mmv_copy_error = 0;
 static __device__ int g_mmv_peer_error = 0;   // (one per translation unit: one per weight type)
 
 __device__ __forceinline__ void mmv_st_release_sys(uint32_t* p, uint32_t v) {
@@ -353,6 +356,63 @@ __device__ __forceinline__ void stage_x_mmq(const MmvArgs& a, int kb0, int nkb, 
     }
   }
   stage_x_pad<MC, DS>(a.m, nkb, colb, xq, xd, xs, tid);
+}
+
+// XL_ROWS: the quants are [column][K] bytes, the scales (and sums) [K/32][MC] floats with zeros past column m, so the CTA's
+// share is one bulk copy per column and one or two for the scales, with nothing left to do per value, and the warp's first
+// record is loaded meanwhile. Unpacking block_q8_1_mmq (above) takes about 2 us per 1000 32-value blocks of a CTA's share,
+// this 1 to 1.5 (us, blocks -> rows: 17408 x 5120 at 16 rows Q4_K 27.9 -> 26.7, at 32 rows Q4_K 37.8 -> 34.8 and IQ4_XS
+// 39.3 -> 36.8; 5120 x 17408 at 32 rows Q6_K 54.6 -> 50.1, IQ3_S 42.8 -> 40.5).
+__device__ __forceinline__ uint32_t mmv_saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <int MC, bool DS>
+__device__ __forceinline__ void stage_rows_init(const MmvArgs& a, int nkb, uint32_t bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nkb * (32 * a.m + MC * (DS ? 8 : 4))) : "memory");
+}
+__device__ __forceinline__ void mmv_bulk(const void* dst, const void* src, int bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(mmv_saddr(dst)), "l"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
+}
+// one warp, after the thread that initialised the barrier
+template <int MC, bool DS>
+__device__ __forceinline__ void stage_rows_issue(const MmvArgs& a, int kb0, int nkb, int colb, uint8_t* xq, float* xd, float* xs,
+                                                 uint32_t bar, int lane) {
+  const int64_t qbytes = (int64_t)a.m * a.k, dbytes = (int64_t)(a.k >> 5) * MC * 4;
+  if (lane == 31) mmv_bulk(xd, a.xq + qbytes + (int64_t)kb0 * MC * 4, nkb * MC * 4, bar);
+  if (DS && lane == 30) mmv_bulk(xs, a.xq + qbytes + dbytes + (int64_t)kb0 * MC * 4, nkb * MC * 4, bar);
+  for (int c = lane; c < a.m; c += 32) mmv_bulk(xq + c * colb, a.xq + (int64_t)c * a.k + kb0 * 32, nkb * 32, bar);
+}
+// zeros in the quants of columns m .. MC - 1
+template <int MC>
+__device__ __forceinline__ void stage_rows_pad(int m, int nkb, int colb, uint8_t* xq, int tid) {
+  const int n = nkb * 2;
+  for (int c = m; c < MC; ++c) {
+    for (int i = tid; i < n; i += MMV_THREADS) *reinterpret_cast<uint4*>(xq + c * colb + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+// Bounded: after 2^20 tries (each may be suspended by the hardware for a while) it raises the flag, gives the copies in
+// flight as many tries again, and goes on.
+__device__ __forceinline__ void stage_rows_wait(uint32_t bar) {
+#pragma unroll 1
+  for (int round = 0; round < 2; ++round) {
+#pragma unroll 1
+    for (int spin = 0; spin < (1 << 20); ++spin) {
+      uint32_t done;
+      asm volatile(
+          "{\n"
+          ".reg .pred p;\n"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n"
+          "selp.u32 %0, 1, 0, p;\n"
+          "}\n"
+          : "=r"(done)
+          : "r"(bar)
+          : "memory");
+      if (done) return;
+    }
+    atomicExch(&g_mmv_copy_error, 1);
+  }
 }
 
 // X itself (fp32 / fp16 / bf16): every CTA quantises its share of K for itself, to the quantisers' values
@@ -1069,6 +1129,9 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
     for (int r2 = 0; r2 < GRID / 512 / 16; ++r2)
       dst[r2] = iq3_single(NTL) ? make_uint4(gv, gv, gv, gv) : make_uint4(gv, gv ^ 0xFEFEFEFEu, gv, gv ^ 0xFEFEFEFEu);
   }
+  // (the barrier of the bulk copies: in the padding behind the last quant column, which nothing else touches)
+  const uint32_t xbar = mmv_saddr(xq + (size_t)colb * MC - 16);
+  if (XL == XL_ROWS && tid == 0) stage_rows_init<MC, DS>(a, nkb, xbar);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // fused sum over GPUs: this call's number (the same in every CTA and on every rank) picks the slot pair. Read after
   // the wait: the kernel before this one in a programmatic-launch chain may be the call that publishes it.
@@ -1076,7 +1139,15 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
   const uint32_t epoch = fused ? *reinterpret_cast<volatile uint32_t*>(a.pr_state) + 1u : 0u;
   const int64_t push_off = fused ? (int64_t)((epoch & 1u) * a.pr_world + a.pr_rank) * a.pr_slot_bytes : 0;
   auto nothing = []() {};
-  if (XL == XL_XQ81 || XL == XL_XMMQ) {
+  Rec cur;
+  if (XL == XL_ROWS) {
+    if (warp == 0) {
+      __syncwarp();
+      stage_rows_issue<MC, DS>(a, sb0 * 8, nkb, colb, xq, xd, xs, xbar, lane);
+    }
+    if (have_first) cur.load(a, (tile_begin + first_tl) * MMV_TR, sb0 + first_rec, lane);
+    stage_rows_pad<MC>(a.m, nkb, colb, xq, tid);
+  } else if (XL == XL_XQ81 || XL == XL_XMMQ) {
     stage_x_raw<MC, DS, MmvKind<KIND>::PERM, XL == XL_XMMQ>(a, sb0 * 8, nkb, colb, xq, xd, xs, tid);
   } else if (XL == XL_Q81) {
     stage_x_q81<MC, DS, MmvKind<KIND>::PERM>(a, sb0 * 8, nkb, colb, xq, xd, xs, tid, nothing);
@@ -1084,9 +1155,9 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
     stage_x_mmq<MC, DS, MmvKind<KIND>::PERM>(a, sb0 * 8, nkb, colb, xq, xd, xs, tid, nothing);
   }
   __syncthreads();
+  if (XL == XL_ROWS) stage_rows_wait(xbar);
   mmv_stamp(a, 1);
-  Rec cur;
-  if (have_first) cur.load(a, (tile_begin + first_tl) * MMV_TR, sb0 + first_rec, lane);
+  if (XL != XL_ROWS && have_first) cur.load(a, (tile_begin + first_tl) * MMV_TR, sb0 + first_rec, lane);
   XSmem xlane;
   xlane.q = xq + g * colb + 8 * t;
   xlane.q8 = 8 * colb;
@@ -1515,7 +1586,7 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
   cfg.attrs = attr;
   cfg.numAttrs = g_mmv_pdl ? 2 : 1;
   if (a.pr_world > 1) {
-    if constexpr (DUMP || XL == XL_XQ81 || XL == XL_XMMQ) {
+    if constexpr (DUMP || XL >= XL_XQ81) {
       return GSQ_ERR_UNSUPPORTED;
     } else {
       static bool configured[32];
@@ -1545,15 +1616,17 @@ static int mmv_launch_n(const MmvArgs& a, int sm_count, int max_smem, cudaStream
            : ntl == 2 ? mmv_launch_t<KIND, 2, XL, false>(a, sm_count, max_smem, st)
                       : MMV_DECLINED;
   } else {
-    if (a.dump) {
-      switch (ntl) {
-        case 1: return mmv_launch_t<KIND, 1, XL, true>(a, sm_count, max_smem, st);
-        case 2: return mmv_launch_t<KIND, 2, XL, true>(a, sm_count, max_smem, st);
-        case 3: return mmv_launch_t<KIND, 3, XL, true>(a, sm_count, max_smem, st);
-        case 4: return mmv_launch_t<KIND, 4, XL, true>(a, sm_count, max_smem, st);
-        case 5:
-        case 6: return mmv_launch_t<KIND, 6, XL, true>(a, sm_count, max_smem, st);
-        default: return MMV_DECLINED;
+    if constexpr (XL != XL_ROWS) {
+      if (a.dump) {
+        switch (ntl) {
+          case 1: return mmv_launch_t<KIND, 1, XL, true>(a, sm_count, max_smem, st);
+          case 2: return mmv_launch_t<KIND, 2, XL, true>(a, sm_count, max_smem, st);
+          case 3: return mmv_launch_t<KIND, 3, XL, true>(a, sm_count, max_smem, st);
+          case 4: return mmv_launch_t<KIND, 4, XL, true>(a, sm_count, max_smem, st);
+          case 5:
+          case 6: return mmv_launch_t<KIND, 6, XL, true>(a, sm_count, max_smem, st);
+          default: return MMV_DECLINED;
+        }
       }
     }
     switch (ntl) {
@@ -1572,11 +1645,13 @@ template <int KIND>
 static int mmv_launch_kind(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st) {
   return x_layout == XL_Q81    ? mmv_launch_n<KIND, XL_Q81>(a, sm_count, max_smem, st)
          : x_layout == XL_MMQ  ? mmv_launch_n<KIND, XL_MMQ>(a, sm_count, max_smem, st)
+         : x_layout == XL_ROWS ? mmv_launch_n<KIND, XL_ROWS>(a, sm_count, max_smem, st)
          : x_layout == XL_XQ81 ? mmv_launch_n<KIND, XL_XQ81>(a, sm_count, max_smem, st)
                                : mmv_launch_n<KIND, XL_XMMQ>(a, sm_count, max_smem, st);
 }
-static int mmv_peer_error(int* flag) {
-  GSQ_CUDA_TRY(cudaMemcpyFromSymbol(flag, g_mmv_peer_error, sizeof(int)));
+static int mmv_errors(int* peer, int* copy) {
+  GSQ_CUDA_TRY(cudaMemcpyFromSymbol(peer, g_mmv_peer_error, sizeof(int)));
+  GSQ_CUDA_TRY(cudaMemcpyFromSymbol(copy, g_mmv_copy_error, sizeof(int)));
   return GSQ_OK;
 }
 

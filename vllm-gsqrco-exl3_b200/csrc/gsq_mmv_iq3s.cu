@@ -5,5 +5,5 @@ namespace gsq {
 int mmv_launch_iq3s(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st) {
   return mmv_launch_kind<MK_IQ3S>(a, x_layout, sm_count, max_smem, st);
 }
-int mmv_peer_error_iq3s(int* flag) { return mmv_peer_error(flag); }
+int mmv_errors_iq3s(int* peer, int* copy) { return mmv_errors(peer, copy); }
 }  // namespace gsq

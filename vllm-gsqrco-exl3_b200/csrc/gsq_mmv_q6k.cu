@@ -5,5 +5,5 @@ namespace gsq {
 int mmv_launch_q6k(const MmvArgs& a, int x_layout, int sm_count, int max_smem, cudaStream_t st) {
   return mmv_launch_kind<MK_Q6K>(a, x_layout, sm_count, max_smem, st);
 }
-int mmv_peer_error_q6k(int* flag) { return mmv_peer_error(flag); }
+int mmv_errors_q6k(int* peer, int* copy) { return mmv_errors(peer, copy); }
 }  // namespace gsq

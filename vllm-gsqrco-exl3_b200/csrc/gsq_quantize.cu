@@ -73,6 +73,32 @@ __global__ void __launch_bounds__(256) quantize_q8_1_kernel(const T* __restrict_
   q8_1_store8(v, live, out + (row * (k >> 5) + (c8 >> 2)) * 36, (int)(c8 & 3));
 }
 
+// 8 consecutive values (a quarter of a 32-value block, 4 adjacent lanes) -> quants, the block's d and (DS) sum. All 32
+// lanes of the warp must call it.
+template <bool DS>
+__device__ __forceinline__ void mmq_quant8(const float (&v)[8], float (&q)[8], float& d, float& sum) {
+  float amax = 0.0f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
+  amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+  amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+  sum = 0.0f;
+  if constexpr (DS) {
+    // the reference sums 4 values per thread, then lane offsets 4, 2, 1 over 8 threads
+    float pa = ((v[0] + v[1]) + v[2]) + v[3];
+    float pb = ((v[4] + v[5]) + v[6]) + v[7];
+    pa += __shfl_xor_sync(0xFFFFFFFFu, pa, 2);
+    pb += __shfl_xor_sync(0xFFFFFFFFu, pb, 2);
+    pa += __shfl_xor_sync(0xFFFFFFFFu, pa, 1);
+    pb += __shfl_xor_sync(0xFFFFFFFFu, pb, 1);
+    sum = pa + pb;
+  }
+  const float d_inv = div_approx(127.0f, amax);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) q[e] = roundf(v[e] * d_inv);
+  d = rcp_approx(d_inv);
+}
+
 // 128-value blocks: 16 scale bytes + 128 x int8, block (kb, row) at (kb * m + row) * 144.
 template <typename T, bool VEC, int LAYOUT>
 __global__ void __launch_bounds__(256) quantize_q8_1_mmq_kernel(const T* __restrict__ x, uint8_t* __restrict__ out,
@@ -93,28 +119,9 @@ __global__ void __launch_bounds__(256) quantize_q8_1_mmq_kernel(const T* __restr
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = 0.0f;
   }
-  float amax = 0.0f;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
-  amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
-  amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-  float sum = 0.0f;
-  if constexpr (LAYOUT == GSQ_Q8_LAYOUT_DS4) {
-    // the reference sums 4 values per thread, then lane offsets 4, 2, 1 over 8 threads
-    float pa = ((v[0] + v[1]) + v[2]) + v[3];
-    float pb = ((v[4] + v[5]) + v[6]) + v[7];
-    pa += __shfl_xor_sync(0xFFFFFFFFu, pa, 2);
-    pb += __shfl_xor_sync(0xFFFFFFFFu, pb, 2);
-    pa += __shfl_xor_sync(0xFFFFFFFFu, pa, 1);
-    pb += __shfl_xor_sync(0xFFFFFFFFu, pb, 1);
-    sum = pa + pb;
-  }
+  float q[8], d, sum;
+  mmq_quant8<LAYOUT == GSQ_Q8_LAYOUT_DS4>(v, q, d, sum);
   if (!live) return;
-  const float d_inv = div_approx(127.0f, amax);
-  float q[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) q[e] = roundf(v[e] * d_inv);
-  const float d = rcp_approx(d_inv);
   const int64_t kb = c8 >> 4;             // 128-value block along k
   const int iqs = (int)(c8 & 15) * 8;     // value offset inside the block
   uint8_t* b = out + (kb * m + row) * 144;
@@ -124,6 +131,53 @@ __global__ void __launch_bounds__(256) quantize_q8_1_mmq_kernel(const T* __restr
       reinterpret_cast<__half2*>(b)[iqs >> 5] = __floats2half2_rn(d, sum);
     } else {
       reinterpret_cast<float*>(b)[iqs >> 5] = d;
+    }
+  }
+}
+
+// The same values in the order of the small-batch product's staging area (gsq_mmv.cuh, XL_ROWS), which then takes them in
+// with bulk copies: quants [row][k] (PERM: the words of a 32-value block in the order 0 4 1 5 2 6 3 7), then d
+// [k/32][mc] as floats, then (DS) the sums likewise, d and sum rounded to half as in the blocks. Columns m .. mc - 1 of
+// d and sum are zeros.
+template <typename T, bool VEC, bool DS, bool PERM>
+__global__ void __launch_bounds__(256) quantize_q8_1_rows_kernel(const T* __restrict__ x, uint8_t* __restrict__ out,
+                                                                int m, int mc, int k, int64_t stride) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, per_row = k >> 3;
+  const int row = t / per_row, c8 = t - row * per_row;
+  float v[8];
+  if (row < m) {
+    load8<T, VEC>(x, row * stride + (int64_t)c8 * 8, v);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+  }
+  float q[8], d, sum;
+  mmq_quant8<DS>(v, q, d, sum);
+  if (row >= mc) return;
+  const int kb = c8 >> 2, piece = c8 & 3;
+  if (row < m) {
+    uint8_t* dst = out + (int64_t)row * k + kb * 32;
+    const uint32_t lo = pack4(q[0], q[1], q[2], q[3]), hi = pack4(q[4], q[5], q[6], q[7]);
+    if constexpr (PERM) {
+      const int w = 2 * piece, s = ((w & 3) << 1) | (w >> 2);   // word w goes to slot s, word w + 1 two further
+      reinterpret_cast<uint32_t*>(dst)[s] = lo;
+      reinterpret_cast<uint32_t*>(dst)[s + 2] = hi;
+    } else {
+      *reinterpret_cast<uint2*>(dst + 8 * piece) = make_uint2(lo, hi);
+    }
+  } else {
+    d = 0.0f;
+  }
+  if (piece == 0) {
+    float* dd = reinterpret_cast<float*>(out + (int64_t)m * k) + (int64_t)kb * mc + row;
+    if constexpr (DS) {
+      const float2 h = __half22float2(__floats2half2_rn(d, sum));
+      dd[0] = h.x;
+      dd[(int64_t)(k >> 5) * mc] = h.y;
+    } else {
+      dd[0] = d;
     }
   }
 }
@@ -373,6 +427,30 @@ static int launch_q8_1_tiles(const void* x, int64_t m, int64_t k, int64_t stride
     GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, quantize_q8_1_tiles_kernel<T, false, LAYOUT>, (const T*)x, (uint8_t*)out, m, k, stride));
   }
   return GSQ_OK;
+}
+
+template <typename T, bool DS, bool PERM>
+static int launch_q8_1_rows(const void* x, int64_t m, int mc, int64_t k, int64_t stride, void* out, cudaStream_t st) {
+  const unsigned grid = (unsigned)((mc * (k >> 3) + 255) / 256);
+  const bool vec = ((uintptr_t)x % 16 == 0) && ((stride * (int64_t)sizeof(T)) % 16 == 0);
+  return vec ? launch_pdl(quantize_q8_1_rows_kernel<T, true, DS, PERM>, grid, st, (const T*)x, (uint8_t*)out, (int)m, mc, (int)k, stride)
+             : launch_pdl(quantize_q8_1_rows_kernel<T, false, DS, PERM>, grid, st, (const T*)x, (uint8_t*)out, (int)m, mc, (int)k, stride);
+}
+// x [m, k] -> the small-batch product's staging order (see quantize_q8_1_rows_kernel); m <= mc <= 48, k % 256 == 0.
+int quantize_rows_host(const void* x, int x_dtype, int64_t m, int mc, int64_t k, int64_t stride, int ggml_type, void* out, void* stream) {
+  if (m <= 0 || m > mc || mc > 48 || k <= 0 || k % 256 != 0 || k > (1 << 24) || !x || !out) return GSQ_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)stream;
+#define GSQ_ROWS_CASE(T)                                                                               \
+  return ggml_type == GSQ_TYPE_Q4_K     ? launch_q8_1_rows<T, true, false>(x, m, mc, k, stride, out, st) \
+         : ggml_type == GSQ_TYPE_IQ4_XS ? launch_q8_1_rows<T, false, true>(x, m, mc, k, stride, out, st) \
+                                        : launch_q8_1_rows<T, false, false>(x, m, mc, k, stride, out, st)
+  switch (x_dtype) {
+    case GSQ_F32: GSQ_ROWS_CASE(float);
+    case GSQ_F16: GSQ_ROWS_CASE(__half);
+    case GSQ_BF16: GSQ_ROWS_CASE(__nv_bfloat16);
+    default: return GSQ_ERR_UNSUPPORTED;
+  }
+#undef GSQ_ROWS_CASE
 }
 
 // x [m, k] -> activation tiles for the prefill GEMM (see quantize_q8_1_tiles_kernel); k % 256 == 0.
