@@ -298,8 +298,9 @@ struct WRegs<GK_IQ4XS, P> {
   static __device__ __forceinline__ void lookup(uint32_t v, uint32_t& lo, uint32_t& hi) {
     const uint32_t t0 = c_iq4nl_words_gemm[0], t1 = c_iq4nl_words_gemm[1], t2 = c_iq4nl_words_gemm[2],
                    t3 = c_iq4nl_words_gemm[3];
-    const uint32_t s01 = v & 0x7777u, s23 = (v >> 16) & 0x7777u;
-    const uint32_t pick01 = 0x3210u | ((v & 0x8888u) >> 1), pick23 = 0x3210u | (((v >> 16) & 0x8888u) >> 1);
+    // (a byte permute reads the low 16 bits of its selector, so the upper four nibbles' selectors are one shift away)
+    const uint32_t s01 = v & 0x77777777u, s23 = s01 >> 16;
+    const uint32_t pick01 = ((v >> 1) & 0x44444444u) | 0x32103210u, pick23 = pick01 >> 16;
     const uint32_t r01 = gprmt(gprmt(t0, t1, s01), gprmt(t2, t3, s01), pick01);
     const uint32_t r23 = gprmt(gprmt(t0, t1, s23), gprmt(t2, t3, s23), pick23);
     lo = gprmt(r01, r23, 0x6420u);

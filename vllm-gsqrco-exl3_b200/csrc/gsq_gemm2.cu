@@ -214,8 +214,9 @@ __device__ __forceinline__ void decode_q4k(const uint8_t* raw, uint8_t* a, float
 // IQ4_XS: item (row r, slice p): 16 bytes of 4-bit indices into the 16-entry table; low nibbles are values 0..15 of
 // the slice, high nibbles 16..31.
 __device__ __forceinline__ void iq4_lookup(uint32_t v, const uint32_t (&tb)[4], uint32_t& lo, uint32_t& hi) {
-  const uint32_t s01 = v & 0x7777u, s23 = (v >> 16) & 0x7777u;
-  const uint32_t pick01 = 0x3210u | ((v & 0x8888u) >> 1), pick23 = 0x3210u | (((v >> 16) & 0x8888u) >> 1);
+  // (a byte permute reads the low 16 bits of its selector, so the upper four nibbles' selectors are one shift away)
+  const uint32_t s01 = v & 0x77777777u, s23 = s01 >> 16;
+  const uint32_t pick01 = ((v >> 1) & 0x44444444u) | 0x32103210u, pick23 = pick01 >> 16;
   const uint32_t r01 = prmt(prmt(tb[0], tb[1], s01), prmt(tb[2], tb[3], s01), pick01);
   const uint32_t r23 = prmt(prmt(tb[0], tb[1], s23), prmt(tb[2], tb[3], s23), pick23);
   lo = prmt(r01, r23, 0x6420u);

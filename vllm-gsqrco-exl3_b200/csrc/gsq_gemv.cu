@@ -368,8 +368,9 @@ __device__ __forceinline__ void accumulate(const Rec<KIND_IQ3S_RAW>& r, int row0
 // 8 four-bit indices of v -> the table bytes: lo = entries of the 4 low nibbles, hi = of the 4 high nibbles.
 __device__ __forceinline__ void iq4_lookup(uint32_t v, uint32_t& lo, uint32_t& hi) {
   const uint32_t t0 = c_iq4nl_words[0], t1 = c_iq4nl_words[1], t2 = c_iq4nl_words[2], t3 = c_iq4nl_words[3];
-  const uint32_t s01 = v & 0x7777u, s23 = (v >> 16) & 0x7777u;
-  const uint32_t pick01 = 0x3210u | ((v & 0x8888u) >> 1), pick23 = 0x3210u | (((v >> 16) & 0x8888u) >> 1);
+  // (a byte permute reads the low 16 bits of its selector, so the upper four nibbles' selectors are one shift away)
+  const uint32_t s01 = v & 0x77777777u, s23 = s01 >> 16;
+  const uint32_t pick01 = ((v >> 1) & 0x44444444u) | 0x32103210u, pick23 = pick01 >> 16;
   const uint32_t r01 = prmt(prmt(t0, t1, s01), prmt(t2, t3, s01), pick01);  // nibbles 0..3 of v
   const uint32_t r23 = prmt(prmt(t0, t1, s23), prmt(t2, t3, s23), pick23);  // nibbles 4..7 of v
   lo = prmt(r01, r23, 0x6420u);
