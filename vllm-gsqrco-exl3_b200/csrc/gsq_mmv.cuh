@@ -512,7 +512,31 @@ __device__ __forceinline__ void stage_x_raw(const MmvArgs& a, int kb0, int nkb, 
 // ---------------------------------------------------------------------------------------------
 // Q4_K
 
+// Whether a record's registers are refilled part by part with the next record's while it is multiplied: the loads of a
+// whole next record cost its registers twice (up to 16 columns: nothing left to keep the tensor cores' results in flight)
+// or, where there is no room for that, the latency of L2 after every record. Measured at 17408 x 5120 (us, without ->
+// with): 16 rows Q4_K 26.5 -> 23.0, Q6_K 31.5 -> 27.0; 24 rows IQ4_XS 31.8 -> 30.5, Q6_K 35.4 -> 33.9; 48 rows Q6_K
+// 56.1 -> 53.2, IQ3_S 47.0 -> 45.5; 5120 x 17408, 16 rows Q4_K 34.8 -> 26.4, Q6_K 40.9 -> 31.5. Not where it gains nothing: one column
+// group (the registers suffice; IQ4_XS up to two, IQ3_S with its small records up to three), Q4_K from 25 columns on (0.99
+// to 1.07 of the time without).
+__host__ __device__ constexpr bool mmv_roll(int kind, int ntl) {
+  return kind == MK_Q4K ? ntl == 2 || ntl == 3 : kind == MK_Q6K ? ntl >= 2 : kind == MK_IQ4XS ? ntl >= 3 : ntl >= 4;
+}
+
 struct RecQ4K {
+  struct Src { const uint8_t* b[2]; };
+  static __device__ __forceinline__ Src src(const MmvArgs& a, int row0, int sb, int lane) {
+    Src n;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      n.b[h] = a.w + (int64_t)min(row0 + (lane >> 2) + 8 * h, a.nrows - 1) * a.row_bytes + (int64_t)sb * 144;
+    return n;
+  }
+  __device__ __forceinline__ void refill_header(const Src& n) { hdr[0] = ldg_stream_v4(n.b[0]); hdr[1] = ldg_stream_v4(n.b[1]); }
+  __device__ __forceinline__ void refill(const Src& n, int p, int lane) {
+    q[0][p] = ldg_stream_v2(n.b[0] + 16 + 32 * p + 8 * (lane & 3));
+    q[1][p] = ldg_stream_v2(n.b[1] + 16 + 32 * p + 8 * (lane & 3));
+  }
   uint4 hdr[2];     // rows g, g + 8: d, dmin, 12 scale bytes
   uint2 q[2][4];    // [row][64-value group p]: qs words 2t, 2t + 1 of the group's 32 bytes
   __device__ __forceinline__ void load(const MmvArgs& a, int row0, int sb, int lane) {
@@ -543,7 +567,7 @@ __device__ __forceinline__ float byte_float(uint32_t word, int byte) {
 // xl: this lane's view of the staged activations of the record's superblock: quants at xl.q + j * xl.q8 + 32 s,
 // scales of its two accumulator columns at xl.d + s * MC + 8 j.
 template <int NTL, bool DUMP>
-__device__ __forceinline__ void process(const RecQ4K& r, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
+__device__ __forceinline__ void process(RecQ4K& r, const RecQ4K::Src& nx, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
                                         const uint8_t*, uint64_t (&acc)[NTL][2]) {
   constexpr int MC = 8 * NTL;
   constexpr bool DEFER = NTL <= 2;  // keep the record's sums unscaled by d / dmin until its end (more registers)
@@ -562,6 +586,7 @@ __device__ __forceinline__ void process(const RecQ4K& r, const MmvArgs& ar, int 
     d[h] = h2f(r.hdr[h].x);
     ndm[h] = -h2f(r.hdr[h].x >> 16);
   }
+  if constexpr (mmv_roll(MK_Q4K, NTL)) r.refill_header(nx);
   const uint64_t nm2 = pk2(-MAGIC_F, -MAGIC_F);
   const uint64_t d02 = pk2(d[0], d[0]), d12 = pk2(d[1], d[1]);
   uint64_t tt[NTL][2], uu[NTL][2];
@@ -577,6 +602,7 @@ __device__ __forceinline__ void process(const RecQ4K& r, const MmvArgs& ar, int 
     uint32_t a[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) a[i] = ((s & 1) ? (w[i] >> 4) : w[i]) & 0x0F0F0F0Fu;
+    if (mmv_roll(MK_Q4K, NTL) && (s & 1)) r.refill(nx, p, lane);
     float m0 = byte_float(mnw[0][s >> 2], s & 3), m1 = byte_float(mnw[1][s >> 2], s & 3);
     if constexpr (!DEFER) {
       m0 *= ndm[0];
@@ -660,6 +686,22 @@ __host__ __device__ constexpr bool iq3_single(int ntl) { return ntl >= 4; }
 constexpr int IQ3_REPLICAS = 16;
 
 struct RecIQ3S {
+  struct Src { const uint8_t* p; };
+  static __device__ __forceinline__ Src src(const MmvArgs& a, int row0, int sb, int lane) {
+    return Src{a.w + (int64_t)row0 * a.row_bytes + (int64_t)sb * 1760};
+  }
+  __device__ __forceinline__ void refill_header(const Src& n, int lane) {
+    sc = ldg_stream_v2(n.p + 1664 + 8 * (lane >> 2));
+    dd = ldg_stream_u32(n.p + 1728 + 4 * (lane >> 2));
+  }
+  // half 0: used up after slice 3 (indices to bit 127, signs of slices 0..3); half 1: first needed again at slice 3
+  __device__ __forceinline__ void refill(const Src& n, int half, int lane) {
+    const uint4 i4 = ldg_stream_v4(n.p + 512 * half + 16 * lane);
+    const uint2 s2 = ldg_stream_v2(n.p + 1152 + 16 * lane + 8 * half);
+    idx[4 * half] = i4.x; idx[4 * half + 1] = i4.y; idx[4 * half + 2] = i4.z; idx[4 * half + 3] = i4.w;
+    sg[2 * half] = s2.x; sg[2 * half + 1] = s2.y;
+    if (half == 1) idx[8] = ldg_stream_u32(n.p + 1024 + 4 * lane);
+  }
   uint32_t idx[9], sg[4];
   uint2 sc;      // sub-scale nibbles of rows g, g + 8
   uint32_t dd;   // fp16 d of rows g, g + 8
@@ -755,7 +797,7 @@ __device__ __forceinline__ void iq3_slice(const RecIQ3S& r, const MmvArgs& ar, i
 }
 
 template <int NTL, bool DUMP>
-__device__ __forceinline__ void process(const RecIQ3S& r, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
+__device__ __forceinline__ void process(RecIQ3S& r, const RecIQ3S::Src& nx, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
                                         const uint8_t* grid, uint64_t (&acc)[NTL][2]) {
   constexpr bool DEFER = NTL <= 2;
   const char* gbase = reinterpret_cast<const char*>(grid);
@@ -770,6 +812,8 @@ __device__ __forceinline__ void process(const RecIQ3S& r, const MmvArgs& ar, int
     const float d = h2f(r.dd >> (16 * h));
     d2[h] = pk2(d, d);
   }
+  constexpr bool ROLL = mmv_roll(MK_IQ3S, NTL);
+  if constexpr (ROLL) r.refill_header(nx, lane);
   uint64_t tt[NTL][2];
   if constexpr (DEFER) {
 #pragma unroll
@@ -779,10 +823,12 @@ __device__ __forceinline__ void process(const RecIQ3S& r, const MmvArgs& ar, int
   iq3_slice<1, NTL, DUMP>(r, ar, row0, sb, lane, xl, gbase, lane_off, iscw, d2, acc, tt);
   iq3_slice<2, NTL, DUMP>(r, ar, row0, sb, lane, xl, gbase, lane_off, iscw, d2, acc, tt);
   iq3_slice<3, NTL, DUMP>(r, ar, row0, sb, lane, xl, gbase, lane_off, iscw, d2, acc, tt);
+  if constexpr (ROLL) r.refill(nx, 0, lane);
   iq3_slice<4, NTL, DUMP>(r, ar, row0, sb, lane, xl, gbase, lane_off, iscw, d2, acc, tt);
   iq3_slice<5, NTL, DUMP>(r, ar, row0, sb, lane, xl, gbase, lane_off, iscw, d2, acc, tt);
   iq3_slice<6, NTL, DUMP>(r, ar, row0, sb, lane, xl, gbase, lane_off, iscw, d2, acc, tt);
   iq3_slice<7, NTL, DUMP>(r, ar, row0, sb, lane, xl, gbase, lane_off, iscw, d2, acc, tt);
+  if constexpr (ROLL) r.refill(nx, 1, lane);
   if constexpr (!mmv_float_scale(NTL)) {
 #pragma unroll
     for (int j = 0; j < NTL; ++j) {
@@ -801,6 +847,19 @@ __device__ __forceinline__ void process(const RecIQ3S& r, const MmvArgs& ar, int
 static __constant__ __align__(16) int8_t c_iq4nl_mmv[16] = GSQ_IQ4NL_VALUES_INIT;
 
 struct RecIQ4XS {
+  struct Src { const uint8_t* b[2]; };
+  static __device__ __forceinline__ Src src(const MmvArgs& a, int row0, int sb, int lane) {
+    Src n;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      n.b[h] = a.w + (int64_t)min(row0 + (lane >> 2) + 8 * h, a.nrows - 1) * a.row_bytes + (int64_t)sb * 136;
+    return n;
+  }
+  __device__ __forceinline__ void refill_header(const Src& n) { hdr[0] = ldg_stream_v2(n.b[0]); hdr[1] = ldg_stream_v2(n.b[1]); }
+  __device__ __forceinline__ void refill(const Src& n, int s, int lane) {
+    q[0][s] = __ldg(reinterpret_cast<const uint32_t*>(n.b[0] + 8 + 16 * s + 4 * (lane & 3)));
+    q[1][s] = __ldg(reinterpret_cast<const uint32_t*>(n.b[1] + 8 + 16 * s + 4 * (lane & 3)));
+  }
   uint2 hdr[2];
   uint32_t q[2][8];
   __device__ __forceinline__ void load(const MmvArgs& a, int row0, int sb, int lane) {
@@ -833,27 +892,30 @@ __device__ __forceinline__ void iq4_lookup_mmv(uint32_t v, const uint32_t (&tb)[
 }
 
 template <int NTL, bool DUMP>
-__device__ __forceinline__ void process(const RecIQ4XS& r, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
+__device__ __forceinline__ void process(RecIQ4XS& r, const RecIQ4XS::Src& nx, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
                                         const uint8_t*, uint64_t (&acc)[NTL][2]) {
   constexpr int MC = 8 * NTL;
   const uint32_t* tw = reinterpret_cast<const uint32_t*>(c_iq4nl_mmv);
   const uint32_t tb[4] = {tw[0], tw[1], tw[2], tw[3]};
   uint64_t d2[2];
-  uint32_t sh4[2];  // the 2-bit high parts, pre-shifted to bits 4, 5
+  uint32_t scl[2], sh4[2];  // scale low nibbles; the 2-bit high parts, pre-shifted to bits 4, 5
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const float d = h2f(r.hdr[h].x);
     d2[h] = pk2(d, d);
     sh4[h] = (r.hdr[h].x >> 16) << 4;
+    scl[h] = r.hdr[h].y;
   }
+  if constexpr (mmv_roll(MK_IQ4XS, NTL)) r.refill_header(nx);
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
     uint32_t a[4];
     iq4_lookup_mmv(r.q[0][s], tb, a[0], a[2]);
     iq4_lookup_mmv(r.q[1][s], tb, a[1], a[3]);
+    if constexpr (mmv_roll(MK_IQ4XS, NTL)) r.refill(nx, s, lane);
     // 6-bit sub-scale minus 32: low nibble from scales_l, bits 4, 5 from scales_h
-    const int sc0 = (int)(((r.hdr[0].y >> (4 * s)) & 0xFu) | ((sh4[0] >> (2 * s)) & 0x30u)) - 32;
-    const int sc1 = (int)(((r.hdr[1].y >> (4 * s)) & 0xFu) | ((sh4[1] >> (2 * s)) & 0x30u)) - 32;
+    const int sc0 = (int)(((scl[0] >> (4 * s)) & 0xFu) | ((sh4[0] >> (2 * s)) & 0x30u)) - 32;
+    const int sc1 = (int)(((scl[1] >> (4 * s)) & 0xFu) | ((sh4[1] >> (2 * s)) & 0x30u)) - 32;
     // d * sub-scale, applied on the floating-point side (|sum| <= 32 * 127 * 127 < 2^22)
     float h0, h1;
     upk2(d2[0], h0, h1);
@@ -884,6 +946,20 @@ __device__ __forceinline__ void process(const RecIQ4XS& r, const MmvArgs& ar, in
 // (sum_a * sc_a + sum_b * sc_b, below 2^24 in magnitude) and converted once.
 
 struct RecQ6K {
+  struct Src { const uint8_t* p; };
+  static __device__ __forceinline__ Src src(const MmvArgs& a, int row0, int sb, int lane) {
+    return Src{a.w + (int64_t)row0 * a.row_bytes + (int64_t)sb * 3360};
+  }
+  __device__ __forceinline__ void refill(const Src& n, int half, int lane) {
+    ql[half] = ldg_stream_v4(n.p + 64 * lane + 16 * half);
+    ql[2 + half] = ldg_stream_v4(n.p + 64 * lane + 16 * (2 + half));
+    if (half == 1) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) qh[i] = ldg_stream_v4(n.p + 2048 + 32 * lane + 16 * i);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) sc[i] = ldg_stream_v4(n.p + 3072 + 32 * (lane >> 2) + 16 * i);
+    }
+  }
   uint4 ql[4];   // [2 h + n]: words (qb, is) = x y z w
   uint4 qh[2];   // [h]: words (n, is)
   uint4 sc[2];   // [h]: 16 int8
@@ -940,7 +1016,7 @@ __device__ __forceinline__ void dump_c16(const MmvArgs& ar, const int (&c)[4], i
 }
 
 template <int NTL, bool DUMP>
-__device__ __forceinline__ void process(const RecQ6K& r, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
+__device__ __forceinline__ void process(RecQ6K& r, const RecQ6K::Src& nx, const MmvArgs& ar, int row0, int sb, int lane, const XSmem& xl,
                                         const uint8_t*, uint64_t (&acc)[NTL][2]) {
   constexpr int MC = 8 * NTL;
   const int t = lane & 3;
@@ -992,9 +1068,11 @@ __device__ __forceinline__ void process(const RecQ6K& r, const MmvArgs& ar, int 
         tt[j][1] = vfma2(pk2(f2, f3), dv2, tt[j][1]);
       }
     }
+    if constexpr (mmv_roll(MK_Q6K, NTL)) r.refill(nx, n, lane);
   }
   const float d0 = h2f(r.dd), d1 = h2f(r.dd >> 16);
   const uint64_t d02 = pk2(d0, d0), d12 = pk2(d1, d1);
+  if constexpr (mmv_roll(MK_Q6K, NTL)) r.dd = ldg_stream_u32(nx.p + 3328 + 4 * (lane >> 2));
 #pragma unroll
   for (int j = 0; j < NTL; ++j) {
     acc[j][0] = vfma2(d02, tt[j][0], acc[j][0]);
@@ -1184,12 +1262,17 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
         const bool has_next = idx + 1 < idx1;
         const bool wrap = rec + 1 == nsr;
         const int ntl = wrap ? tl + 1 : tl, nrc = wrap ? 0 : rec + 1;
-        // Up to 16 columns the next record is loaded into registers while this one is multiplied. Wider than
-        // that the accumulators need the registers: the next record is only requested from L2 and loaded after
-        // the arithmetic (the other warps of the SM cover the wait; a record then takes ~1000 instructions).
-        constexpr bool REGPF = NTL <= 2;
+        // Rolling (mmv_roll): the multiplication replaces each part of the record by the next one's as soon as it has used
+        // it. Else up to 16 columns the next record is loaded into registers of its own while this one is multiplied;
+        // wider than that the accumulators need the registers: the next record is only requested from L2 and loaded
+        // after the arithmetic.
+        constexpr bool ROLL = mmv_roll(KIND, NTL), REGPF = NTL <= 2 && !ROLL;
         Rec nxt;
-        if (has_next) {
+        if (has_next && ROLL) {
+          // (two ahead: the refills below are the requests one ahead)
+          const int n2r = nrc + 1 == nsr ? 0 : nrc + 1, n2t = nrc + 1 == nsr ? ntl + 1 : ntl;
+          if (idx + 2 < idx1) Rec::prefetch(a, (tile_begin + t0 + n2t) * MMV_TR, sb0 + n2r, lane);
+        } else if (has_next) {
           if constexpr (REGPF) {
             nxt.load(a, (tile_begin + t0 + ntl) * MMV_TR, sb0 + nrc, lane);
           } else {
@@ -1201,7 +1284,8 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
         xl.q8 = xlane.q8;
         xl.d = xlane.d + rec * (8 * MC);
         xl.s = xlane.s + rec * (8 * MC);
-        process<NTL, DUMP>(cur, a, (tile_begin + t0 + tl) * MMV_TR, sb0 + rec, lane, xl, grid, acc);
+        const typename Rec::Src nx = Rec::src(a, (tile_begin + t0 + (has_next ? ntl : tl)) * MMV_TR, sb0 + (has_next ? nrc : rec), lane);
+        process<NTL, DUMP>(cur, nx, a, (tile_begin + t0 + tl) * MMV_TR, sb0 + rec, lane, xl, grid, acc);
         if (!has_next || wrap) {
           // leaving tile tl, [row][column]: a tile this warp covered whole is final for this CTA; otherwise the
           // sums are parked, slot 0 for the tile the chunk started in, slot 1 for the one it ends in
@@ -1224,7 +1308,7 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
             acc[j][0] = acc[j][1] = 0ull;
           }
         }
-        if (has_next) {
+        if (has_next && !ROLL) {
           if constexpr (REGPF) {
             cur = nxt;
           } else {
