@@ -90,12 +90,18 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, bool s
 }
 
 // Whether the small-batch tensor-core kernel is tried first. It serves 1..48 rows; for the types in GGUF order, whose
-// decoding it repeats per lane, the kernel with evenly cut work is faster from 33 rows on (48 rows, us: IQ4_XS 5120 x 17408
-// 64 -> 58, Q4_K 17408 x 5120 59 -> 52, 2048 x 2048 16.5 -> 13.5; at 32 rows they are level; repacked IQ3_S 44 against 54).
-static bool small_batch(int ggml_type, int packed, int64_t rows, int64_t m) {
+// decoding it repeats per lane, the kernel with evenly cut work is the faster one from 33 rows on, except (us, small-batch
+// kernel / evenly cut work):
+//   * IQ4_XS while the activations are few: 40 rows 17408 x 5120 45.5 / 54.6, 48 rows 34816 x 5120 82.2 / 95.6, but
+//     48 rows 2048 x 8192 23.9 / 23.0; weights so tall that it would decline, and small ones, go on;
+//   * Q4_K while the weight has too few 128-row tiles to cut evenly: 48 rows 1024 x 5120 17.4 / 21.8, 5120 x 2048
+//     16.3 / 17.0, but 5120 x 5120 25.5 / 24.2.
+static bool small_batch(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k) {
   if (gemm_variant() == 10 || !mmv_applies(ggml_type, packed, rows, m)) return false;
-  const bool gguf = ggml_type == GSQ_TYPE_IQ4_XS || ggml_type == GSQ_TYPE_Q4_K;
-  return !(gguf && m > 32 && gemm_variant() == 0 && !gemm_dump_pointer());
+  if (m <= 32 || gemm_variant() != 0 || gemm_dump_pointer()) return true;
+  if (ggml_type == GSQ_TYPE_IQ4_XS) return m * k <= 320000 && rows <= 40000 && rows * k > (4 << 20);
+  if (ggml_type == GSQ_TYPE_Q4_K) return rows * k <= (12 << 20) && rows * k > (4 << 20);
+  return true;
 }
 
 static size_t way_scratch(Way way, int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
@@ -129,7 +135,7 @@ static size_t linear_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, in
     b = b > plane ? b : plane;
   }
   // (the small-batch kernel takes 128-value blocks, and may decline the shape)
-  size_t mmq = small_batch(ggml_type, packed, rows, m) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
+  size_t mmq = small_batch(ggml_type, packed, rows, m, k) ? (size_t)(k / 128) * (size_t)m * 144 : 0;
   if (mmq && !small && mmv_rows_wins(ggml_type, rows, m, k) && mmv_rows_bytes(ggml_type, m, k) > mmq) mmq = mmv_rows_bytes(ggml_type, m, k);
   b = b > mmq ? b : mmq;
   return align256(b > 0 ? b : 1);
@@ -155,7 +161,7 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
   const int layout = gsq_q8_layout_for_type(ggml_type);
   int rc;
   // 1..48 rows: the small-batch tensor-core kernel on 128-value blocks, where it serves the type and the shape fits
-  if (small_batch(ggml_type, packed, rows, m)) {
+  if (small_batch(ggml_type, packed, rows, m, k)) {
     if (!gemm_dump_pointer() && mmv_raw_applies(ggml_type, packed, rows, m, k, 0)) {
       rc = mmv_host(w, row_bytes, rows, ggml_type, packed, x, 3, m, k, y, y_dtype, y_row_stride, stream, nullptr, nullptr, x_dtype, x_row_stride);
       if (rc != 1000) return rc;

@@ -1543,26 +1543,26 @@ struct MmvCost {
 __host__ __device__ constexpr MmvCost mmv_cost(int kind, int ntl) {
   if (kind == MK_Q4K)
     return ntl == 1   ? MmvCost{0.3f, 0.0656f, 0.1f, 0.11f, 3.0f, 0.165f, 6.1f}
-           : ntl == 2 ? MmvCost{0.915f, 0.136f, 0.366f, 0.0f, 1.94f, 0.349f, 3.54f}
-           : ntl == 3 ? MmvCost{0.639f, 0.157f, 1.58f, 0.12f, 2.49f, 0.618f, 20.0f}
-           : ntl == 4 ? MmvCost{0.745f, 0.202f, 2.6f, 0.0f, 2.13f, 0.877f, 2.02f}
+           : ntl == 2 ? MmvCost{0.524f, 0.119f, 1.04f, 0.384f, 1.32f, 0.351f, 25.0f}
+           : ntl == 3 ? MmvCost{0.533f, 0.168f, 2.15f, 0.0f, 1.13f, 0.344f, 24.8f}
+           : ntl == 4 ? MmvCost{0.76f, 0.204f, 2.05f, 0.0f, 1.29f, 0.539f, 2.99f}
                       : MmvCost{0.3f, 0.204f, 0.442f, 0.0f, 1.71f, 1.07f, 2.23f};
   if (kind == MK_Q6K)
     return ntl == 1   ? MmvCost{0.657f, 0.0959f, 0.546f, 0.0f, 0.907f, 0.1f, 20.0f}
            : ntl == 2 ? MmvCost{1.12f, 0.167f, 0.199f, 0.317f, 1.5f, 0.1f, 20.0f}
-           : ntl == 3 ? MmvCost{0.839f, 0.185f, 1.73f, 0.0f, 1.87f, 0.546f, 15.7f}
-           : ntl == 4 ? MmvCost{1.07f, 0.228f, 2.19f, 0.0146f, 2.07f, 0.791f, 12.0f}
+           : ntl == 3 ? MmvCost{0.663f, 0.179f, 1.57f, 0.0f, 1.03f, 0.351f, 13.1f}
+           : ntl == 4 ? MmvCost{0.753f, 0.233f, 2.58f, 0.0f, 0.95f, 0.442f, 12.9f}
                       : MmvCost{1.35f, 0.319f, 3.94f, 0.0f, 3.01f, 1.33f, 13.6f};
   if (kind == MK_IQ3S)
     return ntl == 1   ? MmvCost{0.584f, 0.0743f, 0.745f, 0.0f, 1.57f, 0.1f, 2.04f}
            : ntl == 2 ? MmvCost{0.545f, 0.102f, 1.05f, 0.142f, 1.41f, 0.1f, 6.95f}
            : ntl == 3 ? MmvCost{0.582f, 0.127f, 1.41f, 0.102f, 2.66f, 0.266f, 7.45f}
-           : ntl == 4 ? MmvCost{0.764f, 0.174f, 2.79f, 0.0f, 1.72f, 1.17f, 2.12f}
+           : ntl == 4 ? MmvCost{0.541f, 0.161f, 2.37f, 0.0f, 1.0f, 0.726f, 1.42f}
                       : MmvCost{0.629f, 0.204f, 3.31f, 0.0f, 2.38f, 1.15f, 2.04f};
   return ntl == 1   ? MmvCost{0.3f, 0.103f, 0.1f, 0.0228f, 2.5f, 0.175f, 3.12f}
          : ntl == 2 ? MmvCost{0.614f, 0.146f, 0.847f, 0.031f, 1.71f, 0.221f, 3.02f}
-         : ntl == 3 ? MmvCost{0.781f, 0.166f, 1.3f, 0.0f, 2.27f, 0.592f, 7.33f}
-         : ntl == 4 ? MmvCost{0.829f, 0.199f, 2.36f, 0.0f, 2.35f, 0.932f, 2.06f}
+         : ntl == 3 ? MmvCost{0.534f, 0.154f, 1.69f, 0.0f, 0.946f, 0.422f, 7.74f}
+         : ntl == 4 ? MmvCost{0.609f, 0.183f, 2.46f, 0.0f, 0.763f, 0.445f, 15.6f}
                     : MmvCost{0.3f, 0.245f, 0.371f, 0.0f, 1.62f, 1.04f, 2.11f};
 }
 
