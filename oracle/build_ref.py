@@ -27,9 +27,10 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 
 def reference_root() -> str | None:
-    """Where the reference tree is: $GSQ_REFERENCE, else a checkout named `reference` beside this repository."""
+    """Where the reference tree is: $GSQ_REFERENCE, else a checkout named `reference` beside this repository (None where
+    there is none, or an empty directory in its place)."""
     cand = os.environ.get("GSQ_REFERENCE") or os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference")
-    return cand if os.path.isdir(cand) else None
+    return cand if os.path.isdir(os.path.join(cand, "plugin", "vllm_gguf_plugin")) else None
 
 
 def build(ref: str | None = None, force: bool = False) -> str:

@@ -35,4 +35,5 @@ def golden_dir():
 
 @pytest.fixture(scope="session")
 def reference_dir():
-    return REFERENCE if os.path.isdir(REFERENCE) else None
+    """The reference tree, None where there is none (or an empty directory in its place)."""
+    return REFERENCE if os.path.isdir(os.path.join(REFERENCE, "plugin", "vllm_gguf_plugin")) else None

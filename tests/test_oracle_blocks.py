@@ -62,3 +62,12 @@ def test_integer_decode_consistent_with_float(name):
         assert dec.isc.min() >= 1 and dec.isc.max() <= 31
     if name == "Q6_K":
         assert dec.w8.min() >= -32 and dec.w8.max() <= 31 and dec.g == 16
+
+
+def test_an_empty_directory_is_no_reference_tree(monkeypatch, tmp_path):
+    from oracle import build_ref
+
+    monkeypatch.setenv("GSQ_REFERENCE", str(tmp_path))
+    assert build_ref.reference_root() is None
+    (tmp_path / "plugin" / "vllm_gguf_plugin").mkdir(parents=True)
+    assert build_ref.reference_root() == str(tmp_path)
