@@ -242,6 +242,7 @@ int gsq_mul_mat_q8(const void* w, int64_t row_bytes, int64_t rows, int ggml_type
  *                fastest kernels run: the prefill GEMM then keeps the expanded weights there, 2 bytes per weight (4 for
  *                Q6_K), at most 512 MB at a time. gsq_linear_scratch_bytes(...) bytes, the least, have no room for that:
  *                the kernels that decode the weights as they go run instead
+ * Repacked weights (packed != 0) have a multiple of 16 rows; any other count is refused (GSQ_ERR_UNSUPPORTED, sizes 0).
  */
 size_t gsq_linear_scratch_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed);
 size_t gsq_linear_workspace_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed);

@@ -34,3 +34,22 @@ def test_host_only_entry_points():
     assert lib.gsq_mul_mat_vec_q8(None, 0, 0, 21, 1, None, 0, 5120, None, 0, 0, None) == 0
     assert lib.gsq_quantize_q8_1(None, 1, 0, 512, 512, None, None) == 0
     assert lib.gsq_iq3s_repack(None, 0, 220, 0, None) == 0
+
+
+def test_repacked_weights_of_ragged_rows_are_refused():
+    """Repacked IQ3_S / Q6_K are records of 16 rows. gsq_linear and gsq_linear_vec refuse any other row count before they
+    touch the device, at every number of activation rows (from 25 on the weights used to be expanded record by record,
+    past the last row)."""
+    lib = _cabi.lib
+    buf = ctypes.create_string_buffer(1 << 20)
+    at = (ctypes.addressof(buf) + 255) // 256 * 256
+    for t, bs in ((21, 110), (14, 210)):
+        for rows in (1, 15, 24, 40, 17400):
+            for m in (1, 8, 9, 24, 25, 32, 48, 97, 128, 300):
+                k = 1024
+                args = (at, k // 256 * bs, rows, t, 1, at, 2, m, k, k, at, 2, rows)
+                assert lib.gsq_linear_workspace_bytes(rows, m, k, t, 1) == 0 and lib.gsq_linear_scratch_bytes(rows, m, k, t, 1) == 0
+                assert lib.gsq_linear(*args, at, 1 << 30, None) == _cabi.ERR_UNSUPPORTED, (t, rows, m)
+                assert lib.gsq_linear_vec(*args, None) == _cabi.ERR_UNSUPPORTED, (t, rows, m)
+                assert lib.gsq_linear_allreduce(*args, at, 1 << 30, ctypes.byref(_cabi.PeerReduce()), None) != 0
+        assert lib.gsq_linear_workspace_bytes(32, 128, 1024, t, 1) > 0

@@ -535,7 +535,7 @@ static void choose_tiles(Plan* p, int64_t n_rp, int64_t rows, int64_t m) {
 }
 
 int make_plan(Plan* p, int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu) {
-  p->kind = kind_of(ggml_type, packed);
+  p->kind = kind_of(ggml_type, packed, rows);
   if (p->kind == K_NONE || rows <= 0 || m <= 0 || k <= 0 || k % 256 != 0) return GSQ_ERR_UNSUPPORTED;
   if (form_of(p->kind) == F_Q81) hu = 2;
   if (p->kind == K_Q4K) hu = 1;
@@ -580,6 +580,8 @@ int gemm4_error_flag(int* flag) {
   GSQ_CUDA_TRY(cudaMemcpyFromSymbol(flag, pl::g4_error, sizeof(int)));
   return GSQ_OK;
 }
+
+bool gemm4_applies(int ggml_type, int packed, int64_t rows) { return pl::kind_of(ggml_type, packed, rows) != pl::K_NONE; }
 
 size_t gemm4_scratch_bytes(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu) {
   pl::Plan p;

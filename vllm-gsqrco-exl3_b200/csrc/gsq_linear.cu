@@ -34,6 +34,7 @@ size_t gemm5_scratch_bytes(int ggml_type, int packed, int64_t rows, int64_t m, i
 int gemm5_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
                  int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* scratch, void* stream);
 // gsq_gemm4.cu
+bool gemm4_applies(int ggml_type, int packed, int64_t rows);
 size_t gemm4_scratch_bytes(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu);
 int gemm4_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
                  int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* scratch, int hu, void* stream);
@@ -46,6 +47,11 @@ int gemm_variant();
 static size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 static int g_prefill_precision = GSQ_PREFILL_ROUNDED;
+
+// Repacked weights are records of 16 rows: no kernel takes a part of one.
+static bool ragged(int ggml_type, int packed, int64_t rows) {
+  return packed && (ggml_type == GSQ_TYPE_IQ3_S || ggml_type == GSQ_TYPE_Q6_K) && rows % 16 != 0;
+}
 
 // The kernels of a product above the small-batch tensor-core kernel's rows (or of a type or shape it does not serve).
 enum Way {
@@ -85,7 +91,7 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, bool s
   const bool q6 = ggml_type == GSQ_TYPE_Q6_K, q6_packed = q6 && packed && rows % 16 == 0;
   // Q6_K, IQ3_S in GGUF order and the low-bit types: the two steps once they cost less than the repeated launches of the
   // small-batch kernels (48 or 8 rows each), at fp32 accuracy, unless integer sums are asked for.
-  if (!small && !dump && g_prefill_precision != GSQ_PREFILL_INTEGER && m >= (q6_packed ? 97 : q6 || ggml_type == GSQ_TYPE_IQ3_S ? 25 : 9)) return W_PLANES2;
+  if (!small && !dump && g_prefill_precision != GSQ_PREFILL_INTEGER && gemm4_applies(ggml_type, packed, rows) && m >= (q6_packed ? 97 : q6 || ggml_type == GSQ_TYPE_IQ3_S ? 25 : 9)) return W_PLANES2;
   return q6_packed ? W_MMV_LOOP : W_GEMV_LOOP;
 }
 
@@ -126,7 +132,7 @@ extern "C" int gsq_prefill_precision(int mode) {
 
 static size_t linear_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed, bool small) {
   using namespace gsq;
-  if (m <= 0 || k <= 0 || rows <= 0) return 0;
+  if (m <= 0 || k <= 0 || rows <= 0 || ragged(ggml_type, packed, rows)) return 0;
   const Way way = choose_way(ggml_type, packed, rows, m, small);
   size_t b = way_scratch(way, rows, m, k, ggml_type, packed);
   if (small && gemm2_applies(ggml_type, packed, rows) && choose_way(ggml_type, packed, rows, m, false) == W_PLANES1) {
@@ -155,7 +161,7 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
   if (m == 0 || rows == 0) return GSQ_OK;
   if (m < 0 || rows < 0 || k <= 0 || k % 256 != 0 || !w || !x || !y) return GSQ_ERR_UNSUPPORTED;
   const int bs = block_bytes(ggml_type);
-  if (bs == 0 || row_bytes != (k / 256) * bs) return GSQ_ERR_UNSUPPORTED;
+  if (bs == 0 || row_bytes != (k / 256) * bs || ragged(ggml_type, packed, rows)) return GSQ_ERR_UNSUPPORTED;
   if (y_dtype != GSQ_F32 && y_dtype != GSQ_F16 && y_dtype != GSQ_BF16) return GSQ_ERR_UNSUPPORTED;
   if (!scratch || scratch_bytes < gsq_linear_scratch_bytes(rows, m, k, ggml_type, packed)) return GSQ_ERR_SCRATCH;
   const int layout = gsq_q8_layout_for_type(ggml_type);

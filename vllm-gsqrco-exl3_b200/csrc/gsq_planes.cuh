@@ -24,7 +24,9 @@ __host__ __device__ constexpr int a_planes(int kind) { return kind == K_Q6K || k
 // planes of per-superblock extra columns (16 of them): Q4_K's minimum and correction terms, Q2_K's minimum terms as a pair
 __host__ __device__ constexpr int t_planes(int kind) { return kind == K_Q4K ? 1 : kind == K_Q2K ? 2 : 0; }
 
-inline int kind_of(int ggml_type, int packed) {
+// (repacked weights: whole 16-row records, which the expanding kernel reads and writes as such)
+inline int kind_of(int ggml_type, int packed, int64_t rows) {
+  if (packed && rows % 16 != 0) return K_NONE;
   switch (ggml_type) {
     case GSQ_TYPE_Q4_K: return packed ? K_NONE : K_Q4K;
     case GSQ_TYPE_IQ4_XS: return packed ? K_NONE : K_IQ4XS;
