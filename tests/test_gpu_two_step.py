@@ -96,3 +96,24 @@ def test_least_scratch(name, packed, m):
     got = _run(t, packed, raw, x.to(DEV), rows, least=True)
     q, d, _ = q8_1.quantize_q8_1(x.numpy())
     assert product.rel_err(got, product.product_q81(blocks.decode(raw, t), q, d)) <= 3e-3   # (d in half or in fp32; Q4_K: sums of x or of q)
+
+
+def test_long_prompt_with_k_in_parts():
+    """More tokens than a grid's y takes, on a weight small enough that K is cut into parts whose sums a second kernel adds."""
+    from oracle import prefill_forms
+
+    name, rows, k, m = "IQ4_XS", 16, 5632, 65537
+    t, lib = TYPES[name], _cabi.lib
+    # (64 rows of this K are not cut; beside the parts their scratch is the same, one pair of row tiles)
+    assert lib.gsq_linear_workspace_bytes(rows, m, k, t, 0) - lib.gsq_linear_workspace_bytes(64, m, k, t, 0) >= 2 * m * rows * 4
+    raw = synth.make_weight(t, rows, k, 90)
+    x = torch.randn(m, k, device=DEV, generator=torch.Generator(DEV).manual_seed(91), dtype=torch.bfloat16)
+    at = [0, 1, 4095, 65534, 65535, 65536]
+    few = synth.nudge_ties_torch(torch.from_numpy(synth.make_activation(len(at), k, 92)).to(torch.bfloat16))
+    x[at] = few.to(DEV)
+    w = torch.from_numpy(raw).to(DEV)
+    y = torch.ops._C_gguf.lcpp_mul_mat_q(w, x, t, rows)
+    got = y[at].float().cpu().numpy()
+    assert bool(torch.isfinite(y).all())
+    # 3e-6 for the sums, and the rounding of the result to bf16 (8 significant bits: at most 2^-8 of a value)
+    assert product.rel_err(got, prefill_forms.product(raw, t, few.float().numpy())) <= 2.0 ** -8 + 3e-6

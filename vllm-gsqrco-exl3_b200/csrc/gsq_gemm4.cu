@@ -476,13 +476,14 @@ static int gemm4_launch(const Plan& p, uint8_t* scratch, int64_t rows, int64_t m
   return p.hu == 2 ? launch_gemm4<2, 1, 0>(g, stage, sm_count, st) : launch_gemm4<1, 1, 0>(g, stage, sm_count, st);
 }
 
-// y = the sum of the parts, in their order; a thread takes one result of every part
+// y = the sum of the parts, in their order; a thread takes one result of every part. Tokens are the grid's x: a prompt may
+// have more than the 65535 blocks of y (row blocks of a call: 4096 at most, by the bound on expanded weights).
 template <typename T>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ part, T* __restrict__ y, int64_t m, int64_t rows, int64_t ldy,
                                                        int splits) {
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int64_t row = (int64_t)blockIdx.x * 256 + threadIdx.x, tok = blockIdx.y;
+  const int64_t row = (int64_t)blockIdx.y * 256 + threadIdx.x, tok = blockIdx.x;
   if (row >= rows) return;
   const float* p = part + tok * rows + row;
   float s = __ldcg(p);
@@ -492,7 +493,7 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict_
 
 static int sum_parts(const Plan& p, const uint8_t* scratch, int64_t rows, int64_t m, void* y, int y_dtype, int64_t ldy, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((rows + 255) / 256), (unsigned)m);
+  cfg.gridDim = dim3((unsigned)m, (unsigned)((rows + 255) / 256));
   cfg.blockDim = dim3(256);
   cfg.stream = st;
   cudaLaunchAttribute attr;
