@@ -53,3 +53,11 @@ def test_repacked_weights_of_ragged_rows_are_refused():
                 assert lib.gsq_linear_vec(*args, None) == _cabi.ERR_UNSUPPORTED, (t, rows, m)
                 assert lib.gsq_linear_allreduce(*args, at, 1 << 30, ctypes.byref(_cabi.PeerReduce()), None) != 0
         assert lib.gsq_linear_workspace_bytes(32, 128, 1024, t, 1) > 0
+
+
+def test_packed_flag_means_nothing_for_types_of_one_layout():
+    lib = _cabi.lib
+    for t in (12, 23):
+        for rows in (16, 24, 5120, 17408):
+            for m in (1, 8, 9, 40, 100, 200, 256, 777):
+                assert lib.gsq_linear_workspace_bytes(rows, m, 2048, t, 1) == lib.gsq_linear_workspace_bytes(rows, m, 2048, t, 0), (t, rows, m)

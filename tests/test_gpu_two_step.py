@@ -117,3 +117,19 @@ def test_long_prompt_with_k_in_parts():
     assert bool(torch.isfinite(y).all())
     # 3e-6 for the sums, and the rounding of the result to bf16 (8 significant bits: at most 2^-8 of a value)
     assert product.rel_err(got, prefill_forms.product(raw, t, few.float().numpy())) <= 2.0 ** -8 + 3e-6
+
+
+@pytest.mark.parametrize("m", [1, 40, 100, 300])
+@pytest.mark.parametrize("name", ["Q4_K", "IQ4_XS"])
+def test_packed_flag_on_a_type_of_one_layout(name, m):
+    rows, k, t, lib = 24, 1024, TYPES[name], _cabi.lib
+    w = torch.from_numpy(synth.make_weight(t, rows, k, 95)).to(DEV)
+    x = torch.from_numpy(synth.make_activation(m, k, 96)).to(DEV)
+    y = []
+    for packed in (0, 1):
+        n = lib.gsq_linear_workspace_bytes(rows, m, k, t, packed)
+        scratch, out = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty(m, rows, device=DEV)
+        assert lib.gsq_linear(w.data_ptr(), w.shape[1], rows, t, packed, x.data_ptr(), 0, m, k, k, out.data_ptr(), 0, rows, scratch.data_ptr(), n,
+                              torch.cuda.current_stream().cuda_stream) == 0
+        y.append(out)
+    assert torch.equal(*y)

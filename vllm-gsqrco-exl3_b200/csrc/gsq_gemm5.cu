@@ -114,8 +114,8 @@ static void tiles_of(Tiles* t, int kind, int64_t rows, int64_t m, int64_t k, int
 }
 static int kind_of(int ggml_type, int packed, int64_t rows) {
   if (ggml_type == GSQ_TYPE_IQ3_S && packed && rows % 16 == 0) return G5_IQ3S;
-  if (ggml_type == GSQ_TYPE_IQ4_XS && !packed) return G5_IQ4XS;
-  if (ggml_type == GSQ_TYPE_Q4_K && !packed) return G5_Q4K;
+  if (ggml_type == GSQ_TYPE_IQ4_XS) return G5_IQ4XS;   // (one layout, whatever the flag says)
+  if (ggml_type == GSQ_TYPE_Q4_K) return G5_Q4K;
   return -1;
 }
 

@@ -24,12 +24,13 @@ __host__ __device__ constexpr int a_planes(int kind) { return kind == K_Q6K || k
 // planes of per-superblock extra columns (16 of them): Q4_K's minimum and correction terms, Q2_K's minimum terms as a pair
 __host__ __device__ constexpr int t_planes(int kind) { return kind == K_Q4K ? 1 : kind == K_Q2K ? 2 : 0; }
 
-// (repacked weights: whole 16-row records, which the expanding kernel reads and writes as such)
+// (repacked weights: whole 16-row records, which the expanding kernel reads and writes as such; Q4_K and IQ4_XS have one
+// layout, whatever the flag says, as in the kernels of fewer rows)
 inline int kind_of(int ggml_type, int packed, int64_t rows) {
+  if (ggml_type == GSQ_TYPE_Q4_K) return K_Q4K;
+  if (ggml_type == GSQ_TYPE_IQ4_XS) return K_IQ4XS;
   if (packed && rows % 16 != 0) return K_NONE;
   switch (ggml_type) {
-    case GSQ_TYPE_Q4_K: return packed ? K_NONE : K_Q4K;
-    case GSQ_TYPE_IQ4_XS: return packed ? K_NONE : K_IQ4XS;
     case GSQ_TYPE_IQ3_S: return packed ? K_IQ3S_PACKED : K_IQ3S;
     case GSQ_TYPE_Q6_K: return packed ? K_Q6K_PACKED : K_Q6K;
     case GSQ_TYPE_Q2_K: return packed ? K_NONE : K_Q2K;
