@@ -6,7 +6,7 @@ import torch
 import torch.utils._python_dispatch
 
 import gsq_b200  # noqa: F401
-from gsq_b200 import _gsq_ops, synth
+from gsq_b200 import _gsq_ops, lcpp_ops, synth
 from gsq_b200.quantization import iq3_pack, linear
 
 TYPES = {**synth.TYPE_IDS, **synth.LOW_BIT_TYPE_IDS}
@@ -38,17 +38,22 @@ def test_native_errors_are_python_exceptions():
         _gsq_ops.linear_runs(x[:4], w, [0, 16, 112, 29], False)
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("m", [1, 4, 8, 9, 40, 70])
-@pytest.mark.parametrize("names", [("IQ3_S", "IQ3_S", "Q6_K"), ("Q4_K", "IQ4_XS", "Q4_K"), ("IQ3_S", "IQ2_XS", "Q2_K")])
-def test_runs_of_a_fused_layer(m, names):
-    k, rows = 1024, (160, 48, 64)
+def _fused_layer(names, rows, k):
     layer, method = torch.nn.Module(), linear.GGUFLinearMethod(None)
     method.create_weights(layer, k, list(rows), k, sum(rows), torch.bfloat16)
     for i, (sid, name, r) in enumerate(zip("qkv", names, rows)):
         layer.weight.load_shard(torch.from_numpy(synth.make_weight(TYPES[name], r, k, 20 + i)).cuda(), sid)
         layer.weight_type.shard_weight_type[sid] = TYPES[name]
     method.process_weights_after_loading(layer)
+    return layer, method
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 4, 8, 9, 40, 70])
+@pytest.mark.parametrize("names", [("IQ3_S", "IQ3_S", "Q6_K"), ("Q4_K", "IQ4_XS", "Q4_K"), ("IQ3_S", "IQ2_XS", "Q2_K")])
+def test_runs_of_a_fused_layer(m, names):
+    k, rows = 1024, (160, 48, 64)
+    layer, method = _fused_layer(names, rows, k)
     x = torch.from_numpy(synth.make_activation(m, k, 30 + m)).to(torch.bfloat16).cuda()
     got = method.apply(layer, x)
     w = layer.weight
@@ -66,3 +71,24 @@ def test_runs_of_a_fused_layer(m, names):
     with Watch():   # someone intercepts: through the custom op, same result
         assert torch.equal(method.apply(layer, x), want)
     assert "_C_gguf.gsq_linear_runs.default" in seen
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 4, 40])
+def test_output_into_of_a_fused_layer(m):
+    """output_into holds for a layer whose shards are of several types: the caller's tensor, strided rows included, or an
+    error if it does not fit."""
+    k, rows = 1024, (160, 48, 64)
+    layer, method = _fused_layer(("IQ3_S", "IQ3_S", "Q6_K"), rows, k)
+    x = torch.from_numpy(synth.make_activation(m, k, 31)).to(torch.bfloat16).cuda()
+    want = method.apply(layer, x)
+    buf = torch.full((m, 300), -1.0, dtype=torch.bfloat16, device="cuda")
+    into = buf[:, 8:8 + sum(rows)]
+    with lcpp_ops.output_into(into):
+        got = method.apply(layer, x)
+    assert got.data_ptr() == into.data_ptr() and torch.equal(into, want)
+    assert bool((buf[:, :8] == -1).all()) and bool((buf[:, 8 + sum(rows):] == -1).all())
+    for bad in (torch.empty(m, 160, dtype=torch.bfloat16, device="cuda"), torch.empty(m, sum(rows), device="cuda")):
+        with pytest.raises(RuntimeError, match="output_into"), lcpp_ops.output_into(bad):
+            method.apply(layer, x)
+    assert torch.equal(method.apply(layer, x), want)

@@ -296,8 +296,8 @@ Tensor linear_runs(const Tensor& x, const Tensor& w, at::IntArrayRef runs, bool 
     bool pk = packed;
     const int op = op_for(n, type, rows, x.size(1), pk);
     if (!x.is_cuda()) guard(kSpec[op], wt, x, type, rows);
-    if (!y.defined()) y = at::empty({n, total}, x.options());
-    product_of_run(op, wt, x, type, rows, q, (char*)y.mutable_data_ptr() + col * x.element_size(), total,
+    if (!y.defined()) y = result(n, total, x);
+    product_of_run(op, wt, x, type, rows, q, (char*)y.mutable_data_ptr() + col * x.element_size(), y.stride(0),
                    c10::cuda::getCurrentCUDAStream().stream());
     col += rows;
   }

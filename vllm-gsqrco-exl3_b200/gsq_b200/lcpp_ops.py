@@ -45,7 +45,7 @@ class output_into:
     """with output_into(t): the next op call of this module on this thread writes its [rows of X, row] result into `t`
     (same shape and dtype as it would have returned, unit inner stride, any row stride) and returns `t`: the kernels take
     any row stride, so a tensor-parallel runtime can have a shard's result land in its slot of a collective's buffer
-    instead of copying it there."""
+    instead of copying it there. A fused layer of several types is one call (gsq_linear_runs): `t` takes all its columns."""
 
     def __init__(self, t: torch.Tensor):
         self.t = t
