@@ -6,7 +6,7 @@ import torch
 import torch.utils._python_dispatch
 
 import gsq_b200  # noqa: F401
-from gsq_b200 import _gsq_ops, lcpp_ops, synth
+from gsq_b200 import _cabi, _gsq_ops, lcpp_ops, synth
 from gsq_b200.quantization import iq3_pack, linear
 
 TYPES = {**synth.TYPE_IDS, **synth.LOW_BIT_TYPE_IDS}
@@ -92,3 +92,30 @@ def test_output_into_of_a_fused_layer(m):
         with pytest.raises(RuntimeError, match="output_into"), lcpp_ops.output_into(bad):
             method.apply(layer, x)
     assert torch.equal(method.apply(layer, x), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,m", [("Q6_K", 128), ("IQ2_S", 64), ("IQ4_XS", 300)])
+def test_short_of_memory(name, m):
+    """Where the allocator has no room for expanded weights the product runs in the least scratch, with that form's result."""
+    t, rows, k = TYPES[name], 4096, 17408
+    w = torch.from_numpy(synth.make_weight(t, 64, k, 40)).cuda().repeat(rows // 64, 1)
+    if t in iq3_pack.PACKABLE_TYPES:
+        iq3_pack.pack_(w, t)
+    packed, x = t in iq3_pack.PACKABLE_TYPES, torch.from_numpy(synth.make_activation(m, k, 41)).to(torch.bfloat16).cuda()
+    lib = _cabi.lib
+    most, least = lib.gsq_linear_workspace_bytes(rows, m, k, t, packed), lib.gsq_linear_scratch_bytes(rows, m, k, t, packed)
+    assert most > (128 << 20) and least < (32 << 20)
+    want, scratch = torch.empty(m, rows, dtype=torch.bfloat16, device="cuda"), torch.empty(least, dtype=torch.uint8, device="cuda")
+    assert lib.gsq_linear(w.data_ptr(), w.shape[1], rows, t, packed, x.data_ptr(), _cabi.BF16, m, k, k, want.data_ptr(), _cabi.BF16, rows,
+                          scratch.data_ptr(), least, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (100 << 20)) / total)
+    try:
+        got = _gsq_ops.linear(x, w, t, None, packed)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got, want)
+    torch.testing.assert_close(_gsq_ops.linear(x, w, t, None, packed).float(), want.float(), rtol=2e-2, atol=2e-2 * want.float().abs().mean().item())
