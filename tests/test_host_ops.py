@@ -1,6 +1,9 @@
 """The native host path (module _gsq_ops): its routing against the Python table that is API, and on the GPU the fused
 layer of several runs against one product per run, direct calls against the custom ops."""
 
+import threading
+import time
+
 import pytest
 import torch
 import torch.utils._python_dispatch
@@ -36,6 +39,33 @@ def test_native_errors_are_python_exceptions():
         _gsq_ops.linear(x, w, 8, None, False)
     with pytest.raises(RuntimeError, match="must be CUDA tensors"):
         _gsq_ops.linear_runs(x[:4], w, [0, 16, 112, 29], False)
+
+
+def test_interpreter_runs_while_a_call_does():
+    """A native call lets other Python threads run (an unquantised product on the host stands in for one that waits)."""
+    x, w = torch.randn(512, 4096), torch.randn(4096, 4096)
+    state = {"done": False}
+
+    def work():
+        state["t"] = -time.perf_counter()
+        for _ in range(5):
+            _gsq_ops.linear(x, w, 0, None, False)
+        state["t"] += time.perf_counter()
+        state["done"] = True
+
+    old = torch.get_num_threads()
+    torch.set_num_threads(1)
+    try:
+        thread, ticks = threading.Thread(target=work), 0
+        thread.start()
+        while not state["done"]:
+            time.sleep(1e-3)
+            ticks += 1
+        thread.join()
+    finally:
+        torch.set_num_threads(old)
+    # one tick a millisecond or so where the interpreter is free, about one per call (of 5) where it is not
+    assert state["t"] < 0.1 or ticks > 20, (state["t"], ticks)
 
 
 def _fused_layer(names, rows, k):

@@ -439,10 +439,13 @@ void implement_vllm(const std::string& name) {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("implement", &implement);
   m.def("implement_vllm", &implement_vllm);
-  m.def("linear", &linear);
-  m.def("linear_runs", [](const Tensor& x, const Tensor& w, const std::vector<int64_t>& runs, bool packed) { return linear_runs(x, w, runs, packed); });
-  m.def("rmsnorm_quantize", &rmsnorm_quantize);
-  m.def("silu_mul_quantize", &silu_mul_quantize);
+  // The calls that launch let go of the interpreter, as the custom ops do: the allocator may wait for the driver in them.
+  using free_interpreter = pybind11::call_guard<pybind11::gil_scoped_release>;
+  m.def("linear", &linear, free_interpreter());
+  m.def("linear_runs", [](const Tensor& x, const Tensor& w, const std::vector<int64_t>& runs, bool packed) { return linear_runs(x, w, runs, packed); },
+        free_interpreter());
+  m.def("rmsnorm_quantize", &rmsnorm_quantize, free_interpreter());
+  m.def("silu_mul_quantize", &silu_mul_quantize, free_interpreter());
   m.def("route", [](int64_t n, int64_t type, int64_t rows, int64_t k, bool packed) -> std::optional<std::string> {
     const int op = route(n, type, rows, k, packed);
     return op < 0 ? std::nullopt : std::optional<std::string>(kSpec[op].name);
