@@ -78,6 +78,32 @@ def _fused_layer(names, rows, k):
     return layer, method
 
 
+def test_a_layer_is_read_at_every_call(monkeypatch):
+    """apply() follows a layer whose types or shard map change after its first call."""
+    layer, method, calls = torch.nn.Module(), linear.GGUFLinearMethod(None), []
+    method.create_weights(layer, 512, [32, 16, 16], 512, 64, torch.bfloat16)
+    for sid, rows in zip("qkv", (32, 16, 16)):
+        layer.weight.load_shard(torch.zeros(rows, 512 // 256 * 144, dtype=torch.uint8), sid)
+        layer.weight_type.shard_weight_type[sid] = 12
+    layer.weight_type.shard_weight_type["v"] = 23
+    method._create_padded_weight_param(layer)
+    monkeypatch.setattr(linear, "fused_mul_mat_gguf", lambda x, w, t, *a: calls.append(t) or x)
+    monkeypatch.setattr(torch.ops._C_gguf, "gsq_linear_runs", lambda x, w, runs, packed: calls.append(runs) or x, raising=False)
+    x, w, size = torch.zeros(1, 512, dtype=torch.bfloat16), layer.weight, 288
+    assert w.shard_offset_map == {"q": (0, 32, size), "k": (32, 48, size), "v": (48, 64, size)}
+    method.apply(layer, x)
+    layer.weight_type.shard_weight_type["k"] = 23          # another type of one shard
+    method.apply(layer, x)
+    w.shard_offset_map["v"] = (48, 56, size)               # another shard map
+    method.apply(layer, x)
+    layer.weight_type.shard_weight_type.update(q=12, k=12, v=12)
+    method.apply(layer, x)
+    w.shard_id = []                                        # one product of the layer's own type
+    layer.weight_type.weight_type = 21
+    method.apply(layer, x)
+    assert calls == [[0, 48, size, 12, 48, 16, size, 23], [0, 32, size, 12, 32, 32, size, 23], [0, 32, size, 12, 32, 24, size, 23], 12, 21]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m", [1, 4, 8, 9, 40, 70])
 @pytest.mark.parametrize("names", [("IQ3_S", "IQ3_S", "Q6_K"), ("Q4_K", "IQ4_XS", "Q4_K"), ("IQ3_S", "IQ2_XS", "Q2_K")])

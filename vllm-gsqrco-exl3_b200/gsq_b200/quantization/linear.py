@@ -30,7 +30,7 @@ import torch
 
 from .. import _gsq_ops, ops
 from . import iq3_pack
-from .params import GGUFWeightParameter, GGUFWeightTypeParameter, _gguf_ordered_shard_ids
+from .params import _QKV_ORDER, GGUFWeightParameter, GGUFWeightTypeParameter, _gguf_ordered_shard_ids
 
 Q2_K, Q4_K, Q6_K = ops.GGML_TYPE_Q2_K, ops.GGML_TYPE_Q4_K, ops.GGML_TYPE_Q6_K
 IQ2_S, IQ3_S, IQ3_XXS = ops.GGML_TYPE_IQ2_S, ops.GGML_TYPE_IQ3_S, ops.GGML_TYPE_IQ3_XXS
@@ -318,38 +318,36 @@ class GGUFLinearMethod:
         layer.register_parameter("weight", new)
 
     @staticmethod
-    def _plan(layer: torch.nn.Module, weight) -> tuple:
+    def _products(layer: torch.nn.Module, weight) -> tuple:
         """(type, None) of a layer that is one product, (None, runs) of one that is several, runs = start row, rows, row
         bytes and type of each in one flat list (gsq_linear_runs), or (None, None) if one of them is not quantised.
-        Worked out at the first call on a weight and kept with it."""
-        shard_id = weight.shard_id
+        Read from the layer at every call: its types and its shard map may change between two (1 us)."""
+        shard_id, types = weight.shard_id, layer.weight_type
+        fallback = types.weight_type
         if not shard_id:
-            return layer.weight_type.weight_type, None
-        shard_id = ["q", "k", "v"] if "q" in shard_id else shard_id
-        fallback = layer.weight_type.weight_type
-        types = [layer.weight_type.shard_weight_type.get(i, fallback) for i in shard_id]
-        if len(set(types)) == 1:
-            return types[0], None
-        if any(t in ops.UNQUANTIZED_TYPES for t in types) or not weight.is_contiguous():
-            return None, None
-        runs, offsets = [], weight.shard_offset_map
-        for t, run in groupby(zip(shard_id, types), key=lambda p: p[1]):
-            ids = [i for i, _ in run]
-            start, _, size = offsets[ids[0]]
-            runs += [start, offsets[ids[-1]][1] - start, size, t]
-        return None, runs
+            return fallback, None
+        ids, types = _QKV_ORDER if "q" in shard_id else shard_id, types.shard_weight_type
+        kinds = [types.get(i, fallback) for i in ids]
+        if kinds.count(kinds[0]) == len(kinds):
+            return kinds[0], None
+        runs, last, offsets = [], None, weight.shard_offset_map
+        for sid, t in zip(ids, kinds):
+            start, end, size = offsets[sid]
+            if t == last:
+                runs[-3] = end - runs[-4]
+            elif t in ops.UNQUANTIZED_TYPES:
+                return None, None
+            else:
+                runs += (start, end - start, size, t)
+                last = t
+        return None, runs if weight.is_contiguous() else None
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         if self.layout is not None:
             x = self.layout.input_to_gguf(x)
         weight = layer.weight
         packed = getattr(weight, "iq3_packed", False)
-        plan = getattr(weight, "gsq_plan", None)
-        if plan is None:
-            plan = self._plan(layer, weight)
-            if weight.numel():
-                weight.gsq_plan = plan
-        weight_type, runs = plan
+        weight_type, runs = self._products(layer, weight)
         # a plain CUDA tensor and nobody tracing or intercepting: straight to the native code under the custom ops
         direct = type(x) is torch.Tensor and x.is_cuda and not torch.compiler.is_compiling() and not torch._C._len_torch_dispatch_stack()
         if weight_type is not None:
