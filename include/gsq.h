@@ -252,8 +252,10 @@ int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, in
 
 /*
  * How gsq_linear forms the prefill product of repacked IQ3_S, of IQ4_XS and of Q4_K (256 tokens and up, 128 on tall
- * weights). Q6_K, IQ3_S in GGUF order and the low-bit types have the accuracy of the split form in the first two modes
- * and their small-batch kernels' integer sums in the third; the other routes are not affected.
+ * weights). Q6_K, IQ3_S in GGUF order, Q2_K and IQ1_M keep exact integer slice sums in every mode, at many rows by the GEMM
+ * in the first two and by repeated launches of their small-batch kernels in the third. IQ2_XXS, IQ2_XS, IQ2_S and IQ3_XXS
+ * have the accuracy of the split form at many rows in the first two modes (their small-batch kernels truncate integer
+ * divisions as the reference's do, 1e-5 .. 5e-5) and those kernels' sums in the third. The other routes are not affected.
  * The reference's kernels keep an exact int32 sum per 32-value slice and scale it in fp32
  * (lcpp_owned_iq3_mma.cu:768-970, mmq.cuh:961-1385). Sets the mode, returns the previous one:
  *   GSQ_PREFILL_ROUNDED (default)  d_x * q goes into the tensor-core operand as one fp16 number and tensor memory

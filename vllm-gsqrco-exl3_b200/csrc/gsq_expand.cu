@@ -32,8 +32,8 @@ struct ExpandArgs {
   int n_items;    // half row tiles x superblocks
   int nsb;
   uint8_t* a;     // [row tile][k-block][plane][16 KB]
-  float* dw;      // [row tile][superblock][128]
-  uint8_t* ta;    // [row tile][superblock][plane][4096]
+  float *dw, *dm; // [row tile][superblock][128]
+  uint8_t* ta;    // [row tile][superblock][4096]
 };
 
 constexpr int XROWS = 64, XTHREADS = 256;
@@ -308,9 +308,10 @@ __device__ __forceinline__ void x_q6k(const uint8_t* s, uint8_t* out, int r, int
 
 // The low-bit types: decoded by the codec they share with the dp4a kernel and the row dequantiser. Factor per row and
 // superblock: the truncating integer divisions of the reference's small-row kernels (its many-row kernels scale in
-// floating point, as here) become the exact fractions d / 8, d / 4.
+// floating point, as here) become the exact fractions d / 8, d / 4. (The truncation is 1e-5 to 5e-5 of a result's norm, so
+// a type's results change by that where its rows pass from the one kernel to the other, and are nearer to 64 bits above.)
 template <int F1>
-__device__ __forceinline__ void x_f1(const uint8_t* s, uint8_t* out, int r, int kb, float* dw, uint8_t* ta) {
+__device__ __forceinline__ void x_f1(const uint8_t* s, uint8_t* out, int r, int kb, float* dw, float* dm, uint8_t* ta) {
 #pragma unroll
   for (int sl = 0; sl < 2; ++sl) {
     Raw<F1> raw;
@@ -322,9 +323,8 @@ __device__ __forceinline__ void x_f1(const uint8_t* s, uint8_t* out, int r, int 
     else if (F1 == F1_IQ2XS || F1 == F1_IQ2S) { f0 = 2 * v.p0 + 1; f1 = 2 * v.p1 + 1; }
     else { f0 = v.p0; f1 = v.p1; }
     if constexpr (F1 == F1_Q2K) {
-      // (d / sigma) * sc is the integer sc unless the minimums dwarf the scale
-      const float sigma = sigma_of(raw.r[9]), ratio = v.d / sigma;
-      const __half h0 = __float2half_rn(ratio * (float)f0), h1 = __float2half_rn(ratio * (float)f1);
+      // 0..3 under the high byte 0x64: (1024 + value) * sc - 1024 * sc, exact
+      const __half h0 = __int2half_rn(f0), h1 = __int2half_rn(f1);
       const __half2 m0 = __half2half2(h0), m1 = __half2half2(h1);
       const __half2 n0 = __half2half2(__hmul(__float2half_rn(-1024.0f), h0)), n1 = __half2half2(__hmul(__float2half_rn(-1024.0f), h1));
 #pragma unroll
@@ -335,15 +335,12 @@ __device__ __forceinline__ void x_f1(const uint8_t* s, uint8_t* out, int r, int 
             make_uint4(x_hfma2(prmt(a, 0x64646464u, 0x4140u), f, nb), x_hfma2(prmt(a, 0x64646464u, 0x4342u), f, nb),
                        x_hfma2(prmt(b, 0x64646464u, 0x4140u), f, nb), x_hfma2(prmt(b, 0x64646464u, 0x4342u), f, nb));
       }
-      // minimum terms of the two 16-value groups, hi and lo: -(dmin / sigma) * m * 16
-      const float fm = -16.0f * v.dmin / sigma;
-      const float ma = fm * (float)v.p2, mb = fm * (float)v.p3;
-      const __half2 hi = __floats2half2_rn(ma, mb);
-      const float2 back = __half22float2(hi);
-      uint8_t* t = ta + (kb >> 1) * 128 + (kb & 1) * 8 + 4 * sl;
-      *reinterpret_cast<__half2*>(t) = hi;
-      *reinterpret_cast<__half2*>(t + 4096) = __floats2half2_rn(ma - back.x, mb - back.y);
-      if (kb == 0 && sl == 0) *dw = sigma;
+      // the minimums of the two 16-value groups, against the sums of their quants; -dmin scales them
+      *reinterpret_cast<__half2*>(ta + (kb >> 1) * 128 + (kb & 1) * 8 + 4 * sl) = __halves2half2(__int2half_rn(v.p2), __int2half_rn(v.p3));
+      if (kb == 0 && sl == 0) {
+        *dw = v.d;
+        *dm = -v.dmin;
+      }
     } else {
       const Sub s0(f0), s1(f1);
 #pragma unroll
@@ -418,7 +415,8 @@ __global__ void __launch_bounds__(XTHREADS) expand_kernel(const ExpandArgs g) {
     __syncthreads();
     const int ht = item / g.nsb, sb = item - ht * g.nsb, rt = ht >> 1, half = ht & 1;
     float* const dw = g.dw + ((int64_t)rt * g.nsb + sb) * TR + half * XROWS;
-    uint8_t* const ta = TP ? g.ta + ((int64_t)rt * g.nsb + sb) * (TP * 4096) + half * (XROWS / 8 * 256) : nullptr;
+    float* const dm = KIND == K_Q2K ? g.dm + (dw - g.dw) : nullptr;
+    uint8_t* const ta = TP ? g.ta + ((int64_t)rt * g.nsb + sb) * 4096 + half * (XROWS / 8 * 256) : nullptr;
     if constexpr (x_packed(KIND)) {
       const int rec = warp >> 1, hf = warp & 1;
       if (ht * XROWS + 16 * rec < g.nrows) {
@@ -448,15 +446,14 @@ __global__ void __launch_bounds__(XTHREADS) expand_kernel(const ExpandArgs g) {
         else if (KIND == K_IQ3S) x_iq3s(s, out, grid, r, kb, dw + r);
         else if (KIND == K_Q6K) x_q6k(s, out, r, kb, dw + r);
         else x_f1<KIND == K_Q2K ? F1_Q2K : KIND == K_IQ2XXS ? F1_IQ2XXS : KIND == K_IQ2XS ? F1_IQ2XS : KIND == K_IQ2S ? F1_IQ2S
-                  : KIND == K_IQ3XXS ? F1_IQ3XXS : F1_IQ1M>(s, out, r, kb, dw + r, tar);
+                  : KIND == K_IQ3XXS ? F1_IQ3XXS : F1_IQ1M>(s, out, r, kb, dw + r, dm + r, tar);
       } else {
         for (int pln = 0; pln < AP; ++pln)
 #pragma unroll
           for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(out + out_at(kb, pln, AP, r, c)) = make_uint4(0, 0, 0, 0);
         if (kb == 0) dw[r] = 0.0f;
-        for (int pln = 0; pln < TP; ++pln) {
-          if (kb < 2) *reinterpret_cast<uint4*>(tar + pln * 4096 + kb * 128) = make_uint4(0, 0, 0, 0);
-        }
+        if (KIND == K_Q2K && kb == 0) dm[r] = 0.0f;
+        if (TP && kb < 2) *reinterpret_cast<uint4*>(tar + kb * 128) = make_uint4(0, 0, 0, 0);
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -516,6 +513,7 @@ int expand_host(const Plan& p, const uint8_t* w, int64_t row_bytes, int64_t rows
   g.n_items = (int)((rows + 255) / 256 * 4) * p.nsb;
   g.a = scratch + p.a;
   g.dw = reinterpret_cast<float*>(scratch + p.dw);
+  g.dm = reinterpret_cast<float*>(scratch + p.dm);
   g.ta = scratch + p.ta;
   switch (p.kind) {
     case K_Q4K: return launch_expand<K_Q4K>(g, sm_count, st);

@@ -17,29 +17,17 @@
 // share both operands in L2. Every wait is bounded and raises the device flag instead of hanging.
 #include <cuda_fp16.h>
 
+#include "gsq_pair.cuh"
 #include "gsq_planes.cuh"
-#include "gsq_tc.cuh"
 
 namespace gsq {
 namespace pl {
 
-using namespace tc;
-
-constexpr int G_THREADS = 384;
-constexpr int CONS_WARP0 = 4, CONS_WARPS = 8;
-constexpr int IDLE_REGS = 40, CONS_REGS = 232;   // 128 x 40 + 256 x 232 = the 384 x 168 the block is launched with
-constexpr int MAX_STAGES = 8;
-constexpr int G_TMEM = 512;
-constexpr int SMEM_HEAD = 1024;                  // barriers; the stages start 1024-byte aligned
-constexpr int SMEM_MAX = 227 * 1024;
-constexpr int ROW_GROUP = 8;                     // row tiles of a rasterisation group
 constexpr int MODEL_PAIRS = 74;                  // pairs of SMs the plan is made for
 
 // k-blocks per stage: 128 values of K of the one-plane form, so that the MMA warp's waits and commits (about 400 cycles)
-// stay behind the 1024 cycles of tensor work they belong to; 64 values of the others, which have two or three MMAs for each
+// stay behind the 1024 cycles of tensor work they belong to; 64 values of the other, which has two MMAs for each
 __host__ __device__ constexpr int stage_kblocks(int hu) { return hu == 1 ? 2 : 1; }
-
-__device__ int g4_error = 0;
 
 struct GemmArgs {
   const uint8_t *a, *ta, *b, *tb;
@@ -53,88 +41,6 @@ struct GemmArgs {
   float* part;
   int stages;
 };
-
-struct Cursor {
-  uint32_t i, ph;
-  __device__ __forceinline__ void next(uint32_t n) {
-    if (++i == n) { i = 0; ph ^= 1u; }
-  }
-};
-
-// Bounded: gives up about a second after the first failed try (SM clocks; the global timer takes about a microsecond to
-// read), or when another thread of the CTA has. The hardware suspends a waiting thread inside try_wait.
-__device__ __forceinline__ bool try_bar(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (try_bar(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (int spin = 1; spin < (1 << 28); ++spin) {
-    if (try_bar(bar, parity)) return true;
-    if ((spin & 15) == 0 && (*abort_flag || clock64() - t0 > 2000000000ll)) break;
-  }
-  if (!*abort_flag) {
-    *abort_flag = 1;
-    atomicExch(&g4_error, 1);
-  }
-  return false;
-}
-
-// Arrival on a barrier of the other CTA. No cluster-scope release: it would wait for every outstanding store of the SM
-// (about 1000 cycles under this kernel's traffic, on every stage), and nothing here is handed over through ordinary
-// stores -- what the waiting side uses are bytes that bulk copies have landed and tensor-memory reads that have completed.
-__device__ __forceinline__ void arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-
-// K-major tile of 8-row groups of 1024 bytes under the 128-byte swizzle; one MMA (K = 16) takes 32 bytes of a row, the
-// next one starts 32 bytes further
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
-  uint64_t d = (uint64_t)((addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-__device__ __forceinline__ bool elect_one() {
-  uint32_t r;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
-  return r != 0;
-}
-// the MMAs issued so far have completed -> one arrival on the barrier at this offset in each CTA of the pair
-__device__ __forceinline__ void commit_both(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
-      "%28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-        "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-        "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-}
-// what follows may not use the loaded registers before this point (the wait above it)
-__device__ __forceinline__ void pin32(uint32_t* v) {
-#pragma unroll
-  for (int i = 0; i < 32; i += 8)
-    asm volatile("" : "+r"(v[i]), "+r"(v[i + 1]), "+r"(v[i + 2]), "+r"(v[i + 3]), "+r"(v[i + 4]), "+r"(v[i + 5]), "+r"(v[i + 6]), "+r"(v[i + 7]));
-}
 
 // A row's n tokens (32 lanes: 32 neighbouring rows); lane l holds the reciprocal scales of tokens 4 l .. 4 l + 3.
 template <typename T>
@@ -154,14 +60,14 @@ __device__ __forceinline__ void store_tokens(T* y, int64_t ldy, const float2 (&a
   }
 }
 
-template <int HU, int AP, int TP>
+template <int HU, int TP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1) gemm4_kernel(const GemmArgs g) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t crank = cluster_ctarank();
   const int nth = g.nt >> 1;
   constexpr int KS = stage_kblocks(HU);
-  const uint32_t b_plane = (uint32_t)nth * (KB * 2), b_bytes = HU * b_plane, a_bytes = AP * A_TILE;   // of one k-block
+  const uint32_t b_plane = (uint32_t)nth * (KB * 2), b_bytes = HU * b_plane, a_bytes = A_TILE;   // of one k-block
   const uint32_t ta_bytes = TP * 4096, tb_bytes = (uint32_t)(TP * nth * 32);
   const uint32_t b_off = KS * a_bytes, t_off = b_off + KS * b_bytes, stage_bytes = t_off + (TP ? TP * 8192 : 0);
   const int n_stages = g.stages;
@@ -194,17 +100,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1) gemm4_
 
   const int pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
   const int n_items = g.n_rp * g.n_tb * g.splits, nkb = 4 * g.nsb;
-  // item -> tile and its superblocks [sb0, sb1); the parts of a tile run side by side
-  auto place = [&](int item, int& rp, int& tb, int& sb0, int& sb1) {
-    const int split = g.splits > 1 ? item % g.splits : 0;
-    if (g.splits > 1) item /= g.splits;
-    sb0 = split * g.nsb / g.splits;
-    sb1 = (split + 1) * g.nsb / g.splits;
-    const int per = ROW_GROUP * g.n_tb, grp = item / per, rem = item - grp * per;
-    const int in_grp = min(ROW_GROUP, g.n_rp - grp * ROW_GROUP);
-    tb = rem / in_grp;
-    rp = grp * ROW_GROUP + rem - tb * in_grp;
-  };
+  auto place = [&](int item, int& rp, int& tb, int& sb0, int& sb1) { place_item(item, g.splits, g.nsb, g.n_tb, g.n_rp, rp, tb, sb0, sb1); };
   // the operands are written by the kernels before this one
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
@@ -296,12 +192,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1) gemm4_
             if (one) {
               uint32_t acc = kb > 0 ? 1u : 0u;
               if (TP && kb == 0) {
-                const uint32_t ta = as + t_off, tb = ta + ta_bytes, tp = (uint32_t)nth * 32;
+                const uint32_t ta = as + t_off, tb = ta + ta_bytes;
                 mma_f16_pair(d, smem_desc(ta, 128, 256), smem_desc(tb, 128, 256), id, 0u);
-                if (TP == 2) {
-                  mma_f16_pair(d, smem_desc(ta, 128, 256), smem_desc(tb + tp, 128, 256), id, 1u);
-                  mma_f16_pair(d, smem_desc(ta + 4096, 128, 256), smem_desc(tb, 128, 256), id, 1u);
-                }
                 acc = 1u;
               }
               if (HU == 1) {
@@ -320,10 +212,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1) gemm4_
                   mma_f16_pair(d, ad + 4 * s + 2, bd + 4 * s + 2, id, 1u);
                   mma_f16_pair(d, ad + 4 * s, bl + 4 * s, id, 1u);
                   mma_f16_pair(d, ad + 4 * s + 2, bl + 4 * s + 2, id, 1u);
-                }
-                if (AP == 2) {
-#pragma unroll
-                  for (int k = 0; k < 4; ++k) mma_f16_pair(d, ad + (A_TILE >> 4) + 2 * k, bd + 2 * k, id, 1u);
                 }
               }
               commit_both(empty + 8 * c.i);
@@ -405,48 +293,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1) gemm4_
 // ---------------------------------------------------------------------------------------------
 
 static int stage_bytes_of(const Plan& p) {
-  return stage_kblocks(p.hu) * (a_planes(p.kind) * A_TILE + p.hu * (p.nt / 2) * KB * 2) + t_planes(p.kind) * 8192;
+  return stage_kblocks(p.hu) * (A_TILE + p.hu * (p.nt / 2) * KB * 2) + t_planes(p.kind) * 8192;
 }
 
-template <int HU, int AP, int TP>
+template <int HU, int TP>
 static int launch_gemm4(GemmArgs& g, int stage, int sm_count, cudaStream_t st) {
   static int max_pairs[64];
-  int dev = 0;
-  GSQ_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return GSQ_ERR_UNSUPPORTED;
-  auto kern = gemm4_kernel<HU, AP, TP>;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(G_THREADS);
-  cfg.stream = st;
-  if (!max_pairs[dev]) {
-    GSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-    // how many pairs the device runs at once (an SM without a free neighbour in its GPC stays out)
-    cudaLaunchAttribute ca;
-    ca.id = cudaLaunchAttributeClusterDimension;
-    ca.val.clusterDim.x = 2;
-    ca.val.clusterDim.y = 1;
-    ca.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2u * (unsigned)sm_count);
-    cfg.dynamicSmemBytes = SMEM_MAX;
-    cfg.attrs = &ca;
-    cfg.numAttrs = 1;
-    int n = 0;
-    GSQ_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
-    if (n < 1) return GSQ_ERR_UNSUPPORTED;
-    max_pairs[dev] = n;
-  }
-  const int items = g.n_rp * g.n_tb * g.splits, pairs = items < max_pairs[dev] ? items : max_pairs[dev];
   g.stages = (SMEM_MAX - SMEM_HEAD) / stage;
   if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
-  cfg.gridDim = dim3(2u * (unsigned)pairs);
-  cfg.dynamicSmemBytes = SMEM_HEAD + g.stages * stage;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, g));
-  return GSQ_OK;
+  return launch_pairs(gemm4_kernel<HU, TP>, G_THREADS, g, max_pairs, (int64_t)g.n_rp * g.n_tb * g.splits, SMEM_HEAD + g.stages * stage, sm_count, st);
 }
 
 static int gemm4_launch(const Plan& p, uint8_t* scratch, int64_t rows, int64_t m, void* y, int y_dtype, int64_t ldy, int sm_count,
@@ -470,10 +325,8 @@ static int gemm4_launch(const Plan& p, uint8_t* scratch, int64_t rows, int64_t m
   g.splits = p.splits;
   g.part = (float*)(scratch + p.part);
   const int stage = stage_bytes_of(p);
-  if (a_planes(p.kind) == 2) return launch_gemm4<2, 2, 0>(g, stage, sm_count, st);
-  if (t_planes(p.kind) == 2) return launch_gemm4<2, 1, 2>(g, stage, sm_count, st);
-  if (t_planes(p.kind) == 1) return launch_gemm4<1, 1, 1>(g, stage, sm_count, st);
-  return p.hu == 2 ? launch_gemm4<2, 1, 0>(g, stage, sm_count, st) : launch_gemm4<1, 1, 0>(g, stage, sm_count, st);
+  if (t_planes(p.kind)) return launch_gemm4<1, 1>(g, stage, sm_count, st);
+  return p.hu == 2 ? launch_gemm4<2, 0>(g, stage, sm_count, st) : launch_gemm4<1, 0>(g, stage, sm_count, st);
 }
 
 // y = the sum of the parts, in their order; a thread takes one result of every part. Tokens are the grid's x: a prompt may
@@ -514,14 +367,22 @@ static int sum_parts(const Plan& p, const uint8_t* scratch, int64_t rows, int64_
 // superblock's drain, stores); waves are whole. Splitting K writes and reads fp32 partial sums: 5000 for the extra kernel
 // and their bytes at 2 KB per cycle.
 static void choose_tiles(Plan* p, int64_t n_rp, int64_t rows, int64_t m) {
-  const int ap = a_planes(p->kind), products = ap == 2 ? 3 : p->hu;
+  const bool ints = int_sums(p->kind);
+  const int ap = a_planes(p->kind), hu = ints ? 1 : p->hu, products = ints ? ap : hu, max_nt = !ints ? MAX_NT : int_comp(p->kind) ? INT_NT_COMP : INT_NT;
+  const int parts = ints && !int_comp(p->kind) ? (p->nsb + INT_PART - 1) / INT_PART : 1;   // the least
   double best = 1e300;
-  const int64_t first = (m + MAX_NT - 1) / MAX_NT;
+  const int64_t first = (m + max_nt - 1) / max_nt;
   for (int64_t b = first; b <= first + 8 && (b == first || (m + b - 1) / b >= 48); ++b) {
     const int64_t t = ((m + b - 1) / b + 15) / 16 * 16, blocks = (m + t - 1) / t;
-    const double mma = 2.0 * t * products, load = (ap * 16384.0 + p->hu * 64.0 * t) / 40.0;
-    const double kblock = (mma > load ? mma : load) + 20.0;
-    for (int s = 1; s <= 8 && (s == 1 || p->nsb / s >= 4); ++s) {
+    double kblock = 2.0 * t * products, load = ap * 16384.0 + hu * 64.0 * t;
+    if (ints) {
+      // the chain of a k-block through the consumers (Q2_K: twice), and their scales
+      const double cons = (1 + t_planes(p->kind)) * (2.5 * t + 900.0);
+      kblock = cons > kblock ? cons : kblock;
+      load += 8.0 * t + t_planes(p->kind) * (1024.0 + 32.0 * t);
+    }
+    kblock = (kblock > load / 40.0 ? kblock : load / 40.0) + 20.0;
+    for (int s = parts; s <= (parts > 8 ? parts : 8) && (s == parts || p->nsb / s >= 4); ++s) {
       const double waves = (double)((n_rp * blocks * s + MODEL_PAIRS - 1) / MODEL_PAIRS);
       double cost = waves * (4.0 * ((p->nsb + s - 1) / s) * kblock + 4000.0);
       if (s > 1) cost += 5000.0 + (double)s * m * rows * 8.0 / 2048.0;
@@ -538,16 +399,17 @@ static void choose_tiles(Plan* p, int64_t n_rp, int64_t rows, int64_t m) {
 int make_plan(Plan* p, int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu) {
   p->kind = kind_of(ggml_type, packed, rows);
   if (p->kind == K_NONE || rows <= 0 || m <= 0 || k <= 0 || k % 256 != 0) return GSQ_ERR_UNSUPPORTED;
-  if (form_of(p->kind) == F_Q81) hu = 2;
+  const bool ints = int_sums(p->kind);
+  if (form_of(p->kind) == F_Q81) hu = ints ? 0 : 2;
   if (p->kind == K_Q4K) hu = 1;
   p->hu = hu;
   p->nsb = (int)(k / 256);
   p->nkb = 4 * p->nsb;
   const int ap = a_planes(p->kind), tp = t_planes(p->kind);
   const int64_t rows_pad = (rows + 255) / 256 * 256;
-  // the expanded weights of a call are bounded (512 MB); taller ones go a chunk of rows at a time
-  const int64_t per_row = (int64_t)ap * k * 2;
-  int64_t chunk = ((int64_t)512 << 20) / per_row / 256 * 256;
+  // the expanded weights of a call (with the least of partial sums) are bounded (512 MB); taller ones go a chunk of rows at a time
+  const int64_t per_row = (int64_t)ap * k * 2, parts = ints && !int_comp(p->kind) ? (p->nsb + INT_PART - 1) / INT_PART : 1;
+  int64_t chunk = ((int64_t)512 << 20) / (per_row + (parts > 1 ? parts * m * 4 : 0)) / 256 * 256;
   if (chunk < 256) chunk = 256;
   p->chunk_rows = rows_pad < chunk ? rows_pad : chunk;
   choose_tiles(p, p->chunk_rows / 256, p->chunk_rows < rows ? p->chunk_rows : rows, m);
@@ -558,14 +420,18 @@ int make_plan(Plan* p, int ggml_type, int packed, int64_t rows, int64_t m, int64
   at = up(at + c * (size_t)per_row);
   p->dw = at;
   at = up(at + c * p->nsb * 4);
+  p->dm = at;
+  if (ints && tp) at = up(at + c * p->nsb * 4);
   p->ta = at;
   at = up(at + (size_t)tp * c * p->nsb * 32);
   p->b = at;
-  at = up(at + (size_t)p->hu * tokens * (size_t)k * 2);
+  at = up(at + (size_t)(ints ? 1 : p->hu) * tokens * (size_t)k * 2);
   p->tb = at;
-  at = up(at + (size_t)tp * tokens * p->nsb * 32);
+  at = up(at + (size_t)tp * tokens * p->nsb * 32 * (ints ? 8 : 1));
   p->inv = at;
-  at = up(at + tokens * 4);
+  if (!ints) at = up(at + tokens * 4);
+  p->dx = at;
+  if (ints) at = up(at + tokens * (size_t)(k / 32) * 4);
   p->part = at;
   if (p->splits > 1) at = up(at + (size_t)p->splits * m * (size_t)(p->chunk_rows < rows ? p->chunk_rows : rows) * 4);
   p->total = at;
@@ -574,12 +440,18 @@ int make_plan(Plan* p, int ggml_type, int packed, int64_t rows, int64_t m, int64
 
 int planes_host(const Plan& p, const void* x, int x_dtype, int64_t m, int64_t k, int64_t stride, uint8_t* scratch, cudaStream_t st);
 int expand_host(const Plan& p, const uint8_t* w, int64_t row_bytes, int64_t rows, uint8_t* scratch, int sm_count, cudaStream_t st);
+int gemm6_launch(const Plan& p, uint8_t* scratch, int64_t rows, int64_t m, void* y, int y_dtype, int64_t ldy, int sm_count, cudaStream_t st);
 
 }  // namespace pl
 
+int gemm6_error_flag(int* flag);   // gsq_gemm6.cu
+
 int gemm4_error_flag(int* flag) {
-  GSQ_CUDA_TRY(cudaMemcpyFromSymbol(flag, pl::g4_error, sizeof(int)));
-  return GSQ_OK;
+  int a = 0, b = 0;
+  GSQ_CUDA_TRY(cudaMemcpyFromSymbol(&a, pl::pair_error, sizeof(int)));
+  const int rc = gemm6_error_flag(&b);
+  *flag = a | b;
+  return rc;
 }
 
 bool gemm4_applies(int ggml_type, int packed, int64_t rows) { return pl::kind_of(ggml_type, packed, rows) != pl::K_NONE; }
@@ -605,7 +477,9 @@ int gemm4_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, 
   for (int64_t r0 = 0; r0 < rows && rc == GSQ_OK; r0 += p.chunk_rows) {
     const int64_t n = rows - r0 < p.chunk_rows ? rows - r0 : p.chunk_rows;
     rc = pl::expand_host(p, (const uint8_t*)w + r0 * row_bytes, row_bytes, n, (uint8_t*)scratch, di.sm_count, st);
-    if (rc == GSQ_OK) rc = pl::gemm4_launch(p, (uint8_t*)scratch, n, m, (uint8_t*)y + r0 * ysz, y_dtype, y_row_stride, di.sm_count, st);
+    if (rc == GSQ_OK)
+      rc = (pl::int_sums(p.kind) ? pl::gemm6_launch : pl::gemm4_launch)(p, (uint8_t*)scratch, n, m, (uint8_t*)y + r0 * ysz, y_dtype, y_row_stride,
+                                                                        di.sm_count, st);
     if (rc == GSQ_OK && p.splits > 1) rc = pl::sum_parts(p, (const uint8_t*)scratch, n, m, (uint8_t*)y + r0 * ysz, y_dtype, y_row_stride, st);
   }
   return rc;

@@ -56,7 +56,7 @@ static bool ragged(int ggml_type, int packed, int64_t rows) {
 // The kernels of a product above the small-batch tensor-core kernel's rows (or of a type or shape it does not serve).
 enum Way {
   W_PLANES1,    // two steps, operands expanded to fp16: one plane of scaled activations (rounded)
-  W_PLANES2,    // the same with the activations as hi + lo: fp32 accuracy
+  W_PLANES2,    // the same at fp32 accuracy: the activations as hi + lo, or bare quants and integer slice sums (gsq_gemm6.cu)
   W_IQ3_INT,    // gsq_gemm3.cu: fp16 operands, integer slice sums
   W_I8,         // gsq_gemm2.cu: int8 prefill GEMM
   W_BATCH,      // gsq_gemm5.cu: up to 256 rows, int8 operands decoded in the kernel, work cut evenly over the SMs
@@ -90,7 +90,7 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, bool s
   }
   const bool q6 = ggml_type == GSQ_TYPE_Q6_K, q6_packed = q6 && packed && rows % 16 == 0;
   // Q6_K, IQ3_S in GGUF order and the low-bit types: the two steps once they cost less than the repeated launches of the
-  // small-batch kernels (48 or 8 rows each), at fp32 accuracy, unless integer sums are asked for.
+  // small-batch kernels (48 or 8 rows each), no less exact than those, unless they are asked for.
   if (!small && !dump && g_prefill_precision != GSQ_PREFILL_INTEGER && gemm4_applies(ggml_type, packed, rows) && m >= (q6_packed ? 97 : q6 || ggml_type == GSQ_TYPE_IQ3_S ? 25 : 9)) return W_PLANES2;
   return q6_packed ? W_MMV_LOOP : W_GEMV_LOOP;
 }

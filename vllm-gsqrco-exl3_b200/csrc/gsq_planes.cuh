@@ -1,4 +1,4 @@
-// Operand layout of the two-step tensor-core product (gsq_expand.cu -> gsq_planes.cu -> gsq_gemm4.cu) and the geometry all
+// Operand layout of the two-step tensor-core product (gsq_expand.cu, gsq_planes.cu -> gsq_gemm4.cu, gsq_gemm6.cu) and the geometry all
 // three agree on. Everything is fp16, K-major, in tiles of 64 values of K ("k-blocks", 4 per superblock), stored in
 // global memory exactly as the tensor cores read them from shared memory, so that a stage is filled by plain bulk copies:
 // 8-row groups of 1024 bytes, row r of a group at r * 128, its 16-byte chunk c (8 values) at ((c ^ r) * 16) -- the
@@ -18,11 +18,21 @@ constexpr int TR = 128;         // weight rows of a tile (one CTA of a pair)
 constexpr int KB = 64;          // values of K per k-block
 constexpr int A_TILE = TR * KB * 2;
 constexpr int MAX_NT = 256;     // most tokens of a block
+constexpr int INT_NT = 128;     // the same of the form with integer slice sums (gsq_gemm6.cu)
+constexpr int INT_NT_COMP = 64; // ... where the sum over K carries its rounding error along
+constexpr int INT_PART = 12;    // most superblocks that it adds up in one sum, where that does not carry its error along
 
 // fp16 planes of the weight operand: 2 for Q6_K, whose sub-scale times value reaches 4096 and needs 13 bits
 __host__ __device__ constexpr int a_planes(int kind) { return kind == K_Q6K || kind == K_Q6K_PACKED ? 2 : 1; }
-// planes of per-superblock extra columns (16 of them): Q4_K's minimum and correction terms, Q2_K's minimum terms as a pair
-__host__ __device__ constexpr int t_planes(int kind) { return kind == K_Q4K ? 1 : kind == K_Q2K ? 2 : 0; }
+// planes of per-superblock extra columns (16 of them): Q4_K's minimum and correction terms, Q2_K's minimums
+__host__ __device__ constexpr int t_planes(int kind) { return kind == K_Q4K || kind == K_Q2K ? 1 : 0; }
+// Types whose kernels of few rows keep exact integer sums up to the fp32 scaling: so does their two-step product
+// (gsq_gemm6.cu). Error against 64 bits, 2-norm over 1024 to 17408 columns: scaled products in two planes 4e-7 to 7e-7, the
+// kernels of few rows 0.7e-7 to 1.1e-7. (The other low-bit types' few-row kernels truncate integer divisions as the
+// reference's do, 1e-5 to 5e-5: two planes, 6e-7, are the more exact.)
+__host__ __device__ constexpr bool int_sums(int kind) {
+  return kind == K_Q6K || kind == K_Q6K_PACKED || kind == K_IQ3S || kind == K_Q2K || kind == K_IQ1M;
+}
 
 // (repacked weights: whole 16-row records, which the expanding kernel reads and writes as such; Q4_K and IQ4_XS have one
 // layout, whatever the flag says, as in the kernels of fewer rows)
@@ -41,7 +51,8 @@ inline int kind_of(int ggml_type, int packed, int64_t rows) {
     case GSQ_TYPE_IQ1_M: return packed ? K_NONE : K_IQ1M;
     default: return K_NONE;
   }
-}
+}// ... with a sum over K that carries its rounding error along: the types whose kernel of few rows is the most exact
+__host__ __device__ constexpr bool int_comp(int kind) { return kind == K_Q2K || kind == K_IQ1M; }
 
 // How X is quantised: as the 128-value blocks with fp32 d or with half (d, sum x), or as block_q8_1 (half d). The same
 // per type as in the kernels that serve it at fewer rows.
@@ -52,12 +63,12 @@ __host__ __device__ constexpr int form_of(int kind) {
 
 // Sizes and places (bytes from the scratch buffer's start) of one product's operands.
 struct Plan {
-  int kind, hu;              // hu: planes of scaled products (1 = rounded, 2 = hi + lo)
+  int kind, hu;              // hu: planes of scaled products (1 = rounded, 2 = hi + lo); 0: the bare quants (int_sums)
   int nt, n_tb;              // tokens per block (a multiple of 16), blocks
   int splits;                // parts that K is cut into (few tiles: partial sums in fp32, then their sum)
   int nsb, nkb;
   int64_t chunk_rows;        // weight rows expanded and multiplied at a time (a multiple of 256)
-  size_t a, dw, ta, b, tb, inv, part, total;
+  size_t a, dw, dm, ta, b, tb, inv, dx, part, total;
 };
 int make_plan(Plan* p, int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu);   // gsq_gemm4.cu
 
