@@ -139,6 +139,38 @@ def test_numbers_that_are_not_finite(name, packed):
     assert np.linalg.norm(got[ok] - want[ok]) <= 2e-4 * np.linalg.norm(want[ok])   # (truncating divisions: 5e-5)
 
 
+def test_weights_expanded_in_several_chunks():
+    """A weight above the bound on expanded weights goes a range of rows at a time through one buffer: results on both sides
+    of each seam, and the whole against the same rows called by themselves."""
+    t, rows, k, m = 14, 7680 + 272, 17408, 100
+    assert rows * k * 4 > 512 << 20
+    g = torch.Generator(DEV).manual_seed(93)
+    w = torch.randint(0, 256, (rows, k // 256, 210), dtype=torch.uint8, device=DEV, generator=g)
+    w[..., 208:210] = (torch.randn(rows, k // 256, device=DEV, generator=g).abs() * 1e-2).to(torch.float16).unsqueeze(-1).view(torch.uint8)
+    w = w.view(rows, -1)
+    sample = [0, 1, 6911, 6912, 7167, 7168, 7169, 7424, 7679, 7680, 7681, rows - 1]
+    raw = w[sample].cpu().numpy()
+    iq3_pack.pack_(w, t)
+    x = synth.nudge_ties_torch(torch.from_numpy(synth.make_activation(m, k, 94)).to(torch.bfloat16)).float()
+    lib, xd = _cabi.lib, x.to(DEV)
+
+    def run(w):
+        n = w.shape[0]
+        size = lib.gsq_linear_workspace_bytes(n, m, k, t, 1)
+        scratch = torch.full((size,), 0xFF, dtype=torch.uint8, device=DEV)
+        y = torch.full((m, n), float("nan"), device=DEV)
+        assert lib.gsq_linear(w.data_ptr(), w.shape[1], n, t, 1, xd.data_ptr(), 0, m, k, k, y.data_ptr(), 0, n, scratch.data_ptr(), size,
+                              torch.cuda.current_stream().cuda_stream) == 0
+        return y
+
+    y = run(w)
+    q, d, _ = q8_1.quantize_q8_1(x.numpy())
+    assert product.rel_err(y[:, sample].cpu().numpy(), product.product_q81(blocks.decode(raw, t), q, d)) <= 2.5e-7
+    for a in range(0, rows, 2048):
+        part = run(w[a:a + 2048])
+        assert bool(((part - y[:, a:a + 2048]).norm(dim=1) <= 2.5e-7 * part.norm(dim=1)).all())
+
+
 @pytest.mark.parametrize("m", [256, 257, 272, 511, 529])
 @pytest.mark.parametrize("name", ["IQ3_S", "IQ4_XS", "Q4_K"])
 def test_rounded_kinds_over_token_blocks(name, m):
@@ -152,6 +184,22 @@ def test_rounded_kinds_over_token_blocks(name, m):
     assert product.rel_err(got, prefill_forms.product(raw, t, x.numpy())) <= 3e-6
 
 
+def _integer_sums(raw, t, packed, x):
+    """The arithmetic of the kernels with integer slice sums, the scaling in float64: 128-value blocks for repacked IQ3_S,
+    IQ4_XS and Q4_K (there d, sum x, d * sc and dmin * m in half, as the int8 GEMM keeps them), block_q8_1 for the others."""
+    dec = blocks.decode(raw, t)
+    if t == 14 or (t == 21 and not packed):
+        q, d, _ = q8_1.quantize_q8_1(x)
+        return product.product_q81(dec, q, d)
+    q, d, s = q8_1.quantize_mmq(x, q8_1.LAYOUT_DS4 if t == 12 else q8_1.LAYOUT_D4)
+    if t == 12:
+        f16, f64 = np.float16, np.float64
+        scale, least = [(np.repeat(a, 8, axis=1).astype(f16) * i.astype(f16)).astype(f64) for a, i in ((dec.d, dec.isc), (dec.dmin, dec.imin))]
+        y = np.einsum("mns,ns,ms->mn", product.block_sums(dec, q).astype(f64), scale, d.astype(f16).astype(f64), optimize=True)
+        return y - s.astype(f16).astype(f64) @ least.T
+    return product.product_q81(dec, q, d)
+
+
 @pytest.mark.parametrize("name,packed,m", [("IQ3_S", True, 256), ("IQ4_XS", False, 300), ("Q4_K", False, 520), ("Q6_K", True, 99),
                                            ("Q6_K", False, 26)])
 def test_least_scratch(name, packed, m):
@@ -162,8 +210,7 @@ def test_least_scratch(name, packed, m):
     lib = _cabi.lib
     assert lib.gsq_linear_scratch_bytes(rows, m, k, t, int(packed)) < lib.gsq_linear_workspace_bytes(rows, m, k, t, int(packed))
     got = _run(t, packed, raw, x.to(DEV), rows, least=True)
-    q, d, _ = q8_1.quantize_q8_1(x.numpy())
-    assert product.rel_err(got, product.product_q81(blocks.decode(raw, t), q, d)) <= 3e-3   # (d in half or in fp32; Q4_K: sums of x or of q)
+    assert product.rel_err(got, _integer_sums(raw, t, packed, x.numpy())) <= 2e-6
 
 
 def test_long_prompt_with_k_in_parts():
