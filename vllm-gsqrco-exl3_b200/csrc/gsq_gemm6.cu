@@ -8,7 +8,7 @@
 // Two levels and short parts because every fp32 sum over n terms rounds n times: error against 64 bits, 2-norm, 1024 to
 // 17408 columns 0.67e-7 to 0.95e-7, the kernels of few rows 0.69e-7 to 1.08e-7; scaled products accumulated in tensor memory,
 // whose adder cuts off, 7e-7. For Q2_K and IQ1_M, whose kernel of few rows is the most exact (0.65e-7 at 1024 columns), t
-// covers 4 slices and the sum over K carries its rounding error along: 0.57e-7 to 0.81e-7. Q2_K's minimums are 8 more sums per
+// covers 4 slices and the sum over K carries its rounding error along: 0.55e-7 to 0.81e-7. Q2_K's minimums are 8 more sums per
 // superblock, over the slice's two groups of m * (sum of q), scaled by -dmin the same way.
 //
 // A pair of CTAs owns 256 weight rows x nt tokens, 128 at most: two (three) fp32 numbers per result in the consumers'

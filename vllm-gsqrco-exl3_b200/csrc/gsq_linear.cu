@@ -65,8 +65,28 @@ enum Way {
   W_GEMV_LOOP   // GGUF-order blocks: the dp4a kernels, 8 rows per launch
 };
 
+// The fewest activation rows from which the two-step product takes the place of repeated launches of the small-batch
+// kernels. Where the two cross, us two steps / launches (weights cycled through HBM; profiles/two_step_thresholds.txt):
+//   Q6_K repacked (48 rows a launch)  97: 5120 x 5120 50 / 69, 5120 x 17408 158 / 183, but 17408 x 5120 154 / 143
+//                                     (112 rows 156 / 150, 128 rows 158 / 164)
+//   Q6_K, IQ3_S in GGUF order (8)     25: 512 x 1024 16 / 21 and 15 / 32, 17408 x 5120 148 / 281 and 95 / 176
+//   Q2_K                              25: 5120 x 5120 47 / 70, 17408 x 5120 120 / 155; 512 x 1024 22 / 18, at 40 rows 23 / 26
+//   IQ1_M                             12: 5120 x 5120 32 / 40, 17408 x 5120 81 / 89; 1024 x 2048 16.5 / 13.9, at 17 rows 17.4 / 18.9
+//   the others                        9: 2048 x 8192 22 / 36 (IQ2_XXS) to 23 / 34 (IQ2_S); tall weights 78 / 75 (IQ2_S
+//                                     17408 x 5120), at 12 rows 78 / 87; IQ2_S 2048 x 2048 14.8 / 13.6, at 12 rows 14.8 / 15.7
+static int two_step_rows(int ggml_type, bool q6_packed, int64_t rows, int64_t k) {
+  const int64_t values = rows * k;
+  switch (ggml_type) {
+    case GSQ_TYPE_Q6_K: return !q6_packed ? 25 : rows > 8192 ? 113 : 97;
+    case GSQ_TYPE_IQ3_S: return 25;
+    case GSQ_TYPE_Q2_K: return values <= (1 << 20) ? 33 : 25;
+    case GSQ_TYPE_IQ1_M: return values <= (4 << 20) ? 17 : 12;
+    default: return rows > 8192 || (ggml_type == GSQ_TYPE_IQ2_S && values <= (4 << 20)) ? 12 : 9;
+  }
+}
+
 // small: the scratch has no room for expanded weights: the forms that need none instead, none less exact
-static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, bool small) {
+static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, bool small) {
   const int variant = gemm_variant();
   const bool dump = gemm_dump_pointer() != nullptr;   // (per-slice integer sums: only the integer forms have them)
   if (variant == 10 && !dump && gemm5_applies(ggml_type, packed, rows, m)) return W_BATCH;
@@ -88,10 +108,12 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, bool s
     if (variant == 3 || variant == 4 || variant >= 5 || (variant == 0 && big)) return W_I8;
     return variant == 0 && !dump && gemm5_applies(ggml_type, packed, rows, m) ? W_BATCH : W_LOCKSTEP;
   }
-  const bool q6 = ggml_type == GSQ_TYPE_Q6_K, q6_packed = q6 && packed && rows % 16 == 0;
+  const bool q6_packed = ggml_type == GSQ_TYPE_Q6_K && packed && rows % 16 == 0;
   // Q6_K, IQ3_S in GGUF order and the low-bit types: the two steps once they cost less than the repeated launches of the
   // small-batch kernels (48 or 8 rows each), no less exact than those, unless they are asked for.
-  if (!small && !dump && g_prefill_precision != GSQ_PREFILL_INTEGER && gemm4_applies(ggml_type, packed, rows) && m >= (q6_packed ? 97 : q6 || ggml_type == GSQ_TYPE_IQ3_S ? 25 : 9)) return W_PLANES2;
+  if (!small && !dump && g_prefill_precision != GSQ_PREFILL_INTEGER && gemm4_applies(ggml_type, packed, rows) &&
+      m >= two_step_rows(ggml_type, q6_packed, rows, k))
+    return W_PLANES2;
   return q6_packed ? W_MMV_LOOP : W_GEMV_LOOP;
 }
 
@@ -133,9 +155,9 @@ extern "C" int gsq_prefill_precision(int mode) {
 static size_t linear_bytes(int64_t rows, int64_t m, int64_t k, int ggml_type, int packed, bool small) {
   using namespace gsq;
   if (m <= 0 || k <= 0 || rows <= 0 || ragged(ggml_type, packed, rows)) return 0;
-  const Way way = choose_way(ggml_type, packed, rows, m, small);
+  const Way way = choose_way(ggml_type, packed, rows, m, k, small);
   size_t b = way_scratch(way, rows, m, k, ggml_type, packed);
-  if (small && gemm2_applies(ggml_type, packed, rows) && choose_way(ggml_type, packed, rows, m, false) == W_PLANES1) {
+  if (small && gemm2_applies(ggml_type, packed, rows) && choose_way(ggml_type, packed, rows, m, k, false) == W_PLANES1) {
     // one fp16 plane of activations (and Q4_K's block sums): room for any of the forms of the default precision
     const size_t plane = gemm3_tile_bytes(m, k) + (ggml_type == GSQ_TYPE_Q4_K ? (size_t)((m + 255) / 256) * (k / 256) * 8192 : 0);
     b = b > plane ? b : plane;
@@ -181,7 +203,7 @@ extern "C" int gsq_linear(const void* w, int64_t row_bytes, int64_t rows, int gg
     rc = mmv_host(w, row_bytes, rows, ggml_type, packed, scratch, in_rows ? 4 : 1, m, k, y, y_dtype, y_row_stride, stream, gemm_dump_pointer());
     if (rc != 1000) return rc;  // 1000: declined, the activations of this shape do not fit its staging area
   }
-  const Way way = choose_way(ggml_type, packed, rows, m, scratch_bytes < gsq_linear_workspace_bytes(rows, m, k, ggml_type, packed));
+  const Way way = choose_way(ggml_type, packed, rows, m, k, scratch_bytes < gsq_linear_workspace_bytes(rows, m, k, ggml_type, packed));
   const int64_t ysz = y_dtype == GSQ_F32 ? 4 : 2;
   switch (way) {
     case W_PLANES1:
