@@ -58,9 +58,9 @@ extern "C" {
 /* kernel selectors returned by gsq_route / accepted by gsq_mul_mat */
 #define GSQ_KERNEL_NONE 0
 #define GSQ_KERNEL_GEMV 1 /* dp4a streaming GEMV, 1..8 activation rows per launch, reads block_q8_1 */
-#define GSQ_KERNEL_GEMM 2 /* tcgen05 kind::i8 GEMM, 64-token tiles in lockstep, reads 128-value q8_1 blocks */
+#define GSQ_KERNEL_GEMM 2 /* tcgen05 kind::i8 GEMMs: evenly cut work, one or two token blocks (gsq_linear); 64-token tiles (gsq_mul_mat_q8) */
 #define GSQ_KERNEL_MMV 3  /* register-operand tensor-core kernel, 1..48 activation rows per launch */
-#define GSQ_KERNEL_GEMM_PREFILL 4 /* tcgen05 prefill GEMMs: weights expanded to fp16 operands, or (integer sums) decoded in the kernel */
+#define GSQ_KERNEL_GEMM_PREFILL 4 /* tcgen05 prefill GEMMs: weights expanded to fp16 operands, or (integer setting) decoded in the kernel */
 
 const char* gsq_strerror(int status);
 /* cudaError_t of the last failing CUDA call made by this library on this thread (0 if none). */
@@ -337,11 +337,11 @@ int gsq_linear_allreduce(const void* w, int64_t row_bytes, int64_t rows, int ggm
 int gsq_peer_reduce_error_flag(int* flag);
 
 /*
- * Kernel family that serves (activation rows m, type, weight rows, k, packed) on B200: GSQ_KERNEL_*, the choice
- * gsq_mul_mat_vec_q8 and, for repacked IQ3_S, IQ4_XS and Q4_K, gsq_linear make (for the other types: the small-batch
- * kernel; gsq_linear leaves it for the prefill GEMM once it would take several launches). The op-level routing table of the reference (_lcpp_op,
- * quantization/linear.py:85-114) stays in the Python layer because its op names are API; this is the choice made
- * underneath those names.
+ * Kernel family that serves (activation rows m, type, weight rows, k, packed) on B200: GSQ_KERNEL_*, the choice that
+ * gsq_mul_mat_vec_q8 makes up to 8 activation rows and gsq_linear above (for the precision that is set, with
+ * gsq_linear_workspace_bytes of scratch; a family that takes fewer rows per launch is launched several times). The op-level
+ * routing table of the reference (_lcpp_op, quantization/linear.py:85-114) stays in the Python layer because its op names
+ * are API; this is the choice made underneath those names.
  */
 int gsq_route(int64_t m, int ggml_type, int64_t rows, int64_t k, int packed);
 

@@ -92,8 +92,8 @@ def test_zero_rows_return_before_routing():
 
 
 def test_c_route():
-    """gsq_route names the kernel family the library runs underneath the op names (what gsq_mul_mat_vec_q8 and
-    gsq_linear choose)."""
+    """gsq_route names the kernel family the library runs underneath the op names: what gsq_mul_mat_vec_q8 (up to 8 rows)
+    and gsq_linear choose."""
     from gsq_b200 import _cabi
 
     r = _cabi.lib.gsq_route
@@ -102,14 +102,28 @@ def test_c_route():
     assert r(1, IQ3_S, BIG, K, 0) == _cabi.KERNEL_GEMV         # GGUF order: dp4a
     assert r(1, Q4_K, BIG, K, 0) == _cabi.KERNEL_GEMV and r(2, Q4_K, BIG, K, 0) == _cabi.KERNEL_MMV
     assert r(3, IQ4_XS, BIG, K, 0) == _cabi.KERNEL_GEMV and r(4, IQ4_XS, BIG, K, 0) == _cabi.KERNEL_MMV
-    assert r(48, Q4_K, BIG, K, 0) == _cabi.KERNEL_MMV and r(49, Q4_K, BIG, K, 0) == _cabi.KERNEL_GEMM
+    assert r(32, Q4_K, BIG, K, 0) == _cabi.KERNEL_MMV and r(33, Q4_K, BIG, K, 0) == _cabi.KERNEL_GEMM   # evenly cut work
+    assert r(48, Q4_K, 1024, K, 0) == _cabi.KERNEL_MMV and r(49, Q4_K, 1024, K, 0) == _cabi.KERNEL_GEMM
+    assert r(48, IQ4_XS, BIG, K, 0) == _cabi.KERNEL_MMV and r(48, IQ4_XS, 2048, 8192, 0) == _cabi.KERNEL_GEMM
+    assert r(48, IQ3_S, BIG, K, 1) == _cabi.KERNEL_MMV and r(49, IQ3_S, 5120, K, 1) == _cabi.KERNEL_GEMM
     assert r(512, Q4_K, BIG, K, 0) == _cabi.KERNEL_GEMM_PREFILL and r(256, Q4_K, 5120, K, 0) == _cabi.KERNEL_GEMM_PREFILL
     assert r(255, Q4_K, 5120, K, 0) == _cabi.KERNEL_GEMM and r(128, Q4_K, BIG, K, 0) == _cabi.KERNEL_GEMM_PREFILL
     assert r(256, IQ4_XS, 5120, K, 0) == _cabi.KERNEL_GEMM_PREFILL and r(255, IQ4_XS, 5120, K, 0) == _cabi.KERNEL_GEMM
     assert r(128, IQ3_S, 17408, K, 1) == _cabi.KERNEL_GEMM_PREFILL and r(128, IQ3_S, 5120, K, 1) == _cabi.KERNEL_GEMM
-    assert r(8192, Q6_K, 151936, K, 1) == _cabi.KERNEL_MMV     # repacked Q6_K: 48 rows per launch
-    assert r(33, Q6_K, BIG, K, 0) == _cabi.KERNEL_GEMV         # GGUF order: dp4a, 8 rows per launch
-    assert r(4, IQ2_S, BIG, K, 0) == _cabi.KERNEL_GEMV and r(300, IQ2_S, BIG, K, 0) == _cabi.KERNEL_GEMV   # low-bit types: dp4a
+    # launches of the few-row kernel, then the two steps: per type, height and size of the weight
+    for t, packed, rows, k, first, few in ((Q6_K, 1, 5120, BIG, 97, "MMV"), (Q6_K, 1, BIG, K, 113, "MMV"), (Q6_K, 1, 151936, K, 113, "MMV"),
+                                           (Q6_K, 0, BIG, K, 25, "GEMV"), (IQ3_S, 0, 512, 1024, 25, "GEMV"), (10, 0, BIG, K, 25, "GEMV"),
+                                           (10, 0, 512, 1024, 33, "GEMV"), (IQ1_M, 0, BIG, K, 12, "GEMV"), (IQ1_M, 0, 1024, 2048, 17, "GEMV"),
+                                           (IQ2_S, 0, 2048, 8192, 9, "GEMV"), (IQ2_S, 0, 2048, 2048, 12, "GEMV"), (IQ2_XS, 0, 2048, 2048, 9, "GEMV"),
+                                           (IQ2_XS, 0, BIG, K, 12, "GEMV"), (18, 0, 5120, BIG, 9, "GEMV"), (16, 0, BIG, K, 12, "GEMV")):
+        below = first - 1
+        assert r(first, t, rows, k, packed) == _cabi.KERNEL_GEMM_PREFILL and r(8192, t, rows, k, packed) == _cabi.KERNEL_GEMM_PREFILL, (t, rows, k)
+        assert r(below, t, rows, k, packed) == getattr(_cabi, "KERNEL_" + few), (t, rows, k)
+        # the choice gsq_linear sizes its workspace by
+        w = _cabi.lib.gsq_linear_workspace_bytes
+        assert w(rows, first, k, t, packed) > min(rows * k * 2, 480 << 20) > w(rows, below, k, t, packed), (t, rows, k)   # (in chunks)
+    assert r(4, IQ2_S, BIG, K, 0) == _cabi.KERNEL_GEMV
+    assert r(32, Q6_K, 24, 1024, 1) == _cabi.KERNEL_NONE       # repacked rows that are no whole records: refused
     assert r(4, 8, BIG, K, 0) == _cabi.KERNEL_NONE             # Q8_0: not a type of this route
 
 

@@ -160,25 +160,15 @@ extern "C" int gsq_check_inputs(const gsq_guard_args* a, int64_t* k_out, char* m
 }
 
 namespace gsq {
-bool mmv_applies(int ggml_type, int packed, int64_t rows, int64_t m);   // gsq_mmv.cu
-bool gemm2_applies(int ggml_type, int packed, int64_t rows);            // gsq_gemm2.cu
+bool mmv_applies(int ggml_type, int packed, int64_t rows, int64_t m);                          // gsq_mmv.cu
+int linear_kernel(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k);              // gsq_linear.cu
 }
 
-// The choice gsq_mul_mat_vec_q8 (m <= 8) and gsq_linear (any m) make, in the same order (a shape whose activations do
-// not fit the small-batch kernel's staging area falls through to the next family at launch).
+// (A shape whose activations do not fit the small-batch kernel's staging area goes on to the next family at launch.)
 extern "C" int gsq_route(int64_t m, int ggml_type, int64_t rows, int64_t k, int packed) {
-  (void)k;
   if (gsq::block_bytes(ggml_type) == 0 || m <= 0 || rows <= 0) return GSQ_KERNEL_NONE;
-  if (ggml_type == GSQ_TYPE_Q6_K && packed && rows % 16 == 0) return GSQ_KERNEL_MMV;   // 48 rows per launch above 48
-  if (m <= 48 && gsq::mmv_applies(ggml_type, packed, rows, m)) return GSQ_KERNEL_MMV;
-  if (m <= 8) return GSQ_KERNEL_GEMV;
-  if (gsq::gemm2_applies(ggml_type, packed, rows)) {
-    const bool tall = (rows + 127) / 128 >= 74;
-    const bool fp16_operands = true;   // gsq_gemm3.cu serves all three types of gemm2_applies in the default precision
-    const bool big = fp16_operands ? (m >= 256 || (m >= 128 && tall)) : (m >= 512 || (m >= 192 && tall));
-    return big ? GSQ_KERNEL_GEMM_PREFILL : GSQ_KERNEL_GEMM;
-  }
-  return GSQ_KERNEL_GEMV;   // Q6_K / IQ3_S in GGUF order: the dp4a kernel, 8 rows per launch
+  if (m <= 8) return gsq::mmv_applies(ggml_type, packed, rows, m) ? GSQ_KERNEL_MMV : GSQ_KERNEL_GEMV;
+  return gsq::linear_kernel(ggml_type, packed, rows, m, k);
 }
 
 extern "C" int gsq_q8_layout_for_type(int ggml_type) {

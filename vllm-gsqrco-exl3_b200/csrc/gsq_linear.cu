@@ -132,6 +132,22 @@ static bool small_batch(int ggml_type, int packed, int64_t rows, int64_t m, int6
   return true;
 }
 
+// GSQ_KERNEL_* of a gsq_linear call with the scratch it wants most
+int linear_kernel(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k) {
+  if (ragged(ggml_type, packed, rows)) return GSQ_KERNEL_NONE;
+  if (small_batch(ggml_type, packed, rows, m, k)) return GSQ_KERNEL_MMV;
+  switch (choose_way(ggml_type, packed, rows, m, k, false)) {
+    case W_PLANES1:
+    case W_PLANES2:
+    case W_IQ3_INT:
+    case W_I8: return GSQ_KERNEL_GEMM_PREFILL;
+    case W_BATCH:
+    case W_LOCKSTEP: return GSQ_KERNEL_GEMM;
+    case W_MMV_LOOP: return GSQ_KERNEL_MMV;
+    default: return GSQ_KERNEL_GEMV;
+  }
+}
+
 static size_t way_scratch(Way way, int64_t rows, int64_t m, int64_t k, int ggml_type, int packed) {
   switch (way) {
     case W_PLANES1: return gemm4_scratch_bytes(ggml_type, packed, rows, m, k, 1);
