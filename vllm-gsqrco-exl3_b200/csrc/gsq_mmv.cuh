@@ -416,7 +416,7 @@ __device__ __forceinline__ void stage_rows_wait(uint32_t bar) {
 }
 
 // X itself (fp32 / fp16 / bf16): every CTA quantises its share of K for itself, to the quantisers' values
-// (gsq_quantize.cu): a thread takes 8 consecutive values, four neighbouring threads a 32-value block. See mmv_raw_wins for
+// (gsq_quantize.cu): a thread takes 8 consecutive values, four neighbouring threads a 32-value block. See mmv_raw_applies for
 // what this costs against a quantiser kernel in front.
 __device__ __forceinline__ void load_x8(const MmvArgs& a, int64_t off, float (&v)[8]) {
   if (a.x_dtype == GSQ_F32) {
@@ -1533,8 +1533,9 @@ static int mmv_max_clusters(int cs, size_t smem, int sm_count, int* out) {
 // Constants of a launch plan's estimated time, us: a record of the busiest warp and of an SM (whichever binds), parked
 // segments (equal chunks) and what they add per tile of a cluster's other CTAs, staging per 1000 32-value blocks of
 // activations, doubling the cluster, a further round. Fitted per type and column groups to a sweep of cluster sizes and
-// chunkings over 11 shapes from 1024 x 2048 to 34816 x 5120 (and the 151936 x 5120 head): the chosen plan is then within 1 %
-// of the fastest one on average. One set of constants for all, which the sweep replaced, was 4.8 % off, and up to 1.7x (us,
+// chunkings over 11 shapes from 1024 x 2048 to 34816 x 5120 (and the 151936 x 5120 head). Over 292 cells of the kernel as it is
+// (profiles/mmv_plans.txt) the chosen plan takes 1.5 % longer than the fastest one on average, half of them 0.3 % or less,
+// the worst (Q4_K 1024 x 5120 at 4 rows) 14 %. One set of constants for all was 4.8 % off on average, and up to 1.7x (us,
 // before -> after: 9216 x 2560 at 32 rows IQ3_S 27.1 -> 16.1; 4096 x 11264 at 48 rows Q6_K 54 -> 46; the head at 16 rows
 // 319 -> 211).
 struct MmvCost {

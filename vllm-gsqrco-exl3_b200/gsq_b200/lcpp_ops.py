@@ -85,9 +85,9 @@ PREFILL_ROUNDED, PREFILL_SPLIT, PREFILL_INTEGER = 0, 1, 2
 
 
 def set_prefill_precision(mode: int) -> int:
-    """How the prefill product of repacked IQ3_S is formed (gsq_prefill_precision): PREFILL_ROUNDED (default; within
-    about 3e-4 of a row's norm of the reference kernels' result), PREFILL_SPLIT (about 1e-6), PREFILL_INTEGER (the
-    reference's exact integer slice sums). Returns the previous mode. The environment variable GSQ_PREFILL_PRECISION
+    """How the prefill products of repacked IQ3_S, IQ4_XS and Q4_K are formed (gsq_prefill_precision): PREFILL_ROUNDED
+    (default; within about 4e-4 of a row's norm of the reference kernels' result), PREFILL_SPLIT (IQ3_S: about 1e-6),
+    PREFILL_INTEGER (the reference's exact integer slice sums, which Q6_K keeps in every mode). Returns the previous mode. The environment variable GSQ_PREFILL_PRECISION
     (rounded / split / integer) sets it at import."""
     return int(_cabi.lib.gsq_prefill_precision(int(mode)))
 
