@@ -49,13 +49,15 @@ struct SliceArgs {
   int stages;
 };
 
-// Tensor memory -> registers in the layout of 16 rows x 8 columns per 4 registers: lane l holds columns 2 (l % 4), + 1 of row
-// l / 4 and of row l / 4 + 8. A thread then has a quarter of the tokens of four rows (two loads, 16 tensor-memory lanes each)
-// instead of all tokens of one, and reads a quarter of the scales from shared memory: with one row a thread (32 x 32b) these
-// reads, 128 of 16 bytes per slice, took as long as the tensor-memory loads, 560 cycles a slice together.
+// Tensor memory -> registers in the layout of 16 rows x 4 columns per 2 registers: lane l holds column l % 4 of row l / 4 and of
+// row l / 4 + 8. A thread then has a quarter of the tokens of four rows (two loads, 16 tensor-memory lanes each) instead of
+// all tokens of one, and reads a quarter of the scales from shared memory: with one row a thread (32 x 32b) these reads, 128 of
+// 16 bytes per slice, took as long as the tensor-memory loads, 560 cycles a slice together. Tensor memory gives an SM 512 bytes
+// a cycle in this shape, 905 in that of 32 x 32b, but 256 in that of 8 columns per 4 registers (16 x 256b): 256 cycles for the
+// 128 x 128 sums of a slice instead of 128, and with it Q6_K 5120 x 17408, 512 tokens, took 352 us, now 344.
 __device__ __forceinline__ void tmem_rows16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      "tcgen05.ld.sync.aligned.16x128b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
         "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr)
@@ -63,7 +65,7 @@ __device__ __forceinline__ void tmem_rows16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 
 __device__ __forceinline__ void tmem_rows16(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+  asm volatile("tcgen05.ld.sync.aligned.16x128b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(taddr)
                : "memory");
@@ -75,24 +77,24 @@ __device__ __forceinline__ void pin(uint32_t (&v)[N]) {
     asm volatile("" : "+r"(v[i]), "+r"(v[i + 1]), "+r"(v[i + 2]), "+r"(v[i + 3]), "+r"(v[i + 4]), "+r"(v[i + 5]), "+r"(v[i + 6]), "+r"(v[i + 7]));
 }
 
-// Results of a thread: pairs of tokens (8 i + 2 (lane % 4), + 1) of its four rows (8 apart), acc[4 * i + row]; y at its first
+// Results of a thread: tokens 4 i + lane % 4 of its four rows (8 apart), acc[2 * i + h] rows 2 h and 2 h + 1; y at its first
 // token and row, `n` tokens from there, `rows` rows.
 template <int ACC, typename T>
 __device__ __forceinline__ void store_results(T* y, int64_t ldy, const float2 (&acc)[ACC], int n, int rows) {
 #pragma unroll
-  for (int i = 0; i < ACC / 4; ++i) {
+  for (int i = 0; i < ACC / 2; ++i) {
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      if (8 * h < rows) {
-        if (8 * i < n) store_out<T>(y + 8 * h, acc[4 * i + h].x);
-        if (8 * i + 1 < n) store_out<T>(y + ldy + 8 * h, acc[4 * i + h].y);
+    for (int h = 0; h < 2; ++h) {
+      if (4 * i < n) {
+        if (16 * h < rows) store_out<T>(y + 16 * h, acc[2 * i + h].x);
+        if (16 * h + 8 < rows) store_out<T>(y + 16 * h + 8, acc[2 * i + h].y);
       }
     }
-    y += 8 * ldy;
+    y += 4 * ldy;
   }
 }
 
-// acc += t * f with the rounding error of the sum carried along in e (Kahan); f the same in both halves. An infinite sum
+// acc += t * f with the rounding error of the sum carried along in e (Kahan). An infinite sum
 // stays infinite: its error, which would be NaN, is cut to a number.
 __device__ __forceinline__ void add_carried(float2& acc, float2& e, const float2& t, const float2& f) {
   const float2 minus = make_float2(-1.0f, -1.0f);
@@ -107,7 +109,7 @@ __device__ __forceinline__ void add_carried(float2& acc, float2& e, const float2
 template <int AP, int TP, bool COMP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(S_THREADS, 1) gemm6_kernel(const SliceArgs g) {
   constexpr int FOLD = COMP ? 2 : 4;   // pairs of slices
-  constexpr int WT = warp_tokens(COMP), ACC = WT / 2;   // tokens of a warp; pairs of results of a thread
+  constexpr int WT = warp_tokens(COMP), ACC = WT / 2;   // tokens of a warp; pairs of results (rows 8 apart) of a thread
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t crank = cluster_ctarank();
@@ -295,7 +297,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(S_THREADS, 1) gemm6_
     // ------------------------------------------------------------------------------------ consumers
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S_CONS_REGS));
     const int q4 = warp & 3, tok_w = ((warp - CONS_WARP0) >> 2) * WT;   // lane quarter, first token
-    const int r_in = 32 * q4 + (lane >> 2), t_in = tok_w + 2 * (lane & 3);   // first row of the tile, first token of the thread
+    const int r_in = 32 * q4 + (lane >> 2), t_in = tok_w + (lane & 3);   // first row of the tile, first token of the thread
     const uint32_t t_warp = tmem_base + ((uint32_t)(32 * q4) << 16) + (uint32_t)tok_w;
     const uint32_t d_empty0 = mapa(d_empty, 0u);
     Cursor rd = {0u, 0u}, x = {0u, 0u};
@@ -334,10 +336,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(S_THREADS, 1) gemm6_
 #pragma unroll
               for (int s = 0; s < 2; ++s) {
                 const uint32_t ta = t_warp + rd.i * (2 * d_cols) + s * d_cols;
-                const uint8_t* ds = slot + (((2 * (part * FOLD + j) + s) & 7) * g.nt + t_in) * 4;
-                float2 d[WT / 8];
+                // (tokens 4 i + lane % 4 lie side by side: gsq_planes.cu)
+                const uint8_t* ds = slot + (((2 * (part * FOLD + j) + s) & 7) * g.nt + tok_w + 4 * (lane & 3)) * 4;
+                float4 d[WT / 16];
 #pragma unroll
-                for (int i = 0; i < WT / 8; ++i) d[i] = *reinterpret_cast<const float2*>(ds + 32 * i);
+                for (int i = 0; i < WT / 16; ++i) d[i] = *reinterpret_cast<const float4*>(ds + 64 * i);
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                   uint32_t v[WT / 2];
@@ -345,12 +348,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(S_THREADS, 1) gemm6_
                   tmem_ld_wait();
                   pin(v);
                   if (s == 1 && hh == 1) release();
-                  // t += S * d_x: four registers per 8 columns, rows 16 hh + l / 4 and + 8
+                  // t += S * d_x: two registers per 4 columns, rows 16 hh + l / 4 and + 8
 #pragma unroll
-                  for (int i = 0; i < WT / 8; ++i) {
-                    float2 &t0 = t[4 * i + 2 * hh], &t1 = t[4 * i + 2 * hh + 1];
-                    t0 = __ffma2_rn(make_float2(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1])), d[i], t0);
-                    t1 = __ffma2_rn(make_float2(__uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3])), d[i], t1);
+                  for (int i = 0; i < WT / 4; ++i) {
+                    const float4& q = d[i >> 2];
+                    const float dx = (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w;
+                    t[2 * i + hh] = __ffma2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), make_float2(dx, dx), t[2 * i + hh]);
                   }
                 }
               }
@@ -359,12 +362,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(S_THREADS, 1) gemm6_
           }
           const float* f = reinterpret_cast<const float*>(slot + dx_bytes + (TP && part >= 4 / FOLD ? 512 : 0)) + r_in;
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const float2 scale = make_float2(f[8 * h], f[8 * h]);
+          for (int h = 0; h < 2; ++h) {
+            const float2 scale = make_float2(f[16 * h], f[16 * h + 8]);
 #pragma unroll
-            for (int i = 0; i < ACC / 4; ++i) {
-              if (COMP) add_carried(acc[4 * i + h], err[COMP ? 4 * i + h : 0], t[4 * i + h], scale);
-              else acc[4 * i + h] = __ffma2_rn(t[4 * i + h], scale, acc[4 * i + h]);
+            for (int i = 0; i < ACC / 2; ++i) {
+              if (COMP) add_carried(acc[2 * i + h], err[COMP ? 2 * i + h : 0], t[2 * i + h], scale);
+              else acc[2 * i + h] = __ffma2_rn(t[2 * i + h], scale, acc[2 * i + h]);
             }
           }
         }

@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(QTHREADS) planes_kernel(const T* __restrict__ 
 #pragma unroll
       for (int e = 0; e < 4; ++e) h[e] = __floats2half2_rn(q[2 * e], q[2 * e + 1]);
       *reinterpret_cast<uint4*>(b0 + (int64_t)(4 * sb + (lane >> 3)) * (2 * unit)) = *reinterpret_cast<const uint4*>(h);
-      if ((lane & 3) == 0) g.dx[((blk * g.nsb + sb) * 8 + (lane >> 2)) * g.nt + ti] = live ? d : 0.0f;
+      // (of 16 tokens, 4 i + j at place 4 j + i: a thread of the GEMM has those of one j)
+      if ((lane & 3) == 0) g.dx[((blk * g.nsb + sb) * 8 + (lane >> 2)) * g.nt + (ti & ~15) + 4 * (ti & 3) + ((ti >> 2) & 3)] = live ? d : 0.0f;
       if constexpr (TP) {
         float sum = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
         sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
