@@ -329,24 +329,44 @@ static int gemm4_launch(const Plan& p, uint8_t* scratch, int64_t rows, int64_t m
   return p.hu == 2 ? launch_gemm4<2, 0>(g, stage, sm_count, st) : launch_gemm4<1, 0>(g, stage, sm_count, st);
 }
 
-// y = the sum of the parts, in their order; a thread takes one result of every part. Tokens are the grid's x: a prompt may
-// have more than the 65535 blocks of y (row blocks of a call: 4096 at most, by the bound on expanded weights).
-template <typename T>
+// y = the sum of the parts, in their order; a thread takes V rows of a token (4 where rows and y allow it: 16-byte loads, all of
+// a thread's in flight; with one row Q6_K 5120 rows x 512 tokens in 6 parts, 63 MB, took 19.6 us). Tokens are the grid's x: a
+// prompt may have more than the 65535 blocks of y (row blocks of a call: 4096 at most, by the bound on expanded weights).
+template <typename T, int V>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ part, T* __restrict__ y, int64_t m, int64_t rows, int64_t ldy,
                                                        int splits) {
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int64_t row = (int64_t)blockIdx.y * 256 + threadIdx.x, tok = blockIdx.x;
+  const int64_t row = ((int64_t)blockIdx.y * 256 + threadIdx.x) * V, tok = blockIdx.x;
   if (row >= rows) return;
   const float* p = part + tok * rows + row;
-  float s = __ldcg(p);
-  for (int i = 1; i < splits; ++i) s += __ldcg(p + i * m * rows);
-  store_out<T>(y + tok * ldy + row, s);
+  if constexpr (V == 1) {
+    float s = __ldcg(p);
+    for (int i = 1; i < splits; ++i) s += __ldcg(p + i * m * rows);
+    store_out<T>(y + tok * ldy + row, s);
+  } else {
+    float4 s = __ldcg(reinterpret_cast<const float4*>(p));
+#pragma unroll 8
+    for (int i = 1; i < splits; ++i) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(p + i * m * rows));
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    alignas(16) T r[4];
+    store_out<T>(r, s.x);
+    store_out<T>(r + 1, s.y);
+    store_out<T>(r + 2, s.z);
+    store_out<T>(r + 3, s.w);
+    if constexpr (sizeof(T) == 4) *reinterpret_cast<uint4*>(y + tok * ldy + row) = *reinterpret_cast<const uint4*>(r);
+    else *reinterpret_cast<uint2*>(y + tok * ldy + row) = *reinterpret_cast<const uint2*>(r);
+  }
 }
 
-static int sum_parts(const Plan& p, const uint8_t* scratch, int64_t rows, int64_t m, void* y, int y_dtype, int64_t ldy, cudaStream_t st) {
+template <typename T>
+static int launch_sum_parts(const Plan& p, const float* part, int64_t rows, int64_t m, T* y, int64_t ldy, cudaStream_t st) {
+  const bool vec = rows % 4 == 0 && ldy % 4 == 0 && (uintptr_t)y % (4 * sizeof(T)) == 0;
+  const int64_t per = vec ? 1024 : 256;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)m, (unsigned)((rows + 255) / 256));
+  cfg.gridDim = dim3((unsigned)m, (unsigned)((rows + per - 1) / per));
   cfg.blockDim = dim3(256);
   cfg.stream = st;
   cudaLaunchAttribute attr;
@@ -354,11 +374,14 @@ static int sum_parts(const Plan& p, const uint8_t* scratch, int64_t rows, int64_
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  const float* part = reinterpret_cast<const float*>(scratch + p.part);
-  if (y_dtype == GSQ_BF16) GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, sum_parts_kernel<__nv_bfloat16>, part, (__nv_bfloat16*)y, m, rows, ldy, p.splits));
-  else if (y_dtype == GSQ_F16) GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, sum_parts_kernel<__half>, part, (__half*)y, m, rows, ldy, p.splits));
-  else GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, sum_parts_kernel<float>, part, (float*)y, m, rows, ldy, p.splits));
+  GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, vec ? sum_parts_kernel<T, 4> : sum_parts_kernel<T, 1>, part, y, m, rows, ldy, p.splits));
   return GSQ_OK;
+}
+static int sum_parts(const Plan& p, const uint8_t* scratch, int64_t rows, int64_t m, void* y, int y_dtype, int64_t ldy, cudaStream_t st) {
+  const float* part = reinterpret_cast<const float*>(scratch + p.part);
+  if (y_dtype == GSQ_BF16) return launch_sum_parts(p, part, rows, m, (__nv_bfloat16*)y, ldy, st);
+  if (y_dtype == GSQ_F16) return launch_sum_parts(p, part, rows, m, (__half*)y, ldy, st);
+  return launch_sum_parts(p, part, rows, m, (float*)y, ldy, st);
 }
 
 // Tokens per block, blocks and parts of K of a product of n_rp pairs of row tiles and m tokens, by an estimate in SM
