@@ -364,7 +364,6 @@ __device__ __forceinline__ void x_f1(const uint8_t* s, uint8_t* out, int r, int 
 
 template <int KIND>
 __global__ void __launch_bounds__(XTHREADS) expand_kernel(const ExpandArgs g) {
-  asm volatile("griddepcontrol.launch_dependents;");
   extern __shared__ __align__(1024) uint8_t smem[];
   using T = typename Unit<x_unit(KIND)>::T;
   constexpr int PER = x_segment(KIND) / x_unit(KIND), UNITS = x_segments(KIND) * PER, NLD = (UNITS + XTHREADS - 1) / XTHREADS;
@@ -406,6 +405,9 @@ __global__ void __launch_bounds__(XTHREADS) expand_kernel(const ExpandArgs g) {
   if (item < g.n_items) load(item);
   // the weights may be read before the previous kernel has finished; the operand buffer may not be written
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  // Only now may the next kernel start: where that is the one that quantises the activations (gsq_planes.cu), it takes it that
+  // whatever ran before this kernel has finished, and runs beside this one.
+  asm volatile("griddepcontrol.launch_dependents;");
   for (int n = 0; item < g.n_items; ++n) {
     uint8_t* const raw = raw0 + (n & 1) * x_raw(KIND);
     stash(raw);

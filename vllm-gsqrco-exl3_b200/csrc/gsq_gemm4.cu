@@ -495,11 +495,12 @@ int gemm4_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, 
   rc = device_info(&di);
   if (rc != GSQ_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = pl::planes_host(p, x, x_dtype, m, k, x_row_stride, (uint8_t*)scratch, st);
   const int64_t ysz = y_dtype == GSQ_F32 ? 4 : 2;
   for (int64_t r0 = 0; r0 < rows && rc == GSQ_OK; r0 += p.chunk_rows) {
     const int64_t n = rows - r0 < p.chunk_rows ? rows - r0 : p.chunk_rows;
     rc = pl::expand_host(p, (const uint8_t*)w + r0 * row_bytes, row_bytes, n, (uint8_t*)scratch, di.sm_count, st);
+    // (beside the first expansion: the order of these two launches matters, see planes_kernel)
+    if (rc == GSQ_OK && r0 == 0) rc = pl::planes_host(p, x, x_dtype, m, k, x_row_stride, (uint8_t*)scratch, st);
     if (rc == GSQ_OK)
       rc = (pl::int_sums(p.kind) ? pl::gemm6_launch : pl::gemm4_launch)(p, (uint8_t*)scratch, n, m, (uint8_t*)y + r0 * ysz, y_dtype, y_row_stride,
                                                                         di.sm_count, st);

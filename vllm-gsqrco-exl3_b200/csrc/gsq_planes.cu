@@ -41,8 +41,10 @@ __device__ __forceinline__ uint32_t half_bits(float v) { return (uint32_t)__half
 
 template <typename T, bool VEC, int FORM, int HU, int TP>
 __global__ void __launch_bounds__(QTHREADS) planes_kernel(const T* __restrict__ x, const QuantArgs g) {
+  // Starts once every block of the expanding kernel has seen the kernels before it finish, and runs beside it: 4 to 16 us of
+  // latency and reads that fit into the 40 to 75 us in which that one writes the weights. Only the last block waits for it, at
+  // the end: so this grid finishes after it, and the GEMM, which waits for this grid, finds both.
   asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ float wmax[QTHREADS / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t tok = blockIdx.x;
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(QTHREADS) planes_kernel(const T* __restrict__ 
       }
     }
   }
+  if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <typename T, int FORM, int HU, int TP>
