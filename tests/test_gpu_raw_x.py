@@ -65,3 +65,32 @@ def test_quantised_in_the_product(name, dtype, rows, k, ms, pad):
             want = product.product_q81(dec, q, d)
         assert bool(torch.isnan(y[:, rows:]).all())
         assert product.rel_err(y[:, :rows].cpu().numpy(), want) <= 2e-6
+
+
+@pytest.mark.parametrize("name,ms", [("Q4_K", (1,)), ("IQ4_XS", (1, 2, 3))])
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("rows,k,pad", [(12301, 256, 0), (3077, 1280, 1), (2050, 5120, 8), (516, 8192, 0), (516, 8448, 3)])
+def test_dp4a_product_quantises_as_the_kernel_in_front(name, ms, dtype, rows, k, pad):
+    """The dp4a kernel with X quantised inside: bit for bit what the quantiser kernel and the product on its blocks give."""
+    t = TYPES[name]
+    lib, code, tdt = _cabi.lib, DTYPES[dtype][0], DTYPES[dtype][1]
+    w = torch.from_numpy(synth.make_weight(t, rows, k, 95 + rows)).to(DEV)
+    st = torch.cuda.current_stream().cuda_stream
+    for m in ms:
+        buf = torch.empty((m, k + pad), dtype=tdt, device=DEV)
+        buf[:, :k] = torch.from_numpy(synth.make_activation(m, k, 96 + m)).to(tdt).to(DEV)
+        buf[0, :64] = 0.0
+        out = [torch.full((m, rows + 3), float("nan"), dtype=torch.float32, device=DEV) for _ in range(2)]
+        args = (w.data_ptr(), w.shape[1], rows, t, 0)
+        rc = lib.gsq_linear_vec(*args, buf.data_ptr(), code, m, k, k + pad, out[0].data_ptr(), 0, rows + 3, st)
+        if m * k > 8192:   # (the two calls are faster)
+            assert rc == UNSUPPORTED
+            continue
+        assert rc == 0, lib.gsq_strerror(rc)
+        q8 = torch.empty(m * k // 32 * 36, dtype=torch.uint8, device=DEV)
+        assert lib.gsq_quantize_q8_1(buf.data_ptr(), code, m, k, k + pad, q8.data_ptr(), st) == 0
+        assert lib.gsq_mul_mat_vec_q8(*args, q8.data_ptr(), m, k, out[1].data_ptr(), 0, rows + 3, st) == 0
+        if rows * k > 3 << 20:   # (smaller ones: the tensor-core kernel, which adds in another order)
+            assert torch.equal(out[0][:, :rows], out[1][:, :rows])
+        assert product.rel_err(out[0][:, :rows].cpu().numpy(), out[1][:, :rows].cpu().numpy().astype(np.float64)) <= 1e-6
+        assert bool(torch.isnan(out[0][:, rows:]).all())

@@ -27,7 +27,10 @@
 //     lane l at word 32 i + l), so the data-dependent lookups never collide on a bank.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "gsq_common.cuh"
+#include "gsq_quant.cuh"
 #include "gsq_tables.h"
 
 namespace cg = cooperative_groups;
@@ -51,7 +54,9 @@ struct GemvArgs {
   int64_t row_bytes;
   int nrows;
   int k;
-  const uint8_t* xq8;
+  const uint8_t* xq8;  // block_q8_1; RAWX: X [m, k] in x_dtype, rows x_stride elements apart, x_vec: 16-byte aligned
+  int x_dtype, x_vec;
+  int64_t x_stride;
   void* y;
   int y_dtype;
   int64_t ldy;
@@ -232,9 +237,10 @@ struct Rec<KIND_Q6K> {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Decode + dot. Activations are block_q8_1 in global memory (L1-cached reads).
+// Decode + dot. Activations are block_q8_1 in global memory (L1-cached reads) or, CtxShared, in shared memory.
 
 struct Ctx {
+  static constexpr bool shared_x = false;
   const uint8_t* xq8;    // [m][k/32] blocks of 36 bytes
   const uint32_t* grid;  // replicated IQ3_S codebook (shared memory)
   int k;
@@ -243,6 +249,14 @@ struct Ctx {
   int* dump;
   int dump_rows, dump_m0;
 };
+struct CtxShared : Ctx {
+  static constexpr bool shared_x = true;
+};
+template <typename C>
+__device__ __forceinline__ uint32_t ldx(const uint32_t* p) {
+  if constexpr (C::shared_x) return *p;
+  else return __ldg(p);
+}
 
 __device__ __forceinline__ void dump_add(const Ctx& cx, int m, int row, int group, int groups, int v) {
   if (row < cx.dump_rows) atomicAdd(cx.dump + ((int64_t)(cx.dump_m0 + m) * cx.dump_rows + row) * groups + group, v);
@@ -260,9 +274,9 @@ __device__ __forceinline__ const uint32_t* q8_block(const Ctx& cx, int m, int bl
 
 // wv[i][e] = 4 signed int8 of group e (values 4e..4e+3 of the lane's slice) of row i; common dot loop of
 // the kinds whose lane owns one whole 32-value slice with a single integer sub-scale.
-template <int M, bool DUMP>
+template <int M, bool DUMP, typename C>
 __device__ __forceinline__ void dot_slice(const int (&wv)[4][8], const int (&isc)[4], const float (&dw)[4],
-                                          const Ctx& cx, int blk, int row_base, int row_step, float (&acc)[4][M]) {
+                                          const C& cx, int blk, int row_base, int row_step, float (&acc)[4][M]) {
   float dws[4];  // d_w times the integer sub-scale: exact in fp32 (11-bit by 6-bit significands)
 #pragma unroll
   for (int i = 0; i < 4; ++i) dws[i] = dw[i] * (float)isc[i];
@@ -271,8 +285,8 @@ __device__ __forceinline__ void dot_slice(const int (&wv)[4][8], const int (&isc
     const uint32_t* b = q8_block(cx, m, blk);
     int u[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) u[e] = (int)__ldg(b + 1 + e);  // word 0 of a block is (d, sum), the quants follow
-    const float d8 = h2f(__ldg(b));
+    for (int e = 0; e < 8; ++e) u[e] = (int)ldx<C>(b + 1 + e);  // word 0 of a block is (d, sum), the quants follow
+    const float d8 = h2f(ldx<C>(b));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       int sumi = 0;
@@ -291,9 +305,9 @@ __device__ __forceinline__ void dot_slice(const int (&wv)[4][8], const int (&isc
 // A group's signed word is then one byte permute of the pair, the selector built from the record's sign bits.
 // The lane dots its two groups of each slice of rows g and g + 8 (accumulator rows 0 and 1; 2 and 3 stay zero);
 // the four lanes of a row group add up when the tile is left.
-template <int M, int RS, bool DUMP>
+template <int M, int RS, bool DUMP, typename C>
 __device__ __forceinline__ void accumulate(const Rec<KIND_IQ3S_PACKED>& r, int row0, int rec, int lane, bool ok,
-                                           const Ctx& cx, float (&acc)[4][M]) {
+                                           const C& cx, float (&acc)[4][M]) {
   (void)ok;
   const uint32_t lane_off = (uint32_t)(lane & 15) << 3;
   const char* gbase = reinterpret_cast<const char*>(cx.grid);
@@ -327,8 +341,8 @@ __device__ __forceinline__ void accumulate(const Rec<KIND_IQ3S_PACKED>& r, int r
 #pragma unroll
     for (int m = 0; m < M; ++m) {
       const uint32_t* b = q8_block(cx, m, blk);
-      const int u0 = (int)__ldg(b + 1 + 2 * t), u1 = (int)__ldg(b + 2 + 2 * t);
-      const float d8 = h2f(__ldg(b));
+      const int u0 = (int)ldx<C>(b + 1 + 2 * t), u1 = (int)ldx<C>(b + 2 + 2 * t);
+      const float d8 = h2f(ldx<C>(b));
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int sumi = dp4a(wv[h][1], u1, dp4a(wv[h][0], u0, 0));
@@ -340,9 +354,9 @@ __device__ __forceinline__ void accumulate(const Rec<KIND_IQ3S_PACKED>& r, int r
   }
 }
 
-template <int M, int RS, bool DUMP>
+template <int M, int RS, bool DUMP, typename C>
 __device__ __forceinline__ void accumulate(const Rec<KIND_IQ3S_RAW>& r, int row0, int rec, int lane, bool ok,
-                                           const Ctx& cx, float (&acc)[4][M]) {
+                                           const C& cx, float (&acc)[4][M]) {
   if (!ok) return;
   const uint32_t lane_off = (uint32_t)(lane & 15) << 3;
   const char* gbase = reinterpret_cast<const char*>(cx.grid);
@@ -377,9 +391,9 @@ __device__ __forceinline__ void iq4_lookup(uint32_t v, uint32_t& lo, uint32_t& h
   hi = prmt(r01, r23, 0x7531u);
 }
 
-template <int M, int RS, bool DUMP>
+template <int M, int RS, bool DUMP, typename C>
 __device__ __forceinline__ void accumulate(const Rec<KIND_IQ4XS>& r, int row0, int rec, int lane, bool ok,
-                                           const Ctx& cx, float (&acc)[4][M]) {
+                                           const C& cx, float (&acc)[4][M]) {
   if (!ok) return;
   const int p = lane & 7;
   int wv[4][8];
@@ -410,9 +424,9 @@ __device__ __forceinline__ void accumulate(const Rec<KIND_IQ4XS>& r, int row0, i
 // with q16[] the bytes taken as six halfwords. Integer sums become floats by adding the bit pattern of
 // 1.5 * 2^23 inside the integer multiply-add and subtracting it again as a float (exact below 2^22), which
 // keeps the conversions off the slow conversion pipe.
-template <int M, int RS, bool DUMP>
+template <int M, int RS, bool DUMP, typename C>
 __device__ __forceinline__ void accumulate(const Rec<KIND_Q4K>& r, int row0, int rec, int lane, bool ok,
-                                           const Ctx& cx, float (&acc)[4][M]) {
+                                           const C& cx, float (&acc)[4][M]) {
   if (!ok) return;
   const int p = lane & 7, jj = p >> 1, half = p & 1;
   const bool lo4 = jj < 2;
@@ -450,10 +464,10 @@ __device__ __forceinline__ void accumulate(const Rec<KIND_Q4K>& r, int row0, int
     int u0[4], u1[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      u0[e] = (int)__ldg(bm + e);
-      u1[e] = (int)__ldg(bm + 9 + e);
+      u0[e] = (int)ldx<C>(bm + e);
+      u1[e] = (int)ldx<C>(bm + 9 + e);
     }
-    const float d80 = h2f(__ldg(bm - 1 - 4 * half)), d81 = h2f(__ldg(bm + 8 - 4 * half));
+    const float d80 = h2f(ldx<C>(bm - 1 - 4 * half)), d81 = h2f(ldx<C>(bm + 8 - 4 * half));
     // sum of the activation quants this lane pairs with its 16 + 16 weights (the min term's factor)
     int q0 = 0, q1 = 0;
 #pragma unroll
@@ -482,9 +496,9 @@ __device__ __forceinline__ void accumulate(const Rec<KIND_Q4K>& r, int row0, int
   }
 }
 
-template <int M, int RS, bool DUMP>
+template <int M, int RS, bool DUMP, typename C>
 __device__ __forceinline__ void accumulate(const Rec<KIND_Q6K>& r, int row0, int rec, int lane, bool ok,
-                                           const Ctx& cx, float (&acc)[4][M]) {
+                                           const C& cx, float (&acc)[4][M]) {
   (void)ok;
   const int n = lane >> 4, w16 = lane & 15;
   const int blk = rec * 8 + 4 * n + (w16 >> 3);
@@ -505,8 +519,8 @@ __device__ __forceinline__ void accumulate(const Rec<KIND_Q6K>& r, int row0, int
   for (int m = 0; m < M; ++m) {
     const uint32_t* b0 = q8_block(cx, m, blk);
     const uint32_t* b1 = q8_block(cx, m, blk + 2);  // 64 values further
-    const int u0 = (int)__ldg(b0 + 1 + (w16 & 7)), u1 = (int)__ldg(b1 + 1 + (w16 & 7));
-    const float d80 = h2f(__ldg(b0)), d81 = h2f(__ldg(b1));
+    const int u0 = (int)ldx<C>(b0 + 1 + (w16 & 7)), u1 = (int)ldx<C>(b1 + 1 + (w16 & 7));
+    const float d80 = h2f(ldx<C>(b0)), d81 = h2f(ldx<C>(b1));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int p0 = dp4a(v0[i], u0, 0), p1 = dp4a(v1[i], u1, 0);
@@ -603,7 +617,35 @@ __host__ __device__ inline size_t gemv_smem_bytes(int kind, int rs, int m, int s
 }
 
 // TMA: weights come through a per-warp ring of bulk copies (cp.async.bulk + mbarrier) instead of direct loads.
-template <int KIND, int M, int RS, bool DUMP, bool TMA>
+// X -> block_q8_1 in shared memory (RAWX): the quantiser's own arithmetic (gsq_quantize.cu), all of X in every CTA.
+template <typename T, bool VEC, int M>
+__device__ __forceinline__ void stage_x(const GemvArgs& a, uint8_t* blocks) {
+  const int per_row = a.k >> 3, total = M * per_row;
+  // all of a thread's loads before the first value is used; whole warps stay together (the shuffles of a 32-value block)
+  constexpr int U = 4;
+  for (int t0 = 0; t0 < total; t0 += U * GEMV_THREADS) {
+    float v[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * GEMV_THREADS + (int)threadIdx.x, row = M == 1 ? 0 : t / per_row;
+      if (t < total) {
+        load8<T, VEC>(reinterpret_cast<const T*>(a.xq8), row * a.x_stride + (t - row * per_row) * 8, v[u]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[u][e] = 0.0f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * GEMV_THREADS + (int)threadIdx.x;
+      if (t0 + u * GEMV_THREADS < total) q8_1_store8(v[u], t < total, blocks + (t >> 2) * 36, t & 3);   // (k % 32 == 0: block t / 4 of all rows)
+    }
+  }
+  __syncthreads();
+}
+
+// RAWX: X itself comes in and is quantised by every CTA (gemv_raw_host).
+template <int KIND, int M, int RS, bool DUMP, bool TMA, bool RAWX>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_kernel(const GemvArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int TR = KindTraits<KIND>::tile_rows;
@@ -630,7 +672,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_kernel(const GemvArgs a)
   const uint32_t ring_u32 = smem_u32(ring);
   const uint32_t bars_u32 = smem_u32(sp + (size_t)GEMV_WARPS * stages * RECB) + (uint32_t)(warp * stages * 8);
 
-  Ctx cx;
+  std::conditional_t<RAWX, CtxShared, Ctx> cx;
   cx.xq8 = a.xq8; cx.grid = grid_s; cx.k = a.k; cx.nb32 = a.k >> 5;
   cx.dump = a.dump; cx.dump_rows = a.nrows; cx.dump_m0 = a.dump_m0;
 
@@ -685,6 +727,21 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_kernel(const GemvArgs a)
   // Up to here nothing depends on the kernel that wrote the activations: launched with programmatic stream
   // serialisation, the first weight loads and the codebook copy overlap its tail (a no-op otherwise).
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if constexpr (RAWX) {
+    // (behind the ring and its barriers; 16-byte aligned, as are they)
+    uint8_t* const blocks = sp + (TMA ? (size_t)GEMV_WARPS * stages * (RECB + 8) : 0);
+    if (a.x_dtype == GSQ_F32) {
+      if (a.x_vec) stage_x<float, true, M>(a, blocks);
+      else stage_x<float, false, M>(a, blocks);
+    } else if (a.x_dtype == GSQ_F16) {
+      if (a.x_vec) stage_x<__half, true, M>(a, blocks);
+      else stage_x<__half, false, M>(a, blocks);
+    } else {
+      if (a.x_vec) stage_x<__nv_bfloat16, true, M>(a, blocks);
+      else stage_x<__nv_bfloat16, false, M>(a, blocks);
+    }
+    cx.xq8 = blocks;
+  }
   for (int t0 = 0; t0 < tile_cnt; t0 += a.tiles_round) {
     const int tiles_r = min(a.tiles_round, tile_cnt - t0);
     const int rr = tiles_r * nrec;
@@ -831,7 +888,7 @@ struct ClusterPlan {
 };
 
 // Per kernel instantiation and device: the cluster size that keeps most SMs busy with every cluster resident.
-template <int KIND, int M, int RS, bool DUMP, bool TMA>
+template <int KIND, int M, int RS, bool DUMP, bool TMA, bool RAWX>
 static int plan_clusters(size_t smem, int sm_count, ClusterPlan* out) {
   static ClusterPlan cache[32];
   static bool have[32];
@@ -841,7 +898,7 @@ static int plan_clusters(size_t smem, int sm_count, ClusterPlan* out) {
     *out = cache[dev];
     return GSQ_OK;
   }
-  auto kern = gemv_kernel<KIND, M, RS, DUMP, TMA>;
+  auto kern = gemv_kernel<KIND, M, RS, DUMP, TMA, RAWX>;
   GSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   ClusterPlan best{1, sm_count};
   for (int cs : {4, 2}) {
@@ -873,20 +930,22 @@ static int plan_clusters(size_t smem, int sm_count, ClusterPlan* out) {
   return GSQ_OK;
 }
 
-template <int KIND, int M, int RS, bool DUMP, bool TMA>
+template <int KIND, int M, int RS, bool DUMP, bool TMA, bool RAWX>
 static int launch_gemv_t(GemvArgs a, int sm_count, int max_smem, cudaStream_t st) {
-  // ring depth: the deepest power of two that fits beside the codebook and the partial sums
+  // ring depth: the deepest power of two that fits beside the codebook and the partial sums (and the blocks of X)
+  const size_t blocks = RAWX ? (size_t)M * (a.k >> 5) * 36 : 0;
   int shift = 0;
   if (TMA) {
     shift = 2;
-    while (shift > 1 && gemv_smem_bytes(KIND, RS, M, 1 << shift) > (size_t)max_smem) --shift;
+    while (shift > 1 && gemv_smem_bytes(KIND, RS, M, 1 << shift) + blocks > (size_t)max_smem) --shift;
   }
   a.stage_shift = shift;
   if (TMA) a.nrec = ((a.k >> 8) + KindTraits<KIND>::rec_sb * SUB - 1) / (KindTraits<KIND>::rec_sb * SUB);
-  const size_t smem = gemv_smem_bytes(KIND, RS, M, TMA ? 1 << shift : 0);
+  const size_t smem = gemv_smem_bytes(KIND, RS, M, TMA ? 1 << shift : 0) + blocks;
   if (smem > (size_t)max_smem) return GSQ_ERR_TOO_LARGE;
   ClusterPlan plan;
-  int rc = plan_clusters<KIND, M, RS, DUMP, TMA>(smem, sm_count, &plan);
+  // (kept per instantiation: with X inside for the most shared memory that it may take, which differs with K)
+  int rc = plan_clusters<KIND, M, RS, DUMP, TMA, RAWX>(RAWX ? (size_t)max_smem : smem, sm_count, &plan);
   if (rc != GSQ_OK) return rc;
   const int wc = plan.cs * GEMV_WARPS;
   a.tiles_base = a.ntiles / plan.clusters;
@@ -906,19 +965,19 @@ static int launch_gemv_t(GemvArgs a, int sm_count, int max_smem, cudaStream_t st
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_kernel<KIND, M, RS, DUMP, TMA>, a));
+  GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_kernel<KIND, M, RS, DUMP, TMA, RAWX>, a));
   return GSQ_OK;
 }
 
 // The staged variant needs 16-byte aligned row segments of whole 16-byte multiples: always true for packed
 // IQ3_S and Q4_K (144-byte blocks), for IQ4_XS (136-byte blocks) only when K is a multiple of 1024.
-template <int KIND, int M, int RS, bool DUMP = false>
+template <int KIND, int M, int RS, bool DUMP = false, bool RAWX = false>
 static int launch_gemv(const GemvArgs& a, int sm_count, int max_smem, cudaStream_t st) {
   constexpr bool can = KIND == KIND_IQ3S_PACKED || KIND == KIND_Q4K || KIND == KIND_IQ4XS;
   if constexpr (can && !DUMP) {
-    if (!a.force_direct && (KIND != KIND_IQ4XS || a.k % 1024 == 0)) return launch_gemv_t<KIND, M, RS, DUMP, true>(a, sm_count, max_smem, st);
+    if (!a.force_direct && (KIND != KIND_IQ4XS || a.k % 1024 == 0)) return launch_gemv_t<KIND, M, RS, DUMP, true, RAWX>(a, sm_count, max_smem, st);
   }
-  return launch_gemv_t<KIND, M, RS, DUMP, false>(a, sm_count, max_smem, st);
+  return launch_gemv_t<KIND, M, RS, DUMP, false, RAWX>(a, sm_count, max_smem, st);
 }
 
 template <int KIND, int RS>
@@ -946,7 +1005,7 @@ int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int 
 
 static int gemv_host_dp4a(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x_q8,
                           int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
-                          int dump_m0);
+                          int dump_m0, int x_dtype = -1, int64_t x_row_stride = 0);
 
 // gsq_gemv_f1.cu
 bool gemv_f1_applies(int ggml_type);
@@ -997,10 +1056,10 @@ static int gemv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_ty
   return gemv_host_dp4a(w, row_bytes, rows, ggml_type, packed, x_q8, m, k, y, y_dtype, y_row_stride, stream, dump, dump_m0);
 }
 
-// The dp4a kernel proper: 1..8 activation rows.
+// The dp4a kernel proper: 1..8 activation rows. x_dtype >= 0: x_q8 is X itself (rows x_row_stride elements apart).
 static int gemv_host_dp4a(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x_q8,
                           int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
-                          int dump_m0) {
+                          int dump_m0, int x_dtype, int64_t x_row_stride) {
   if (m == 0 || rows == 0) return GSQ_OK;
   if (m < 0 || m > 8 || rows < 0 || k <= 0 || k % 256 != 0 || !w || !x_q8 || !y) return GSQ_ERR_UNSUPPORTED;
   if (rows > INT32_MAX || k > INT32_MAX) return GSQ_ERR_TOO_LARGE;
@@ -1029,6 +1088,9 @@ static int gemv_host_dp4a(const void* w, int64_t row_bytes, int64_t rows, int gg
   a.nrows = (int)rows;
   a.k = (int)k;
   a.xq8 = (const uint8_t*)x_q8;
+  a.x_dtype = x_dtype;
+  a.x_vec = (uintptr_t)x_q8 % 16 == 0 && (x_row_stride * (x_dtype == GSQ_F32 ? 4 : 2)) % 16 == 0;
+  a.x_stride = x_row_stride;
   a.y = y;
   a.y_dtype = y_dtype;
   a.ldy = y_row_stride;
@@ -1053,6 +1115,13 @@ static int gemv_host_dp4a(const void* w, int64_t row_bytes, int64_t rows, int gg
       default: return launch_gemv<KIND_Q6K, 1, 7, true>(a, sms, smem, st);
     }
   }
+  if (x_dtype >= 0) {
+    if (kind == KIND_Q4K && m == 1) return launch_gemv<KIND_Q4K, 1, 7, false, true>(a, sms, smem, st);
+    if (kind == KIND_IQ4XS && m == 1) return launch_gemv<KIND_IQ4XS, 1, 7, false, true>(a, sms, smem, st);
+    if (kind == KIND_IQ4XS && m == 2) return launch_gemv<KIND_IQ4XS, 2, 7, false, true>(a, sms, smem, st);
+    if (kind == KIND_IQ4XS && m == 3) return launch_gemv<KIND_IQ4XS, 3, 7, false, true>(a, sms, smem, st);
+    return GSQ_ERR_UNSUPPORTED;
+  }
   switch (kind) {
     case KIND_IQ3S_PACKED: return launch_gemv_m<KIND_IQ3S_PACKED, 7>((int)m, a, sms, smem, st);
     case KIND_IQ3S_RAW: return launch_gemv_m<KIND_IQ3S_RAW, 7>((int)m, a, sms, smem, st);
@@ -1060,6 +1129,19 @@ static int gemv_host_dp4a(const void* w, int64_t row_bytes, int64_t rows, int gg
     case KIND_IQ4XS: return launch_gemv_m<KIND_IQ4XS, 7>((int)m, a, sms, smem, st);
     default: return launch_gemv_m<KIND_Q6K, 7>((int)m, a, sms, smem, st);
   }
+}
+
+// The same with X quantised inside the kernel: one launch instead of two, at the rows at which these types have this kernel, up
+// to 8192 values of X. There the GPU needs as long either way (us, here / two kernels: Q4_K 1 row 5120 x 5120 8.8 / 8.8,
+// 17408 x 5120 16.6 / 17.2, 2048 x 5120 6.7 / 6.4; IQ4_XS 10.3 / 10.1 and 21.0 / 20.8) and the host 2 us less, which is what
+// calls one by one wait for (Q4_K 5120 x 5120, 1 row: 9.65 -> 7.58). Beyond, every CTA quantising all of X costs more than the
+// launch (Q4_K 5120 x 17408 1 row 18.5 / 17.3; IQ4_XS 5120 x 5120 2 rows 11.8 / 10.9): GSQ_ERR_UNSUPPORTED.
+int gemv_raw_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
+                  int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* stream) {
+  if (packed || m < 1 || m > (ggml_type == GSQ_TYPE_Q4_K ? 1 : ggml_type == GSQ_TYPE_IQ4_XS ? 3 : 0) || m * k > 8192 || g_force_direct || g_force_cluster ||
+      (x_dtype != GSQ_F32 && x_dtype != GSQ_F16 && x_dtype != GSQ_BF16))
+    return GSQ_ERR_UNSUPPORTED;
+  return gemv_host_dp4a(w, row_bytes, rows, ggml_type, packed, x, m, k, y, y_dtype, y_row_stride, stream, nullptr, 0, x_dtype, x_row_stride);
 }
 
 }  // namespace gsq

@@ -38,6 +38,9 @@ bool gemm4_applies(int ggml_type, int packed, int64_t rows);
 size_t gemm4_scratch_bytes(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k, int hu);
 int gemm4_linear(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
                  int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* scratch, int hu, void* stream);
+// gsq_gemv.cu
+int gemv_raw_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
+                  int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* stream);
 // gsq_quantize.cu
 int quantize_tiles_host(const void* x, int x_dtype, int64_t m, int64_t k, int64_t stride, int layout, void* out, void* stream);
 // gsq_gemm.cu
@@ -283,7 +286,11 @@ extern "C" int gsq_linear_vec(const void* w, int64_t row_bytes, int64_t rows, in
   using namespace gsq;
   if (m == 0 || rows == 0) return GSQ_OK;
   if (m < 0 || m > 8 || rows < 0 || k <= 0 || k % 256 != 0 || !w || !x || !y) return GSQ_ERR_UNSUPPORTED;
-  if (!mmv_raw_applies(ggml_type, packed, rows, m, k, 1)) return GSQ_ERR_UNSUPPORTED;
+  if (!mmv_raw_applies(ggml_type, packed, rows, m, k, 1)) {
+    if (small_batch(ggml_type, packed, rows, m, k)) return GSQ_ERR_UNSUPPORTED;   // (that kernel on blocks)
+    const int rc = gemv_raw_host(w, row_bytes, rows, ggml_type, packed, x, x_dtype, m, k, x_row_stride, y, y_dtype, y_row_stride, stream);
+    return rc == GSQ_ERR_TOO_LARGE ? GSQ_ERR_UNSUPPORTED : rc;   // (X does not fit)
+  }
   const int rc = mmv_host(w, row_bytes, rows, ggml_type, packed, x, 2, m, k, y, y_dtype, y_row_stride, stream, nullptr, nullptr, x_dtype,
                           x_row_stride);
   return rc == 1000 ? GSQ_ERR_UNSUPPORTED : rc;

@@ -12,40 +12,6 @@
 
 namespace gsq {
 
-__device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d) {
-  // float -> int8 as the C conversion in the reference (round toward zero of an already rounded value)
-  const int ia = (int)a, ib = (int)b, ic = (int)c, id = (int)d;
-  return (uint32_t)(ia & 0xFF) | ((uint32_t)(ib & 0xFF) << 8) | ((uint32_t)(ic & 0xFF) << 16) | ((uint32_t)(id & 0xFF) << 24);
-}
-
-// This thread's 8 consecutive values (piece `piece` of the 32-value block its 4 adjacent lanes share) -> block_q8_1 at
-// `b`. All 32 lanes of the warp must call it (shuffles); dead lanes pass zeros and live = false.
-__device__ __forceinline__ void q8_1_store8(const float (&v)[8], bool live, uint8_t* b, int piece) {
-  float amax = 0.0f;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
-  amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
-  amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-  float s[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) s[e] = v[e] + __shfl_xor_sync(0xFFFFFFFFu, v[e], 2);  // lane offset 16
-#pragma unroll
-  for (int e = 0; e < 8; ++e) s[e] = s[e] + __shfl_xor_sync(0xFFFFFFFFu, s[e], 1);  // lane offset 8
-  const float s0 = s[0] + s[4], s1 = s[1] + s[5], s2 = s[2] + s[6], s3 = s[3] + s[7];  // offset 4
-  const float sum = (s0 + s2) + (s1 + s3);                                              // offsets 2, 1
-  if (!live) return;
-  const float d = div_approx(amax, 127.0f);
-  float q[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) q[e] = amax == 0.0f ? 0.0f : roundf(div_approx(v[e], d));
-  uint32_t* q32 = reinterpret_cast<uint32_t*>(b + 4 + piece * 8);  // the quants follow the (d, sum) pair
-  q32[0] = pack4(q[0], q[1], q[2], q[3]);
-  q32[1] = pack4(q[4], q[5], q[6], q[7]);
-  if (piece == 0) {
-    *reinterpret_cast<__half2*>(b) = __floats2half2_rn(d, sum);
-  }
-}
-
 // MMVQ layout: block_q8_1 = half d, half sum, 32 x int8 (36 bytes).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) quantize_q8_1_kernel(const T* __restrict__ x, uint8_t* __restrict__ out,
