@@ -183,6 +183,23 @@ int gsq_linear_vec(const void* w, int64_t row_bytes, int64_t rows, int ggml_type
                    int64_t m, int64_t k, int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* stream);
 
 /*
+ * Two 1..8-row products of the same activations in one launch: a fused layer whose shards are of two types (Q4_K, IQ3_S or
+ * IQ4_XS first and Q6_K second, IQ3_S first and IQ4_XS second). x: block_q8_1 of m rows (x_dtype = -1) or X as for
+ * gsq_linear_vec. Results: those of gsq_mul_mat_vec_q8 per weight up to the order of the fp32 sums. Not in the reference.
+ * GSQ_ERR_UNSUPPORTED, nothing launched, for other types and for shapes that one launch does not serve: use two calls then.
+ */
+typedef struct gsq_weight {
+  const void* w;
+  int64_t row_bytes, rows;
+  int ggml_type, packed;
+  void* y;               /* first result of its rows; rows y_row_stride elements apart */
+} gsq_weight;
+int gsq_linear_vec_pair(const gsq_weight* a, const gsq_weight* b, const void* x, int x_dtype, int64_t m, int64_t k, int64_t x_row_stride,
+                        int y_dtype, int64_t y_row_stride, void* stream);
+/* 1 where the call above has a kernel for the two weights' types and layouts at m rows of block_q8_1 (it may still refuse the shape) */
+int gsq_linear_vec_pair_serves(const gsq_weight* a, const gsq_weight* b, int64_t m);
+
+/*
  * No counterpart in the reference (its shim always takes scratch from torch's allocator, lcpp_shim.cu:250-263).
  * Quantise X and run the 1..8-row GEMV in one call without any buffer from the caller besides X, W and Y:
  * the q8_1 blocks in between are kept in a fixed device array inside the library. For hosts that cannot

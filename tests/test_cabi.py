@@ -36,6 +36,29 @@ def test_host_only_entry_points():
     assert lib.gsq_iq3s_repack(None, 0, 220, 0, None) == 0
 
 
+def test_pairs_that_one_launch_serves():
+    """Two weights of a fused layer: the listed pairs of types, at the rows of the small-batch kernel, repacked where that reads
+    repacked weights; everything else is refused before the GPU is touched."""
+    lib, first = _cabi.lib, {12: 2, 21: 1, 23: 4}      # fewest rows of Q4_K, IQ3_S, IQ4_XS
+
+    def weight(t, rows=64, k=512):
+        return _cabi.Weight(1, k // 256 * lib.gsq_type_block_bytes(t), rows, t, int(t in (14, 21)), 1)
+
+    for ta in (10, 12, 14, 21, 23):
+        for tb in (10, 12, 14, 21, 23):
+            for m in range(0, 10):
+                want = (tb == 14 and ta in first or (ta, tb) == (21, 23)) and max(first[ta], first.get(tb, 1)) <= m <= 8
+                a, b = weight(ta), weight(tb)
+                assert lib.gsq_linear_vec_pair_serves(a, b, m) == int(want), (ta, tb, m)
+                if not want:
+                    assert lib.gsq_linear_vec_pair(a, b, 1, -1, m, 512, 0, 0, 128, None) == _cabi.ERR_UNSUPPORTED
+    for bad in (weight(14, rows=40), weight(14, k=768)):
+        assert lib.gsq_linear_vec_pair(weight(21), bad, 1, -1, 4, 512, 0, 0, 128, None) == _cabi.ERR_UNSUPPORTED
+    unpacked = weight(21)
+    unpacked.packed = 0
+    assert lib.gsq_linear_vec_pair_serves(unpacked, weight(14), 4) == 0
+
+
 def test_repacked_weights_of_ragged_rows_are_refused():
     """Repacked IQ3_S / Q6_K are records of 16 rows. gsq_linear and gsq_linear_vec refuse any other row count before they
     touch the device, at every number of activation rows (from 25 on the weights used to be expanded record by record,

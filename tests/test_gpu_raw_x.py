@@ -94,3 +94,44 @@ def test_dp4a_product_quantises_as_the_kernel_in_front(name, ms, dtype, rows, k,
             assert torch.equal(out[0][:, :rows], out[1][:, :rows])
         assert product.rel_err(out[0][:, :rows].cpu().numpy(), out[1][:, :rows].cpu().numpy().astype(np.float64)) <= 1e-6
         assert bool(torch.isnan(out[0][:, rows:]).all())
+
+
+@pytest.mark.parametrize("pair", [("Q4_K", "Q6_K"), ("IQ3_S", "Q6_K"), ("IQ4_XS", "Q6_K"), ("IQ3_S", "IQ4_XS")])
+@pytest.mark.parametrize("rows,k", [((16, 16), 256), ((48, 2064), 768), ((6144, 1024), 5120), ((1024, 34816), 2560), ((512, 256), 17408)])
+def test_two_products_in_one_launch(pair, rows, k):
+    """A fused layer of two types in one launch: what a call per type gives, up to the order of the fp32 sums; from blocks and, where
+    both products take X, from X."""
+    lib, st = _cabi.lib, torch.cuda.current_stream().cuda_stream
+    raws = [synth.make_weight(TYPES[n], r, k, 97 + r) for n, r in zip(pair, rows)]
+    ws = [torch.from_numpy(raw).to(DEV) for raw in raws]
+    for n, w in zip(pair, ws):
+        if n in ("IQ3_S", "Q6_K"):
+            iq3_pack.pack_(w, TYPES[n])
+    total = sum(rows)
+    for m in (1, 2, 4, 7, 8):
+        x = torch.from_numpy(synth.make_activation(m, k, 98 + m)).to(torch.bfloat16).to(DEV)
+        q8 = torch.empty(m * k // 32 * 36, dtype=torch.uint8, device=DEV)
+        assert lib.gsq_quantize_q8_1(x.data_ptr(), 2, m, k, k, q8.data_ptr(), st) == 0
+        want = torch.full((m, total + 1), float("nan"), device=DEV)
+        y = [torch.full_like(want, float("nan")) for _ in range(2)]
+
+        def weights(out):
+            return [_cabi.Weight(w.data_ptr(), w.shape[1], r, TYPES[n], int(n in ("IQ3_S", "Q6_K")), out.data_ptr() + 4 * c)
+                    for n, w, r, c in zip(pair, ws, rows, (0, rows[0]))]
+
+        for g in weights(want):
+            assert lib.gsq_mul_mat_vec_q8(g.w, g.row_bytes, g.rows, g.ggml_type, g.packed, q8.data_ptr(), m, k, g.y, 0, total + 1, st) == 0
+        a, b = weights(y[0])
+        served = lib.gsq_linear_vec_pair_serves(a, b, m)
+        rc = lib.gsq_linear_vec_pair(a, b, q8.data_ptr(), -1, m, k, 0, 0, total + 1, st)
+        assert rc == (0 if served else UNSUPPORTED)
+        a, b = weights(y[1])
+        rx = lib.gsq_linear_vec_pair(a, b, x.data_ptr(), 2, m, k, k, 0, total + 1, st)
+        assert rx in (0, UNSUPPORTED) and (rx == UNSUPPORTED or served)
+        for code, got in ((rc, y[0]), (rx, y[1])):
+            if code == 0:
+                assert bool(torch.isnan(got[:, total:]).all())
+                for c, r in ((0, rows[0]), (rows[0], rows[1])):
+                    assert product.rel_err(got[:, c:c + r].cpu().numpy(), want[:, c:c + r].cpu().numpy().astype(np.float64)) <= 1e-6
+            else:
+                assert bool(torch.isnan(got).all())

@@ -70,21 +70,9 @@ bool mmv_raw_applies(int ggml_type, int packed, int64_t rows, int64_t m, int64_t
   }
 }
 
-// x_layout: 0 = block_q8_1, 1 = block_q8_1_mmq. Returns MMV_DECLINED when the shape does not fit.
-// x_layout 4: quantize_rows_host's. x_layout 2 / 3: xq is X itself (x_dtype, rows x_row_stride elements apart), up to 8 / 16 rows.
-int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* xq, int x_layout,
-             int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
-             const gsq_peer_reduce* pr, int x_dtype, int64_t x_row_stride) {
-  if (pr && (m == 0 || rows == 0)) return GSQ_ERR_UNSUPPORTED;   // every rank must launch: nothing to skip
-  if (m == 0 || rows == 0) return GSQ_OK;
-  if (m < 0 || m > 48 || rows < 0 || k <= 0 || k % 256 != 0 || !w || !xq || !y) return GSQ_ERR_UNSUPPORTED;
-  if (rows > INT32_MAX || k > INT32_MAX) return GSQ_ERR_TOO_LARGE;
-  const int bs = block_bytes(ggml_type);
-  if (bs == 0 || row_bytes != (k / 256) * bs) return GSQ_ERR_UNSUPPORTED;
-  if (y_dtype != GSQ_F32 && y_dtype != GSQ_F16 && y_dtype != GSQ_BF16) return GSQ_ERR_UNSUPPORTED;
-  DeviceInfo di;
-  const int rc = device_info(&di);
-  if (rc != GSQ_OK) return rc;
+// the arguments of a product, but for what its launch plan sets
+static MmvArgs mmv_args(const void* w, int64_t row_bytes, int64_t rows, const void* xq, int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride,
+                        int* dump, int x_dtype, int64_t x_row_stride) {
   MmvArgs a;
   a.w = (const uint8_t*)w;
   a.row_bytes = row_bytes;
@@ -110,6 +98,25 @@ int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int 
   a.x_dtype = x_dtype;
   a.x_stride = x_row_stride;
   a.x_vec = (uintptr_t)xq % 16 == 0 && (x_row_stride * (x_dtype == GSQ_F32 ? 4 : 2)) % 16 == 0;
+  return a;
+}
+
+// x_layout: 0 = block_q8_1, 1 = block_q8_1_mmq. Returns MMV_DECLINED when the shape does not fit.
+// x_layout 4: quantize_rows_host's. x_layout 2 / 3: xq is X itself (x_dtype, rows x_row_stride elements apart), up to 8 / 16 rows.
+int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* xq, int x_layout,
+             int64_t m, int64_t k, void* y, int y_dtype, int64_t y_row_stride, void* stream, int* dump,
+             const gsq_peer_reduce* pr, int x_dtype, int64_t x_row_stride) {
+  if (pr && (m == 0 || rows == 0)) return GSQ_ERR_UNSUPPORTED;   // every rank must launch: nothing to skip
+  if (m == 0 || rows == 0) return GSQ_OK;
+  if (m < 0 || m > 48 || rows < 0 || k <= 0 || k % 256 != 0 || !w || !xq || !y) return GSQ_ERR_UNSUPPORTED;
+  if (rows > INT32_MAX || k > INT32_MAX) return GSQ_ERR_TOO_LARGE;
+  const int bs = block_bytes(ggml_type);
+  if (bs == 0 || row_bytes != (k / 256) * bs) return GSQ_ERR_UNSUPPORTED;
+  if (y_dtype != GSQ_F32 && y_dtype != GSQ_F16 && y_dtype != GSQ_BF16) return GSQ_ERR_UNSUPPORTED;
+  DeviceInfo di;
+  const int rc = device_info(&di);
+  if (rc != GSQ_OK) return rc;
+  MmvArgs a = mmv_args(w, row_bytes, rows, xq, m, k, y, y_dtype, y_row_stride, dump, x_dtype, x_row_stride);
   if (x_layout == XL_ROWS && (dump || pr || (uintptr_t)xq % 16 != 0)) return GSQ_ERR_UNSUPPORTED;
   if ((x_layout == XL_XQ81 || x_layout == XL_XMMQ) && ((x_dtype != GSQ_F32 && x_dtype != GSQ_F16 && x_dtype != GSQ_BF16) || dump || pr)) return GSQ_ERR_UNSUPPORTED;
   if (pr) {
@@ -133,6 +140,41 @@ int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int 
     case GSQ_TYPE_Q6_K: return mmv_launch_q6k(a, x_layout, di.sm_count, di.max_smem_optin, st);
     default: return MMV_DECLINED;
   }
+}
+
+// the pairs that mmv_pair_kernel is instantiated for
+static bool mmv_pair_types(int ta, int tb) {
+  return (tb == GSQ_TYPE_Q6_K && (ta == GSQ_TYPE_Q4_K || ta == GSQ_TYPE_IQ3_S || ta == GSQ_TYPE_IQ4_XS)) ||
+         (tb == GSQ_TYPE_IQ4_XS && ta == GSQ_TYPE_IQ3_S);
+}
+bool mmv_pair_serves(const gsq_weight* a, const gsq_weight* b, int64_t m) {
+  return m >= 1 && m <= 8 && mmv_pair_types(a->ggml_type, b->ggml_type) && mmv_applies(a->ggml_type, a->packed, a->rows, m) &&
+         mmv_applies(b->ggml_type, b->packed, b->rows, m);
+}
+
+int mmv_launch_pair_q81(int ta, int tb, const MmvArgs& a, const MmvArgs& b, int sm_count, int max_smem, cudaStream_t st);    // gsq_mmv_pair.cu
+int mmv_launch_pair_xq81(int ta, int tb, const MmvArgs& a, const MmvArgs& b, int sm_count, int max_smem, cudaStream_t st);   // gsq_mmv_pair_x.cu
+
+// Two products of the same activations in one launch (mmv_pair_kernel): 1..8 rows, both types at row counts that this kernel
+// serves. x: block_q8_1 (x_dtype < 0), or X itself where both products would take that (mmv_raw_applies).
+int mmv_pair_host(const gsq_weight* wa, const gsq_weight* wb, const void* x, int x_dtype, int64_t m, int64_t k, int64_t x_row_stride, int y_dtype,
+                  int64_t y_row_stride, void* stream) {
+  if (!mmv_pair_serves(wa, wb, m) || k <= 0 || k % 256 != 0 || k > INT32_MAX || !x || (y_dtype != GSQ_F32 && y_dtype != GSQ_F16 && y_dtype != GSQ_BF16) ||
+      (x_dtype >= 0 && x_dtype != GSQ_F32 && x_dtype != GSQ_F16 && x_dtype != GSQ_BF16))
+    return GSQ_ERR_UNSUPPORTED;
+  for (const gsq_weight* w : {wa, wb}) {
+    const int bs = block_bytes(w->ggml_type);
+    if (!w->w || !w->y || w->rows < 1 || w->rows > INT32_MAX || bs == 0 || w->row_bytes != (k / 256) * bs || (x_dtype >= 0 && !mmv_raw_applies(w->ggml_type, w->packed, w->rows, m, k, 1)))
+      return GSQ_ERR_UNSUPPORTED;
+  }
+  DeviceInfo di;
+  const int rc = device_info(&di);
+  if (rc != GSQ_OK) return rc;
+  const MmvArgs a = mmv_args(wa->w, wa->row_bytes, wa->rows, x, m, k, wa->y, y_dtype, y_row_stride, nullptr, x_dtype, x_row_stride);
+  const MmvArgs b = mmv_args(wb->w, wb->row_bytes, wb->rows, x, m, k, wb->y, y_dtype, y_row_stride, nullptr, x_dtype, x_row_stride);
+  const int r = (x_dtype < 0 ? mmv_launch_pair_q81 : mmv_launch_pair_xq81)(wa->ggml_type, wb->ggml_type, a, b, di.sm_count, di.max_smem_optin,
+                                                                          (cudaStream_t)stream);
+  return r == MMV_DECLINED ? GSQ_ERR_UNSUPPORTED : r;
 }
 
 // Sticky flags of bounded waits that gave up: on a peer GPU, on a bulk copy.
@@ -226,3 +268,10 @@ extern "C" int gsq_debug_mmv_cluster_size(int cs) {
   gsq::g_mmv_cluster = (cs == 1 || cs == 2 || cs == 4 || cs == 8) ? cs : 0;
   return old;
 }
+
+extern "C" int gsq_linear_vec_pair(const gsq_weight* a, const gsq_weight* b, const void* x, int x_dtype, int64_t m, int64_t k, int64_t x_row_stride,
+                                   int y_dtype, int64_t y_row_stride, void* stream) {
+  if (!a || !b) return GSQ_ERR_UNSUPPORTED;
+  return gsq::mmv_pair_host(a, b, x, x_dtype, m, k, x_row_stride, y_dtype, y_row_stride, stream);
+}
+extern "C" int gsq_linear_vec_pair_serves(const gsq_weight* a, const gsq_weight* b, int64_t m) { return a && b && gsq::mmv_pair_serves(a, b, m) ? 1 : 0; }

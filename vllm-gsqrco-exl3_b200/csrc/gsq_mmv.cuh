@@ -32,6 +32,7 @@
 #include <cooperative_groups.h>
 
 #include <cstdio>
+#include <type_traits>
 
 #include "gsq_common.cuh"
 #include "gsq_quant.cuh"
@@ -1136,9 +1137,10 @@ __host__ __device__ inline void mmv_k_range(int nsb, int cs, int rank, int* firs
 }
 
 // FUSED: the instantiation that also sums the result over the GPUs (see the end of the kernel); the plain product is
-// a separate instantiation so that it carries none of that code or of its registers.
-template <int KIND, int NTL, int XL, bool DUMP, bool FUSED = false>
-__global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
+// a separate instantiation so that it carries none of that code or of its registers. `block`: this CTA's number among those of
+// the product.
+template <int KIND, int NTL, int XL, bool DUMP, bool FUSED>
+__device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
   extern __shared__ __align__(128) uint8_t smem[];
   using Rec = typename MmvKind<KIND>::Rec;
   constexpr bool DS = MmvKind<KIND>::DS;
@@ -1146,7 +1148,7 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
   constexpr int SEGF = MMV_TR * MC;          // floats per parked tile segment
   cg::cluster_group cluster = cg::this_cluster();
   const int cs = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-  const int cluster_id = (int)blockIdx.x / cs;
+  const int cluster_id = block / cs;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int nsb = a.k >> 8;
@@ -1477,6 +1479,21 @@ __global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
   }
 }
 
+template <int KIND, int NTL, int XL, bool DUMP, bool FUSED = false>
+__global__ void __launch_bounds__(MMV_THREADS, 1) mmv_kernel(const MmvArgs a) {
+  mmv_body<KIND, NTL, XL, DUMP, FUSED>(a, (int)blockIdx.x);
+}
+
+// Two products of the same activations with weights of two types (a fused layer whose shards differ), side by side: the first
+// `blocks_a` CTAs work on the one, the rest on the other. A launch of its own for the smaller one costs what a small product
+// costs at least, 5 to 7 us, and waits for the larger one to finish (qkv of 5120 + 1024 rows IQ3_S and 1024 rows Q6_K x 5120, 4
+// rows: 17.7 -> 12.5 us with the quantiser in front).
+template <int KA, int KB, int XL>
+__global__ void __launch_bounds__(MMV_THREADS, 1) mmv_pair_kernel(const MmvArgs a, const MmvArgs b, const int blocks_a) {
+  if ((int)blockIdx.x < blocks_a) mmv_body<KA, 1, XL, false, false>(a, (int)blockIdx.x);
+  else mmv_body<KB, 1, XL, false, false>(b, (int)blockIdx.x - blocks_a);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Launch. (The experiment settings are defined in gsq_mmv.cu.)
 
@@ -1484,25 +1501,25 @@ extern int g_mmv_cluster, g_mmv_pdl, g_mmv_pf_first, g_mmv_aligned, g_mmv_trace;
 
 constexpr int MMV_DECLINED = 1000;  // mmv_host: this shape does not fit; use another kernel
 
-// co-resident clusters of `cs` CTAs with `smem` bytes each (cached per device / size class)
-template <int KIND, int NTL, int XL, bool DUMP>
-static int mmv_max_clusters(int cs, size_t smem, int sm_count, int* out) {
+// co-resident clusters of `cs` CTAs with `smem` bytes each (cached per kernel, device and size class)
+struct MmvOccupancy {
   struct Entry { int dev, cs, kb, n; };
-  static Entry cache[64];
-  static int used = 0;
-  static bool configured[32];
+  Entry cache[64];
+  int used;
+  bool configured[32];
+};
+static int mmv_max_clusters(MmvOccupancy& o, const void* kern, int cs, size_t smem, int sm_count, int* out) {
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
-  auto kern = mmv_kernel<KIND, NTL, XL, DUMP>;
-  if (dev >= 32 || !configured[dev]) {
+  if (dev >= 32 || !o.configured[dev]) {
     GSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     GSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 0));
-    if (dev < 32) configured[dev] = true;
+    if (dev < 32) o.configured[dev] = true;
   }
   const int kb = (int)((smem + 8191) / 8192);
-  for (int i = 0; i < used; ++i) {
-    if (cache[i].dev == dev && cache[i].cs == cs && cache[i].kb == kb) {
-      *out = cache[i].n;
+  for (int i = 0; i < o.used; ++i) {
+    if (o.cache[i].dev == dev && o.cache[i].cs == cs && o.cache[i].kb == kb) {
+      *out = o.cache[i].n;
       return GSQ_OK;
     }
   }
@@ -1525,7 +1542,7 @@ static int mmv_max_clusters(int cs, size_t smem, int sm_count, int* out) {
     n = 0;
   }
   n = n < sm_count / cs ? n : sm_count / cs;
-  if (used < 64) cache[used++] = Entry{dev, cs, kb, n};
+  if (o.used < 64) o.cache[o.used++] = MmvOccupancy::Entry{dev, cs, kb, n};
   *out = n;
   return GSQ_OK;
 }
@@ -1567,94 +1584,110 @@ __host__ __device__ constexpr MmvCost mmv_cost(int kind, int ntl) {
                     : MmvCost{0.3f, 0.245f, 0.371f, 0.0f, 1.62f, 1.04f, 2.11f};
 }
 
-template <int KIND, int NTL, int XL, bool DUMP>
-static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) {
+// A launch plan of one product on `clusters` clusters of cs CTAs (cs = 0: none), and its estimated time.
+struct MmvPlan {
+  int cs, clusters, cap, round, bufs, aligned;
+  double t;
+};
+
+// The plan with cluster size `cs` and up to `n` clusters. A cluster takes its tiles in rounds of as many as the gather areas
+// have room for. False: it does not fit.
+template <int KIND, int NTL>
+static bool mmv_plan(const MmvArgs& a, int cs, int n, int aligned, int max_smem, MmvPlan* out) {
   constexpr int MC = 8 * NTL;
   constexpr bool DS = MmvKind<KIND>::DS;
   const int nsb = a.k >> 8;
-  // Cluster size: the CTAs of a cluster split K, so each stages 1 / cs of the activations, and the cluster takes
-  // its tiles in rounds of as many as the gather areas have room for. Chunking: equal chunks per warp, or (from
-  // 17 columns on, where the parked segments take a third of shared memory) whole tiles per warp. Among the
-  // combinations that fit, the one with the least estimated time.
-  struct Plan { int cs, clusters, cap, round, bufs, per; double t; };
-  Plan plans[2] = {{0, 0, 0, 0, 1, 0, 0.0}, {0, 0, 0, 0, 1, 0, 0.0}};
-  const int force_aligned = g_mmv_aligned;
-  for (int aligned = 0; aligned <= 1; ++aligned) {
-    if (force_aligned >= 0 && aligned != force_aligned) continue;
-    const size_t fixed = MmvKind<KIND>::grid_bytes(NTL) + (aligned ? 0 : mmv_partial_bytes(MC));
-    Plan& best = plans[aligned];
-    for (int cs : {1, 2, 4, 8}) {
-      if (g_mmv_cluster && cs != g_mmv_cluster) continue;
-      if (cs > nsb) break;
-      const int cap_kb = ((nsb + cs - 1) / cs) * 8;
-      const size_t xb = mmv_x_bytes(cap_kb, MC, DS);
-      if (fixed + xb + (size_t)cs * MMV_TR * MC * 4 > (size_t)max_smem) continue;
-      // occupancy is asked for with the largest footprint this cluster size could use
-      int n = 0;
-      const int rc = mmv_max_clusters<KIND, NTL, XL, DUMP>(cs, (size_t)max_smem, sm_count, &n);
-      if (rc != GSQ_OK) return rc;
-      if (n <= 0) continue;
-      const int clusters = n < a.ntiles ? n : a.ntiles;
-      const int per = (a.ntiles + clusters - 1) / clusters;
-      // tiles per round: all of a cluster's tiles if one gather area for them fits, else rounds that alternate
-      // between two areas
-      const size_t avail = (size_t)max_smem - fixed - xb, tile_b = (size_t)MMV_TR * MC * 4;
-      int round = per, bufs = 1;
-      if ((size_t)cs * ((per + cs - 1) / cs) * tile_b > avail) {
-        bufs = 2;
-        round = (int)(avail / (2 * tile_b)) / cs * cs;
-        if (round < cs) continue;
-      }
-      const int rounds = (per + round - 1) / round;
-      // measured: beyond 24 rows a second round costs more than the tcgen05 GEMM (repacked Q6_K has no other kernel)
-      if (NTL >= 4 && rounds > 1 && KIND != MK_Q6K) continue;
-      // estimated time (us; constants: MmvCost)
-      const int nsr = (nsb + cs - 1) / cs;
-      int rec_warp = 0, rec_sm = 0;
-      for (int left = per; left > 0; left -= round) {
-        const int x = left < round ? left : round;
-        rec_warp += aligned ? (x + MMV_WARPS - 1) / MMV_WARPS * nsr : (x * nsr + MMV_WARPS - 1) / MMV_WARPS;
-        rec_sm += x * nsr;
-      }
-      constexpr MmvCost q = mmv_cost(KIND, NTL);
-      const double by_warp = q.rec_warp * rec_warp, by_sm = q.rec_sm * rec_sm;
-      const double log2cs = cs == 1 ? 0.0 : cs == 2 ? 1.0 : cs == 4 ? 2.0 : 3.0;
-      const double t = (by_warp > by_sm ? by_warp : by_sm) + q.stage * ((double)a.m * cap_kb / 1000.0) + q.cluster * log2cs +
-                       q.round * (rounds - 1) + (aligned ? 0.0 : q.park + (cs > 1 ? q.park_remote * rec_warp / nsr : 0.0));
-      if (!best.cs || t < best.t) best = Plan{cs, clusters, cap_kb, round, bufs, per, t};
-    }
+  const size_t fixed = MmvKind<KIND>::grid_bytes(NTL) + (aligned ? 0 : mmv_partial_bytes(MC));
+  const int cap_kb = ((nsb + cs - 1) / cs) * 8;
+  const size_t xb = mmv_x_bytes(cap_kb, MC, DS);
+  if (cs > nsb || n <= 0 || fixed + xb + (size_t)cs * MMV_TR * MC * 4 > (size_t)max_smem) return false;
+  const int clusters = n < a.ntiles ? n : a.ntiles;
+  const int per = (a.ntiles + clusters - 1) / clusters;
+  // tiles per round: all of a cluster's tiles if one gather area for them fits, else rounds that alternate
+  // between two areas
+  const size_t avail = (size_t)max_smem - fixed - xb, tile_b = (size_t)MMV_TR * MC * 4;
+  int round = per, bufs = 1;
+  if ((size_t)cs * ((per + cs - 1) / cs) * tile_b > avail) {
+    bufs = 2;
+    round = (int)(avail / (2 * tile_b)) / cs * cs;
+    if (round < cs) return false;
   }
-  const int best_aligned = plans[1].cs && (!plans[0].cs || plans[1].t <= plans[0].t) ? 1 : 0;
-  const int best_cs = plans[best_aligned].cs, best_clusters = plans[best_aligned].clusters, best_cap = plans[best_aligned].cap,
-            best_round = plans[best_aligned].round, best_bufs = plans[best_aligned].bufs;
-  const double best_t = plans[best_aligned].t;
-  const size_t fixed = MmvKind<KIND>::grid_bytes(NTL) + (best_aligned ? 0 : mmv_partial_bytes(MC));
-  if (g_mmv_trace) {
-    fprintf(stderr, "mmv plan kind=%d ntl=%d xl=%d m=%d rows=%d k=%d: cs=%d clusters=%d round=%d bufs=%d aligned=%d est=%.1f us%s\n",
-            KIND, NTL, XL, a.m, a.nrows, a.k, best_cs, best_clusters, best_round, best_bufs, best_aligned, best_t,
-            best_cs ? "" : " (declined)");
+  const int rounds = (per + round - 1) / round;
+  // measured: beyond 24 rows a second round costs more than the tcgen05 GEMM (repacked Q6_K has no other kernel)
+  if (NTL >= 4 && rounds > 1 && KIND != MK_Q6K) return false;
+  // estimated time (us; constants: MmvCost)
+  const int nsr = (nsb + cs - 1) / cs;
+  int rec_warp = 0, rec_sm = 0;
+  for (int left = per; left > 0; left -= round) {
+    const int x = left < round ? left : round;
+    rec_warp += aligned ? (x + MMV_WARPS - 1) / MMV_WARPS * nsr : (x * nsr + MMV_WARPS - 1) / MMV_WARPS;
+    rec_sm += x * nsr;
   }
-  if (!best_cs) return MMV_DECLINED;
-  a.xcap_kb = best_cap;
-  a.nsr_lo = nsb / best_cs;
+  constexpr MmvCost q = mmv_cost(KIND, NTL);
+  const double by_warp = q.rec_warp * rec_warp, by_sm = q.rec_sm * rec_sm;
+  const double log2cs = cs == 1 ? 0.0 : cs == 2 ? 1.0 : cs == 4 ? 2.0 : 3.0;
+  const double t = (by_warp > by_sm ? by_warp : by_sm) + q.stage * ((double)a.m * cap_kb / 1000.0) + q.cluster * log2cs +
+                   q.round * (rounds - 1) + (aligned ? 0.0 : q.park + (cs > 1 ? q.park_remote * rec_warp / nsr : 0.0));
+  *out = MmvPlan{cs, clusters, cap_kb, round, bufs, aligned, t};
+  return true;
+}
+
+// the plan's values of the arguments; returns the dynamic shared memory
+template <int KIND, int NTL>
+static size_t mmv_set_plan(MmvArgs& a, const MmvPlan& p) {
+  constexpr int MC = 8 * NTL;
+  a.xcap_kb = p.cap;
+  a.nsr_lo = (a.k >> 8) / p.cs;
   for (int i = 0; i < 2; ++i) {
     a.inv_gpc[i] = fast_div_inv((a.nsr_lo + i) * 18);
     a.inv_nkb[i] = fast_div_inv((a.nsr_lo + i) * 8);
     a.inv_ppc[i] = fast_div_inv((a.nsr_lo + i) * 32);
   }
   a.inv_per = fast_div_inv(a.m * 9);
-  a.tiles_base = a.ntiles / best_clusters;
-  a.tiles_extra = a.ntiles % best_clusters;
-  a.tiles_round = best_round;
-  a.share_cap = (best_round + best_cs - 1) / best_cs;
-  a.gather_bufs = best_bufs;
-  a.aligned = best_aligned;
+  a.tiles_base = a.ntiles / p.clusters;
+  a.tiles_extra = a.ntiles % p.clusters;
+  a.tiles_round = p.round;
+  a.share_cap = (p.round + p.cs - 1) / p.cs;
+  a.gather_bufs = p.bufs;
+  a.aligned = p.aligned;
   a.pf_first = g_mmv_pf_first;
+  return MmvKind<KIND>::grid_bytes(NTL) + (p.aligned ? 0 : mmv_partial_bytes(MC)) + mmv_x_bytes(p.cap, MC, MmvKind<KIND>::DS) +
+         (size_t)p.bufs * p.cs * a.share_cap * MMV_TR * MC * 4;
+}
+
+template <int KIND, int NTL, int XL, bool DUMP>
+static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) {
+  static MmvOccupancy occupancy;
+  // Cluster size: the CTAs of a cluster split K, so each stages 1 / cs of the activations. Chunking: equal chunks per warp, or
+  // (from 17 columns on, where the parked segments take a third of shared memory) whole tiles per warp. Among the
+  // combinations that fit, the one with the least estimated time.
+  MmvPlan plans[2] = {};
+  for (int aligned = 0; aligned <= 1; ++aligned) {
+    if (g_mmv_aligned >= 0 && aligned != g_mmv_aligned) continue;
+    for (int cs : {1, 2, 4, 8}) {
+      if (g_mmv_cluster && cs != g_mmv_cluster) continue;
+      if (cs > (a.k >> 8)) break;
+      // occupancy is asked for with the largest footprint this cluster size could use
+      int n = 0;
+      MmvPlan p;
+      const int rc = mmv_max_clusters(occupancy, (const void*)mmv_kernel<KIND, NTL, XL, DUMP>, cs, (size_t)max_smem, sm_count, &n);
+      if (rc != GSQ_OK) return rc;
+      if (mmv_plan<KIND, NTL>(a, cs, n, aligned, max_smem, &p) && (!plans[aligned].cs || p.t < plans[aligned].t)) plans[aligned] = p;
+    }
+  }
+  const MmvPlan& best = plans[plans[1].cs && (!plans[0].cs || plans[1].t <= plans[0].t) ? 1 : 0];
+  if (g_mmv_trace) {
+    fprintf(stderr, "mmv plan kind=%d ntl=%d xl=%d m=%d rows=%d k=%d: cs=%d clusters=%d round=%d bufs=%d aligned=%d est=%.1f us%s\n",
+            KIND, NTL, XL, a.m, a.nrows, a.k, best.cs, best.clusters, best.round, best.bufs, best.aligned, best.t,
+            best.cs ? "" : " (declined)");
+  }
+  if (!best.cs) return MMV_DECLINED;
+  const size_t smem = mmv_set_plan<KIND, NTL>(a, best);
   // measured: the early start pays where the next product has a codebook to copy meanwhile and this grid leaves
   // some SMs free for the waiting quantiser (IQ3_S, 132 of 148 SMs: -1 us); it costs up to 1 us elsewhere (on a
   // full GPU the quantiser's blocks all land on the few SMs that drained first)
+  const int best_cs = best.cs, best_clusters = best.clusters;
   a.early = g_mmv_pdl >= 3 || (g_mmv_pdl == 2 && KIND == MK_IQ3S && best_clusters * best_cs + 8 <= sm_count);
-  const size_t smem = fixed + mmv_x_bytes(best_cap, MC, DS) + (size_t)best_bufs * best_cs * a.share_cap * MMV_TR * MC * 4;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(best_clusters * best_cs));
   cfg.blockDim = dim3(MMV_THREADS);
@@ -1689,6 +1722,66 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
     }
   }
   GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, mmv_kernel<KIND, NTL, XL, DUMP>, a));
+  return GSQ_OK;
+}
+
+// The pair: one cluster size for both, the clusters shared out by the products' work; among the cluster sizes and the shares next
+// to that one the least time of the slower product.
+template <int KA, int KB, int XL>
+static int mmv_launch_pair(MmvArgs a, MmvArgs b, int sm_count, int max_smem, cudaStream_t st) {
+  static MmvOccupancy occupancy;
+  auto kern = mmv_pair_kernel<KA, KB, XL>;
+  MmvPlan pa = {}, pb = {};
+  double best = 0.0;
+  auto plan = [&](auto kind, const MmvArgs& g, int cs, int n, MmvPlan* out) {
+    constexpr int K = decltype(kind)::value;
+    MmvPlan p;
+    out->cs = 0;
+    for (int aligned = 0; aligned <= 1; ++aligned)
+      if (mmv_plan<K, 1>(g, cs, n, aligned, max_smem, &p) && (!out->cs || p.t < out->t)) *out = p;
+    return out->cs != 0;
+  };
+  const double wa = (double)a.ntiles * mmv_cost(KA, 1).rec_sm, wb = (double)b.ntiles * mmv_cost(KB, 1).rec_sm;
+  for (int cs : {1, 2, 4, 8}) {
+    if (cs > (a.k >> 8) || (g_mmv_cluster && cs != g_mmv_cluster)) continue;
+    int n = 0;
+    const int rc = mmv_max_clusters(occupancy, (const void*)kern, cs, (size_t)max_smem, sm_count, &n);
+    if (rc != GSQ_OK) return rc;
+    const int share = (int)(n * wa / (wa + wb) + 0.5);
+    for (int na = share - 1; na <= share + 1; ++na) {
+      MmvPlan x, y;
+      if (na < 1 || n - na < 1 || !plan(std::integral_constant<int, KA>{}, a, cs, na, &x) || !plan(std::integral_constant<int, KB>{}, b, cs, n - na, &y))
+        continue;
+      const double t = x.t > y.t ? x.t : y.t;
+      if (!pa.cs || t < best) {
+        pa = x;
+        pb = y;
+        best = t;
+      }
+    }
+  }
+  if (g_mmv_trace)
+    fprintf(stderr, "mmv pair kinds=%d,%d xl=%d m=%d rows=%d,%d k=%d: cs=%d clusters=%d,%d est=%.1f,%.1f us%s\n", KA, KB, XL, a.m, a.nrows, b.nrows, a.k,
+            pa.cs, pa.clusters, pb.clusters, pa.t, pb.t, pa.cs ? "" : " (declined)");
+  if (!pa.cs) return MMV_DECLINED;
+  const size_t sa = mmv_set_plan<KA, 1>(a, pa), sb = mmv_set_plan<KB, 1>(b, pb);
+  a.early = b.early = 0;
+  const int blocks_a = pa.clusters * pa.cs;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(blocks_a + pb.clusters * pa.cs));
+  cfg.blockDim = dim3(MMV_THREADS);
+  cfg.dynamicSmemBytes = sa > sb ? sa : sb;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = pa.cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_mmv_pdl ? 2 : 1;
+  GSQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, b, blocks_a));
   return GSQ_OK;
 }
 

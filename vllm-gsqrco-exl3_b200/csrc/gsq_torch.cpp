@@ -263,6 +263,30 @@ void product_of_run(int op, const Weight& w, const Tensor& x, int64_t type, int6
     product(s, w, x, i, std::min(per_call, n - i), type, rows, k, q, y + i * ldy * x.element_size(), ldy, stream);
 }
 
+// Two runs' products at 1..8 rows in one launch, side by side in y. False: no such kernel, nothing done.
+bool product_of_two(const Weight& wa, int64_t ta, const Weight& wb, int64_t tb, const Tensor& x, bool packed, Tensor& q, char* y, int64_t ldy,
+                    void* stream) {
+  if (ta == tb || (tb != Q6_K && !(ta == IQ3_S && tb == IQ4_XS)) || (ta != Q4_K && ta != IQ3_S && ta != IQ4_XS) || dtype_code(x.scalar_type()) == GSQ_DTYPE_OTHER)
+    return false;
+  const int64_t n = x.size(0);
+  bool pa = packed, pb = packed;
+  const int oa = op_for(n, ta, wa.size0, x.size(1), pa), ob = op_for(n, tb, wb.size0, x.size(1), pb);
+  if (!kSpec[oa].vec || !kSpec[ob].vec) return false;
+  const int64_t k = guard(kSpec[oa], wa, x, ta, wa.size0);
+  guard(kSpec[ob], wb, x, tb, wb.size0);
+  const gsq_weight a = {wa.data, wa.size1, wa.size0, (int)ta, kSpec[oa].packed, y}, b = {wb.data, wb.size1, wb.size0, (int)tb, kSpec[ob].packed, y + wa.size0 * x.element_size()};
+  const int dt = dtype_code(x.scalar_type());
+  int rc = GSQ_ERR_UNSUPPORTED;
+  if (!q.defined()) rc = gsq_linear_vec_pair(&a, &b, x.const_data_ptr(), dt, n, k, row_stride(x, k), dt, ldy, stream);
+  if (rc == GSQ_ERR_UNSUPPORTED && gsq_linear_vec_pair_serves(&a, &b, n)) {
+    if (!q.defined()) q = quantize_blocks(x, k, stream);
+    rc = gsq_linear_vec_pair(&a, &b, q.const_data_ptr(), -1, n, k, 0, dt, ldy, stream);
+  }
+  if (rc == GSQ_ERR_UNSUPPORTED) return false;
+  check(rc, "gsq_linear_vec_pair");
+  return true;
+}
+
 Tensor unquantized(const Tensor& x, const Tensor& w) {
   if (x.size(0) <= 8 && w.size(0) <= 128) return at::bmm(x.unsqueeze(1), w.t().expand({x.size(0), -1, -1})).squeeze(1);
   return at::linear(x, w);
@@ -302,10 +326,24 @@ Tensor linear_runs(const Tensor& x, const Tensor& w, at::IntArrayRef runs, bool 
   const c10::cuda::OptionalCUDAGuard dev(x.is_cuda() ? std::optional<c10::Device>(x.device()) : std::nullopt);
   Tensor y, q;
   int64_t col = 0;
+  auto weight = [&](size_t i) {
+    return Weight{(const uint8_t*)w.const_data_ptr() + runs[i] * w.size(1), 2, runs[i + 1], runs[i + 2], runs[i + 2], 1,
+                  w.scalar_type() == at::kByte, w.is_cuda(), w.device()};
+  };
   for (size_t i = 0; i < runs.size(); i += 4) {
     const int64_t rows = runs[i + 1], type = runs[i + 3];
-    const Weight wt = {(const uint8_t*)w.const_data_ptr() + runs[i] * w.size(1), 2, rows, runs[i + 2], runs[i + 2], 1,
-                       w.scalar_type() == at::kByte, w.is_cuda(), w.device()};
+    const Weight wt = weight(i);
+    if (i + 4 < runs.size() && n <= 8 && x.is_cuda() && t_peers.empty()) {
+      // two runs in one launch, where there is such a kernel
+      const Weight wn = weight(i + 4);
+      if (!y.defined()) y = result(n, total, x);
+      if (product_of_two(wt, type, wn, runs[i + 7], x, packed, q, (char*)y.mutable_data_ptr() + col * x.element_size(), y.stride(0),
+                         c10::cuda::getCurrentCUDAStream().stream())) {
+        col += rows + runs[i + 5];
+        i += 4;
+        continue;
+      }
+    }
     bool pk = packed;
     const int op = op_for(n, type, rows, x.size(1), pk);
     if (!x.is_cuda()) guard(kSpec[op], wt, x, type, rows);

@@ -25,6 +25,7 @@ EXPORTS = (
     "gsq_debug_mmv_mode", "gsq_debug_mmv_min_rows", "gsq_debug_mmv_cluster_size", "gsq_mul_mat_vec_max_rows",
     "gsq_debug_mmv_profile", "gsq_debug_mmv_max_rows", "gsq_debug_mmv_pdl", "gsq_debug_mmv_prefetch_first", "gsq_debug_mmv_chunking", "gsq_debug_mmv_trace",
     "gsq_linear", "gsq_linear_scratch_bytes", "gsq_linear_workspace_bytes", "gsq_debug_gemm_profile", "gsq_q6k_repack", "gsq_allreduce_sum", "gsq_allreduce_error_flag", "gsq_linear_allreduce", "gsq_peer_reduce_error_flag", "gsq_rmsnorm_quantize_q8_1", "gsq_silu_mul_quantize_q8_1", "gsq_dequantize_rows", "gsq_dequantize_bad_index_flag", "gsq_prefill_precision", "gsq_linear_vec",
+    "gsq_linear_vec_pair", "gsq_linear_vec_pair_serves",
 )
 
 
@@ -32,6 +33,11 @@ class PeerReduce(C.Structure):
     """gsq_peer_reduce (include/gsq.h)."""
     _fields_ = [("slots", C.c_void_p), ("flags", C.c_void_p), ("state", C.c_void_p), ("rank", C.c_int), ("world", C.c_int),
                 ("slot_bytes", C.c_int64)]
+
+
+class Weight(C.Structure):
+    """gsq_weight (include/gsq.h)."""
+    _fields_ = [("w", C.c_void_p), ("row_bytes", C.c_int64), ("rows", C.c_int64), ("ggml_type", C.c_int), ("packed", C.c_int), ("y", C.c_void_p)]
 
 
 class GuardArgs(C.Structure):
@@ -109,6 +115,10 @@ def _load() -> C.CDLL:
     lib.gsq_linear.argtypes = [vp, i64, i64, ci, ci, vp, ci, i64, i64, i64, vp, ci, i64, vp, sz, vp]
     lib.gsq_linear_vec.restype = ci
     lib.gsq_linear_vec.argtypes = [vp, i64, i64, ci, ci, vp, ci, i64, i64, i64, vp, ci, i64, vp]
+    lib.gsq_linear_vec_pair.restype = ci
+    lib.gsq_linear_vec_pair.argtypes = [C.POINTER(Weight), C.POINTER(Weight), vp, ci, i64, i64, i64, ci, i64, vp]
+    lib.gsq_linear_vec_pair_serves.restype = ci
+    lib.gsq_linear_vec_pair_serves.argtypes = [C.POINTER(Weight), C.POINTER(Weight), i64]
     lib.gsq_iq3s_repack.restype = ci
     lib.gsq_iq3s_repack.argtypes = [vp, i64, i64, ci, vp]
     lib.gsq_allreduce_sum.restype = ci
