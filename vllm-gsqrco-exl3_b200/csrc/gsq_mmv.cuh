@@ -1136,6 +1136,11 @@ __host__ __device__ inline void mmv_k_range(int nsb, int cs, int rank, int* firs
   *last = (int)((int64_t)nsb * (rank + 1) / cs);
 }
 
+// Place of four columns (group c4) of row r2 in tile sums: rows of MC floats; above 16 columns each row's groups are turned by its
+// number, so that the same group of neighbouring rows falls on different banks (r2 may count over tiles: 16 rows of MC floats each)
+template <int MC>
+__device__ __forceinline__ int mmv_seg(int r2, int c4) { return MC <= 16 ? r2 * MC + 4 * c4 : r2 * MC + 4 * ((c4 + r2 % MMV_TR) % (MC / 4)); }
+
 // FUSED: the instantiation that also sums the result over the GPUs (see the end of the kernel); the plain product is
 // a separate instantiation so that it carries none of that code or of its registers. `block`: this CTA's number among those of
 // the product.
@@ -1305,8 +1310,8 @@ __device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
             float v0, v1, v2, v3;
             upk2(acc[j][0], v0, v1);
             upk2(acc[j][1], v2, v3);
-            *reinterpret_cast<float2*>(seg + g * MC + 8 * j + 2 * t) = make_float2(v0, v1);
-            *reinterpret_cast<float2*>(seg + (g + 8) * MC + 8 * j + 2 * t) = make_float2(v2, v3);
+            *reinterpret_cast<float2*>(seg + mmv_seg<MC>(g, 2 * j + (t >> 1)) + 2 * (t & 1)) = make_float2(v0, v1);
+            *reinterpret_cast<float2*>(seg + mmv_seg<MC>(g + 8, 2 * j + (t >> 1)) + 2 * (t & 1)) = make_float2(v2, v3);
             acc[j][0] = acc[j][1] = 0ull;
           }
         }
@@ -1352,27 +1357,38 @@ __device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
     const int own_tiles = max(0, min(a.share_cap, tiles_r - crank * a.share_cap));
     const float* g0 = gath + (size_t)buf * cs * a.share_cap * SEGF;
     if constexpr (!fused) {
-      for (int r2 = tid; r2 < own_tiles * MMV_TR; r2 += MMV_THREADS) {
+      const int own_rows = own_tiles * MMV_TR;
+      auto put = [&](int r2, int c4) {
         const int row = (tile_begin + t0 + crank * a.share_cap) * MMV_TR + r2;
-        if (row < a.nrows) {
+        if (row < a.nrows && 4 * c4 < a.m) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-          for (int c4 = 0; c4 < MC / 4; ++c4) {
-            if (4 * c4 < a.m) {
-              float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-              for (int r = 0; r < 8; ++r) {
-                if (r < cs) {
-                  const float4 p = *reinterpret_cast<const float4*>(g0 + (size_t)r * a.share_cap * SEGF + r2 * MC + 4 * c4);
-                  v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-                }
-              }
-              const float o[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                if (4 * c4 + e < a.m) store_out_dyn(a.y, a.y_dtype, (int64_t)(4 * c4 + e) * a.ldy + row, o[e]);
-              }
+          for (int r = 0; r < 8; ++r) {
+            if (r < cs) {
+              const float4 p = *reinterpret_cast<const float4*>(g0 + (size_t)r * a.share_cap * SEGF + mmv_seg<MC>(r2, c4));
+              v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
             }
           }
+          const float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (4 * c4 + e < a.m) store_out_dyn(a.y, a.y_dtype, (int64_t)(4 * c4 + e) * a.ldy + row, o[e]);
+          }
+        }
+      };
+      if (MC <= 16 && own_rows >= MMV_THREADS) {
+        // a row a thread (151936 x 5120 Q6_K, 16 rows: 203 us, 206 the other way; but 34816 x 12800, 55 rows, 453 and 417)
+        for (int r2 = tid; r2 < own_rows; r2 += MMV_THREADS) {
+#pragma unroll
+          for (int c4 = 0; c4 < MC / 4; ++c4) put(r2, c4);
+        }
+      } else {
+        // Four columns of a row a thread, rows fastest: all threads work, a warp's stores are contiguous, and its 16-byte loads
+        // fall on different banks (mmv_seg). With a row a thread, 118 of 512 threads were busy at 17408 x 5120 and a warp's loads
+        // in the same four banks at 32 columns: 3.0 of that product's 29.7 us.
+        for (int it = tid; it < own_rows * (MC / 4); it += MMV_THREADS) {
+          const int c4 = it / own_rows;
+          put(it - c4 * own_rows, c4);
         }
       }
     } else {
@@ -1387,7 +1403,7 @@ __device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
 #pragma unroll
           for (int r = 0; r < 8; ++r) {
             if (r < cs) {
-              const float4 p = *reinterpret_cast<const float4*>(g0 + (size_t)r * a.share_cap * SEGF + r2 * MC + 4 * c4);
+              const float4 p = *reinterpret_cast<const float4*>(g0 + (size_t)r * a.share_cap * SEGF + mmv_seg<MC>(r2, c4));
               v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
             }
           }
