@@ -248,3 +248,30 @@ def test_packed_flag_on_a_type_of_one_layout(name, m):
                               torch.cuda.current_stream().cuda_stream) == 0
         y.append(out)
     assert torch.equal(*y)
+
+
+@pytest.mark.parametrize("name,rows,k,m", [("Q6_K", 848, 5120, 49), ("Q6_K", 2048, 5120, 96), ("Q6_K", 2064, 2560, 81), ("Q6_K", 8192, 1024, 96),
+                                           ("IQ4_XS", 23, 512, 33), ("IQ4_XS", 1000, 1024, 48), ("IQ4_XS", 2049, 8448, 41), ("IQ4_XS", 1023, 17408, 48),
+                                           ("Q4_K", 23, 256, 33), ("Q4_K", 777, 2048, 48), ("Q4_K", 5121, 5120, 41), ("Q4_K", 1000, 17408, 34)])
+def test_row_counts_that_two_kernels_serve(name, rows, k, m):
+    """33..48 rows of Q4_K and IQ4_XS, 49..96 of repacked Q6_K: the kernel that the rules choose against the other one that
+    serves the same call. Both round K / 32 fp32 sums of exact integer products (Q4_K: twice as many, of terms that partly
+    cancel): each is within sqrt(K / 32) of an fp32 rounding, 2^-24, and their difference within four times that."""
+    t, packed, lib = TYPES[name], name == "Q6_K", _cabi.lib
+    raw = synth.make_weight(t, rows, k, 69 + rows)
+    x = torch.from_numpy(synth.make_activation(m, k, 70 + m)).float().to(DEV)
+    x[m - 1, :64] = 0.0
+    x[3, :] = 0.0
+    here = _run(t, packed, raw, x, rows, rows + 3)
+    if packed:
+        old = lib.gsq_prefill_precision(2)
+        other = _run(t, packed, raw, x, rows)
+        lib.gsq_prefill_precision(old)
+    else:
+        old = lib.gsq_debug_gemm_variant(10)
+        other = _run(t, packed, raw, x, rows)
+        lib.gsq_debug_gemm_variant(old)
+    assert not here[3].any() and np.isfinite(here).all()
+    assert product.rel_err(here, other) <= 4 * np.sqrt(k / 32) * 2.0 ** -24
+    if packed:
+        assert np.array_equal(_run(t, packed, raw, x, rows, least=True), other)     # no room for expanded weights: launches

@@ -127,6 +127,19 @@ def test_c_route():
     assert r(4, 8, BIG, K, 0) == _cabi.KERNEL_NONE             # Q8_0: not a type of this route
 
 
+@pytest.mark.parametrize("t,packed,rows,k,few,first", [
+    # the last row count of the small-batch kernel, the first of the kernel that takes over
+    (23, 0, 512, 1024, 48, 49), (23, 0, 1024, 8192, 39, 40), (23, 0, 5120, BIG, 48, 49), (23, 0, 40016, K, 32, 33), (23, 0, 34816, 12800, 32, 33),
+    (Q4_K, 0, 512, 1024, 48, 49), (Q4_K, 0, 7168, K, 48, 49), (Q4_K, 0, 9216, K, 32, 33), (Q4_K, 0, 1024, BIG, 48, 49), (Q4_K, 0, 2048, BIG, 32, 33),
+    (14, 1, 2048, 8192, 48, 49), (14, 1, 1024, K, 48, 49), (14, 1, 512, K, 96, 97), (14, 1, 5120, K, 80, 81), (14, 1, 2048, 2048, 96, 97),
+    (14, 1, 8192, 8192, 96, 97), (14, 1, 9216, K, 96, 97), (14, 1, 12288, K, 112, 113)])
+def test_lines_between_the_small_batch_kernel_and_the_next(t, packed, rows, k, few, first):
+    from gsq_b200 import _cabi
+
+    assert _cabi.lib.gsq_route(few, t, rows, k, packed) == _cabi.KERNEL_MMV
+    assert _cabi.lib.gsq_route(first, t, rows, k, packed) == (_cabi.KERNEL_GEMM_PREFILL if t == 14 else _cabi.KERNEL_GEMM)
+
+
 def test_route_switch_keys_the_compile_cache():
     """The switch that changes apply()'s traced graph is registered where vLLM hashes its compile factors
     (plugin.py:156-161 of the reference does the same)."""

@@ -70,8 +70,13 @@ enum Way {
 
 // The fewest activation rows from which the two-step product takes the place of repeated launches of the small-batch
 // kernels. Where the two cross, us two steps / launches (weights cycled through HBM; profiles/two_step_thresholds.txt):
-//   Q6_K repacked (48 rows a launch)  97: 5120 x 5120 50 / 69, 5120 x 17408 158 / 183, but 17408 x 5120 154 / 143
-//                                     (112 rows 156 / 150, 128 rows 158 / 164)
+//   Q6_K repacked (48 rows a launch)  97: 512 x 1024 15.2 / 19.8 (at 96 rows 14.9 / 14.3), 8192 x 8192 113.2 / 113.8 (112.2 / 94.8),
+//                                     5120 x 17408 150 / 166 (151 / 143); 113 rows for tall weights of some size: 17408 x 5120
+//                                     148 / 142 (97 rows 146 / 131), 12288 x 8192 167 / 165 (112 rows), but 9216 x 5120 97 rows 78 / 97;
+//                                     81 where the third 16-row group of a launch costs more than the expansion: 5120 x 5120 (88
+//                                     rows) 44.2 / 49.5, 4096 x 4096 30.9 / 35.0, but 2048 x 2048 20.7 / 18.9, 17408 x 2560 71 / 62;
+//                                     49 where a launch has few rows of long K: 2048 x 8192 29.7 / 31.1 (64 rows 30.5 / 32.7, 96 rows
+//                                     32.2 / 42.3), 1024 x 17408 39.7 / 40.8 (64 rows 39.9 / 46.0), 1024 x 5120 21.1 / 21.7
 //   Q6_K, IQ3_S in GGUF order (8)     25: 512 x 1024 16 / 21 and 15 / 32, 17408 x 5120 148 / 281 and 95 / 176
 //   Q2_K                              25: 5120 x 5120 47 / 70, 17408 x 5120 120 / 155; 512 x 1024 22 / 18, at 40 rows 23 / 26
 //   IQ1_M                             12: 5120 x 5120 32 / 40, 17408 x 5120 81 / 89; 1024 x 2048 16.5 / 13.9, at 17 rows 17.4 / 18.9
@@ -80,7 +85,11 @@ enum Way {
 static int two_step_rows(int ggml_type, bool q6_packed, int64_t rows, int64_t k) {
   const int64_t values = rows * k;
   switch (ggml_type) {
-    case GSQ_TYPE_Q6_K: return !q6_packed ? 25 : rows > 8192 ? 113 : 97;
+    case GSQ_TYPE_Q6_K:
+      if (!q6_packed) return 25;
+      if (rows > 8192) return values > (48 << 20) ? 113 : 97;
+      if (values > (4 << 20) && rows <= 2048 && k >= 5120) return 49;
+      return values > (4 << 20) && values <= (32 << 20) ? 81 : 97;
     case GSQ_TYPE_IQ3_S: return 25;
     case GSQ_TYPE_Q2_K: return values <= (1 << 20) ? 33 : 25;
     case GSQ_TYPE_IQ1_M: return values <= (4 << 20) ? 17 : 12;
@@ -121,17 +130,19 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, int64_
 }
 
 // Whether the small-batch tensor-core kernel is tried first. It serves 1..48 rows; for the types in GGUF order, whose
-// decoding it repeats per lane, the kernel with evenly cut work is the faster one from 33 rows on, except (us, small-batch
-// kernel / evenly cut work):
-//   * IQ4_XS while the activations are few: 40 rows 17408 x 5120 45.5 / 54.6, 48 rows 34816 x 5120 82.2 / 95.6, but
-//     48 rows 2048 x 8192 23.9 / 23.0; weights so tall that it would decline, and small ones, go on;
-//   * Q4_K while the weight has too few 128-row tiles to cut evenly: 48 rows 1024 x 5120 17.4 / 21.8, 5120 x 2048
-//     16.3 / 17.0, but 5120 x 5120 25.5 / 24.2.
+// decoding it repeats per lane, the kernel with evenly cut work takes over from 33 rows on where it is the faster one (us,
+// small-batch kernel / evenly cut work, 33 and 48 rows):
+//   * IQ4_XS: on weights so tall or large that the first one has no even plan: 60000 x 5120 154 / 153, 34816 x 12800 217 / 215,
+//     5120 x 32768 94 / 91, but 34816 x 5120 78 / 94, 17408 x 5120 43 / 53, 5120 x 17408 52.9 / 54.8, 512 x 1024 7.9 / 8.9. To
+//     16 M values the activations' size decides, as callers of gsq_route know it (48 rows 2048 x 8192: 18.3 / 22.9).
+//   * Q4_K: from 40 M values on, 17408 x 5120 52.7 / 50.4 and 54.3 / 50.8, 5120 x 12800 47 / 42, with long K from 20 M on,
+//     2048 x 17408 32.4 / 31.6; but 7168 x 5120 26.0 / 28.0 and 26.6 / 28.3, 5120 x 8192 30.6 / 31.4, 1024 x 17408 26.0 / 28.2,
+//     1024 x 2048 8.6 / 11.3.
 static bool small_batch(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k) {
   if (gemm_variant() == 10 || !mmv_applies(ggml_type, packed, rows, m)) return false;
   if (m <= 32 || gemm_variant() != 0 || gemm_dump_pointer()) return true;
-  if (ggml_type == GSQ_TYPE_IQ4_XS) return m * k <= 320000 && rows <= 40000 && rows * k > (4 << 20);
-  if (ggml_type == GSQ_TYPE_Q4_K) return rows * k <= (12 << 20) && rows * k > (4 << 20);
+  if (ggml_type == GSQ_TYPE_IQ4_XS) return rows <= 40000 && (m * k <= 320000 || (rows * k > (16 << 20) && rows * k <= (100 << 20)));
+  if (ggml_type == GSQ_TYPE_Q4_K) return rows * k <= (k <= 12288 ? 40 << 20 : 20 << 20);
   return true;
 }
 
