@@ -37,3 +37,9 @@ def test_rows_equal_blocks(name, t, rows, k, m):
     assert torch.equal(out[0][:, :rows], out[1][:, :rows])
     flag = ctypes.c_int(-1)
     assert lib.gsq_device_error_flag(ctypes.byref(flag)) == 0 and flag.value == 0
+
+
+@pytest.mark.parametrize("m", [33, 41, 48])
+def test_rows_equal_blocks_on_large_weights_above_32_rows(m):
+    """IQ4_XS weights of more than 64 M values."""
+    test_rows_equal_blocks("IQ4_XS", 23, 13136, 5120, m)

@@ -195,11 +195,14 @@ int mmv_rows_columns(int64_t m) {
   return (int)(8 * (ntl == 5 ? 6 : ntl));
 }
 // Whether that order is the faster one: it is once a CTA's share of a column is some hundred bytes. Small weights are split
-// over clusters of 8 and each copy is short (1024 x 2048 IQ3_S at 40 rows 11.1 us from blocks, 11.9 from rows); above 32 rows
-// the scales of 48 columns and the more copies leave a gain only for the large products of Q6_K (17408 x 5120 at 48
-// rows 60.3 -> 56.1; IQ3_S 47.0 -> 47.5).
+// over clusters of 8 and each copy is short (1024 x 2048 IQ3_S at 40 rows 7.8 us from blocks, 8.5 from rows); above 32 rows
+// the scales of 48 columns and the more copies leave a gain only for large products of Q6_K (17408 x 5120 at 48 rows 55.4 ->
+// 52.0; 5120 x 5120 24.9 -> 24.1, at 33 rows 24.1 -> 24.8) and the largest of IQ4_XS (17408 x 5120 at 33 and 48 rows 42.8 -> 41.2
+// and 44.6 -> 40.9, 34816 x 5120 77.3 -> 75.8 and 79.7 -> 74.7, but 7168 x 5120 at 33 rows 24.9 -> 25.0; IQ3_S 43.7 -> 43.1, Q4_K
+// 51.1 both).
 bool mmv_rows_wins(int ggml_type, int64_t rows, int64_t m, int64_t k) {
-  return rows * k > (4 << 20) && k <= (1 << 24) && (m <= 32 || (ggml_type == GSQ_TYPE_Q6_K && rows * k > (16 << 20)));
+  const int64_t least = m <= 32 ? 4 << 20 : ggml_type == GSQ_TYPE_Q6_K ? 16 << 20 : ggml_type == GSQ_TYPE_IQ4_XS ? 64 << 20 : INT64_MAX;
+  return rows * k > least && k <= (1 << 24);
 }
 size_t mmv_rows_bytes(int ggml_type, int64_t m, int64_t k) {
   return (size_t)(m * k) + (size_t)(k / 32) * mmv_rows_columns(m) * (ggml_type == GSQ_TYPE_Q4_K ? 8 : 4);
