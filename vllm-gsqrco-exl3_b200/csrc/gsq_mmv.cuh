@@ -1358,6 +1358,9 @@ __device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
     const float* g0 = gath + (size_t)buf * cs * a.share_cap * SEGF;
     if constexpr (!fused) {
       const int own_rows = own_tiles * MMV_TR;
+      // IQ3_S at 9 to 16 rows keeps a row a thread: with the other loop the compiler gives the kernel 128 registers instead of
+      // 124, and its main loop is slower by more than this one gains (four linears of a layer, 16 rows: 110.6 us, 100.4 so)
+      constexpr bool ROW_A_THREAD = KIND == MK_IQ3S && NTL == 2;
       auto put = [&](int r2, int c4) {
         const int row = (tile_begin + t0 + crank * a.share_cap) * MMV_TR + r2;
         if (row < a.nrows && 4 * c4 < a.m) {
@@ -1376,7 +1379,7 @@ __device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
           }
         }
       };
-      if (MC <= 16 && own_rows >= MMV_THREADS) {
+      if (ROW_A_THREAD || (MC <= 16 && own_rows >= MMV_THREADS)) {
         // a row a thread (151936 x 5120 Q6_K, 16 rows: 203 us, 206 the other way; but 34816 x 12800, 55 rows, 453 and 417)
         for (int r2 = tid; r2 < own_rows; r2 += MMV_THREADS) {
 #pragma unroll
