@@ -1136,10 +1136,10 @@ __host__ __device__ inline void mmv_k_range(int nsb, int cs, int rank, int* firs
   *last = (int)((int64_t)nsb * (rank + 1) / cs);
 }
 
-// Place of four columns (group c4) of row r2 in tile sums: rows of MC floats; above 16 columns each row's groups are turned by its
+// Place of four columns (group c4) of row r2 in tile sums: rows of MC floats; from 16 columns on each row's groups are turned by its
 // number, so that the same group of neighbouring rows falls on different banks (r2 may count over tiles: 16 rows of MC floats each)
 template <int MC>
-__device__ __forceinline__ int mmv_seg(int r2, int c4) { return MC <= 16 ? r2 * MC + 4 * c4 : r2 * MC + 4 * ((c4 + r2 % MMV_TR) % (MC / 4)); }
+__device__ __forceinline__ int mmv_seg(int r2, int c4) { return MC < 16 ? r2 * MC + 4 * c4 : r2 * MC + 4 * ((c4 + r2 % MMV_TR) % (MC / 4)); }
 
 // FUSED: the instantiation that also sums the result over the GPUs (see the end of the kernel); the plain product is
 // a separate instantiation so that it carries none of that code or of its registers. `block`: this CTA's number among those of
@@ -1358,9 +1358,6 @@ __device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
     const float* g0 = gath + (size_t)buf * cs * a.share_cap * SEGF;
     if constexpr (!fused) {
       const int own_rows = own_tiles * MMV_TR;
-      // IQ3_S at 9 to 16 rows keeps a row a thread: with the other loop the compiler gives the kernel 128 registers instead of
-      // 124, and its main loop is slower by more than this one gains (four linears of a layer, 16 rows: 110.6 us, 100.4 so)
-      constexpr bool ROW_A_THREAD = KIND == MK_IQ3S && NTL == 2;
       auto put = [&](int r2, int c4) {
         const int row = (tile_begin + t0 + crank * a.share_cap) * MMV_TR + r2;
         if (row < a.nrows && 4 * c4 < a.m) {
@@ -1379,16 +1376,17 @@ __device__ __forceinline__ void mmv_body(const MmvArgs& a, int block) {
           }
         }
       };
-      if (ROW_A_THREAD || (MC <= 16 && own_rows >= MMV_THREADS)) {
-        // a row a thread (151936 x 5120 Q6_K, 16 rows: 203 us, 206 the other way; but 34816 x 12800, 55 rows, 453 and 417)
-        for (int r2 = tid; r2 < own_rows; r2 += MMV_THREADS) {
-#pragma unroll
-          for (int c4 = 0; c4 < MC / 4; ++c4) put(r2, c4);
-        }
+      // Four columns of a row a thread, rows fastest: all threads work, a warp's stores are contiguous, and its 16-byte loads fall on
+      // different banks (mmv_seg). With a row a thread, 118 of 512 threads were busy at 17408 x 5120 and a warp's loads in the
+      // same four banks at 32 columns: 3.0 of that product's 29.7 us. To 16 rows a thread's group of columns comes from its
+      // number, without a division: over 18 weights from 512 x 1024 to 34816 x 5120, against a row a thread, 1.5 to 2.9 % (to 8
+      // rows, by type) and 5.3 to 6.0 % (9 to 16 rows) less on average, at most 1.8 % more on any. Q4_K at 9 to 16 rows keeps
+      // the other loop: the compiler makes another main loop beside it, 2.5 % faster over those weights.
+      constexpr bool SHARES = NTL == 1 || (NTL == 2 && KIND != MK_Q4K);
+      if constexpr (SHARES) {
+        const int sh = a.m > 8 ? 7 : a.m > 4 ? 8 : 9;   // threads of a group: 512, 256 or 128
+        for (int r2 = tid & ((1 << sh) - 1); r2 < own_rows; r2 += 1 << sh) put(r2, tid >> sh);
       } else {
-        // Four columns of a row a thread, rows fastest: all threads work, a warp's stores are contiguous, and its 16-byte loads
-        // fall on different banks (mmv_seg). With a row a thread, 118 of 512 threads were busy at 17408 x 5120 and a warp's loads
-        // in the same four banks at 32 columns: 3.0 of that product's 29.7 us.
         for (int it = tid; it < own_rows * (MC / 4); it += MMV_THREADS) {
           const int c4 = it / own_rows;
           put(it - c4 * own_rows, c4);
