@@ -16,17 +16,19 @@ int record_cuda_error(cudaError_t e) {
 
 int gemv_device_init(int device);  // gsq_gemv.cu
 
-static DeviceInfo g_info[64];
+// (threads may be the first to ask at the same time: both write the same, and the flag comes last)
+static std::atomic<int> g_sm_count[64], g_max_smem[64];
+static std::atomic<bool> g_ready[64];
 
 int device_info(DeviceInfo* out) {
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return GSQ_ERR_UNSUPPORTED;
-  if (!g_info[dev].ready) {
+  if (!g_ready[dev]) {
     int rc = gsq_device_init(dev);
     if (rc != GSQ_OK) return rc;
   }
-  *out = g_info[dev];
+  *out = DeviceInfo{g_sm_count[dev], g_max_smem[dev]};
   return GSQ_OK;
 }
 
@@ -54,7 +56,7 @@ extern "C" int gsq_type_block_bytes(int ggml_type) { return gsq::block_bytes(ggm
 extern "C" int gsq_device_init(int device) {
   using namespace gsq;
   if (device < 0 || device >= 64) return GSQ_ERR_UNSUPPORTED;
-  if (g_info[device].ready) return GSQ_OK;
+  if (g_ready[device]) return GSQ_OK;
   int prev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&prev));
   if (prev != device) GSQ_CUDA_TRY(cudaSetDevice(device));
@@ -64,9 +66,9 @@ extern "C" int gsq_device_init(int device) {
   int rc = gemv_device_init(device);
   if (prev != device) cudaSetDevice(prev);
   if (rc != GSQ_OK) return rc;
-  g_info[device].sm_count = sm;
-  g_info[device].max_smem_optin = smem;
-  g_info[device].ready = true;
+  g_sm_count[device] = sm;
+  g_max_smem[device] = smem;
+  g_ready[device] = true;
   return GSQ_OK;
 }
 

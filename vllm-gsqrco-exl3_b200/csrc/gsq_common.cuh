@@ -8,26 +8,18 @@
 
 #include "../../include/gsq.h"
 #include "../../include/gsq_debug.h"
+#include "gsq_host.h"
 
 #define GSQ_WARP 32
 #define GSQ_QK_K 256
 
 namespace gsq {
 
-// thread-local record of the last failing CUDA call (read through gsq_last_cuda_error)
-int record_cuda_error(cudaError_t e);
-#define GSQ_CUDA_TRY(expr)                                   \
-  do {                                                       \
-    cudaError_t _e = (expr);                                 \
-    if (_e != cudaSuccess) return gsq::record_cuda_error(_e); \
-  } while (0)
-
 // activation tiles of the prefill GEMMs: besides GSQ_Q8_LAYOUT_D4 / _DS4, the quants as fp16 with fp32 d (gsq_gemm3.cu)
 constexpr int Q8_TILES_H16 = 2;
 struct DeviceInfo {
   int sm_count;
   int max_smem_optin;
-  bool ready;
 };
 // cached facts about the current device (filled by gsq_device_init)
 int device_info(DeviceInfo* out);

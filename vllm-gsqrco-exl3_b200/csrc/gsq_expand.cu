@@ -479,7 +479,7 @@ template <int KIND>
 static int launch_expand(const ExpandArgs& g, int sm_count, cudaStream_t st) {
   constexpr int smem = x_smem(KIND);
   static_assert(smem <= 227 * 1024, "shared memory budget");
-  static int per_sm[64];
+  static std::atomic<int> per_sm[64];
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return GSQ_ERR_UNSUPPORTED;

@@ -912,7 +912,7 @@ int gemm_variant() { return g_gemm_variant; }
 
 template <int KIND>
 static int launch_gemm(const GemmArgs& g, int sm_count, cudaStream_t st) {
-  static int configured_mask = 0;
+  static std::atomic<uint32_t> configured_mask{0};
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   const bool ws = g_gemm_variant == 1;   // (0 and 2: the lockstep kernel)
@@ -922,7 +922,7 @@ static int launch_gemm(const GemmArgs& g, int sm_count, cudaStream_t st) {
                                       (int)gemm_smem_bytes<KIND>()));
     GSQ_CUDA_TRY(cudaFuncSetAttribute(gemm_ws_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)gemm_ws_smem_bytes<KIND>()));
-    if (dev < 32) configured_mask |= 1 << dev;
+    if (dev < 32) configured_mask |= 1u << dev;
   }
   const int n_items = g.n_row_tiles * g.n_tok_tiles;
   // split K over a cluster when there are too few tiles to occupy the SMs (decode-sized token counts)

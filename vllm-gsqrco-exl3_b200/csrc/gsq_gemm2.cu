@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm2_kernel(const Args g) {
 
 template <int KIND>
 static int launch(const Args& g, int sm_count, cudaStream_t st) {
-  static bool configured[64];
+  static std::atomic<bool> configured[64];
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   constexpr int smem = Smem<KIND>::TOTAL;

@@ -298,7 +298,7 @@ static int stage_bytes_of(const Plan& p) {
 
 template <int HU, int TP>
 static int launch_gemm4(GemmArgs& g, int stage, int sm_count, cudaStream_t st) {
-  static int max_pairs[64];
+  static std::atomic<int> max_pairs[64];
   g.stages = (SMEM_MAX - SMEM_HEAD) / stage;
   if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
   return launch_pairs(gemm4_kernel<HU, TP>, G_THREADS, g, max_pairs, (int64_t)g.n_rp * g.n_tb * g.splits, SMEM_HEAD + g.stages * stage, sm_count, st);

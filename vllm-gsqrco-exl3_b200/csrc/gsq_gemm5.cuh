@@ -598,7 +598,7 @@ static int launch_pdl(void (*kern)(KA...), dim3 grid, int threads, int smem, cud
 
 template <int KIND, int CP>
 static int launch_t(const Args& g, int n_cta, cudaStream_t st) {
-  static bool configured[64];
+  static std::atomic<bool> configured[64];
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return GSQ_ERR_UNSUPPORTED;

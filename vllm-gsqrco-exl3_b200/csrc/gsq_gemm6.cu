@@ -395,7 +395,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(S_THREADS, 1) gemm6_
 
 template <int AP, int TP, bool COMP>
 static int launch_gemm6(SliceArgs& g, int sm_count, cudaStream_t st) {
-  static int max_pairs[64];
+  static std::atomic<int> max_pairs[64];
   const int stage = AP * A_TILE + g.nt / 2 * (KB * 2), dx = DX_SLOTS * (g.nt * 32 + (1 + TP) * 512);
   static_assert(!TP || 4096 + 8 * 32 * INT_NT / 2 <= AP * A_TILE + INT_NT / 2 * KB * 2, "a term unit fits into a stage");
   g.stages = (SMEM_MAX - SMEM_HEAD - dx) / stage;

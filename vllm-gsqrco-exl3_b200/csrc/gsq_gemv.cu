@@ -890,12 +890,12 @@ struct ClusterPlan {
 // Per kernel instantiation and device: the cluster size that keeps most SMs busy with every cluster resident.
 template <int KIND, int M, int RS, bool DUMP, bool TMA, bool RAWX>
 static int plan_clusters(size_t smem, int sm_count, ClusterPlan* out) {
-  static ClusterPlan cache[32];
-  static bool have[32];
+  static std::atomic<ClusterPlan> cache[32];   // (eight bytes: read and written whole; no cluster: not asked yet)
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 32 && have[dev] && !g_force_cluster) {
-    *out = cache[dev];
+  const ClusterPlan kept = dev < 32 && !g_force_cluster ? cache[dev].load() : ClusterPlan{};
+  if (kept.cs) {
+    *out = kept;
     return GSQ_OK;
   }
   auto kern = gemv_kernel<KIND, M, RS, DUMP, TMA, RAWX>;
@@ -922,10 +922,7 @@ static int plan_clusters(size_t smem, int sm_count, ClusterPlan* out) {
     n = n < sm_count / cs ? n : sm_count / cs;
     if (n * cs > best.cs * best.clusters || (best.cs == 1 && n * cs >= (sm_count * 15) / 16)) best = ClusterPlan{cs, n};
   }
-  if (dev < 32 && !g_force_cluster) {
-    cache[dev] = best;
-    have[dev] = true;
-  }
+  if (dev < 32 && !g_force_cluster) cache[dev] = best;
   *out = best;
   return GSQ_OK;
 }

@@ -1518,52 +1518,6 @@ extern int g_mmv_cluster, g_mmv_pdl, g_mmv_pf_first, g_mmv_aligned, g_mmv_trace;
 
 constexpr int MMV_DECLINED = 1000;  // mmv_host: this shape does not fit; use another kernel
 
-// co-resident clusters of `cs` CTAs with `smem` bytes each (cached per kernel, device and size class)
-struct MmvOccupancy {
-  struct Entry { int dev, cs, kb, n; };
-  Entry cache[64];
-  int used;
-  bool configured[32];
-};
-static int mmv_max_clusters(MmvOccupancy& o, const void* kern, int cs, size_t smem, int sm_count, int* out) {
-  int dev = 0;
-  GSQ_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev >= 32 || !o.configured[dev]) {
-    GSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    GSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 0));
-    if (dev < 32) o.configured[dev] = true;
-  }
-  const int kb = (int)((smem + 8191) / 8192);
-  for (int i = 0; i < o.used; ++i) {
-    if (o.cache[i].dev == dev && o.cache[i].cs == cs && o.cache[i].kb == kb) {
-      *out = o.cache[i].n;
-      return GSQ_OK;
-    }
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(sm_count / cs * cs));
-  cfg.blockDim = dim3(MMV_THREADS);
-  cfg.dynamicSmemBytes = (size_t)kb * 8192 > 227 * 1024 ? 227 * 1024 : (size_t)kb * 8192;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = cs;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cs == 1) {
-    n = sm_count;
-  } else if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    n = 0;
-  }
-  n = n < sm_count / cs ? n : sm_count / cs;
-  if (o.used < 64) o.cache[o.used++] = MmvOccupancy::Entry{dev, cs, kb, n};
-  *out = n;
-  return GSQ_OK;
-}
-
 // Constants of a launch plan's estimated time, us: a record of the busiest warp and of an SM (whichever binds), parked
 // segments (equal chunks) and what they add per tile of a cluster's other CTAs, staging per 1000 32-value blocks of
 // activations, doubling the cluster, a further round. Fitted per type and column groups to a sweep of cluster sizes and
@@ -1674,7 +1628,7 @@ static size_t mmv_set_plan(MmvArgs& a, const MmvPlan& p) {
 
 template <int KIND, int NTL, int XL, bool DUMP>
 static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) {
-  static MmvOccupancy occupancy;
+  static ClusterCount occupancy;
   // Cluster size: the CTAs of a cluster split K, so each stages 1 / cs of the activations. Chunking: equal chunks per warp, or
   // (from 17 columns on, where the parked segments take a third of shared memory) whole tiles per warp. Among the
   // combinations that fit, the one with the least estimated time.
@@ -1687,7 +1641,7 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
       // occupancy is asked for with the largest footprint this cluster size could use
       int n = 0;
       MmvPlan p;
-      const int rc = mmv_max_clusters(occupancy, (const void*)mmv_kernel<KIND, NTL, XL, DUMP>, cs, (size_t)max_smem, sm_count, &n);
+      const int rc = max_clusters(occupancy, (const void*)mmv_kernel<KIND, NTL, XL, DUMP>, cs, MMV_THREADS, (size_t)max_smem, sm_count, &n);
       if (rc != GSQ_OK) return rc;
       if (mmv_plan<KIND, NTL>(a, cs, n, aligned, max_smem, &p) && (!plans[aligned].cs || p.t < plans[aligned].t)) plans[aligned] = p;
     }
@@ -1725,7 +1679,7 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
     if constexpr (DUMP || XL >= XL_XQ81) {
       return GSQ_ERR_UNSUPPORTED;
     } else {
-      static bool configured[32];
+      static std::atomic<bool> configured[32];
       int dev = 0;
       GSQ_CUDA_TRY(cudaGetDevice(&dev));
       auto kern = mmv_kernel<KIND, NTL, XL, false, true>;
@@ -1746,7 +1700,7 @@ static int mmv_launch_t(MmvArgs a, int sm_count, int max_smem, cudaStream_t st) 
 // to that one the least time of the slower product.
 template <int KA, int KB, int XL>
 static int mmv_launch_pair(MmvArgs a, MmvArgs b, int sm_count, int max_smem, cudaStream_t st) {
-  static MmvOccupancy occupancy;
+  static ClusterCount occupancy;
   auto kern = mmv_pair_kernel<KA, KB, XL>;
   MmvPlan pa = {}, pb = {};
   double best = 0.0;
@@ -1762,7 +1716,7 @@ static int mmv_launch_pair(MmvArgs a, MmvArgs b, int sm_count, int max_smem, cud
   for (int cs : {1, 2, 4, 8}) {
     if (cs > (a.k >> 8) || (g_mmv_cluster && cs != g_mmv_cluster)) continue;
     int n = 0;
-    const int rc = mmv_max_clusters(occupancy, (const void*)kern, cs, (size_t)max_smem, sm_count, &n);
+    const int rc = max_clusters(occupancy, (const void*)kern, cs, MMV_THREADS, (size_t)max_smem, sm_count, &n);
     if (rc != GSQ_OK) return rc;
     const int share = (int)(n * wa / (wa + wb) + 0.5);
     for (int na = share - 1; na <= share + 1; ++na) {

@@ -116,7 +116,7 @@ __device__ __forceinline__ void place_item(int item, int splits, int nsb, int n_
 
 // One persistent pair per item, at most as many as the device runs at once (max_pairs: kept per device and kernel).
 template <typename G>
-static int launch_pairs(void (*kern)(G), int threads, const G& g, int (&max_pairs)[64], int64_t items, int smem, int sm_count, cudaStream_t st) {
+static int launch_pairs(void (*kern)(G), int threads, const G& g, std::atomic<int> (&max_pairs)[64], int64_t items, int smem, int sm_count, cudaStream_t st) {
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return GSQ_ERR_UNSUPPORTED;
@@ -141,7 +141,8 @@ static int launch_pairs(void (*kern)(G), int threads, const G& g, int (&max_pair
     if (n < 1) return GSQ_ERR_UNSUPPORTED;
     max_pairs[dev] = n;
   }
-  cfg.gridDim = dim3(2u * (unsigned)(items < max_pairs[dev] ? items : max_pairs[dev]));
+  const int most = max_pairs[dev];
+  cfg.gridDim = dim3(2u * (unsigned)(items < most ? items : most));
   cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -472,7 +472,7 @@ namespace gsq {
 template <typename T>
 static int launch_rmsnorm_q8_1(const void* x, int64_t m, int64_t k, int64_t stride, void* residual, const void* gamma, float eps,
                                void* out, void* y_out, cudaStream_t st) {
-  static bool configured[64];
+  static std::atomic<bool> configured[64];
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return GSQ_ERR_UNSUPPORTED;

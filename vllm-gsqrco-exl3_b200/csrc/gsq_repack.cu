@@ -195,12 +195,12 @@ extern "C" int gsq_q6k_repack(void* w, int64_t rows, int64_t row_bytes, int dire
   if (rc != GSQ_OK) return rc;
   const size_t smem = (size_t)16 * row_bytes;
   if (smem > (size_t)di.max_smem_optin) return GSQ_ERR_TOO_LARGE;
-  static int configured_mask = 0;
+  static std::atomic<uint32_t> configured_mask{0};
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 32 || !((configured_mask >> dev) & 1)) {
     GSQ_CUDA_TRY(cudaFuncSetAttribute(q6k_repack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    if (dev < 32) configured_mask |= 1 << dev;
+    if (dev < 32) configured_mask |= 1u << dev;
   }
   q6k_repack_kernel<<<(unsigned)(rows / 16), 256, smem, (cudaStream_t)stream>>>((uint8_t*)w, row_bytes,
                                                                                (int)(row_bytes / 210), direction);
@@ -220,12 +220,12 @@ extern "C" int gsq_iq3s_repack(void* w, int64_t rows, int64_t row_bytes, int dir
   if (rc != GSQ_OK) return rc;
   const size_t smem = (size_t)16 * row_bytes;
   if (smem > (size_t)di.max_smem_optin) return GSQ_ERR_TOO_LARGE;
-  static int configured_mask = 0;
+  static std::atomic<uint32_t> configured_mask{0};
   int dev = 0;
   GSQ_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 32 || !((configured_mask >> dev) & 1)) {
     GSQ_CUDA_TRY(cudaFuncSetAttribute(iq3s_repack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    if (dev < 32) configured_mask |= 1 << dev;
+    if (dev < 32) configured_mask |= 1u << dev;
   }
   iq3s_repack_kernel<<<(unsigned)(rows / 16), 256, smem, (cudaStream_t)stream>>>((uint8_t*)w, row_bytes,
                                                                                 (int)(row_bytes / 110), direction);

@@ -20,7 +20,7 @@ static __device__ __align__(256) unsigned char g_static_q8[STATIC_MAX_Q8_BYTES];
 
 // Device address of the array per device. In host code the symbol g_static_q8 is only a handle: its address
 // there is not a device address, so it is resolved once with cudaGetSymbolAddress while that device is current.
-static void* g_static_q8_addr[64];
+static std::atomic<void*> g_static_q8_addr[64];
 
 static int static_q8_address(void** out) {
   int dev = 0;
