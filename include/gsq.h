@@ -172,11 +172,12 @@ int gsq_mul_mat_vec_q8(const void* w, int64_t row_bytes, int64_t rows, int ggml_
                        void* stream);
 
 /*
- * The 1..8-row product from X itself: quantises to block_q8_1 values inside the product kernel (each CTA its share), one
- * launch and no buffer between. The result is that of gsq_quantize_q8_1 + gsq_mul_mat_vec_q8 up to the order of the fp32
+ * The 1..8-row product from X itself: quantises to block_q8_1 values inside the product kernel, one launch and no buffer
+ * between. The result is that of gsq_quantize_q8_1 + gsq_mul_mat_vec_q8 up to the order of the fp32
  * sums. Not in the reference, whose shim quantises with a kernel of its own (lcpp_shim.cu:274-294). Returns
  * GSQ_ERR_UNSUPPORTED, nothing launched, where no kernel does both (the low-bit types, IQ3_S / Q6_K in GGUF order) or where
- * the two calls are faster (many activations): use the two calls then. x as for gsq_quantize_q8_1, the rest as for
+ * the two calls are faster (many activations; Q4_K at 1 row and IQ4_XS at 1..3 while `stream` is capturing, but for the
+ * largest Q4_K): use the two calls then. x as for gsq_quantize_q8_1, the rest as for
  * gsq_mul_mat_vec_q8.
  */
 int gsq_linear_vec(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype,

@@ -96,6 +96,33 @@ def test_dp4a_product_quantises_as_the_kernel_in_front(name, ms, dtype, rows, k,
         assert bool(torch.isnan(out[0][:, rows:]).all())
 
 
+@pytest.mark.parametrize("name,m,rows,inside", [("Q4_K", 1, 2064, False), ("Q4_K", 1, 13312, True), ("IQ4_XS", 1, 2064, False), ("IQ4_XS", 1, 13312, False)])
+def test_dp4a_product_in_a_capture(name, m, rows, inside):
+    """A capture takes the quantiser and the product as two kernels (but for the largest Q4_K); its replay gives what calls one by
+    one give, bit for bit."""
+    from gsq_b200 import _gsq_ops
+
+    t, k = TYPES[name], 5120
+    w = torch.from_numpy(synth.make_weight(t, rows, k, 77)).to(DEV)
+    x = torch.from_numpy(synth.make_activation(m, k, 78)).to(torch.bfloat16).to(DEV)
+    y = torch.empty((m, rows), dtype=torch.bfloat16, device=DEV)
+
+    def vec():
+        return _cabi.lib.gsq_linear_vec(w.data_ptr(), w.shape[1], rows, t, 0, x.data_ptr(), 2, m, k, k, y.data_ptr(), 2, rows,
+                                        torch.cuda.current_stream().cuda_stream)
+
+    assert vec() == 0
+    eager = _gsq_ops.linear(x, w, t, None, False)
+    assert torch.equal(eager, y)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        rc = vec()
+        got = _gsq_ops.linear(x, w, t, None, False)
+    assert rc == (0 if inside else UNSUPPORTED)
+    g.replay()
+    assert torch.equal(got, eager)
+
+
 @pytest.mark.parametrize("pair", [("Q4_K", "Q6_K"), ("IQ3_S", "Q6_K"), ("IQ4_XS", "Q6_K"), ("IQ3_S", "IQ4_XS")])
 @pytest.mark.parametrize("rows,k", [((16, 16), 256), ((48, 2064), 768), ((6144, 1024), 5120), ((1024, 34816), 2560), ((512, 256), 17408)])
 def test_two_products_in_one_launch(pair, rows, k):

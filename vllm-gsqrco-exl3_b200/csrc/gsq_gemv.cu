@@ -616,7 +616,6 @@ __host__ __device__ inline size_t gemv_smem_bytes(int kind, int rs, int m, int s
   return s;
 }
 
-// TMA: weights come through a per-warp ring of bulk copies (cp.async.bulk + mbarrier) instead of direct loads.
 // X -> block_q8_1 in shared memory (RAWX): the quantiser's own arithmetic (gsq_quantize.cu), all of X in every CTA.
 template <typename T, bool VEC, int M>
 __device__ __forceinline__ void stage_x(const GemvArgs& a, uint8_t* blocks) {
@@ -644,6 +643,7 @@ __device__ __forceinline__ void stage_x(const GemvArgs& a, uint8_t* blocks) {
   __syncthreads();
 }
 
+// TMA: weights come through a per-warp ring of bulk copies (cp.async.bulk + mbarrier) instead of direct loads.
 // RAWX: X itself comes in and is quantised by every CTA (gemv_raw_host).
 template <int KIND, int M, int RS, bool DUMP, bool TMA, bool RAWX>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_kernel(const GemvArgs a) {
@@ -1128,16 +1128,28 @@ static int gemv_host_dp4a(const void* w, int64_t row_bytes, int64_t rows, int gg
   }
 }
 
-// The same with X quantised inside the kernel: one launch instead of two, at the rows at which these types have this kernel, up
-// to 8192 values of X. There the GPU needs as long either way (us, here / two kernels: Q4_K 1 row 5120 x 5120 8.8 / 8.8,
-// 17408 x 5120 16.6 / 17.2, 2048 x 5120 6.7 / 6.4; IQ4_XS 10.3 / 10.1 and 21.0 / 20.8) and the host 2 us less, which is what
-// calls one by one wait for (Q4_K 5120 x 5120, 1 row: 9.65 -> 7.58). Beyond, every CTA quantising all of X costs more than the
-// launch (Q4_K 5120 x 17408 1 row 18.5 / 17.3; IQ4_XS 5120 x 5120 2 rows 11.8 / 10.9): GSQ_ERR_UNSUPPORTED.
+// The same with X quantised inside the kernel, by every CTA all of it, up to 8192 values of X: one launch instead of two, at the
+// rows at which these types have this kernel. Which way is faster depends on who launches (us, here / two kernels, weights from
+// HBM):
+//   * calls one by one: here on every weight, host-bound or not, Q4_K 1 row 2048 x 2048 6.0 / 10.2, 5120 x 5120 8.4 / 9.0,
+//     34816 x 5120 29.2 / 33.1, IQ4_XS 1 row 5120 x 5120 9.7 / 10.0, 34816 x 5120 38.2 / 39.8, 3 rows 2048 x 2048 6.8 / 8.4;
+//   * replayed from a graph, where a launch costs next to nothing: two kernels, IQ4_XS 1 row 1024 x 5120 6.4 / 5.8, 5120 x 5120
+//     10.4 / 10.0, 34816 x 5120 39.5 / 38.5, 3 rows 2048 x 2048 7.2 / 6.4, Q4_K 2048 x 5120 6.9 / 6.5, 12288 x 5120 13.2 / 12.8;
+//     but Q4_K from 64 M values on 34816 x 2048 18.0 / 18.2, 17408 x 5120 16.8 / 17.3, 34816 x 5120 30.7 / 31.4.
+// So a stream that is capturing takes the two kernels but for such Q4_K. Beyond 8192 values X costs more in every CTA than the
+// launch (Q4_K 5120 x 17408 1 row 18.5 / 17.3; IQ4_XS 5120 x 5120 2 rows 11.8 / 10.9). GSQ_ERR_UNSUPPORTED: the two calls.
+static bool capturing(void* stream) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing((cudaStream_t)stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+  cudaGetLastError();   // (the legacy stream while another one captures: the launch will say so)
+  return false;
+}
 int gemv_raw_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int packed, const void* x, int x_dtype, int64_t m, int64_t k,
                   int64_t x_row_stride, void* y, int y_dtype, int64_t y_row_stride, void* stream) {
   if (packed || m < 1 || m > (ggml_type == GSQ_TYPE_Q4_K ? 1 : ggml_type == GSQ_TYPE_IQ4_XS ? 3 : 0) || m * k > 8192 || g_force_direct || g_force_cluster ||
       (x_dtype != GSQ_F32 && x_dtype != GSQ_F16 && x_dtype != GSQ_BF16))
     return GSQ_ERR_UNSUPPORTED;
+  if (!(ggml_type == GSQ_TYPE_Q4_K && rows * k > (64 << 20)) && capturing(stream)) return GSQ_ERR_UNSUPPORTED;
   return gemv_host_dp4a(w, row_bytes, rows, ggml_type, packed, x, m, k, y, y_dtype, y_row_stride, stream, nullptr, 0, x_dtype, x_row_stride);
 }
 
