@@ -187,7 +187,8 @@ int gsq_linear_vec(const void* w, int64_t row_bytes, int64_t rows, int ggml_type
  * Two 1..8-row products of the same activations in one launch: a fused layer whose shards are of two types (Q4_K, IQ3_S or
  * IQ4_XS first and Q6_K second, IQ3_S first and IQ4_XS second). x: block_q8_1 of m rows (x_dtype = -1) or X as for
  * gsq_linear_vec. Results: those of gsq_mul_mat_vec_q8 per weight up to the order of the fp32 sums. Not in the reference.
- * GSQ_ERR_UNSUPPORTED, nothing launched, for other types and for shapes that one launch does not serve: use two calls then.
+ * GSQ_ERR_UNSUPPORTED, nothing launched, for other types or orders, for shapes that one launch does not serve and where the smaller
+ * product is so large (more than 96 M weight values) that two calls are faster: use two calls then.
  */
 typedef struct gsq_weight {
   const void* w;

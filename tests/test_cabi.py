@@ -84,3 +84,15 @@ def test_packed_flag_means_nothing_for_types_of_one_layout():
         for rows in (16, 24, 5120, 17408):
             for m in (1, 8, 9, 40, 100, 200, 256, 777):
                 assert lib.gsq_linear_workspace_bytes(rows, m, 2048, t, 1) == lib.gsq_linear_workspace_bytes(rows, m, 2048, t, 0), (t, rows, m)
+
+
+def test_which_pairs_one_launch_serves():
+    """The size of the smaller product decides, whichever of the two it is."""
+    def weight(t, rows, k):
+        bs = {12: 144, 14: 210, 21: 110, 23: 136}[t]
+        return _cabi.Weight(4096, k // 256 * bs, rows, t, int(t in (14, 21)), 4096)
+
+    for a, b in ((12, 14), (21, 14), (23, 14), (21, 23)):
+        for ra, rb, k, served in ((5120, 1024, 5120, 1), (34816, 1024, 17408, 1), (1024, 34816, 17408, 1), (12288, 60000, 8192, 1),
+                                  (60000, 12288, 8192, 1), (12304, 60000, 8192, 0), (60000, 12304, 8192, 0)):
+            assert _cabi.lib.gsq_linear_vec_pair_serves(weight(a, ra, k), weight(b, rb, k), 4) == served, (a, b, ra, rb, k)

@@ -147,9 +147,22 @@ static bool mmv_pair_types(int ta, int tb) {
   return (tb == GSQ_TYPE_Q6_K && (ta == GSQ_TYPE_Q4_K || ta == GSQ_TYPE_IQ3_S || ta == GSQ_TYPE_IQ4_XS)) ||
          (tb == GSQ_TYPE_IQ4_XS && ta == GSQ_TYPE_IQ3_S);
 }
+// weight values of which one launch for two products still serves the smaller of them
+constexpr int64_t MMV_PAIR_VALUES = 96 << 20;
+
+// Whether the pair serves two weights at m rows. One launch saves the smaller product its start, staging and last step and the
+// wait for the larger one, 5 to 8 us, but gives both one cluster size and leaves the clusters of the product that ends first
+// idle. Measured against two launches in a graph over 1892 cells of the four pairs of types, 19 pairs of row counts from 512 + 256 to
+// 34816 + 34816, K 1024 to 17408, 1 to 8 rows (profiles/mmv_pair.txt): 28 % less on average. Where the smaller product alone takes
+// 20 us and more the saving no longer covers the rest: 17408 + 17408 rows IQ3_S + IQ4_XS, 4 rows, K 17408 122.7 / 111.4 us, K 8192
+// 61.4 / 59.8 (but K 5120, 89 M values, 41.6 / 43.3, and Q4_K + Q6_K 35.1 / 37.0). Below that line the pair loses on some
+// weights of K 17408, at most 7 %, and nowhere to K 8192.
 bool mmv_pair_serves(const gsq_weight* a, const gsq_weight* b, int64_t m) {
-  return m >= 1 && m <= 8 && mmv_pair_types(a->ggml_type, b->ggml_type) && mmv_applies(a->ggml_type, a->packed, a->rows, m) &&
-         mmv_applies(b->ggml_type, b->packed, b->rows, m);
+  if (m < 1 || m > 8 || !mmv_pair_types(a->ggml_type, b->ggml_type) || !mmv_applies(a->ggml_type, a->packed, a->rows, m) ||
+      !mmv_applies(b->ggml_type, b->packed, b->rows, m))
+    return false;
+  const int64_t va = a->row_bytes / block_bytes(a->ggml_type) * 256 * a->rows, vb = b->row_bytes / block_bytes(b->ggml_type) * 256 * b->rows;
+  return (va < vb ? va : vb) <= MMV_PAIR_VALUES;
 }
 
 int mmv_launch_pair_q81(int ta, int tb, const MmvArgs& a, const MmvArgs& b, int sm_count, int max_smem, cudaStream_t st);    // gsq_mmv_pair.cu
