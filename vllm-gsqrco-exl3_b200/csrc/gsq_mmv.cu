@@ -142,11 +142,6 @@ int mmv_host(const void* w, int64_t row_bytes, int64_t rows, int ggml_type, int 
   }
 }
 
-// the pairs that mmv_pair_kernel is instantiated for
-static bool mmv_pair_types(int ta, int tb) {
-  return (tb == GSQ_TYPE_Q6_K && (ta == GSQ_TYPE_Q4_K || ta == GSQ_TYPE_IQ3_S || ta == GSQ_TYPE_IQ4_XS)) ||
-         (tb == GSQ_TYPE_IQ4_XS && ta == GSQ_TYPE_IQ3_S);
-}
 // weight values of which one launch for two products still serves the smaller of them
 constexpr int64_t MMV_PAIR_VALUES = 96 << 20;
 

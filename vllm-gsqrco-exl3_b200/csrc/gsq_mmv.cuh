@@ -1766,6 +1766,35 @@ static int mmv_launch_pair(MmvArgs a, MmvArgs b, int sm_count, int max_smem, cud
   return GSQ_OK;
 }
 
+// Which pairs there are: a main type first and the one that a file keeps some shards at second.
+static constexpr bool mmv_pair_types(int ta, int tb) {
+  return (tb == GSQ_TYPE_Q6_K && (ta == GSQ_TYPE_Q4_K || ta == GSQ_TYPE_IQ3_S || ta == GSQ_TYPE_IQ4_XS)) ||
+         (tb == GSQ_TYPE_IQ4_XS && ta == GSQ_TYPE_IQ3_S);
+}
+static constexpr int mmv_kind(int t) {
+  return t == GSQ_TYPE_Q4_K ? MK_Q4K : t == GSQ_TYPE_Q6_K ? MK_Q6K : t == GSQ_TYPE_IQ3_S ? MK_IQ3S : MK_IQ4XS;
+}
+template <int TA, int TB, int XL>
+static int mmv_launch_pair_if(int ta, int tb, const MmvArgs& a, const MmvArgs& b, int sm_count, int max_smem, cudaStream_t st) {
+  if constexpr (mmv_pair_types(TA, TB)) {
+    if (ta == TA && tb == TB) return mmv_launch_pair<mmv_kind(TA), mmv_kind(TB), XL>(a, b, sm_count, max_smem, st);
+  }
+  return MMV_DECLINED;
+}
+template <int XL>
+static int mmv_launch_pair_of(int ta, int tb, const MmvArgs& a, const MmvArgs& b, int sm_count, int max_smem, cudaStream_t st) {
+  int rc = MMV_DECLINED;
+  auto first = [&](auto t) {
+    constexpr int TA = decltype(t)::value;
+    if (rc == MMV_DECLINED) rc = mmv_launch_pair_if<TA, GSQ_TYPE_Q6_K, XL>(ta, tb, a, b, sm_count, max_smem, st);
+    if (rc == MMV_DECLINED) rc = mmv_launch_pair_if<TA, GSQ_TYPE_IQ4_XS, XL>(ta, tb, a, b, sm_count, max_smem, st);
+  };
+  first(std::integral_constant<int, GSQ_TYPE_Q4_K>{});
+  first(std::integral_constant<int, GSQ_TYPE_IQ3_S>{});
+  first(std::integral_constant<int, GSQ_TYPE_IQ4_XS>{});
+  return rc;
+}
+
 template <int KIND, int XL>
 static int mmv_launch_n(const MmvArgs& a, int sm_count, int max_smem, cudaStream_t st) {
   const int ntl = (a.m + 7) / 8;

@@ -266,19 +266,20 @@ void product_of_run(int op, const Weight& w, const Tensor& x, int64_t type, int6
 // Two runs' products at 1..8 rows in one launch, side by side in y. False: no such kernel, nothing done.
 bool product_of_two(const Weight& wa, int64_t ta, const Weight& wb, int64_t tb, const Tensor& x, bool packed, Tensor& q, char* y, int64_t ldy,
                     void* stream) {
-  if (ta == tb || (tb != Q6_K && !(ta == IQ3_S && tb == IQ4_XS)) || (ta != Q4_K && ta != IQ3_S && ta != IQ4_XS) || dtype_code(x.scalar_type()) == GSQ_DTYPE_OTHER)
-    return false;
   const int64_t n = x.size(0);
+  gsq_weight a = {wa.data, wa.size1, wa.size0, (int)ta, packed && packable(ta), y}, b = {wb.data, wb.size1, wb.size0, (int)tb, packed && packable(tb), y + wa.size0 * x.element_size()};
+  if (!gsq_linear_vec_pair_serves(&a, &b, n) || dtype_code(x.scalar_type()) == GSQ_DTYPE_OTHER) return false;
   bool pa = packed, pb = packed;
   const int oa = op_for(n, ta, wa.size0, x.size(1), pa), ob = op_for(n, tb, wb.size0, x.size(1), pb);
   if (!kSpec[oa].vec || !kSpec[ob].vec) return false;
   const int64_t k = guard(kSpec[oa], wa, x, ta, wa.size0);
   guard(kSpec[ob], wb, x, tb, wb.size0);
-  const gsq_weight a = {wa.data, wa.size1, wa.size0, (int)ta, kSpec[oa].packed, y}, b = {wb.data, wb.size1, wb.size0, (int)tb, kSpec[ob].packed, y + wa.size0 * x.element_size()};
+  a.packed = kSpec[oa].packed;
+  b.packed = kSpec[ob].packed;
   const int dt = dtype_code(x.scalar_type());
   int rc = GSQ_ERR_UNSUPPORTED;
   if (!q.defined()) rc = gsq_linear_vec_pair(&a, &b, x.const_data_ptr(), dt, n, k, row_stride(x, k), dt, ldy, stream);
-  if (rc == GSQ_ERR_UNSUPPORTED && gsq_linear_vec_pair_serves(&a, &b, n)) {
+  if (rc == GSQ_ERR_UNSUPPORTED) {
     if (!q.defined()) q = quantize_blocks(x, k, stream);
     rc = gsq_linear_vec_pair(&a, &b, q.const_data_ptr(), -1, n, k, 0, dt, ldy, stream);
   }
