@@ -16,10 +16,11 @@
 //   warp 0        copies: k-blocks, `stages` deep; d_x, d and dmin of a superblock, 3 deep
 //   warp 1        CTA 0: MMA issue, two slices (a k-block) at a time; CTA 1: reports each landed stage to CTA 0
 //   warps 4..19   scaling: four warps per tensor-memory lane quarter, a quarter of the most tokens each
-// What bounds it: the chain of each k-block, 1200 cycles at 128 tokens (Q6_K 5120 x 17408, clock64 stamps): the hand-over
-// between MMAs and scaling takes about 500 of them, four dependent tensor-memory loads per warp most of the rest; operands
-// are in after about 1050 (40 KB), the tensor pipe needs 512. 8 consumer warps took 1450 (one row a thread) and 1250 (four).
-// Q6_K 5120 x 17408, 512 tokens: 355 us, scaled products (two planes, 256 tokens a block) 325, few-row launches 861.
+// What bounds it: no unit is full (Q6_K 5120 x 17408, 512 tokens: tensor pipe 44 %, issue 53 %, shared memory 36 %, L2 31 %). By
+// clock64 stamps, taken when tensor memory was read by 16x256b loads, a k-block of 128 tokens took 1200 cycles, its operands (40 KB)
+// were in after about 1050 and the tensor pipe needs 512; the loads of today took 7 us of 235 off this kernel. 8 consumer warps took
+// 1450 cycles (one row a thread) and 1250 (four). The case: 331 us with expansion and sum, scaled products (two planes, 256
+// tokens a block) 325, few-row launches 861.
 // Every wait is bounded and raises the device flag instead of hanging.
 #include <cuda_fp16.h>
 
@@ -54,7 +55,8 @@ struct SliceArgs {
 // all tokens of one, and reads a quarter of the scales from shared memory: with one row a thread (32 x 32b) these reads, 128 of
 // 16 bytes per slice, took as long as the tensor-memory loads, 560 cycles a slice together. Tensor memory gives an SM 512 bytes
 // a cycle in this shape, 905 in that of 32 x 32b, but 256 in that of 8 columns per 4 registers (16 x 256b): 256 cycles for the
-// 128 x 128 sums of a slice instead of 128, and with it Q6_K 5120 x 17408, 512 tokens, took 352 us, now 344.
+// 128 x 128 sums of a slice instead of 128, and with it Q6_K 5120 x 17408, 512 tokens, took 352 us, in this shape 344 (331 with the sum
+// of the parts as it is now).
 __device__ __forceinline__ void tmem_rows16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.16x128b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"

@@ -76,7 +76,11 @@ enum Way {
 //                                     81 where the third 16-row group of a launch costs more than the expansion: 5120 x 5120 (88
 //                                     rows) 44.2 / 49.5, 4096 x 4096 30.9 / 35.0, but 2048 x 2048 20.7 / 18.9, 17408 x 2560 71 / 62;
 //                                     49 where a launch has few rows of long K: 2048 x 8192 29.7 / 31.1 (64 rows 30.5 / 32.7, 96 rows
-//                                     32.2 / 42.3), 1024 x 17408 39.7 / 40.8 (64 rows 39.9 / 46.0), 1024 x 5120 21.1 / 21.7
+//                                     32.2 / 42.3), 1024 x 17408 39.7 / 40.8 (64 rows 39.9 / 46.0), 1024 x 5120 21.1 / 21.7.
+//                                     The steps are coarse; cells of the sweep more than 4 % off: two steps too late for 512 x 8192
+//                                     (64 to 96 rows 21.3 / 23.3 to 22.4 / 26.3), 9216 x 2560 and 9216 x 5120 (88, 96 rows 38 / 41,
+//                                     77 / 82) and 17408 x 12800 (97 to 112 rows 364 / 412 to 365 / 428), too early for 34816 x 5120
+//                                     (128 to 144 rows 316 / 274 to 363 / 309) and 151936 x 5120 (144 rows 1529 / 1452)
 //   Q6_K, IQ3_S in GGUF order (8)     25: 512 x 1024 16 / 21 and 15 / 32, 17408 x 5120 148 / 281 and 95 / 176
 //   Q2_K                              25: 5120 x 5120 47 / 70, 17408 x 5120 120 / 155; 512 x 1024 22 / 18, at 40 rows 23 / 26
 //   IQ1_M                             12: 5120 x 5120 32 / 40, 17408 x 5120 81 / 89; 1024 x 2048 16.5 / 13.9, at 17 rows 17.4 / 18.9
@@ -134,10 +138,12 @@ static Way choose_way(int ggml_type, int packed, int64_t rows, int64_t m, int64_
 // small-batch kernel / evenly cut work, 33 and 48 rows):
 //   * IQ4_XS: on weights so tall or large that the first one has no even plan: 60000 x 5120 154 / 153, 34816 x 12800 217 / 215,
 //     5120 x 32768 94 / 91, but 34816 x 5120 78 / 94, 17408 x 5120 43 / 53, 5120 x 17408 52.9 / 54.8, 512 x 1024 7.9 / 8.9. To
-//     16 M values the activations' size decides, as callers of gsq_route know it (48 rows 2048 x 8192: 18.3 / 22.9).
+//     16 M values the activations' size decides, as callers of gsq_route know it; that is not where the two cross (2048 x 8192,
+//     40 to 48 rows: 18.2 / 22.8 to 18.3 / 22.9, and the second one runs).
 //   * Q4_K: from 40 M values on, 17408 x 5120 52.7 / 50.4 and 54.3 / 50.8, 5120 x 12800 47 / 42, with long K from 20 M on,
 //     2048 x 17408 32.4 / 31.6; but 7168 x 5120 26.0 / 28.0 and 26.6 / 28.3, 5120 x 8192 30.6 / 31.4, 1024 x 17408 26.0 / 28.2,
-//     1024 x 2048 8.6 / 11.3.
+//     1024 x 2048 8.6 / 11.3. The line by size alone is early for some: 13312 x 4096 32.4 / 35.9, 9216 x 5120 33 rows 30.5 / 33.0
+//     (48 rows 36.0 / 33.2), 4096 x 11264 32.6 / 34.1, 12288 x 5120 36.9 / 38.4.
 static bool small_batch(int ggml_type, int packed, int64_t rows, int64_t m, int64_t k) {
   if (gemm_variant() == 10 || !mmv_applies(ggml_type, packed, rows, m)) return false;
   if (m <= 32 || gemm_variant() != 0 || gemm_dump_pointer()) return true;

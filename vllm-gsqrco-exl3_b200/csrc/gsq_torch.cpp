@@ -263,7 +263,8 @@ void product_of_run(int op, const Weight& w, const Tensor& x, int64_t type, int6
     product(s, w, x, i, std::min(per_call, n - i), type, rows, k, q, y + i * ldy * x.element_size(), ldy, stream);
 }
 
-// Two runs' products at 1..8 rows in one launch, side by side in y. False: no such kernel, nothing done.
+// Two runs' products in one launch, side by side in y, where both ops read block_q8_1: to 7 rows (at 8 the routing table gives one of
+// every pair's types an op on 128-value blocks), the types in the order of mmv_pair_types. False: no such kernel.
 bool product_of_two(const Weight& wa, int64_t ta, const Weight& wb, int64_t tb, const Tensor& x, bool packed, Tensor& q, char* y, int64_t ldy,
                     void* stream) {
   const int64_t n = x.size(0);
