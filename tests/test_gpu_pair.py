@@ -64,28 +64,33 @@ def test_forms_of_x_and_y(pair, dtype, k, pad, shift):
                     assert torch.equal(got[ydt], got[torch.float32].to(ydt))
 
 
+def _layer(names, k, tdt):
+    """A fused layer, q and k of the one type and v of the other; its rows' bytes."""
+    shards = [("q", names[0], 1040), ("k", names[0], 256), ("v", names[1], 256)]
+    layer, method = torch.nn.Module(), linear.GGUFLinearMethod(None)
+    method.create_weights(layer, k, [r for _, _, r in shards], k, sum(r for _, _, r in shards), tdt)
+    raws = []
+    for i, (sid, name, rows) in enumerate(shards):
+        raws.append((name, synth.make_weight(TYPES[name], rows, k, 130 + i)))
+        layer.weight.load_shard(torch.from_numpy(raws[-1][1]).to(DEV), sid)
+        layer.weight_type.shard_weight_type[sid] = TYPES[name]
+    layer.weight_type.weight_type = TYPES[names[0]]
+    method.process_weights_after_loading(layer)
+    return layer, method, raws
+
+
 @pytest.mark.parametrize("pair", PAIRS)
 @pytest.mark.parametrize("dtype", list(DTYPES))
 @pytest.mark.parametrize("order", [0, 1])
 def test_through_apply(pair, dtype, order):
     """A fused layer of two types in either order (the pairs have one: the other is two launches)."""
-    k, names = 2560, pair if order == 0 else pair[::-1]
-    shards = [("q", names[0], 1040), ("k", names[0], 256), ("v", names[1], 256)]
-    layer, method = torch.nn.Module(), linear.GGUFLinearMethod(None)
-    tdt = DTYPES[dtype][1]
-    method.create_weights(layer, k, [r for _, _, r in shards], k, sum(r for _, _, r in shards), tdt)
-    raws = []
-    for i, (sid, name, rows) in enumerate(shards):
-        raws.append(synth.make_weight(TYPES[name], rows, k, 130 + i))
-        layer.weight.load_shard(torch.from_numpy(raws[-1]).to(DEV), sid)
-        layer.weight_type.shard_weight_type[sid] = TYPES[name]
-    layer.weight_type.weight_type = TYPES[shards[0][1]]
-    method.process_weights_after_loading(layer)
+    k, tdt = 2560, DTYPES[dtype][1]
+    layer, method, raws = _layer(pair if order == 0 else pair[::-1], k, tdt)
     bound = {torch.float32: 1e-5, torch.float16: 1e-3, torch.bfloat16: 5e-3}[tdt]
     for m in (1, 2, 4, 7, 8):
         x = synth.nudge_ties_torch(torch.from_numpy(synth.make_activation(m, k, 131 + m)).to(tdt))
         q, d = q8_1.quantize_q8_1(x.float().numpy())[:2]
-        want = np.concatenate([product.product_q81(blocks.decode(raw, TYPES[n]), q, d) for raw, (_, n, _) in zip(raws, shards)], axis=1)
+        want = np.concatenate([product.product_q81(blocks.decode(raw, TYPES[n]), q, d) for n, raw in raws], axis=1)
         wide = torch.empty((m, k + 24), dtype=tdt, device=DEV)
         wide[:, 16:16 + k] = x.to(DEV)
         for xd in (x.to(DEV), wide[:, 16:16 + k]):
@@ -93,3 +98,29 @@ def test_through_apply(pair, dtype, order):
             assert y.dtype == tdt
             # 8 rows of some types go through the ops that read 128-value blocks (Q4_K's minimum from their half sums)
             assert product.rel_err(y.float().cpu().numpy(), want) <= max(bound, 1e-3 if m == 8 else 0), m
+
+
+@pytest.mark.parametrize("pair", PAIRS)
+@pytest.mark.parametrize("order", [0, 1])
+def test_which_launches_apply_takes(pair, order, capfd):
+    """One launch for both types in the pair's order, from the rows at which the small-batch kernel has both (Q4_K 2, IQ4_XS 4) to 7,
+    whether X goes in itself or as blocks; replayed from a graph it gives the same."""
+    k, lib = 2560, _cabi.lib
+    layer, method, _ = _layer(pair if order == 0 else pair[::-1], k, torch.bfloat16)
+    first = max({"Q4_K": 2, "IQ4_XS": 4}.get(n, 1) for n in pair)
+    for m in range(1, 9):
+        x = torch.from_numpy(synth.make_activation(m, k, 140 + m)).to(torch.bfloat16).to(DEV)
+        method.apply(layer, x)
+        capfd.readouterr()
+        old = lib.gsq_debug_mmv_trace(1)
+        y = method.apply(layer, x)
+        lib.gsq_debug_mmv_trace(old)
+        err = capfd.readouterr().err
+        one = order == 0 and first <= m <= 7
+        assert err.count("mmv pair") == int(one) and not (one and "mmv plan" in err), (m, err)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            got = method.apply(layer, x)
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, y)
